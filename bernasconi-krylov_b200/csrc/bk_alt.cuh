@@ -1,0 +1,647 @@
+// Turning-pass engine (sm_100a): one pass over the statevector per Trotter step.
+//
+// A step is psi <- M D psi with M a product of commuting single-qubit rotations,
+// so the qubits of a step may be rotated in any order. With the element bits
+// split into two sets X and Y (each a tile of the statevector can hold), the
+// steps run as
+//   [D_0 X][Y D_1 Y][X D_2 X] ... [. finish]
+// where a bracket is ONE pass over the state: the pass finishes step k - 1 on its
+// set, measures psi_k, applies D_k and starts step k on the same set. Every step
+// costs one pass, where a pass per set costs two. With three sets (large states)
+// a plain pass over the third set A sits between two turning passes:
+//   [D_0 S][A][T D_1 T][A][S D_2 S][A] ...
+// two passes a step instead of three.
+//
+// Tiles. 2^TB 16-byte elements (bk_persist.cuh): the A set is element bits
+// [0, TB), an S set [h0, h0 + w) with the tile's other cp = TB - w bits contiguous
+// low ones. A thread keeps 2^KB elements in registers; round 0 holds the top KB
+// tile bits in registers, round 1 the next KB, round 2 the lowest (those left).
+// A turning pass climbs down the rounds that its set needs, turns (measurement,
+// D, amplitude bit 0 of complex64) in the last of them and climbs back up, so
+// w <= KB needs no shared-memory round trip, w <= 2 KB two, more four. The last
+// round is round 0 again: lanes run over the low tile bits and every global
+// store is a run of min(512, 16 * 2^cp) bytes.
+//
+// What bounds it (B200): up to 2^23 elements shared memory and its latency (N = 23
+// complex64: shared-memory pipe 52%, issue 26% of peak at 16 warps an SM; a step of
+// N = 19 is 5.7 us against 27 us for the persistent task engine, N = 22 25 against
+// 37); beyond, DRAM: N = 28 complex64 1.57 ms a step = 5.8 TB/s over its two passes
+// (2.09 ms with a pass per set and the strided passes fused through L2).
+//
+// All passes of a run are one cooperative launch: a CTA takes tiles
+// rank, rank + G, ... of each pass and a counter barrier over the G CTAs
+// separates the passes (bounded polls, a common abort word). The next tile's TMA
+// load is issued as soon as the current tile's last shared-memory read is done.
+#pragma once
+#include "bk_s23.cuh"
+
+namespace bk {
+
+// Full per-energy phase table: every LABS energy is c0 + 4 j. Entry 0 rotates by
+// nothing, entry 1 + j by level j; a pass without D reads entry 0 through a stride
+// of 0 (a branch around the unrolled phase costs the register allocation more).
+template <class R>
+struct AltPhase;
+struct AltTab {
+  const unsigned char* base;
+  uint32_t stride, c0;
+};
+template <>
+struct AltPhase<float> {
+  using entry = float2;  // {-tan(r/4), sin(r/2)}: two half-angle shear rotations
+  __device__ static void apply(El<float>::T& v, uint32_t e2, const AltTab& t) {
+    const float2 H0 = *reinterpret_cast<const float2*>(t.base + (((e2 & 0xFFFFu) - t.c0) >> 2) * t.stride);
+    const float2 H1 = *reinterpret_cast<const float2*>(t.base + (((e2 >> 16) - t.c0) >> 2) * t.stride);
+    const float2 A = make_float2(H0.x, H1.x), B = make_float2(H0.y, H1.y);
+    PhaseV<float>::shear2(v.re, v.im, A, B);
+    PhaseV<float>::shear2(v.re, v.im, A, B);
+  }
+};
+template <>
+struct AltPhase<double> {
+  using entry = double2;  // {cos r, sin r}
+  __device__ static void apply(El<double>::T& v, uint32_t e, const AltTab& t) {
+    const double2 cs = *reinterpret_cast<const double2*>(t.base + ((e - t.c0) >> 2) * t.stride);
+    v.v = make_double2(fma(v.v.x, cs.x, -v.v.y * cs.y), fma(v.v.x, cs.y, v.v.y * cs.x));
+  }
+};
+
+// TMA coordinates of a set's tiles: the dimensions of the tile id's two parts.
+struct AltSet {
+  int mid_dim, hi_dim, mid_bits, pad;
+};
+
+// One statevector's run (kernel parameter, or device memory for a batch).
+template <class R>
+struct alignas(64) AltInst {
+  CUtensorMap map[3];  // tiles of the A set and of the S sets
+  unsigned char* state;
+  const uint16_t* E;
+  const typename AltPhase<R>::entry* tab;
+  const R* tan;        // [steps]
+  const R* scale;      // [steps]
+  const int* slot;     // [steps + 1] measurement row, or -1
+  double* partials;    // [rows][G][3]: norm, P_<, <d_H> of one CTA's tiles
+  AltSet set[3];
+  uint32_t n_tiles;
+  int n_j, c0;         // levels of the phase table (after its entry 0), lowest level
+  int e0;
+  uint32_t s0;
+  int k0, k1;          // steps [k0, k1)
+  int row0;            // first measurement row of `partials`
+  int meas_first;      // measure psi_k0 (else an earlier segment has)
+};
+
+// Barrier over the G CTAs of a run; `ctr` counts arrivals over all passes.
+struct AltBarrier {
+  unsigned int* ctr;
+  int* err;
+  int* abort;
+  uint32_t poll_limit;
+};
+
+template <int TB, int KB>
+struct AltPlan {
+  static constexpr int kThreads = 1 << (TB - KB);
+  static constexpr int kWarps = kThreads / 32;
+  static constexpr int kPer = 1 << KB;
+  static_assert(TB - KB >= 6 && 3 * KB >= TB && TB - KB <= 9, "three rounds cover the tile");
+  // lowest register bit and number of new tile bits of each round
+  static constexpr int reg_lo(int r) { return r == 0 ? TB - KB : r == 1 ? TB - 2 * KB : 0; }
+  static constexpr int act_hi(int r) { return r < 2 ? KB : TB - 2 * KB; }
+  // tile position of a thread's register element 0. Round 0: lanes over tile bits
+  // 0-4. Round 1: the bits below its registers first, then those from TB - KB up
+  // (with two low bits the third lane takes bit 8, so that the three lowest lanes
+  // fold onto different residues of the swizzle); rounds 1 and 2 share their warp
+  // bits (the top ones), so data moves inside a warp between them.
+  template <int r>
+  __device__ static uint32_t base(uint32_t lane, uint32_t warp) {
+    if constexpr (r == 0) return lane | (warp << 5);
+    constexpr int top = TB - (TB - KB - 5);  // warp bits [top, TB) of rounds 1 and 2
+    if constexpr (r == 2) return (lane << KB) | (warp << top);
+    constexpr int lo = TB - 2 * KB;          // tile bits below round 1's registers
+    if constexpr (lo == 2) {  // the 2^10-element tile
+      return (lane & 3u) | ((lane & 4u) << 6) | ((lane & 24u) << 3) | (warp << top);
+    }
+    return (lane & ((1u << lo) - 1u)) | ((lane >> lo) << (TB - KB)) | (warp << top);
+  }
+};
+
+// element index of tile position p relative to the tile's base: bits at or above CP move to H0
+template <int CP, int H0>
+__device__ __forceinline__ constexpr uint32_t alt_index(uint32_t p) {
+  return (p & ((1u << CP) - 1u)) | ((p >> CP) << H0);
+}
+
+// A value the compiler may not relate to earlier uses: the swizzled addresses of
+// a round are cheap to form again and too many to keep between the rounds.
+__device__ __forceinline__ uint32_t alt_fresh(uint32_t x) {
+  asm volatile("" : "+r"(x));
+  return x;
+}
+
+template <class R, int TB, int KB, int r, bool SWZ>
+__device__ __forceinline__ void alt_load(const unsigned char* s, typename El<R>::T (&v)[1 << KB], uint32_t base) {
+  constexpr int lo = AltPlan<TB, KB>::reg_lo(r);
+  const uint32_t sb = alt_fresh(SWZ ? swz<double>(base) : base);
+#pragma unroll
+  for (int j = 0; j < (1 << KB); ++j)
+    v[j] = El<R>::ld(s + 16u * (sb ^ (SWZ ? swz<double>((uint32_t)j << lo) : (uint32_t)j << lo)));
+}
+template <class R, int TB, int KB, int r>
+__device__ __forceinline__ void alt_store(unsigned char* s, const typename El<R>::T (&v)[1 << KB], uint32_t base) {
+  constexpr int lo = AltPlan<TB, KB>::reg_lo(r);
+  const uint32_t sb = alt_fresh(swz<double>(base));
+#pragma unroll
+  for (int j = 0; j < (1 << KB); ++j) El<R>::st(s + 16u * (sb ^ swz<double>((uint32_t)j << lo)), v[j]);
+}
+// the rotations of round r's new bits that belong to the set (tile bits >= cp)
+template <class R, int TB, int KB, int CP, int r>
+__device__ __forceinline__ void alt_rotate(typename El<R>::T (&v)[1 << KB], R t) {
+  constexpr int lo = AltPlan<TB, KB>::reg_lo(r);
+#pragma unroll
+  for (int k = 0; k < AltPlan<TB, KB>::act_hi(r); ++k) {
+    if (lo + k >= CP) {
+#pragma unroll
+      for (int j = 0; j < (1 << KB); ++j)
+        if (!(j & (1 << k))) El<R>::bfly(v[j], v[j | (1 << k)], t);
+    }
+  }
+}
+// E of the thread's elements in round r's layout, brought into shared memory by
+// asynchronous copies while the tile is on its way (every thread reads back only
+// what it copied: no barrier). Round 2 holds consecutive elements (16-byte copies);
+// the others one 4-byte word per element (complex128: the word around its uint16).
+__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+template <class R, int TB, int KB, int CP, int H0, int r>
+struct AltE {
+  static constexpr int kThreads = AltPlan<TB, KB>::kThreads;
+  static constexpr int lo = AltPlan<TB, KB>::reg_lo(r);
+  static constexpr bool kRun = r == 2 && CP >= KB;             // 2^KB consecutive elements
+  static constexpr int kPieces = (1 << KB) * (int)sizeof(uint16_t) * El<R>::kAmps / 16;  // 16-byte pieces of a run
+  __device__ static void fetch(const uint16_t* __restrict__ E, uint32_t tile_base, uint32_t base, uint32_t es) {
+    const uint32_t g0 = tile_base | alt_index<CP, H0>(base);
+    const uint32_t tid = threadIdx.x;
+    if constexpr (kRun) {
+      const unsigned char* p = reinterpret_cast<const unsigned char*>(E + (size_t)g0 * El<R>::kAmps);
+#pragma unroll
+      for (int q = 0; q < kPieces; ++q) cp_async16(es + 16u * (uint32_t)(q * kThreads + tid), p + 16 * q);
+    } else {
+      const uint32_t* p = reinterpret_cast<const uint32_t*>(E) + (sizeof(R) == 4 ? g0 : g0 >> 1);
+#pragma unroll
+      for (int j = 0; j < (1 << KB); ++j)
+        cp_async4(es + 4u * (uint32_t)(j * kThreads + tid), p + (alt_index<CP, H0>((uint32_t)j << lo) >> (sizeof(R) == 4 ? 0 : 1)));
+    }
+  }
+  // E of element j of the thread
+  __device__ static uint32_t get1(const unsigned char* es, uint32_t base, uint32_t j) {
+    const uint32_t tid = threadIdx.x;
+    if constexpr (kRun) {
+      constexpr uint32_t per = 16 / (sizeof(uint16_t) * El<R>::kAmps);  // elements of a piece
+      const unsigned char* p = es + 16u * ((j / per) * kThreads + tid);
+      if constexpr (sizeof(R) == 4)
+        return reinterpret_cast<const uint32_t*>(p)[j % per];
+      else
+        return reinterpret_cast<const uint16_t*>(p)[j % per];
+    } else {
+      const uint32_t w = *reinterpret_cast<const uint32_t*>(es + 4u * (j * kThreads + tid));
+      return sizeof(R) == 4 ? w : (((base + (j << lo)) & 1u) ? w >> 16 : w & 0xFFFFu);
+    }
+  }
+  // E of elements j0 .. j0 + 7 of the thread (base: tile position of its element 0)
+  __device__ static void get8(const unsigned char* es, uint32_t base, int j0, uint32_t (&ev)[8]) {
+    const uint32_t tid = threadIdx.x;
+    if constexpr (kRun) {
+#pragma unroll
+      for (int q = 0; q < (sizeof(R) == 4 ? 2 : 1); ++q) {
+        const uint4 a = *reinterpret_cast<const uint4*>(es + 16u * (uint32_t)((j0 / (sizeof(R) == 4 ? 4 : 8) + q) * kThreads + tid));
+        const uint32_t w[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          if constexpr (sizeof(R) == 4) {
+            ev[4 * q + i] = w[i];
+          } else {
+            ev[2 * i] = w[i] & 0xFFFFu;
+            ev[2 * i + 1] = w[i] >> 16;
+          }
+        }
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const uint32_t w = *reinterpret_cast<const uint32_t*>(es + 4u * (uint32_t)((j0 + i) * kThreads + tid));
+        if constexpr (sizeof(R) == 4) {
+          ev[i] = w;
+        } else {
+          const uint32_t odd = (base + (((uint32_t)(j0 + i) << lo))) & 1u;  // which uint16 of the word
+          ev[i] = odd ? w >> 16 : w & 0xFFFFu;
+        }
+      }
+    }
+  }
+};
+
+// what a turning pass does at its turn
+template <class R>
+struct AltTurn {
+  R t_pre, t_post, scale;
+  bool post, meas;
+};
+
+// Measurement of the thread's elements at the turn: rolled, from the thread's own
+// slots of the tile and of the staged E (no barrier), so that it costs the passes
+// that measure nothing neither registers nor instruction cache. Unrolled on the
+// register copies it pushed the 2^12-element kernels into spills, which go to L2:
+// next to the tile the L1 has little room.
+template <class R, int TB, int KB, int CP, int H0, int r>
+__device__ __forceinline__ void alt_measure(const typename El<R>::T (&v)[1 << KB], unsigned char* tile,
+                                            const unsigned char* es, const AltInst<R>& D, uint32_t tile_base,
+                                            uint32_t base, double* acc3) {
+  constexpr int lo = AltPlan<TB, KB>::reg_lo(r);
+  alt_store<R, TB, KB, r>(tile, v, base);
+  const uint32_t sb = swz<double>(base), g0 = tile_base | alt_index<CP, H0>(base);
+  MeasureAcc acc;
+#pragma unroll 1
+  for (uint32_t j = 0; j < (1u << KB); ++j) {
+    const typename El<R>::T x = El<R>::ld(tile + 16u * (sb ^ swz<double>(j << lo)));
+    const uint32_t e = AltE<R, TB, KB, CP, H0, r>::get1(es, base, j);
+    measure_el(acc, x, e, g0 + alt_index<CP, H0>(j << lo), D.e0, D.s0);
+  }
+  const double a = warp_sum(acc.norm), b = warp_sum(acc.p_less), c = warp_sum(acc.d_h);
+  if ((threadIdx.x & 31u) == 0) {  // the warp's sums over the CTA's tiles of this pass
+    acc3[0] += a;
+    acc3[1] += b;
+    acc3[2] += c;
+  }
+}
+
+template <class R, int TB, int KB, int CP, int H0, int r>
+__device__ __forceinline__ void alt_turn(typename El<R>::T (&v)[1 << KB], unsigned char* tile, const unsigned char* es,
+                                         const AltInst<R>& D, const AltTurn<R>& T, uint32_t tile_base, uint32_t base,
+                                         const unsigned char* tab, double* acc3) {
+  cp_async_wait();
+  if (T.meas) alt_measure<R, TB, KB, CP, H0, r>(v, tile, es, D, tile_base, base, acc3);
+  constexpr uint32_t kEntry = sizeof(typename AltPhase<R>::entry);
+  const AltTab P{tab + (T.post ? kEntry : 0u), T.post ? kEntry : 0u, (uint32_t)D.c0};
+#pragma unroll
+  for (int j0 = 0; j0 < (1 << KB); j0 += 8) {
+    uint32_t ev[8];
+    AltE<R, TB, KB, CP, H0, r>::get8(es, base, j0, ev);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      AltPhase<R>::apply(v[j0 + i], ev[i], P);
+      El<R>::bfly_inner(v[j0 + i], T.t_post);
+    }
+  }
+  if (T.scale != (R)1) {
+#pragma unroll
+    for (int j = 0; j < (1 << KB); ++j) El<R>::scale(v[j], T.scale);
+  }
+  alt_rotate<R, TB, KB, CP == TB ? 0 : CP, r>(v, T.t_post);
+}
+
+// the round a pass turns in (CP = TB: the A set)
+__host__ __device__ constexpr int alt_turn_round(int TB, int KB, int CP) {
+  return CP == TB ? 2 : (TB - CP + KB - 1) / KB - 1;
+}
+
+// A turning pass on one staged tile (CP = TB: a tile of the A set). `wait()` returns
+// when the tile has landed, `stage_free()` runs in every thread after a barrier
+// behind the last shared-memory read.
+template <class R, int TB, int KB, int CP, int H0, class W, class F>
+__device__ __forceinline__ void alt_tile_turn(unsigned char* tile, const AltInst<R>& D, const AltTurn<R>& T,
+                                              uint32_t tile_base, const unsigned char* tab, unsigned char* es,
+                                              double* acc3, W&& wait, F&& stage_free) {
+  using PL = AltPlan<TB, KB>;
+  constexpr int RT = alt_turn_round(TB, KB, CP);
+  constexpr int LO = CP == TB ? 0 : CP;  // lowest tile bit of the set
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const uint32_t b0 = PL::template base<0>(lane, warp);
+  typename El<R>::T v[1 << KB];
+  wait();
+  alt_load<R, TB, KB, 0, false>(tile, v, b0);
+  if constexpr (RT == 0) {
+    alt_rotate<R, TB, KB, LO, 0>(v, T.t_pre);
+    if (T.meas) __syncwarp();  // the measurement's swizzled slots were other lanes' linear ones
+    alt_turn<R, TB, KB, CP, H0, 0>(v, tile, es, D, T, tile_base, b0, tab, acc3);
+    __syncthreads();
+    stage_free();
+  } else {
+    alt_rotate<R, TB, KB, LO, 0>(v, T.t_pre);
+    __syncwarp();  // the linear tile's reads against swizzled stores: same warp
+    alt_store<R, TB, KB, 0>(tile, v, b0);
+    __syncthreads();
+    const uint32_t b1 = PL::template base<1>(lane, warp);
+    alt_load<R, TB, KB, 1, true>(tile, v, b1);
+    alt_rotate<R, TB, KB, LO, 1>(v, T.t_pre);
+    if constexpr (RT == 1) {
+      alt_turn<R, TB, KB, CP, H0, 1>(v, tile, es, D, T, tile_base, b1, tab, acc3);
+    } else {
+      alt_store<R, TB, KB, 1>(tile, v, b1);
+      __syncwarp();  // rounds 1 and 2 share their warp bits
+      const uint32_t b2 = PL::template base<2>(lane, warp);
+      alt_load<R, TB, KB, 2, true>(tile, v, b2);
+      alt_rotate<R, TB, KB, LO, 2>(v, T.t_pre);
+      alt_turn<R, TB, KB, CP, H0, 2>(v, tile, es, D, T, tile_base, b2, tab, acc3);
+      alt_store<R, TB, KB, 2>(tile, v, b2);
+      __syncwarp();
+      alt_load<R, TB, KB, 1, true>(tile, v, b1);
+      alt_rotate<R, TB, KB, LO, 1>(v, T.t_post);
+    }
+    alt_store<R, TB, KB, 1>(tile, v, b1);
+    __syncthreads();
+    alt_load<R, TB, KB, 0, true>(tile, v, b0);
+    __syncthreads();
+    stage_free();
+    alt_rotate<R, TB, KB, LO, 0>(v, T.t_post);
+  }
+  unsigned char* g = D.state + 16ull * (tile_base | alt_index<CP, H0>(b0));
+#pragma unroll
+  for (int j = 0; j < (1 << KB); ++j)
+    El<R>::st(g + 16ull * alt_index<CP, H0>((uint32_t)j << PL::reg_lo(0)), v[j]);
+}
+
+template <class R>
+__device__ __forceinline__ void alt_issue(const AltInst<R>& D, int s, uint32_t tile, uint32_t bytes,
+                                          unsigned char* stage, uint32_t fb) {
+  const AltSet& S = D.set[s];
+  const int mid = (int)(tile & ((1u << S.mid_bits) - 1u)), hi = (int)(tile >> S.mid_bits);
+  const int md = S.mid_dim, hd = S.hi_dim;
+  fence_proxy_async_shared();  // the CTA's generic accesses of the stage precede the copy's writes
+  mbar_arrive_expect_tx(fb, bytes);
+  tma_load_5d(smem_addr(stage), &D.map[s], tile_coord(0, md, mid, hd, hi), tile_coord(1, md, mid, hd, hi),
+              tile_coord(2, md, mid, hd, hi), tile_coord(3, md, mid, hd, hi), tile_coord(4, md, mid, hd, hi), fb);
+}
+// first element of a tile: the id's low bits are element bits [CP, H0), the others those above the set
+template <int TB, int CP, int H0>
+__device__ __forceinline__ uint32_t alt_tile_base(uint32_t tile) {
+  if constexpr (CP == TB) return tile << TB;
+  constexpr int mb = H0 - CP;
+  return ((tile & ((1u << mb) - 1u)) << CP) | ((tile >> mb) << (H0 + TB - CP));
+}
+
+// A plain pass on one staged tile of the A set (2^12 elements, loaded through the
+// 128-byte TMA swizzle so that the first round reads without bank conflicts; the
+// rounds of the warp-local A1, then the top four bits): three rounds, the last
+// one's lanes over the low bits.
+template <class R, class W, class F>
+__device__ __forceinline__ void alt_tile_plain(unsigned char* tile, const AltInst<R>& D, R t, uint32_t tile_base,
+                                               W&& wait, F&& stage_free) {
+  using PL = PlanA1Warp;
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const uint32_t ba = pdep(lane, PL::R1_LANE) | (warp << 9);
+  typename El<R>::T v[16];
+  wait();
+  {
+    const uint32_t sb = ba ^ ((ba >> 3) & 7u);
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const uint32_t o = pdep((uint32_t)j, PL::R1_REG);
+      v[j] = El<R>::ld(tile + 16u * (sb ^ o ^ ((o >> 3) & 7u)));
+    }
+  }
+  el_bflys<R, PL::R1_REG, PL::R1_REG>(v, t);
+  el_store_swz<R, PL::R1_REG>(tile, v, alt_fresh(ba));  // a thread's 128-byte groups are its own: no hazard
+  __syncwarp();
+  const uint32_t bb = pdep(lane, PL::R2_LANE) | (warp << 9);
+  el_load<R, PL::R2_REG, true>(tile, v, alt_fresh(bb));
+  el_bflys<R, PL::R2_REG, PL::R2_REG>(v, t);
+  el_store_swz<R, PL::R2_REG>(tile, v, alt_fresh(bb));
+  __syncthreads();
+  const uint32_t bc = lane | (warp << 5);
+  el_load<R, 0xF00u, true>(tile, v, bc);
+  __syncthreads();
+  stage_free();
+  el_bflys<R, 0xF00u, 0xF00u>(v, t);
+  unsigned char* g = D.state + 16ull * (tile_base | bc);
+#pragma unroll
+  for (int j = 0; j < 16; ++j) El<R>::st(g + 16ull * ((uint32_t)j << 8), v[j]);
+}
+
+// thread 0: wait until `ctr` reaches `target`; false on timeout or abort
+__device__ __forceinline__ bool alt_wait(const AltBarrier& B, uint32_t target) {
+  uint32_t polls = 0;
+  while ((int32_t)(ld_acquire(B.ctr) - target) < 0) {
+    if (++polls > B.poll_limit) {
+      atomicCAS(B.err, 0, DEV_TIMEOUT);
+      atomicExch(B.abort, 1);
+      return false;
+    }
+    if ((polls & 63u) == 0u && aborted(B.abort)) return false;
+  }
+  fence_proxy_async_global();  // the TMA reads what the barrier released
+  return true;
+}
+
+// dynamic shared memory: the tile, a word of E per element, the CTA's control
+// block, the phase table
+struct AltCtl {
+  uint64_t full_bar;
+  int stop;      // the run has failed: every thread leaves at the end of the pass
+  int inflight;  // thread 0: a tile's copy is on its way
+  double acc[16][3];  // per warp: norm, P_<, <d_H> of the pass
+};
+template <int TB>
+struct AltSmem {
+  static constexpr int kEOff = 16 << TB, kCtlOff = kEOff + (4 << TB), kTabOff = kCtlOff + 512;
+  static_assert(sizeof(AltCtl) <= 512, "the control block's room");
+  // + room to align the tile to 1024 bytes (swizzled loads)
+  static int bytes(int n_j, int entry) { return kTabOff + (((n_j + 1) * entry + 127) & ~127) + 1024; }
+};
+
+// One CTA of a run's group.
+template <class R, int TB, int KB>
+struct AltCta {
+  using PL = AltPlan<TB, KB>;
+  using SM = AltSmem<TB>;
+  static constexpr uint32_t kBytes = 16u << TB;
+  const AltInst<R>& D;
+  const AltBarrier& B;
+  uint32_t rank, G;
+  unsigned char* stage;
+  uint32_t parity, epoch;
+
+  __device__ __forceinline__ volatile AltCtl& ctl() const { return *reinterpret_cast<volatile AltCtl*>(stage + SM::kCtlOff); }
+  __device__ __forceinline__ uint32_t bar() const { return smem_addr(stage) + SM::kCtlOff; }
+  __device__ __forceinline__ unsigned char* es() const { return stage + SM::kEOff; }
+  __device__ __forceinline__ unsigned char* tab() const { return stage + SM::kTabOff; }
+
+  __device__ __forceinline__ void issue(int map, uint32_t tile) {
+    if (threadIdx.x == 0 && tile < D.n_tiles && !ctl().stop) {
+      alt_issue(D, map, tile, kBytes, stage, bar());
+      ctl().inflight = 1;
+    }
+    __syncwarp();
+  }
+  __device__ __forceinline__ void wait() {
+    for (uint32_t i = 0; i < kWaitPolls; ++i) {
+      if (mbar_try_wait(bar(), parity)) {
+        parity ^= 1u;
+        if (threadIdx.x == 0) ctl().inflight = 0;
+        return;
+      }
+      if (ctl().stop) return;
+    }
+    ctl().stop = 1;
+    atomicCAS(B.err, 0, DEV_TIMEOUT);
+    atomicExch(B.abort, 1);
+  }
+  // E of a tile of set (CP, H0) for this thread's elements at the turn
+  template <int CP, int H0>
+  __device__ __forceinline__ void fetch_e(uint32_t tile) {
+    if (tile >= D.n_tiles) return;
+    constexpr int RT = alt_turn_round(TB, KB, CP);
+    AltE<R, TB, KB, CP, H0, RT>::fetch(D.E, alt_tile_base<TB, CP, H0>(tile),
+                                       PL::template base<RT>(threadIdx.x & 31u, threadIdx.x >> 5), smem_addr(es()));
+  }
+  // the turning pass of step k on the tiles of set `s` (E of the first one already fetched)
+  template <int CP, int H0>
+  __device__ __forceinline__ void turn(int s, int k) {
+    AltTurn<R> T;
+    const bool pre = k > D.k0;
+    T.post = k < D.k1;
+    T.t_pre = pre ? D.tan[k - 1] : (R)0;  // a tangent of 0 rotates nothing
+    T.t_post = T.post ? D.tan[k] : (R)0;
+    T.scale = T.post ? D.scale[k] : (R)1;
+    const int slot = (pre || D.meas_first) ? D.slot[k] : -1;
+    T.meas = slot >= 0;
+    const uint32_t warp = threadIdx.x >> 5;
+    double* acc3 = const_cast<double*>(&ctl().acc[warp][0]);
+    if (T.meas && (threadIdx.x & 31u) == 0) acc3[0] = acc3[1] = acc3[2] = 0.0;
+    for (uint32_t tile = rank; tile < D.n_tiles; tile += G) {
+      alt_tile_turn<R, TB, KB, CP, H0>(stage, D, T, alt_tile_base<TB, CP, H0>(tile), tab(), es(), acc3,
+                                       [&]() { wait(); }, [&]() { issue(s, tile + G); });
+      fetch_e<CP, H0>(tile + G);  // after the stores, when the registers are free
+    }
+    if (T.meas) {
+      __syncthreads();
+      if (threadIdx.x < 3u) {
+        double x = 0;
+        for (int w = 0; w < PL::kWarps; ++w) x += ctl().acc[w][threadIdx.x];
+        D.partials[3 * ((size_t)(slot - D.row0) * G + rank) + threadIdx.x] = x;
+      }
+    }
+  }
+  __device__ __forceinline__ void plain(int s, int k) {
+    const R t = D.tan[k];
+    for (uint32_t tile = rank; tile < D.n_tiles; tile += G)
+      alt_tile_plain<R>(stage, D, t, alt_tile_base<TB, TB, TB>(tile), [&]() { wait(); }, [&]() { issue(s, tile + G); });
+  }
+  // the end of a pass: every CTA's stores are in memory, then the next pass's first tile
+  __device__ __forceinline__ bool next_pass(int map) {
+    if (__syncthreads_or(ctl().stop)) return false;  // every store of the CTA is issued
+    if (threadIdx.x == 0) {
+      red_release_add(B.ctr, 1u);  // releases every thread's stores (ordered before it by the CTA barrier)
+      epoch += G;
+      if (!alt_wait(B, epoch)) ctl().stop = 1;
+    }
+    // lane 0's warp waits for it here: its other lanes must not spin on the tile's
+    // barrier while lane 0 polls (a warp in a suspended try_wait polls nothing)
+    __syncwarp();
+    issue(map, rank);
+    return true;
+  }
+  __device__ __forceinline__ void stage_table() {
+    auto* dst = reinterpret_cast<typename AltPhase<R>::entry*>(tab());
+    for (int i = (int)threadIdx.x; i <= D.n_j; i += PL::kThreads) dst[i] = D.tab[i];
+    __syncthreads();
+  }
+  __device__ __forceinline__ void begin() {
+    if (threadIdx.x == 0) {
+      ctl().stop = 0;
+      ctl().inflight = 0;
+      mbar_init(bar(), 1);
+      fence_barrier_init();
+    }
+    parity = epoch = 0u;
+    __syncthreads();
+  }
+  // a copy still on its way after a failure lands before its CTA leaves
+  __device__ __forceinline__ void leave() {
+    if (threadIdx.x == 0 && ctl().stop && ctl().inflight) mbar_wait_bounded(bar(), parity, B.err);
+  }
+};
+
+// Two sets: A (the tile's bits) and the W bits above it.
+template <class R, int TB, int KB, int W>
+__device__ __forceinline__ void alt_run2(AltCta<R, TB, KB>& C) {
+  const AltInst<R>& D = C.D;
+  if (D.k0 & 1) C.template fetch_e<TB - W, TB>(C.rank); else C.template fetch_e<TB, TB>(C.rank);
+  C.issue(D.k0 & 1, C.rank);
+  C.stage_table();
+  for (int k = D.k0;; ++k) {
+    if (k & 1) {
+      C.template turn<TB - W, TB>(1, k);
+      if (k == D.k1) break;
+      C.template fetch_e<TB, TB>(C.rank);
+    } else {
+      C.template turn<TB, TB>(0, k);
+      if (k == D.k1) break;
+      C.template fetch_e<TB - W, TB>(C.rank);
+    }
+    if (!C.next_pass((k + 1) & 1)) break;
+  }
+  C.leave();
+}
+
+// Three sets: turning passes on the W2 bits above the A set and the W3 bits above
+// those in turn, plain passes over the A set between them.
+template <class R, int W2, int W3>
+__device__ __forceinline__ void alt_run3(AltCta<R, 12, 4>& C) {
+  constexpr int TB = 12, C2 = TB - W2, C3 = TB - W3, H3 = TB + W2;
+  const AltInst<R>& D = C.D;
+  if (D.k0 & 1) C.template fetch_e<C3, H3>(C.rank); else C.template fetch_e<C2, TB>(C.rank);
+  C.issue(1 + (D.k0 & 1), C.rank);
+  C.stage_table();
+  for (int k = D.k0;; ++k) {
+    if (k & 1)
+      C.template turn<C3, H3>(2, k);
+    else
+      C.template turn<C2, TB>(1, k);
+    if (k == D.k1 || !C.next_pass(0)) break;
+    C.plain(0, k);
+    if (k & 1) C.template fetch_e<C2, TB>(C.rank); else C.template fetch_e<C3, H3>(C.rank);
+    if (!C.next_pass(1 + ((k + 1) & 1))) break;
+  }
+  C.leave();
+}
+
+// W3 = 0: two sets (A and W2), else three
+template <class R, int TB, int KB, int W2, int W3>
+__global__ void __launch_bounds__(AltPlan<TB, KB>::kThreads, TB == 10 ? 4 : TB == 12 ? 2 : 1)
+    alt_kernel(const __grid_constant__ AltInst<R> D, const __grid_constant__ AltBarrier B) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  AltCta<R, TB, KB> C{D, B, blockIdx.x, gridDim.x, smem_raw + ((1024u - (smem_addr(smem_raw) & 1023u)) & 1023u)};
+  C.begin();
+  if constexpr (W3 == 0)
+    alt_run2<R, TB, KB, W2>(C);
+  else
+    alt_run3<R, W2, W3>(C);
+}
+
+// results[row0 + row] = sum over the G CTAs of a run in index order (one warp a row)
+__global__ void __launch_bounds__(128) alt_reduce_kernel(const double* __restrict__ partials, int rows, int G,
+                                                         double* __restrict__ results) {
+  const int row = (int)(blockIdx.x * 4 + (threadIdx.x >> 5)), lane = (int)(threadIdx.x & 31);
+  if (row >= rows) return;
+  double s[3] = {0, 0, 0};
+  for (int i = lane; i < G; i += 32)
+#pragma unroll
+    for (int q = 0; q < 3; ++q) s[q] += partials[3 * ((size_t)row * G + i) + q];
+#pragma unroll
+  for (int q = 0; q < 3; ++q) s[q] = warp_sum(s[q]);
+  if (lane == 0) {
+    results[4 * (size_t)row + 0] = s[1];
+    results[4 * (size_t)row + 1] = s[2];
+    results[4 * (size_t)row + 2] = s[0];
+  }
+}
+
+}  // namespace bk

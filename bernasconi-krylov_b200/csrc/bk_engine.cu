@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "bk_adjoint.cuh"
+#include "bk_alt.cuh"
 #include "bk_aux.cuh"
 #include "bk_engine.h"
 #include "bk_fused.cuh"
@@ -94,12 +95,17 @@ struct bk_ctx {
   int num_sms = 148;
   bool planar = false;        // complex64 state stored pair-planar (persistent engine)
   int slab_lag = 3;           // persistent engine: S2 queue lag behind A1, in slabs
-  int engine_mode = 0;        // 0 persistent dataflow, 1 one launch per pass (tile grid)
+  int engine_mode = 4;        // 0 persistent dataflow, 1 one launch per pass (tile grid), 4 turning passes
   int force_w2 = 0;           // S2 width when > 0 and valid for the size (else the default split)
   int e_recompute = 0;        // tile engine: 1 = E(s) recomputed from popcounts in A1, 0 = uint16 table
   int a1_wide = 0;            // per-pass schedule A1: 1 = 512 threads x 8 elements, 2 = warp-local (bits 0-8)
   int phase_table = 0;        // complex64 per-pass A1 (kernels 1-3): 1 = the full per-energy phase table
   int adj_a1 = 0;             // adjoint reverse sweep A1: 0 = 12-bit, 1 = warp-local (element bits 0-8)
+  void* d_alt = nullptr;      // turning passes: phase table, per-step arrays, partial sums, counters
+  size_t alt_cap = 0;
+  void* h_stage = nullptr;    // pinned staging of a run's uploads
+  size_t stage_cap = 0;
+  std::map<std::pair<const void*, int>, int> occupancy;  // (kernel, dynamic smem) -> CTAs per SM
   uint32_t wait_polls = 0;    // persistent engine: polls of a dependency wait before it gives up (0 = default)
   uint64_t s23_checked = 0;   // fused strided pass geometry (np, a1, w2, lag) whose closed form was checked
   int64_t hold_step = -1;     // test hook: launch step whose dependency can never be met (-1 = off)
@@ -961,7 +967,7 @@ template <class R>
 int evolve_persist(bk_ctx* c, const bk_evolve_params* p, const Schedule& S, double angle_unit,
                    const std::vector<R>& tans, const std::vector<R>& scales) {
   PersistRun<R> run;
-  BK_TRY(persist_prepare<R>(c, p, S, angle_unit, tans, scales, &run, c->engine_mode != 0));
+  BK_TRY(persist_prepare<R>(c, p, S, angle_unit, tans, scales, &run, c->engine_mode >= 1 && c->engine_mode <= 3));
   const int n = p->n;
   cudaStream_t st = c->stream;
   unsigned int* ctr = run.ctr;
@@ -1079,6 +1085,257 @@ int evolve_persist(bk_ctx* c, const bk_evolve_params* p, const Schedule& S, doub
 }
 
 // ---------------------------------------------------------------------------
+// turning-pass engine (csrc/bk_alt.cuh)
+// ---------------------------------------------------------------------------
+// the phase angles the engine accepts (complex64: those the level table holds)
+template <class R>
+int check_phase(bk_ctx* c, int n, double angle_unit) {
+  if constexpr (sizeof(R) == 4) {
+    const int emax = (n - 1) * n * (2 * n - 1) / 6;
+    const int K = std::max(2, (emax + kPhaseH) / kPhaseH);
+    if (!(std::fabs(angle_unit) * (double)(K - 1) <= 0.5))
+      return fail(c, BK_ERR_UNSUPPORTED, "phase angle per unit energy %g too large for the table", angle_unit);
+  }
+  return BK_OK;
+}
+
+// pinned host memory for a run's uploads (one copy, no staging by the driver)
+int ensure_stage(bk_ctx* c, size_t bytes) {
+  if (c->stage_cap >= bytes) return BK_OK;
+  if (c->h_stage) cudaFreeHost(c->h_stage);
+  c->h_stage = nullptr;
+  c->stage_cap = 0;
+  const size_t room = std::max<size_t>(bytes, 1 << 16);
+  BK_CUDA(c, cudaMallocHost(&c->h_stage, room));
+  c->stage_cap = room;
+  return BK_OK;
+}
+
+template <class R>
+using AltKernel = void (*)(AltInst<R>, AltBarrier);
+struct AltGeo {
+  int tb = 0, w2 = 0, w3 = 0;
+};
+// Tile and split by the number of element bits np (measured on a B200, us a step,
+// complex64 / complex128):
+//   np <= 18: 2^10-element tiles, a 64-thread CTA each, two sets. The barrier and the
+//     exchange through L2 bound these sizes, so small tiles on many SMs win (np = 18:
+//     5.7 / 5.1 against 16.5 / 14.6 for a launch per pass).
+//   np <= 20: 2^12-element tiles, two CTAs an SM, two sets (np = 20: 12.3 / 12.2
+//     against 22.8 / 20.6).
+//   np <= 23: 2^13-element tiles with 32 elements a thread, so that two sets still do
+//     (one pass a step): np = 21 25.4 / 23.9 against 27.8 / 26.7 with 2^12-element
+//     tiles and a 9-bit second set, np = 23 94 / 86 against 103 / 110 with three sets.
+//   beyond: 2^12-element tiles, three sets (two passes a step).
+bool alt_geometry(int np, AltGeo* g) {
+  if (np < kElemBits + 1 || np > 30) return false;
+  g->tb = np <= 18 ? 10 : np <= 20 || np > 23 ? 12 : 13;
+  const int rest = np - g->tb;
+  g->w2 = np <= 23 ? rest : (rest + 1) / 2;
+  g->w3 = rest - g->w2;
+  return true;
+}
+template <class R>
+bool alt_takes(const bk_ctx* c, int n) {
+  AltGeo g;
+  return c->e_recompute == 0 && alt_geometry(sizeof(R) == 4 ? n - 1 : n, &g);
+}
+template <class R>
+AltKernel<R> alt_kernel_of(const AltGeo& g) {
+  switch (g.tb * 256 + g.w2 * 16 + g.w3) {
+    case 0xA30: return alt_kernel<R, 10, 4, 3, 0>;
+    case 0xA40: return alt_kernel<R, 10, 4, 4, 0>;
+    case 0xA50: return alt_kernel<R, 10, 4, 5, 0>;
+    case 0xA60: return alt_kernel<R, 10, 4, 6, 0>;
+    case 0xA70: return alt_kernel<R, 10, 4, 7, 0>;
+    case 0xA80: return alt_kernel<R, 10, 4, 8, 0>;
+    case 0xC70: return alt_kernel<R, 12, 4, 7, 0>;
+    case 0xC80: return alt_kernel<R, 12, 4, 8, 0>;
+    case 0xD80: return alt_kernel<R, 13, 5, 8, 0>;
+    case 0xD90: return alt_kernel<R, 13, 5, 9, 0>;
+    case 0xDA0: return alt_kernel<R, 13, 5, 10, 0>;
+    case 0xC66: return alt_kernel<R, 12, 4, 6, 6>;
+    case 0xC76: return alt_kernel<R, 12, 4, 7, 6>;
+    case 0xC77: return alt_kernel<R, 12, 4, 7, 7>;
+    case 0xC87: return alt_kernel<R, 12, 4, 8, 7>;
+    case 0xC88: return alt_kernel<R, 12, 4, 8, 8>;
+    case 0xC98: return alt_kernel<R, 12, 4, 9, 8>;
+    default: return alt_kernel<R, 12, 4, 9, 9>;
+  }
+}
+int alt_smem_bytes(const AltGeo& g, int n_j, int entry) {
+  return g.tb == 10 ? AltSmem<10>::bytes(n_j, entry) : g.tb == 12 ? AltSmem<12>::bytes(n_j, entry) : AltSmem<13>::bytes(n_j, entry);
+}
+int ctas_per_sm(bk_ctx* c, const void* fn, int threads, int smem, int* out) {
+  auto key = std::make_pair(fn, smem);
+  auto it = c->occupancy.find(key);
+  if (it == c->occupancy.end()) {
+    int n = 0;
+    BK_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, threads, (size_t)smem));
+    it = c->occupancy.emplace(key, n).first;
+  }
+  *out = it->second;
+  return BK_OK;
+}
+
+// Full phase table: entry 0 rotates by nothing, entry 1 + j by level E = c0 + 4 j.
+inline void alt_table(int n, double angle_unit, float2* t, int c0, int n_j) {
+  const double two_pi = 6.283185307179586;
+  *t++ = make_float2(0.f, 0.f);
+  for (int j = 0; j < n_j; ++j) {
+    const double r = std::remainder(-angle_unit * (double)(c0 + 4 * j), two_pi);
+    t[j] = make_float2((float)(-std::tan(0.25 * r)), (float)std::sin(0.5 * r));
+  }
+}
+inline void alt_table(int n, double angle_unit, double2* t, int c0, int n_j) {
+  *t++ = make_double2(1.0, 0.0);
+  for (int j = 0; j < n_j; ++j) {
+    const double r = -angle_unit * (double)(c0 + 4 * j);
+    t[j] = make_double2(std::cos(r), std::sin(r));
+  }
+}
+
+int alt_set(bk_ctx* c, void* state, int np, int cp, int h0, int w, CUtensorMap* map, AltSet* s) {
+  TmaDesc d;
+  BK_TRY(build_amp_map(c, state, np, BK_C128, cp, h0, w, &d));
+  *map = d.map;
+  s->mid_dim = d.mid_dim;
+  s->hi_dim = d.hi_dim;
+  s->mid_bits = w > 0 ? (int)d.mid_bits : 0;
+  return BK_OK;
+}
+
+constexpr size_t kAltPartialBytes = (size_t)64 << 20;  // partial sums of one launch (more rows: more launches)
+
+// A prepared run over c->d_state: geometry, uploads and the kernel; alt_launch
+// runs any range of its steps.
+template <class R>
+struct AltRun {
+  AltInst<R> D{};
+  AltBarrier B{};
+  AltKernel<R> fn = nullptr;
+  int smem = 0, threads = 0;
+  uint32_t G = 0;
+  int max_rows = 1;  // measurement rows the partial sums of one launch have room for
+};
+
+template <class R>
+int alt_prepare(bk_ctx* c, int n, uint64_t s0, int64_t e0, double angle_unit, const Schedule& S,
+                const std::vector<R>& tans, const std::vector<R>& scales, AltRun<R>* run) {
+  using entry = typename AltPhase<R>::entry;
+  const int np = sizeof(R) == 4 ? n - 1 : n, T = (int)tans.size();
+  AltGeo geo;
+  if (!alt_geometry(np, &geo)) return fail(c, BK_ERR_UNSUPPORTED, "turning passes: n = %d", n);
+  AltInst<R>& D = run->D;
+  if (geo.w3 == 0) {
+    BK_TRY(alt_set(c, c->d_state, np, geo.tb, geo.tb, 0, &D.map[0], &D.set[0]));
+  } else {  // the plain pass loads its tiles swizzled
+    TmaDesc d;
+    BK_TRY(build_a1_swizzled_map(c, c->d_state, np, &d));
+    D.map[0] = d.map;
+    D.set[0] = AltSet{-1, d.hi_dim, 0, 0};
+    BK_TRY(alt_set(c, c->d_state, np, geo.tb - geo.w3, geo.tb + geo.w2, geo.w3, &D.map[2], &D.set[2]));
+  }
+  BK_TRY(alt_set(c, c->d_state, np, geo.tb - geo.w2, geo.tb, geo.w2, &D.map[1], &D.set[1]));
+  D.c0 = (n / 2) & 3;
+  D.n_j = ((n - 1) * n * (2 * n - 1) / 6 - D.c0) / 4 + 1;
+  D.n_tiles = 1u << (np - geo.tb);
+  run->fn = alt_kernel_of<R>(geo);
+  run->smem = alt_smem_bytes(geo, D.n_j, (int)sizeof(entry));
+  run->threads = geo.tb == 10 ? 64 : 256;
+  const void* fn = reinterpret_cast<const void*>(run->fn);
+  BK_TRY(allow_smem(c, fn, run->smem));
+  int per_sm = 0;
+  BK_TRY(ctas_per_sm(c, fn, run->threads, run->smem, &per_sm));
+  if (per_sm < 1) return fail(c, BK_ERR_CUDA, "turning pass: no room for a CTA (%d bytes of shared memory)", run->smem);
+  run->G = std::min<uint32_t>(D.n_tiles, (uint32_t)(per_sm * c->num_sms));
+
+  // one upload: phase table, tangents, rescales, measurement rows, zeroed counters
+  Bump b;
+  const size_t o_tab = b.take((size_t)(D.n_j + 1) * sizeof(entry));
+  const size_t o_tan = b.take((size_t)std::max(T, 1) * sizeof(R));
+  const size_t o_sc = b.take((size_t)std::max(T, 1) * sizeof(R));
+  const size_t o_slot = b.take((size_t)(T + 1) * sizeof(int));
+  const size_t o_ctr = b.take(64);
+  const size_t up = b.off;
+  const size_t row_bytes = 3 * sizeof(double) * (size_t)run->G;
+  run->max_rows = (int)std::max<size_t>(kAltPartialBytes / row_bytes, 1);
+  const size_t o_part = b.take(row_bytes * (size_t)std::max(1, std::min(S.n_meas, run->max_rows + 1)));
+  BK_TRY(ensure_buffer(c, &c->d_alt, &c->alt_cap, b.off));
+  BK_TRY(ensure_stage(c, up));
+  char *h = static_cast<char*>(c->h_stage), *d = static_cast<char*>(c->d_alt);
+  alt_table(n, angle_unit, reinterpret_cast<entry*>(h + o_tab), D.c0, D.n_j);
+  std::copy(tans.begin(), tans.end(), reinterpret_cast<R*>(h + o_tan));
+  std::copy(scales.begin(), scales.end(), reinterpret_cast<R*>(h + o_sc));
+  std::copy(S.slot.begin(), S.slot.end(), reinterpret_cast<int*>(h + o_slot));
+  std::memset(h + o_ctr, 0, 64);
+  BK_CUDA(c, cudaMemcpyAsync(d, h, up, cudaMemcpyHostToDevice, c->stream));
+  D.state = static_cast<unsigned char*>(c->d_state);
+  D.E = c->d_E;
+  D.tab = reinterpret_cast<const entry*>(d + o_tab);
+  D.tan = reinterpret_cast<const R*>(d + o_tan);
+  D.scale = reinterpret_cast<const R*>(d + o_sc);
+  D.slot = reinterpret_cast<const int*>(d + o_slot);
+  D.partials = reinterpret_cast<double*>(d + o_part);
+  D.e0 = (int)e0;
+  D.s0 = (uint32_t)(s0 & ((1ull << n) - 1ull));
+  run->B.ctr = reinterpret_cast<unsigned int*>(d + o_ctr);
+  run->B.abort = reinterpret_cast<int*>(d + o_ctr + 8);
+  run->B.err = c->d_err;
+  run->B.poll_limit = c->wait_polls > 0 ? c->wait_polls : kWaitPolls * 4u;
+  return BK_OK;
+}
+
+// Steps [k0, k1) and the measurement of psi_k1; `first`: no launch of this run has
+// measured psi_k0. rows measured, from row0 on. Enqueues only: a device wait that
+// gave up is in the context's error word.
+template <class R>
+int alt_launch(bk_ctx* c, AltRun<R>& r, int k0, int k1, bool first, int row0, int rows) {
+  cudaStream_t st = c->stream;
+  r.D.k0 = k0;
+  r.D.k1 = k1;
+  r.D.row0 = row0;
+  r.D.meas_first = first ? 1 : 0;
+  if (!first) BK_CUDA(c, cudaMemsetAsync(r.B.ctr, 0, sizeof(unsigned int), st));
+  size_t ev = 0;
+  BK_TRY(ev_begin(c, "turn", &ev));
+  void* args[] = {&r.D, &r.B};
+  BK_CUDA(c, cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(r.fn), dim3(r.G), dim3((unsigned)r.threads), args,
+                                         (size_t)r.smem, st));
+  BK_TRY(ev_end(c, ev));
+  if (rows > 0) {
+    alt_reduce_kernel<<<(rows + 3) / 4, 128, 0, st>>>(r.D.partials, rows, (int)r.G, c->d_results + 4 * (size_t)row0);
+    BK_CUDA(c, cudaGetLastError());
+  }
+  return BK_OK;
+}
+
+template <class R>
+int evolve_alt(bk_ctx* c, const bk_evolve_params* p, const Schedule& S, double angle_unit, const std::vector<R>& tans,
+               const std::vector<R>& scales) {
+  using Samp = typename std::conditional<sizeof(R) == 4, Planar64, double2>::type;
+  const int n = p->n, T = p->n_steps;
+  const Samp* psi = reinterpret_cast<const Samp*>(c->d_state);
+  AltRun<R> run;
+  BK_TRY(alt_prepare<R>(c, n, p->s0, p->e0, angle_unit, S, tans, scales, &run));
+  if (S.sample_pt[0] >= 0) BK_TRY(launch_sampling_t(c, psi, n, S.sample_pt[0], S.shots));
+  // segments end at sampling points (which read psi_k) and where the partial sums' room ends
+  int k0 = 0;
+  for (bool first = true;; first = false) {
+    int row0 = 0, rows = 0, k1 = k0;
+    for (int k = k0;; ++k) {
+      if ((k > k0 || first) && S.slot[(size_t)k] >= 0 && rows++ == 0) row0 = S.slot[(size_t)k];
+      k1 = k;
+      if (k == T || (k > k0 && (S.sample_pt[(size_t)k] >= 0 || rows >= run.max_rows))) break;
+    }
+    BK_TRY(alt_launch<R>(c, run, k0, k1, first, row0, rows));
+    if (k1 > 0 && S.sample_pt[(size_t)k1] >= 0) BK_TRY(launch_sampling_t(c, psi, n, S.sample_pt[(size_t)k1], S.shots));
+    if (k1 == T) return BK_OK;
+    k0 = k1;
+  }
+}
+
+// ---------------------------------------------------------------------------
 // batched evolution (persistent engine over many statevectors)
 // ---------------------------------------------------------------------------
 int batch_energy(bk_ctx* c, int n, uint16_t** out) {
@@ -1163,12 +1420,15 @@ int evolve_batch_t(bk_ctx* c, const bk_batch_params* bp, const bk_batch_instance
   std::vector<long double> row_log2((size_t)n_inst * std::max(n_meas, 1), 0.0L);
   for (int i = 0; i < n_inst; ++i) {
     long double lg = 0.0L;
+    double carry = 0.0;
     for (int k = 0; k <= T; ++k) {
       if (slot[(size_t)k] >= 0) row_log2[(size_t)i * n_meas + slot[(size_t)k]] = lg;
       if (k == T) break;
       const double gk = inst[i].g ? inst[i].g[k] : inst[i].g_const;
       if (!is_finite(gk)) return fail(c, BK_ERR_INVALID, "instance %d: g[%d] not finite", i, k);
-      const R tf = (R)std::tan(gk * bp->dt);
+      const double want = std::tan(gk * bp->dt) + carry;  // as in evolve_fused
+      const R tf = (R)want;
+      carry = want - (double)tf;
       R sc = (R)1;
       if (lg >= (long double)kRescaleLog2) {
         sc = (R)std::ldexp(1.0, -kRescaleLog2);
@@ -1424,7 +1684,11 @@ int evolve_fused(bk_ctx* c, const bk_evolve_params* p, const Schedule& S, double
   const int n = p->n;
   const double dt = p->dt;
   typename PhaseOf<R>::params phase{};
-  BK_TRY(build_phase(c, n, angle_unit, &phase));
+  const bool use_alt = n > T && c->engine_mode == 4 && alt_takes<R>(c, n);
+  if (use_alt)
+    BK_TRY(check_phase<R>(c, n, angle_unit));
+  else
+    BK_TRY(build_phase(c, n, angle_unit, &phase));
   const int e0 = (int)p->e0;
   const uint32_t s0 = (uint32_t)(p->s0 & ((1ull << n) - 1ull));
 
@@ -1432,11 +1696,16 @@ int evolve_fused(bk_ctx* c, const bk_evolve_params* p, const Schedule& S, double
   std::vector<R> tans((size_t)p->n_steps), scales((size_t)p->n_steps);
   row_log2->assign((size_t)S.n_meas, 0.0L);
   long double lg = 0.0L;
+  double carry = 0.0;
   for (int k = 0; k <= p->n_steps; ++k) {
     if (S.slot[(size_t)k] >= 0) (*row_log2)[(size_t)S.slot[(size_t)k]] = lg;
     if (k == p->n_steps) break;
     const double gd = S.g[(size_t)k] * dt;
-    tans[(size_t)k] = (R)std::tan(gd);
+    // the rounding of a step's tangent is made up for in the next ones, so a run's
+    // total rotation is not off by its number of steps times one rounding
+    const double want = std::tan(gd) + carry;
+    tans[(size_t)k] = (R)want;
+    carry = want - (double)tans[(size_t)k];
     R sc = (R)1;
     if (lg >= (long double)kRescaleLog2) {
       sc = (R)std::ldexp(1.0, -kRescaleLog2);
@@ -1517,6 +1786,7 @@ int evolve_fused(bk_ctx* c, const bk_evolve_params* p, const Schedule& S, double
     return BK_OK;
   }
 
+  if (use_alt) return evolve_alt<R>(c, p, S, angle_unit, tans, scales);
   return evolve_persist<R>(c, p, S, angle_unit, tans, scales);
 }
 
@@ -1631,10 +1901,13 @@ int adjoint_t(bk_ctx* c, const bk_adjoint_params* p, const std::vector<double>& 
   std::vector<R> tans((size_t)T), scales((size_t)T);
   std::vector<long double> lgf((size_t)T + 1, 0.0L);
   long double lg = 0.0L;
+  double carry = 0.0;
   for (int k = 0; k <= T; ++k) {
     lgf[(size_t)k] = lg;
     if (k == T) break;
-    tans[(size_t)k] = (R)std::tan(g_step[(size_t)k] * p->dt);
+    const double want = std::tan(g_step[(size_t)k] * p->dt) + carry;  // as in evolve_fused
+    tans[(size_t)k] = (R)want;
+    carry = want - (double)tans[(size_t)k];
     R sc = (R)1;
     if (lg >= (long double)kRescaleLog2) {
       sc = (R)std::ldexp(1.0, -kRescaleLog2);
@@ -1678,13 +1951,20 @@ int adjoint_t(bk_ctx* c, const bk_adjoint_params* p, const std::vector<double>& 
   grad_step->assign((size_t)T, 0.0);
   // forward: one persistent launch per window of K steps, psi copied to a
   // checkpoint between windows; enqueued without host synchronisation
+  const bool turning = c->engine_mode == 4 && alt_takes<R>(c, n);  // bk_evolve's choice
+  AltRun<R> arun;
+  if (turning) BK_TRY(alt_prepare<R>(c, n, p->s0, e0, angle_unit, S, tans, scales, &arun));
+  int* fwd_err = turning ? c->d_err : run.err;
   auto enqueue_forward = [&]() -> int {
     BK_CUDA(c, cudaEventRecord(ev[0], st));
     for (int w = 0; w <= n_ckpt; ++w) {
       const int k0 = w * K, k1 = (w == n_ckpt) ? T : (w + 1) * K;
       if (w > 0)
         BK_CUDA(c, cudaMemcpyAsync(ckpt + (size_t)(w - 1) * sbytes, c->d_state, sbytes, cudaMemcpyDeviceToDevice, st));
-      BK_TRY(persist_launch<R>(c, run, k0, k1 - k0, (w == n_ckpt) ? run.n_final : 0, false));
+      if (turning)
+        BK_TRY(alt_launch<R>(c, arun, k0, k1, w == 0, 0, (w == n_ckpt) ? 1 : 0));
+      else
+        BK_TRY(persist_launch<R>(c, run, k0, k1 - k0, (w == n_ckpt) ? run.n_final : 0, false));
     }
     BK_CUDA(c, cudaEventRecord(ev[1], st));
     return BK_OK;
@@ -1692,7 +1972,7 @@ int adjoint_t(bk_ctx* c, const bk_adjoint_params* p, const std::vector<double>& 
   double row[4] = {0, 0, 0, 0};
   int e_fwd = 0;
   auto finish_forward = [&]() -> int {
-    if (e_fwd != 0) return fail(c, BK_ERR_TIMEOUT, "persistent engine: a bounded device wait gave up (%d)", e_fwd);
+    if (e_fwd != 0) return fail(c, BK_ERR_TIMEOUT, "forward run: a bounded device wait gave up (%d)", e_fwd);
     const long double f = std::exp2(-2.0L * lgf[(size_t)T]);
     const double value = (double)((long double)row[p->objective == BK_OBJ_P_LESS ? 0 : 1] * f);
     if (value_out) *value_out = value;
@@ -1712,7 +1992,7 @@ int adjoint_t(bk_ctx* c, const bk_adjoint_params* p, const std::vector<double>& 
   if (T == 0) {
     BK_TRY(enqueue_forward());
     BK_CUDA(c, cudaMemcpyAsync(row, c->d_results, sizeof(row), cudaMemcpyDeviceToHost, st));
-    BK_CUDA(c, cudaMemcpyAsync(&e_fwd, run.err, sizeof(int), cudaMemcpyDeviceToHost, st));
+    BK_CUDA(c, cudaMemcpyAsync(&e_fwd, fwd_err, sizeof(int), cudaMemcpyDeviceToHost, st));
     BK_CUDA(c, cudaStreamSynchronize(st));
     return finish_forward();
   }
@@ -1904,7 +2184,7 @@ int adjoint_t(bk_ctx* c, const bk_adjoint_params* p, const std::vector<double>& 
   BK_CUDA(c, cudaMemcpyAsync(&e_dev, err, sizeof(int), cudaMemcpyDeviceToHost, st));
   // the forward's result row is untouched by the sweep: read it with the rest
   BK_CUDA(c, cudaMemcpyAsync(row, c->d_results, sizeof(row), cudaMemcpyDeviceToHost, st));
-  BK_CUDA(c, cudaMemcpyAsync(&e_fwd, run.err, sizeof(int), cudaMemcpyDeviceToHost, st));
+  BK_CUDA(c, cudaMemcpyAsync(&e_fwd, fwd_err, sizeof(int), cudaMemcpyDeviceToHost, st));
   BK_CUDA(c, cudaStreamSynchronize(st));
   BK_TRY(finish_forward());
   if (e_dev != 0) return fail(c, BK_ERR_TIMEOUT, "adjoint sweep: a bounded device wait gave up (%d)", e_dev);
@@ -2005,8 +2285,9 @@ int bk_destroy(bk_ctx* c) {
     if (p) cudaFree(p);
   for (auto& kv : c->batch_E) cudaFree(kv.second);
   for (void* p : {c->d_batch_state, c->d_batch, (void*)c->d_batch_results, c->d_persist, c->d_lam, c->d_ckpt,
-                  c->d_adj, c->d_descent, c->d_lz, c->d_fsmap})
+                  c->d_adj, c->d_descent, c->d_lz, c->d_fsmap, c->d_alt})
     if (p) cudaFree(p);
+  if (c->h_stage) cudaFreeHost(c->h_stage);
   for (auto& e : c->ev_pool) {
     cudaEventDestroy(e.first);
     cudaEventDestroy(e.second);
@@ -2203,7 +2484,7 @@ int bk_set_option(bk_ctx* c, int option, int64_t value) {
   if (!c) return BK_ERR_INVALID;
   switch (option) {
     case BK_OPT_ENGINE_MODE:
-      if (value < 0 || value > 3) return fail(c, BK_ERR_INVALID, "engine mode %lld", (long long)value);
+      if (value < 0 || value > 4) return fail(c, BK_ERR_INVALID, "engine mode %lld", (long long)value);
       c->engine_mode = (int)value;
       return BK_OK;
     case BK_OPT_SLAB_LAG:

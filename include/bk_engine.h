@@ -269,7 +269,14 @@ void bk_sampling_result_release(bk_sampling_result* r);
 int bk_d_min(bk_ctx* ctx, int n, uint64_t bits, int64_t target, int max_d, int* d_out);
 
 /* Engine options (tuning knobs; the autotuner sets them from its cache):
- *   BK_OPT_ENGINE_MODE: 0 = persistent dataflow kernel (all steps in one launch,
+ *   BK_OPT_ENGINE_MODE: 4 (default) = turning passes: every pass finishes one
+ *       step on its set of qubits, measures, applies the diagonal phase and
+ *       starts the next step on the same set, so a step costs one pass over the
+ *       statevector (two from 25 qubits in complex64, 24 in complex128, on), all
+ *       of them in one cooperative launch; complex64 takes its phase from the full
+ *       per-energy table; the knobs below do not apply to it, and with
+ *       BK_OPT_E_SOURCE = 1 mode 0 runs; bk_adjoint's forward run follows it,
+ *       0 = persistent dataflow kernel (all steps in one launch,
  *       L2 hand-off between the A1 and S2 tasks), 1 = one grid launch per pass,
  *       2 = a grid launch for the A1 pass and ONE persistent launch for both
  *       strided passes (S3 re-reads each slab S2 wrote from L2, so the strided
