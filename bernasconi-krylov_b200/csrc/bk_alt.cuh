@@ -71,30 +71,43 @@ struct AltSet {
   int mid_dim, hi_dim, mid_bits, pad;
 };
 
-// One statevector's run (kernel parameter, or device memory for a batch).
+// A run's geometry and tables (kernel parameter), the same for every statevector of a batch launch.
 template <class R>
-struct alignas(64) AltInst {
-  CUtensorMap map[3];  // tiles of the A set and of the S sets
-  unsigned char* state;
+struct AltRunDesc {
   const uint16_t* E;
   const typename AltPhase<R>::entry* tab;
-  const R* tan;        // [steps]
-  const R* scale;      // [steps]
   const int* slot;     // [steps + 1] measurement row, or -1
   double* partials;    // [rows][G][3]: norm, P_<, <d_H> of one CTA's tiles
-  AltSet set[3];
+  AltSet set[3];       // the A set, the S sets
   uint32_t n_tiles;
   int n_j, c0;         // levels of the phase table (after its entry 0), lowest level
-  int e0;
-  uint32_t s0;
   int k0, k1;          // steps [k0, k1)
   int row0;            // first measurement row of `partials`
   int meas_first;      // measure psi_k0 (else an earlier segment has)
 };
+// One statevector (kernel parameter; device memory for a batch).
+template <class R>
+struct alignas(64) AltInst {
+  CUtensorMap map[3];  // tiles of the A set and of the S sets
+  unsigned char* state;
+  const R* tan;        // [steps]
+  const R* scale;      // [steps]
+  double* results;     // batch: [rows][4]
+  int e0;
+  uint32_t s0;
+};
+// The statevectors of a batch launch: group g of G CTAs takes instances g, g + n_groups, ...
+template <class R>
+struct AltBatch {
+  const AltInst<R>* inst;
+  int n_inst, n_rows;
+  uint32_t G;
+  size_t part_stride;  // doubles of one partial-sum buffer ([n_rows][G][3]); every group has two
+};
 
 // Barrier over the G CTAs of a run; `ctr` counts arrivals over all passes.
 struct AltBarrier {
-  unsigned int* ctr;
+  unsigned int* ctr;   // batch: one per group, 32 words apart
   int* err;
   int* abort;
   uint32_t poll_limit;
@@ -252,7 +265,34 @@ struct AltE {
 template <class R>
 struct AltTurn {
   R t_pre, t_post, scale;
+  uint32_t c0;
   bool post, meas;
+};
+
+// |psi|^2 of an element's amplitudes: their sum, the share with E < e0 and the sum
+// weighted by the Hamming distance to s0 (a small integer becomes a double by an
+// exponent and one subtraction: the conversion unit is a quarter of the FP64 rate)
+__device__ __forceinline__ double alt_small(uint32_t k) { return __hiloint2double(0x43300000, (int)k) - 4503599627370496.0; }
+__device__ __forceinline__ void alt_weights(const El<float>::T& v, uint32_t e2, uint32_t el, int e0, uint32_t s0,
+                                            double& n, double& b, double& f) {
+  const double w0 = (double)fmaf(v.re.x, v.re.x, v.im.x * v.im.x), w1 = (double)fmaf(v.re.y, v.re.y, v.im.y * v.im.y);
+  const uint32_t d = (el << 1) ^ s0;
+  n = w0 + w1;
+  b = ((int)(e2 & 0xFFFFu) < e0 ? w0 : 0.0) + ((int)(e2 >> 16) < e0 ? w1 : 0.0);
+  f = fma(w0, alt_small(__popc(d)), w1 * alt_small(__popc(d ^ 1u)));
+}
+__device__ __forceinline__ void alt_weights(const El<double>::T& v, uint32_t e, uint32_t el, int e0, uint32_t s0,
+                                            double& n, double& b, double& f) {
+  n = fma(v.v.x, v.v.x, v.v.y * v.v.y);
+  b = (int)e < e0 ? n : 0.0;
+  f = n * alt_small(__popc(el ^ s0));
+}
+
+// a warp's sums, and where the threshold and the trap are (read by the passes that measure)
+struct AltMeas {
+  double* acc3;
+  const int* e0;
+  const uint32_t* s0;
 };
 
 // Measurement of the thread's elements at the turn: rolled, from the thread's own
@@ -262,19 +302,28 @@ struct AltTurn {
 // next to the tile the L1 has little room.
 template <class R, int TB, int KB, int CP, int H0, int r>
 __device__ __forceinline__ void alt_measure(const typename El<R>::T (&v)[1 << KB], unsigned char* tile,
-                                            const unsigned char* es, const AltInst<R>& D, uint32_t tile_base,
+                                            const unsigned char* es, int e0, uint32_t s0, uint32_t tile_base,
                                             uint32_t base, double* acc3) {
   constexpr int lo = AltPlan<TB, KB>::reg_lo(r);
   alt_store<R, TB, KB, r>(tile, v, base);
   const uint32_t sb = swz<double>(base), g0 = tile_base | alt_index<CP, H0>(base);
-  MeasureAcc acc;
+  double norm = 0.0, below = 0.0, flips = 0.0;
 #pragma unroll 1
-  for (uint32_t j = 0; j < (1u << KB); ++j) {
-    const typename El<R>::T x = El<R>::ld(tile + 16u * (sb ^ swz<double>(j << lo)));
-    const uint32_t e = AltE<R, TB, KB, CP, H0, r>::get1(es, base, j);
-    measure_el(acc, x, e, g0 + alt_index<CP, H0>(j << lo), D.e0, D.s0);
+  for (uint32_t j0 = 0; j0 < (1u << KB); j0 += 4u) {
+    // four elements at once: short sums over independent terms instead of one chain
+    double n4[4], b4[4], f4[4];
+#pragma unroll
+    for (uint32_t i = 0; i < 4u; ++i) {
+      const uint32_t j = j0 + i;
+      const typename El<R>::T x = El<R>::ld(tile + 16u * (sb ^ swz<double>(j << lo)));
+      const uint32_t e = AltE<R, TB, KB, CP, H0, r>::get1(es, base, j);
+      alt_weights(x, e, g0 + alt_index<CP, H0>(j << lo), e0, s0, n4[i], b4[i], f4[i]);
+    }
+    norm += (n4[0] + n4[1]) + (n4[2] + n4[3]);
+    below += (b4[0] + b4[1]) + (b4[2] + b4[3]);
+    flips += (f4[0] + f4[1]) + (f4[2] + f4[3]);
   }
-  const double a = warp_sum(acc.norm), b = warp_sum(acc.p_less), c = warp_sum(acc.d_h);
+  const double a = warp_sum(norm), b = warp_sum(below), c = warp_sum(flips);
   if ((threadIdx.x & 31u) == 0) {  // the warp's sums over the CTA's tiles of this pass
     acc3[0] += a;
     acc3[1] += b;
@@ -284,12 +333,12 @@ __device__ __forceinline__ void alt_measure(const typename El<R>::T (&v)[1 << KB
 
 template <class R, int TB, int KB, int CP, int H0, int r>
 __device__ __forceinline__ void alt_turn(typename El<R>::T (&v)[1 << KB], unsigned char* tile, const unsigned char* es,
-                                         const AltInst<R>& D, const AltTurn<R>& T, uint32_t tile_base, uint32_t base,
-                                         const unsigned char* tab, double* acc3) {
+                                         const AltTurn<R>& T, uint32_t tile_base, uint32_t base,
+                                         const unsigned char* tab, const AltMeas& M) {
   cp_async_wait();
-  if (T.meas) alt_measure<R, TB, KB, CP, H0, r>(v, tile, es, D, tile_base, base, acc3);
+  if (T.meas) alt_measure<R, TB, KB, CP, H0, r>(v, tile, es, *M.e0, *M.s0, tile_base, base, M.acc3);
   constexpr uint32_t kEntry = sizeof(typename AltPhase<R>::entry);
-  const AltTab P{tab + (T.post ? kEntry : 0u), T.post ? kEntry : 0u, (uint32_t)D.c0};
+  const AltTab P{tab + (T.post ? kEntry : 0u), T.post ? kEntry : 0u, T.c0};
 #pragma unroll
   for (int j0 = 0; j0 < (1 << KB); j0 += 8) {
     uint32_t ev[8];
@@ -316,9 +365,9 @@ __host__ __device__ constexpr int alt_turn_round(int TB, int KB, int CP) {
 // when the tile has landed, `stage_free()` runs in every thread after a barrier
 // behind the last shared-memory read.
 template <class R, int TB, int KB, int CP, int H0, class W, class F>
-__device__ __forceinline__ void alt_tile_turn(unsigned char* tile, const AltInst<R>& D, const AltTurn<R>& T,
+__device__ __forceinline__ void alt_tile_turn(unsigned char* tile, unsigned char* state, const AltTurn<R>& T,
                                               uint32_t tile_base, const unsigned char* tab, unsigned char* es,
-                                              double* acc3, W&& wait, F&& stage_free) {
+                                              const AltMeas& M, W&& wait, F&& stage_free) {
   using PL = AltPlan<TB, KB>;
   constexpr int RT = alt_turn_round(TB, KB, CP);
   constexpr int LO = CP == TB ? 0 : CP;  // lowest tile bit of the set
@@ -330,7 +379,7 @@ __device__ __forceinline__ void alt_tile_turn(unsigned char* tile, const AltInst
   if constexpr (RT == 0) {
     alt_rotate<R, TB, KB, LO, 0>(v, T.t_pre);
     if (T.meas) __syncwarp();  // the measurement's swizzled slots were other lanes' linear ones
-    alt_turn<R, TB, KB, CP, H0, 0>(v, tile, es, D, T, tile_base, b0, tab, acc3);
+    alt_turn<R, TB, KB, CP, H0, 0>(v, tile, es, T, tile_base, b0, tab, M);
     __syncthreads();
     stage_free();
   } else {
@@ -342,14 +391,14 @@ __device__ __forceinline__ void alt_tile_turn(unsigned char* tile, const AltInst
     alt_load<R, TB, KB, 1, true>(tile, v, b1);
     alt_rotate<R, TB, KB, LO, 1>(v, T.t_pre);
     if constexpr (RT == 1) {
-      alt_turn<R, TB, KB, CP, H0, 1>(v, tile, es, D, T, tile_base, b1, tab, acc3);
+      alt_turn<R, TB, KB, CP, H0, 1>(v, tile, es, T, tile_base, b1, tab, M);
     } else {
       alt_store<R, TB, KB, 1>(tile, v, b1);
       __syncwarp();  // rounds 1 and 2 share their warp bits
       const uint32_t b2 = PL::template base<2>(lane, warp);
       alt_load<R, TB, KB, 2, true>(tile, v, b2);
       alt_rotate<R, TB, KB, LO, 2>(v, T.t_pre);
-      alt_turn<R, TB, KB, CP, H0, 2>(v, tile, es, D, T, tile_base, b2, tab, acc3);
+      alt_turn<R, TB, KB, CP, H0, 2>(v, tile, es, T, tile_base, b2, tab, M);
       alt_store<R, TB, KB, 2>(tile, v, b2);
       __syncwarp();
       alt_load<R, TB, KB, 1, true>(tile, v, b1);
@@ -362,21 +411,19 @@ __device__ __forceinline__ void alt_tile_turn(unsigned char* tile, const AltInst
     stage_free();
     alt_rotate<R, TB, KB, LO, 0>(v, T.t_post);
   }
-  unsigned char* g = D.state + 16ull * (tile_base | alt_index<CP, H0>(b0));
+  unsigned char* g = state + 16ull * (tile_base | alt_index<CP, H0>(b0));
 #pragma unroll
   for (int j = 0; j < (1 << KB); ++j)
     El<R>::st(g + 16ull * alt_index<CP, H0>((uint32_t)j << PL::reg_lo(0)), v[j]);
 }
 
-template <class R>
-__device__ __forceinline__ void alt_issue(const AltInst<R>& D, int s, uint32_t tile, uint32_t bytes,
+__device__ __forceinline__ void alt_issue(const AltSet& S, const CUtensorMap* map, uint32_t tile, uint32_t bytes,
                                           unsigned char* stage, uint32_t fb) {
-  const AltSet& S = D.set[s];
   const int mid = (int)(tile & ((1u << S.mid_bits) - 1u)), hi = (int)(tile >> S.mid_bits);
   const int md = S.mid_dim, hd = S.hi_dim;
   fence_proxy_async_shared();  // the CTA's generic accesses of the stage precede the copy's writes
   mbar_arrive_expect_tx(fb, bytes);
-  tma_load_5d(smem_addr(stage), &D.map[s], tile_coord(0, md, mid, hd, hi), tile_coord(1, md, mid, hd, hi),
+  tma_load_5d(smem_addr(stage), map, tile_coord(0, md, mid, hd, hi), tile_coord(1, md, mid, hd, hi),
               tile_coord(2, md, mid, hd, hi), tile_coord(3, md, mid, hd, hi), tile_coord(4, md, mid, hd, hi), fb);
 }
 // first element of a tile: the id's low bits are element bits [CP, H0), the others those above the set
@@ -392,7 +439,7 @@ __device__ __forceinline__ uint32_t alt_tile_base(uint32_t tile) {
 // rounds of the warp-local A1, then the top four bits): three rounds, the last
 // one's lanes over the low bits.
 template <class R, class W, class F>
-__device__ __forceinline__ void alt_tile_plain(unsigned char* tile, const AltInst<R>& D, R t, uint32_t tile_base,
+__device__ __forceinline__ void alt_tile_plain(unsigned char* tile, unsigned char* state, R t, uint32_t tile_base,
                                                W&& wait, F&& stage_free) {
   using PL = PlanA1Warp;
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
@@ -420,15 +467,15 @@ __device__ __forceinline__ void alt_tile_plain(unsigned char* tile, const AltIns
   __syncthreads();
   stage_free();
   el_bflys<R, 0xF00u, 0xF00u>(v, t);
-  unsigned char* g = D.state + 16ull * (tile_base | bc);
+  unsigned char* g = state + 16ull * (tile_base | bc);
 #pragma unroll
   for (int j = 0; j < 16; ++j) El<R>::st(g + 16ull * ((uint32_t)j << 8), v[j]);
 }
 
 // thread 0: wait until `ctr` reaches `target`; false on timeout or abort
-__device__ __forceinline__ bool alt_wait(const AltBarrier& B, uint32_t target) {
+__device__ __forceinline__ bool alt_wait(const AltBarrier& B, const unsigned int* ctr, uint32_t target) {
   uint32_t polls = 0;
-  while ((int32_t)(ld_acquire(B.ctr) - target) < 0) {
+  while ((int32_t)(ld_acquire(ctr) - target) < 0) {
     if (++polls > B.poll_limit) {
       atomicCAS(B.err, 0, DEV_TIMEOUT);
       atomicExch(B.abort, 1);
@@ -447,23 +494,33 @@ struct AltCtl {
   int stop;      // the run has failed: every thread leaves at the end of the pass
   int inflight;  // thread 0: a tile's copy is on its way
   double acc[16][3];  // per warp: norm, P_<, <d_H> of the pass
+  // batch: the statevector the group works on
+  const CUtensorMap* map;
+  unsigned char* state;
+  const void *tan, *scale;
+  double* partials;
+  int e0;
+  uint32_t s0;
 };
 template <int TB>
 struct AltSmem {
-  static constexpr int kEOff = 16 << TB, kCtlOff = kEOff + (4 << TB), kTabOff = kCtlOff + 512;
-  static_assert(sizeof(AltCtl) <= 512, "the control block's room");
+  static constexpr int kEOff = 16 << TB, kCtlOff = kEOff + (4 << TB), kTabOff = kCtlOff + 640;
+  static_assert(sizeof(AltCtl) <= 640, "the control block's room");
   // + room to align the tile to 1024 bytes (swizzled loads)
   static int bytes(int n_j, int entry) { return kTabOff + (((n_j + 1) * entry + 127) & ~127) + 1024; }
 };
 
-// One CTA of a run's group.
-template <class R, int TB, int KB>
+// One CTA of a run's group. kBatch: the statevector's fields come from the control
+// block (the group changes them), else from the kernel parameter.
+template <class R, int TB, int KB, bool kBatch>
 struct AltCta {
   using PL = AltPlan<TB, KB>;
   using SM = AltSmem<TB>;
   static constexpr uint32_t kBytes = 16u << TB;
-  const AltInst<R>& D;
+  const AltRunDesc<R>& D;
+  const AltInst<R>& I;
   const AltBarrier& B;
+  unsigned int* ctr;   // the group's arrivals
   uint32_t rank, G;
   unsigned char* stage;
   uint32_t parity, epoch;
@@ -473,9 +530,21 @@ struct AltCta {
   __device__ __forceinline__ unsigned char* es() const { return stage + SM::kEOff; }
   __device__ __forceinline__ unsigned char* tab() const { return stage + SM::kTabOff; }
 
+  __device__ __forceinline__ unsigned char* state() const { return kBatch ? ctl().state : I.state; }
+  __device__ __forceinline__ const R* tans() const { return kBatch ? static_cast<const R*>(ctl().tan) : I.tan; }
+  __device__ __forceinline__ const R* scales() const { return kBatch ? static_cast<const R*>(ctl().scale) : I.scale; }
+  __device__ __forceinline__ const CUtensorMap* maps() const { return kBatch ? ctl().map : I.map; }
+  __device__ __forceinline__ AltMeas meas() const {
+    double* a = const_cast<double*>(&ctl().acc[threadIdx.x >> 5][0]);
+    if constexpr (kBatch)
+      return AltMeas{a, const_cast<const int*>(&ctl().e0), const_cast<const uint32_t*>(&ctl().s0)};
+    else
+      return AltMeas{a, &I.e0, &I.s0};
+  }
+
   __device__ __forceinline__ void issue(int map, uint32_t tile) {
     if (threadIdx.x == 0 && tile < D.n_tiles && !ctl().stop) {
-      alt_issue(D, map, tile, kBytes, stage, bar());
+      alt_issue(D.set[map], maps() + map, tile, kBytes, stage, bar());
       ctl().inflight = 1;
     }
     __syncwarp();
@@ -507,16 +576,16 @@ struct AltCta {
     AltTurn<R> T;
     const bool pre = k > D.k0;
     T.post = k < D.k1;
-    T.t_pre = pre ? D.tan[k - 1] : (R)0;  // a tangent of 0 rotates nothing
-    T.t_post = T.post ? D.tan[k] : (R)0;
-    T.scale = T.post ? D.scale[k] : (R)1;
+    T.t_pre = pre ? tans()[k - 1] : (R)0;  // a tangent of 0 rotates nothing
+    T.t_post = T.post ? tans()[k] : (R)0;
+    T.scale = T.post ? scales()[k] : (R)1;
+    T.c0 = (uint32_t)D.c0;
     const int slot = (pre || D.meas_first) ? D.slot[k] : -1;
     T.meas = slot >= 0;
-    const uint32_t warp = threadIdx.x >> 5;
-    double* acc3 = const_cast<double*>(&ctl().acc[warp][0]);
-    if (T.meas && (threadIdx.x & 31u) == 0) acc3[0] = acc3[1] = acc3[2] = 0.0;
+    const AltMeas M = meas();
+    if (T.meas && (threadIdx.x & 31u) == 0) M.acc3[0] = M.acc3[1] = M.acc3[2] = 0.0;
     for (uint32_t tile = rank; tile < D.n_tiles; tile += G) {
-      alt_tile_turn<R, TB, KB, CP, H0>(stage, D, T, alt_tile_base<TB, CP, H0>(tile), tab(), es(), acc3,
+      alt_tile_turn<R, TB, KB, CP, H0>(stage, state(), T, alt_tile_base<TB, CP, H0>(tile), tab(), es(), M,
                                        [&]() { wait(); }, [&]() { issue(s, tile + G); });
       fetch_e<CP, H0>(tile + G);  // after the stores, when the registers are free
     }
@@ -525,26 +594,31 @@ struct AltCta {
       if (threadIdx.x < 3u) {
         double x = 0;
         for (int w = 0; w < PL::kWarps; ++w) x += ctl().acc[w][threadIdx.x];
-        D.partials[3 * ((size_t)(slot - D.row0) * G + rank) + threadIdx.x] = x;
+        (kBatch ? ctl().partials : D.partials)[3 * ((size_t)(slot - D.row0) * G + rank) + threadIdx.x] = x;
       }
     }
   }
   __device__ __forceinline__ void plain(int s, int k) {
-    const R t = D.tan[k];
+    const R t = tans()[k];
     for (uint32_t tile = rank; tile < D.n_tiles; tile += G)
-      alt_tile_plain<R>(stage, D, t, alt_tile_base<TB, TB, TB>(tile), [&]() { wait(); }, [&]() { issue(s, tile + G); });
+      alt_tile_plain<R>(stage, state(), t, alt_tile_base<TB, TB, TB>(tile), [&]() { wait(); }, [&]() { issue(s, tile + G); });
   }
-  // the end of a pass: every CTA's stores are in memory, then the next pass's first tile
-  __device__ __forceinline__ bool next_pass(int map) {
+  // the end of a pass: every CTA's stores are in memory
+  __device__ __forceinline__ bool group_barrier() {
     if (__syncthreads_or(ctl().stop)) return false;  // every store of the CTA is issued
     if (threadIdx.x == 0) {
-      red_release_add(B.ctr, 1u);  // releases every thread's stores (ordered before it by the CTA barrier)
+      red_release_add(ctr, 1u);  // releases every thread's stores (ordered before it by the CTA barrier)
       epoch += G;
-      if (!alt_wait(B, epoch)) ctl().stop = 1;
+      if (!alt_wait(B, ctr, epoch)) ctl().stop = 1;
     }
     // lane 0's warp waits for it here: its other lanes must not spin on the tile's
     // barrier while lane 0 polls (a warp in a suspended try_wait polls nothing)
     __syncwarp();
+    return true;
+  }
+  // ... then the next pass's first tile
+  __device__ __forceinline__ bool next_pass(int map) {
+    if (!group_barrier()) return false;
     issue(map, rank);
     return true;
   }
@@ -569,63 +643,123 @@ struct AltCta {
   }
 };
 
-// Two sets: A (the tile's bits) and the W bits above it.
-template <class R, int TB, int KB, int W>
-__device__ __forceinline__ void alt_run2(AltCta<R, TB, KB>& C) {
-  const AltInst<R>& D = C.D;
+// Two sets: A (the tile's bits) and the W bits above it. False when the run has failed.
+template <class R, int TB, int KB, int W, bool kBatch>
+__device__ __forceinline__ bool alt_run2(AltCta<R, TB, KB, kBatch>& C) {
+  const AltRunDesc<R>& D = C.D;
   if (D.k0 & 1) C.template fetch_e<TB - W, TB>(C.rank); else C.template fetch_e<TB, TB>(C.rank);
   C.issue(D.k0 & 1, C.rank);
-  C.stage_table();
   for (int k = D.k0;; ++k) {
     if (k & 1) {
       C.template turn<TB - W, TB>(1, k);
-      if (k == D.k1) break;
+      if (k == D.k1) return true;
       C.template fetch_e<TB, TB>(C.rank);
     } else {
       C.template turn<TB, TB>(0, k);
-      if (k == D.k1) break;
+      if (k == D.k1) return true;
       C.template fetch_e<TB - W, TB>(C.rank);
     }
-    if (!C.next_pass((k + 1) & 1)) break;
+    if (!C.next_pass((k + 1) & 1)) return false;
   }
-  C.leave();
 }
 
 // Three sets: turning passes on the W2 bits above the A set and the W3 bits above
 // those in turn, plain passes over the A set between them.
-template <class R, int W2, int W3>
-__device__ __forceinline__ void alt_run3(AltCta<R, 12, 4>& C) {
+template <class R, int W2, int W3, bool kBatch>
+__device__ __forceinline__ bool alt_run3(AltCta<R, 12, 4, kBatch>& C) {
   constexpr int TB = 12, C2 = TB - W2, C3 = TB - W3, H3 = TB + W2;
-  const AltInst<R>& D = C.D;
+  const AltRunDesc<R>& D = C.D;
   if (D.k0 & 1) C.template fetch_e<C3, H3>(C.rank); else C.template fetch_e<C2, TB>(C.rank);
   C.issue(1 + (D.k0 & 1), C.rank);
-  C.stage_table();
   for (int k = D.k0;; ++k) {
     if (k & 1)
       C.template turn<C3, H3>(2, k);
     else
       C.template turn<C2, TB>(1, k);
-    if (k == D.k1 || !C.next_pass(0)) break;
+    if (k == D.k1) return true;
+    if (!C.next_pass(0)) return false;
     C.plain(0, k);
     if (k & 1) C.template fetch_e<C2, TB>(C.rank); else C.template fetch_e<C3, H3>(C.rank);
-    if (!C.next_pass(1 + ((k + 1) & 1))) break;
+    if (!C.next_pass(1 + ((k + 1) & 1))) return false;
   }
-  C.leave();
+}
+
+__device__ __forceinline__ unsigned char* alt_stage(unsigned char* raw) {
+  return raw + ((1024u - (smem_addr(raw) & 1023u)) & 1023u);
 }
 
 // W3 = 0: two sets (A and W2), else three
 template <class R, int TB, int KB, int W2, int W3>
-__global__ void __launch_bounds__(AltPlan<TB, KB>::kThreads, TB == 10 ? 4 : TB == 12 ? 2 : 1)
-    alt_kernel(const __grid_constant__ AltInst<R> D, const __grid_constant__ AltBarrier B) {
+__global__ void __launch_bounds__(AltPlan<TB, KB>::kThreads, TB == 10 ? 6 : TB == 12 ? 2 : 1)
+    alt_kernel(const __grid_constant__ AltRunDesc<R> D, const __grid_constant__ AltInst<R> I,
+               const __grid_constant__ AltBarrier B) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  AltCta<R, TB, KB> C{D, B, blockIdx.x, gridDim.x, smem_raw + ((1024u - (smem_addr(smem_raw) & 1023u)) & 1023u)};
+  AltCta<R, TB, KB, false> C{D, I, B, B.ctr, blockIdx.x, gridDim.x, alt_stage(smem_raw)};
   C.begin();
+  C.stage_table();
   if constexpr (W3 == 0)
     alt_run2<R, TB, KB, W2>(C);
   else
     alt_run3<R, W2, W3>(C);
+  C.leave();
 }
 
+// Many statevectors of one size: groups of Q.G CTAs work through them on their own,
+// each with its own barrier, so a small statevector's barriers and waits overlap
+// those of the other groups. Results are reduced by the group (CTA sums in index
+// order) after the statevector's last pass, from one of two partial-sum buffers:
+// the next use of a buffer lies behind the barriers of the statevector between.
+template <class R, int TB, int KB, int W2, int W3>
+__global__ void __launch_bounds__(AltPlan<TB, KB>::kThreads, TB == 10 ? 6 : TB == 12 ? 2 : 1)
+    alt_batch_kernel(const __grid_constant__ AltRunDesc<R> D, const __grid_constant__ AltBatch<R> Q,
+                     const __grid_constant__ AltBarrier B) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  const uint32_t group = blockIdx.x / Q.G, n_groups = gridDim.x / Q.G;
+  AltCta<R, TB, KB, true> C{D, *Q.inst, B, B.ctr + 32u * group, blockIdx.x % Q.G, Q.G, alt_stage(smem_raw)};
+  C.begin();
+  C.stage_table();
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  uint32_t turn = 0;
+  bool ok = true;
+  for (int i = (int)group; ok && i < Q.n_inst; i += (int)n_groups, ++turn) {
+    const AltInst<R>& I = Q.inst[i];
+    double* part = D.partials + (2 * (size_t)group + (turn & 1u)) * Q.part_stride;
+    if (threadIdx.x == 0) {
+      volatile AltCtl& c = C.ctl();
+      c.map = I.map;
+      c.state = I.state;
+      c.tan = I.tan;
+      c.scale = I.scale;
+      c.partials = part;
+      c.e0 = I.e0;
+      c.s0 = I.s0;
+    }
+    __syncthreads();
+    if constexpr (W3 == 0)
+      ok = alt_run2<R, TB, KB, W2>(C);
+    else
+      ok = alt_run3<R, W2, W3>(C);
+    if (!ok || !(ok = C.group_barrier())) break;
+    if (__syncthreads_or(C.ctl().stop)) break;  // also: thread 0 has seen every CTA's partial sums
+    for (int row = (int)(C.rank * AltPlan<TB, KB>::kWarps + warp); row < Q.n_rows; row += (int)(Q.G * AltPlan<TB, KB>::kWarps)) {
+      double s[3] = {0, 0, 0};
+      for (uint32_t j = lane; j < Q.G; j += 32u)
+#pragma unroll
+        for (int q = 0; q < 3; ++q) s[q] += __ldcg(&part[3 * ((size_t)row * Q.G + j) + q]);
+#pragma unroll
+      for (int q = 0; q < 3; ++q) s[q] = warp_sum(s[q]);
+      if (lane == 0) {
+        I.results[4 * (size_t)row + 0] = s[1];
+        I.results[4 * (size_t)row + 1] = s[2];
+        I.results[4 * (size_t)row + 2] = s[0];
+      }
+    }
+    __syncthreads();
+  }
+  C.leave();
+}
+
+#ifdef BK_ALT_REDUCE  // defined by the one source that launches it
 // results[row0 + row] = sum over the G CTAs of a run in index order (one warp a row)
 __global__ void __launch_bounds__(128) alt_reduce_kernel(const double* __restrict__ partials, int rows, int G,
                                                          double* __restrict__ results) {
@@ -641,6 +775,44 @@ __global__ void __launch_bounds__(128) alt_reduce_kernel(const double* __restric
     results[4 * (size_t)row + 0] = s[1];
     results[4 * (size_t)row + 1] = s[2];
     results[4 * (size_t)row + 2] = s[0];
+  }
+}
+
+#endif
+
+// The kernel of a geometry (tile bits, set widths), or nullptr: instantiated in
+// bk_alt_f32.cu and bk_alt_f64.cu.
+const void* alt_kernel_f32(int tb, int w2, int w3, bool batch);
+const void* alt_kernel_f64(int tb, int w2, int w3, bool batch);
+
+template <class R, int TB, int KB, int W2, int W3>
+const void* alt_pick(bool batch) {
+  if constexpr (W3 == 0)  // larger statevectors fill the GPU one at a time
+    if (batch) return reinterpret_cast<const void*>(alt_batch_kernel<R, TB, KB, W2, W3>);
+  return batch ? nullptr : reinterpret_cast<const void*>(alt_kernel<R, TB, KB, W2, W3>);
+}
+template <class R>
+const void* alt_kernel_table(int tb, int w2, int w3, bool batch) {
+  switch (tb * 256 + w2 * 16 + w3) {
+    case 0xA30: return alt_pick<R, 10, 4, 3, 0>(batch);
+    case 0xA40: return alt_pick<R, 10, 4, 4, 0>(batch);
+    case 0xA50: return alt_pick<R, 10, 4, 5, 0>(batch);
+    case 0xA60: return alt_pick<R, 10, 4, 6, 0>(batch);
+    case 0xA70: return alt_pick<R, 10, 4, 7, 0>(batch);
+    case 0xA80: return alt_pick<R, 10, 4, 8, 0>(batch);
+    case 0xC70: return alt_pick<R, 12, 4, 7, 0>(batch);
+    case 0xC80: return alt_pick<R, 12, 4, 8, 0>(batch);
+    case 0xD80: return alt_pick<R, 13, 5, 8, 0>(batch);
+    case 0xD90: return alt_pick<R, 13, 5, 9, 0>(batch);
+    case 0xDA0: return alt_pick<R, 13, 5, 10, 0>(batch);
+    case 0xC66: return alt_pick<R, 12, 4, 6, 6>(batch);
+    case 0xC76: return alt_pick<R, 12, 4, 7, 6>(batch);
+    case 0xC77: return alt_pick<R, 12, 4, 7, 7>(batch);
+    case 0xC87: return alt_pick<R, 12, 4, 8, 7>(batch);
+    case 0xC88: return alt_pick<R, 12, 4, 8, 8>(batch);
+    case 0xC98: return alt_pick<R, 12, 4, 9, 8>(batch);
+    case 0xC99: return alt_pick<R, 12, 4, 9, 9>(batch);
+    default: return nullptr;
   }
 }
 

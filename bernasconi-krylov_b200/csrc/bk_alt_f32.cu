@@ -1,0 +1,6 @@
+// The complex64 turning-pass kernels (csrc/bk_alt.cuh), one source per precision so that they build in parallel.
+#include "bk_alt.cuh"
+
+namespace bk {
+const void* alt_kernel_f32(int tb, int w2, int w3, bool batch) { return alt_kernel_table<float>(tb, w2, w3, batch); }
+}  // namespace bk

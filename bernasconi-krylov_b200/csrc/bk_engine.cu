@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "bk_adjoint.cuh"
+#define BK_ALT_REDUCE
 #include "bk_alt.cuh"
 #include "bk_aux.cuh"
 #include "bk_engine.h"
@@ -515,6 +516,22 @@ static void descend(int n, uint64_t start, uint64_t max_evals, uint64_t* fs, int
   *fe = e;
   if (ev) *ev = evals;
 }
+
+// log2(1 + t^2) of a step's tangent: a constant field repeats one or two of them
+template <class R>
+struct Log2Memo {
+  R t[2] = {(R)0, (R)0};
+  long double v[2] = {0.0L, 0.0L};
+  int next = 0;
+  long double log2_1t2(R x) {
+    for (int i = 0; i < 2; ++i)
+      if (t[i] == x) return v[i];
+    const int i = next;
+    next ^= 1;
+    t[i] = x;
+    return v[i] = std::log2(1.0L + (long double)x * (long double)x);
+  }
+};
 
 struct Schedule {
   std::vector<double> g;        // per step
@@ -1111,8 +1128,6 @@ int ensure_stage(bk_ctx* c, size_t bytes) {
   return BK_OK;
 }
 
-template <class R>
-using AltKernel = void (*)(AltInst<R>, AltBarrier);
 struct AltGeo {
   int tb = 0, w2 = 0, w3 = 0;
 };
@@ -1141,27 +1156,8 @@ bool alt_takes(const bk_ctx* c, int n) {
   return c->e_recompute == 0 && alt_geometry(sizeof(R) == 4 ? n - 1 : n, &g);
 }
 template <class R>
-AltKernel<R> alt_kernel_of(const AltGeo& g) {
-  switch (g.tb * 256 + g.w2 * 16 + g.w3) {
-    case 0xA30: return alt_kernel<R, 10, 4, 3, 0>;
-    case 0xA40: return alt_kernel<R, 10, 4, 4, 0>;
-    case 0xA50: return alt_kernel<R, 10, 4, 5, 0>;
-    case 0xA60: return alt_kernel<R, 10, 4, 6, 0>;
-    case 0xA70: return alt_kernel<R, 10, 4, 7, 0>;
-    case 0xA80: return alt_kernel<R, 10, 4, 8, 0>;
-    case 0xC70: return alt_kernel<R, 12, 4, 7, 0>;
-    case 0xC80: return alt_kernel<R, 12, 4, 8, 0>;
-    case 0xD80: return alt_kernel<R, 13, 5, 8, 0>;
-    case 0xD90: return alt_kernel<R, 13, 5, 9, 0>;
-    case 0xDA0: return alt_kernel<R, 13, 5, 10, 0>;
-    case 0xC66: return alt_kernel<R, 12, 4, 6, 6>;
-    case 0xC76: return alt_kernel<R, 12, 4, 7, 6>;
-    case 0xC77: return alt_kernel<R, 12, 4, 7, 7>;
-    case 0xC87: return alt_kernel<R, 12, 4, 8, 7>;
-    case 0xC88: return alt_kernel<R, 12, 4, 8, 8>;
-    case 0xC98: return alt_kernel<R, 12, 4, 9, 8>;
-    default: return alt_kernel<R, 12, 4, 9, 9>;
-  }
+const void* alt_kernel_of(const AltGeo& g, bool batch) {
+  return sizeof(R) == 4 ? alt_kernel_f32(g.tb, g.w2, g.w3, batch) : alt_kernel_f64(g.tb, g.w2, g.w3, batch);
 }
 int alt_smem_bytes(const AltGeo& g, int n_j, int entry) {
   return g.tb == 10 ? AltSmem<10>::bytes(n_j, entry) : g.tb == 12 ? AltSmem<12>::bytes(n_j, entry) : AltSmem<13>::bytes(n_j, entry);
@@ -1207,13 +1203,50 @@ int alt_set(bk_ctx* c, void* state, int np, int cp, int h0, int w, CUtensorMap* 
 
 constexpr size_t kAltPartialBytes = (size_t)64 << 20;  // partial sums of one launch (more rows: more launches)
 
+// levels of the phase table for n
+inline int alt_levels(int n, int* c0) {
+  *c0 = (n / 2) & 3;
+  return ((n - 1) * n * (2 * n - 1) / 6 - *c0) / 4 + 1;
+}
+// the tensor maps and tile coordinates of a statevector's sets
+int alt_maps(bk_ctx* c, void* state, int np, const AltGeo& geo, CUtensorMap* map, AltSet* set) {
+  if (geo.w3 == 0) {
+    BK_TRY(alt_set(c, state, np, geo.tb, geo.tb, 0, &map[0], &set[0]));
+  } else {  // the plain pass loads its tiles swizzled
+    TmaDesc d;
+    BK_TRY(build_a1_swizzled_map(c, state, np, &d));
+    map[0] = d.map;
+    set[0] = AltSet{-1, d.hi_dim, 0, 0};
+    BK_TRY(alt_set(c, state, np, geo.tb - geo.w3, geo.tb + geo.w2, geo.w3, &map[2], &set[2]));
+  }
+  BK_TRY(alt_set(c, state, np, geo.tb - geo.w2, geo.tb, geo.w2, &map[1], &set[1]));
+  if (geo.w3 == 0) {
+    map[2] = map[1];
+    set[2] = set[1];
+  }
+  return BK_OK;
+}
+// the kernel of a geometry, ready to launch: shared memory opted in, CTAs per SM
+template <class R>
+int alt_kernel_ready(bk_ctx* c, const AltGeo& geo, bool batch, int n_j, const void** fn, int* smem, int* threads,
+                     int* per_sm) {
+  *fn = alt_kernel_of<R>(geo, batch);
+  *smem = alt_smem_bytes(geo, n_j, (int)sizeof(typename AltPhase<R>::entry));
+  *threads = geo.tb == 10 ? 64 : 256;
+  BK_TRY(allow_smem(c, *fn, *smem));
+  BK_TRY(ctas_per_sm(c, *fn, *threads, *smem, per_sm));
+  if (*per_sm < 1) return fail(c, BK_ERR_CUDA, "turning pass: no room for a CTA (%d bytes of shared memory)", *smem);
+  return BK_OK;
+}
+
 // A prepared run over c->d_state: geometry, uploads and the kernel; alt_launch
 // runs any range of its steps.
 template <class R>
 struct AltRun {
-  AltInst<R> D{};
+  AltRunDesc<R> D{};
+  AltInst<R> I{};
   AltBarrier B{};
-  AltKernel<R> fn = nullptr;
+  const void* fn = nullptr;
   int smem = 0, threads = 0;
   uint32_t G = 0;
   int max_rows = 1;  // measurement rows the partial sums of one launch have room for
@@ -1226,28 +1259,12 @@ int alt_prepare(bk_ctx* c, int n, uint64_t s0, int64_t e0, double angle_unit, co
   const int np = sizeof(R) == 4 ? n - 1 : n, T = (int)tans.size();
   AltGeo geo;
   if (!alt_geometry(np, &geo)) return fail(c, BK_ERR_UNSUPPORTED, "turning passes: n = %d", n);
-  AltInst<R>& D = run->D;
-  if (geo.w3 == 0) {
-    BK_TRY(alt_set(c, c->d_state, np, geo.tb, geo.tb, 0, &D.map[0], &D.set[0]));
-  } else {  // the plain pass loads its tiles swizzled
-    TmaDesc d;
-    BK_TRY(build_a1_swizzled_map(c, c->d_state, np, &d));
-    D.map[0] = d.map;
-    D.set[0] = AltSet{-1, d.hi_dim, 0, 0};
-    BK_TRY(alt_set(c, c->d_state, np, geo.tb - geo.w3, geo.tb + geo.w2, geo.w3, &D.map[2], &D.set[2]));
-  }
-  BK_TRY(alt_set(c, c->d_state, np, geo.tb - geo.w2, geo.tb, geo.w2, &D.map[1], &D.set[1]));
-  D.c0 = (n / 2) & 3;
-  D.n_j = ((n - 1) * n * (2 * n - 1) / 6 - D.c0) / 4 + 1;
+  AltRunDesc<R>& D = run->D;
+  BK_TRY(alt_maps(c, c->d_state, np, geo, run->I.map, D.set));
+  D.n_j = alt_levels(n, &D.c0);
   D.n_tiles = 1u << (np - geo.tb);
-  run->fn = alt_kernel_of<R>(geo);
-  run->smem = alt_smem_bytes(geo, D.n_j, (int)sizeof(entry));
-  run->threads = geo.tb == 10 ? 64 : 256;
-  const void* fn = reinterpret_cast<const void*>(run->fn);
-  BK_TRY(allow_smem(c, fn, run->smem));
   int per_sm = 0;
-  BK_TRY(ctas_per_sm(c, fn, run->threads, run->smem, &per_sm));
-  if (per_sm < 1) return fail(c, BK_ERR_CUDA, "turning pass: no room for a CTA (%d bytes of shared memory)", run->smem);
+  BK_TRY(alt_kernel_ready<R>(c, geo, false, D.n_j, &run->fn, &run->smem, &run->threads, &per_sm));
   run->G = std::min<uint32_t>(D.n_tiles, (uint32_t)(per_sm * c->num_sms));
 
   // one upload: phase table, tangents, rescales, measurement rows, zeroed counters
@@ -1270,15 +1287,16 @@ int alt_prepare(bk_ctx* c, int n, uint64_t s0, int64_t e0, double angle_unit, co
   std::copy(S.slot.begin(), S.slot.end(), reinterpret_cast<int*>(h + o_slot));
   std::memset(h + o_ctr, 0, 64);
   BK_CUDA(c, cudaMemcpyAsync(d, h, up, cudaMemcpyHostToDevice, c->stream));
-  D.state = static_cast<unsigned char*>(c->d_state);
   D.E = c->d_E;
   D.tab = reinterpret_cast<const entry*>(d + o_tab);
-  D.tan = reinterpret_cast<const R*>(d + o_tan);
-  D.scale = reinterpret_cast<const R*>(d + o_sc);
   D.slot = reinterpret_cast<const int*>(d + o_slot);
   D.partials = reinterpret_cast<double*>(d + o_part);
-  D.e0 = (int)e0;
-  D.s0 = (uint32_t)(s0 & ((1ull << n) - 1ull));
+  AltInst<R>& I = run->I;
+  I.state = static_cast<unsigned char*>(c->d_state);
+  I.tan = reinterpret_cast<const R*>(d + o_tan);
+  I.scale = reinterpret_cast<const R*>(d + o_sc);
+  I.e0 = (int)e0;
+  I.s0 = (uint32_t)(s0 & ((1ull << n) - 1ull));
   run->B.ctr = reinterpret_cast<unsigned int*>(d + o_ctr);
   run->B.abort = reinterpret_cast<int*>(d + o_ctr + 8);
   run->B.err = c->d_err;
@@ -1299,9 +1317,8 @@ int alt_launch(bk_ctx* c, AltRun<R>& r, int k0, int k1, bool first, int row0, in
   if (!first) BK_CUDA(c, cudaMemsetAsync(r.B.ctr, 0, sizeof(unsigned int), st));
   size_t ev = 0;
   BK_TRY(ev_begin(c, "turn", &ev));
-  void* args[] = {&r.D, &r.B};
-  BK_CUDA(c, cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(r.fn), dim3(r.G), dim3((unsigned)r.threads), args,
-                                         (size_t)r.smem, st));
+  void* args[] = {&r.D, &r.I, &r.B};
+  BK_CUDA(c, cudaLaunchCooperativeKernel(r.fn, dim3(r.G), dim3((unsigned)r.threads), args, (size_t)r.smem, st));
   BK_TRY(ev_end(c, ev));
   if (rows > 0) {
     alt_reduce_kernel<<<(rows + 3) / 4, 128, 0, st>>>(r.D.partials, rows, (int)r.G, c->d_results + 4 * (size_t)row0);
@@ -1367,6 +1384,162 @@ __global__ void set_basis_many_kernel(unsigned char* base, const unsigned long l
     reinterpret_cast<double2*>(st)[s] = make_double2(1.0, 0.0);
 }
 
+struct BatchGeo {
+  int n, np, w2, w3, e0;
+  uint32_t n_a1, slabs, s0;
+  size_t state_off;
+  double angle_unit;
+};
+
+// rows [instance][measurement] of the device -> the caller's arrays, scales taken out
+template <class R>
+void batch_rows(const std::vector<double>& rows, const std::vector<long double>& row_log2, double* p_less, double* d_h,
+                double* norm_out) {
+  for (size_t r = 0; r < rows.size() / 4; ++r) {
+    const long double f = std::exp2(-2.0L * row_log2[r]);
+    // complex64: expectation values of the normalised state (see bk_evolve)
+    const long double nrm = (sizeof(R) == 4 && rows[4 * r + 2] > 0.0) ? (long double)rows[4 * r + 2] * f : 1.0L;
+    p_less[r] = (double)((long double)rows[4 * r + 0] * f / nrm);
+    d_h[r] = (double)((long double)rows[4 * r + 1] * f / nrm);
+    if (norm_out) norm_out[r] = (double)((long double)rows[4 * r + 2] * f);
+  }
+}
+
+// The batch through turning passes: the instances of one size per cooperative
+// launch (alt_batch_kernel), largest size first; a launch's CTAs form groups of G.
+// G is a power of two up to the tiles of a statevector: the one with the shortest
+// run by the measured shape of a step, a barrier's 3 us plus the tiles a CTA takes
+// one after another (about 9 us for a tile of each of an SM's resident CTAs).
+template <class R>
+int batch_turning(bk_ctx* c, const std::vector<BatchGeo>& geo, int T, const std::vector<int>& slot, int n_meas,
+                  const std::vector<R>& tans, const std::vector<R>& scales, size_t state_bytes,
+                  const std::vector<long double>& row_log2, double* p_less, double* d_h, double* norm_out) {
+  using entry = typename AltPhase<R>::entry;
+  constexpr bool c64 = sizeof(R) == 4;
+  const int n_inst = (int)geo.size();
+  cudaStream_t st = c->stream;
+  struct Class {
+    int n = 0, per_sm = 0, smem = 0, threads = 0, n_inst = 0, first = 0;
+    uint32_t G = 1, groups = 1;
+    AltGeo geo;
+    const void* fn = nullptr;
+    AltRunDesc<R> D{};
+    size_t o_tab = 0, o_part = 0, o_ctr = 0;
+    double angle_unit = 0;
+  };
+  std::map<int, Class, std::greater<int>> classes;
+  for (const BatchGeo& g : geo) classes[g.n].n_inst++;
+  Bump b;
+  const size_t o_inst = b.take((size_t)n_inst * sizeof(AltInst<R>));
+  const size_t o_tan = b.take(std::max<size_t>(tans.size(), 1) * sizeof(R));
+  const size_t o_scale = b.take(std::max<size_t>(scales.size(), 1) * sizeof(R));
+  const size_t o_slot = b.take(slot.size() * sizeof(int));
+  const size_t o_offs = b.take((size_t)n_inst * sizeof(unsigned long long));
+  const size_t o_idx = b.take((size_t)n_inst * sizeof(unsigned int));
+  int first = 0;
+  for (auto& kv : classes) {
+    Class& k = kv.second;
+    k.n = kv.first;
+    k.first = first;
+    first += k.n_inst;
+    const int np = c64 ? k.n - 1 : k.n;
+    alt_geometry(np, &k.geo);
+    k.D.n_j = alt_levels(k.n, &k.D.c0);
+    k.D.n_tiles = 1u << (np - k.geo.tb);
+    BK_TRY(alt_kernel_ready<R>(c, k.geo, true, k.D.n_j, &k.fn, &k.smem, &k.threads, &k.per_sm));
+    const uint32_t slots = (uint32_t)(k.per_sm * c->num_sms);
+    double best = 0;
+    for (uint32_t G = std::min<uint32_t>(k.D.n_tiles, slots);;) {
+      const uint32_t groups = std::min<uint32_t>((uint32_t)k.n_inst, slots / G);
+      const double rounds = std::ceil((double)k.n_inst / groups);
+      const double busy = std::ceil((double)groups * G / c->num_sms) / k.per_sm;  // share of an SM's residency in use
+      const double t = rounds * (3.0 + std::ceil((double)k.D.n_tiles / G) * 9.0 * std::max(busy, 0.4));
+      if (best == 0 || t < best) {
+        best = t;
+        k.G = G;
+        k.groups = groups;
+      }
+      if (G == 1) break;
+      uint32_t p = 1;  // the next power of two below G
+      while (2 * p < G) p *= 2;
+      G = p;
+    }
+    k.o_tab = b.take((size_t)(k.D.n_j + 1) * sizeof(entry));
+    k.o_ctr = b.take((size_t)k.groups * 128);
+  }
+  const size_t o_glob = b.take(64);
+  const size_t up = b.off;
+  size_t part = 0;  // the classes run one after another: one room for their partial sums
+  for (auto& kv : classes)
+    part = std::max(part, (size_t)kv.second.groups * 2 * 3 * (size_t)std::max(n_meas, 1) * kv.second.G * sizeof(double));
+  const size_t o_part = b.take(part);
+  BK_TRY(ensure_buffer(c, &c->d_batch, &c->batch_cap, b.off));
+  BK_TRY(ensure_stage(c, up));
+  char *h = static_cast<char*>(c->h_stage), *d = static_cast<char*>(c->d_batch);
+  std::copy(tans.begin(), tans.end(), reinterpret_cast<R*>(h + o_tan));
+  std::copy(scales.begin(), scales.end(), reinterpret_cast<R*>(h + o_scale));
+  std::copy(slot.begin(), slot.end(), reinterpret_cast<int*>(h + o_slot));
+  std::memset(h + o_glob, 0, 64);
+  unsigned char* state = static_cast<unsigned char*>(c->d_batch_state);
+  std::map<int, int> at;
+  for (int i = 0; i < n_inst; ++i) {
+    const BatchGeo& g = geo[(size_t)i];
+    Class& k = classes[g.n];
+    k.angle_unit = g.angle_unit;
+    AltInst<R>& I = reinterpret_cast<AltInst<R>*>(h + o_inst)[k.first + at[g.n]++];
+    BK_TRY(alt_maps(c, state + g.state_off, g.np, k.geo, I.map, k.D.set));
+    I.state = state + g.state_off;
+    I.tan = reinterpret_cast<const R*>(d + o_tan) + (size_t)i * T;
+    I.scale = reinterpret_cast<const R*>(d + o_scale) + (size_t)i * T;
+    I.results = c->d_batch_results + (size_t)i * n_meas * 4;
+    I.e0 = g.e0;
+    I.s0 = g.s0;
+    reinterpret_cast<unsigned long long*>(h + o_offs)[i] = g.state_off;
+    reinterpret_cast<unsigned int*>(h + o_idx)[i] = g.s0;
+  }
+  for (auto& kv : classes) {
+    Class& k = kv.second;
+    alt_table(k.n, k.angle_unit, reinterpret_cast<entry*>(h + k.o_tab), k.D.c0, k.D.n_j);
+    std::memset(h + k.o_ctr, 0, (size_t)k.groups * 128);
+    uint16_t* dE = nullptr;
+    BK_TRY(batch_energy(c, k.n, &dE));
+    k.D.E = dE;
+    k.D.tab = reinterpret_cast<const entry*>(d + k.o_tab);
+    k.D.slot = reinterpret_cast<const int*>(d + o_slot);
+    k.D.partials = reinterpret_cast<double*>(d + o_part);
+    k.D.k1 = T;
+    k.D.meas_first = 1;
+  }
+  size_t ev = 0;
+  BK_TRY(ev_begin(c, "batch", &ev));
+  BK_CUDA(c, cudaMemcpyAsync(d, h, up, cudaMemcpyHostToDevice, st));
+  BK_CUDA(c, cudaMemsetAsync(state, 0, state_bytes, st));
+  set_basis_many_kernel<<<(n_inst + 127) / 128, 128, 0, st>>>(state, reinterpret_cast<unsigned long long*>(d + o_offs),
+                                                              reinterpret_cast<unsigned int*>(d + o_idx), c64 ? 1 : 0,
+                                                              n_inst);
+  BK_CUDA(c, cudaGetLastError());
+  for (auto& kv : classes) {
+    Class& k = kv.second;
+    AltBatch<R> Q{reinterpret_cast<const AltInst<R>*>(d + o_inst) + k.first, k.n_inst, n_meas, k.G,
+                  3 * (size_t)std::max(n_meas, 1) * k.G};
+    AltBarrier B{reinterpret_cast<unsigned int*>(d + k.o_ctr), reinterpret_cast<int*>(d + o_glob),
+                 reinterpret_cast<int*>(d + o_glob + 4), c->wait_polls > 0 ? c->wait_polls : kWaitPolls * 4u};
+    void* args[] = {&k.D, &Q, &B};
+    BK_CUDA(c, cudaLaunchCooperativeKernel(k.fn, dim3(k.G * k.groups), dim3((unsigned)k.threads), args, (size_t)k.smem, st));
+  }
+  BK_TRY(ev_end(c, ev));
+  std::vector<double> rows((size_t)n_inst * n_meas * 4);
+  int e = 0;
+  BK_CUDA(c, cudaMemcpyAsync(&e, d + o_glob, sizeof(int), cudaMemcpyDeviceToHost, st));
+  if (!rows.empty())
+    BK_CUDA(c, cudaMemcpyAsync(rows.data(), c->d_batch_results, rows.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
+  BK_CUDA(c, cudaStreamSynchronize(st));
+  BK_TRY(collect_timing(c));
+  if (e != 0) return fail(c, BK_ERR_TIMEOUT, "batched turning passes: a bounded device wait gave up (%d)", e);
+  batch_rows<R>(rows, row_log2, p_less, d_h, norm_out);
+  return BK_OK;
+}
+
 template <class R>
 int evolve_batch_t(bk_ctx* c, const bk_batch_params* bp, const bk_batch_instance* inst, int n_inst,
                    double* p_less, double* d_h, double* norm_out) {
@@ -1378,17 +1551,11 @@ int evolve_batch_t(bk_ctx* c, const bk_batch_params* bp, const bk_batch_instance
     if (bp->measure == nullptr || bp->measure[k]) slot[(size_t)k] = n_meas++;
   if (n_meas > 0 && (!p_less || !d_h)) return fail(c, BK_ERR_INVALID, "output arrays are NULL");
 
-  struct Geo {
-    int n, np, w2, w3, e0;
-    uint32_t n_a1, slabs, s0;
-    size_t state_off;
-    double angle_unit;
-  };
-  std::vector<Geo> geo((size_t)n_inst);
+  std::vector<BatchGeo> geo((size_t)n_inst);
   size_t state_bytes = 0;
   for (int i = 0; i < n_inst; ++i) {
     const bk_batch_instance& b = inst[i];
-    Geo g{};
+    BatchGeo g{};
     g.n = b.n;
     g.np = c64 ? b.n - 1 : b.n;
     if (g.np <= kElemBits || b.n > kMaxN)
@@ -1420,13 +1587,15 @@ int evolve_batch_t(bk_ctx* c, const bk_batch_params* bp, const bk_batch_instance
   std::vector<long double> row_log2((size_t)n_inst * std::max(n_meas, 1), 0.0L);
   for (int i = 0; i < n_inst; ++i) {
     long double lg = 0.0L;
-    double carry = 0.0;
+    double carry = 0.0, last_g = 0.0, exact = 0.0;
+    Log2Memo<R> memo;
     for (int k = 0; k <= T; ++k) {
       if (slot[(size_t)k] >= 0) row_log2[(size_t)i * n_meas + slot[(size_t)k]] = lg;
       if (k == T) break;
       const double gk = inst[i].g ? inst[i].g[k] : inst[i].g_const;
       if (!is_finite(gk)) return fail(c, BK_ERR_INVALID, "instance %d: g[%d] not finite", i, k);
-      const double want = std::tan(gk * bp->dt) + carry;  // as in evolve_fused
+      if (gk != last_g) exact = std::tan((last_g = gk) * bp->dt);
+      const double want = exact + carry;  // as in evolve_fused
       const R tf = (R)want;
       carry = want - (double)tf;
       R sc = (R)1;
@@ -1436,14 +1605,24 @@ int evolve_batch_t(bk_ctx* c, const bk_batch_params* bp, const bk_batch_instance
       }
       tans[(size_t)i * T + k] = tf;
       scales[(size_t)i * T + k] = sc;
-      lg += 0.5L * (long double)geo[(size_t)i].n * std::log2(1.0L + (long double)tf * (long double)tf);
+      lg += 0.5L * (long double)geo[(size_t)i].n * memo.log2_1t2(tf);
     }
+  }
+  bool turning = c->engine_mode == 4 && c->e_recompute == 0;
+  for (const BatchGeo& g : geo) {
+    AltGeo ag;
+    turning = turning && alt_geometry(g.np, &ag) && alt_kernel_of<R>(ag, true) != nullptr;
+  }
+  if (turning) {
+    if constexpr (sizeof(R) == 4)
+      for (const BatchGeo& g : geo) BK_TRY(check_phase<R>(c, g.n, g.angle_unit));
+    return batch_turning<R>(c, geo, T, slot, n_meas, tans, scales, state_bytes, row_log2, p_less, d_h, norm_out);
   }
 
   // phase tables per distinct n
   std::map<int, std::vector<unsigned char>> tables;
   std::map<int, typename PhaseV<R>::params> phase_of;
-  for (const Geo& g : geo) {
+  for (const BatchGeo& g : geo) {
     if (tables.count(g.n)) continue;
     typename PhaseV<R>::params ph{};
     std::vector<unsigned char> bytes;
@@ -1529,7 +1708,7 @@ int evolve_batch_t(bk_ctx* c, const bk_batch_params* bp, const bk_batch_instance
   std::vector<unsigned long long> offs((size_t)n_inst);
   std::vector<unsigned int> idx((size_t)n_inst);
   for (int i = 0; i < n_inst; ++i) {
-    const Geo& g = geo[(size_t)i];
+    const BatchGeo& g = geo[(size_t)i];
     uint16_t* dE = nullptr;
     BK_TRY(batch_energy(c, g.n, &dE));
     void* st = state + g.state_off;
@@ -1661,16 +1840,7 @@ int evolve_batch_t(bk_ctx* c, const bk_batch_params* bp, const bk_batch_instance
   BK_CUDA(c, cudaStreamSynchronize(st));
   BK_TRY(collect_timing(c));
   if (e != 0) return fail(c, BK_ERR_TIMEOUT, "batched persistent engine: a bounded device wait gave up (%d)", e);
-  for (int i = 0; i < n_inst; ++i)
-    for (int m = 0; m < n_meas; ++m) {
-      const size_t r = (size_t)i * n_meas + m;
-      const long double f = std::exp2(-2.0L * row_log2[r]);
-      // complex64: expectation values of the normalised state (see bk_evolve)
-      const long double nrm = (sizeof(R) == 4 && rows[4 * r + 2] > 0.0) ? (long double)rows[4 * r + 2] * f : 1.0L;
-      p_less[r] = (double)((long double)rows[4 * r + 0] * f / nrm);
-      d_h[r] = (double)((long double)rows[4 * r + 1] * f / nrm);
-      if (norm_out) norm_out[r] = (double)((long double)rows[4 * r + 2] * f);
-    }
+  batch_rows<R>(rows, row_log2, p_less, d_h, norm_out);
   return BK_OK;
 }
 

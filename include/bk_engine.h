@@ -155,12 +155,16 @@ typedef struct bk_evolve_params {
  * steps), and norm[m] is always the raw |psi|^2. */
 int bk_evolve(bk_ctx* ctx, const bk_evolve_params* p, double* p_less, double* d_h, double* norm);
 
-/* ---- Batched evolution: many statevectors in one persistent launch ----
+/* ---- Batched evolution: many statevectors in one call ----
  *
  * Every instance has its own n, trap and field; all share dt, the step count and
- * the measurement schedule. The tile tasks of all instances run in ONE
- * persistent kernel (launched through a captured CUDA graph when use_graph is
- * set), interleaved so that each statevector's A1 output is re-read from L2.
+ * the measurement schedule. Up to 24 qubits (complex64) or 23 (complex128) the
+ * instances of one size share a cooperative launch of turning passes, each worked
+ * on by a group of CTAs with its own barrier (use_graph and lag do not apply).
+ * With a larger instance, with E recomputed, or in BK_OPT_ENGINE_MODE 0 to 3 the
+ * tile tasks of all instances run in ONE persistent kernel (launched through a
+ * captured CUDA graph when use_graph is set), interleaved so that each
+ * statevector's A1 output is re-read from L2.
  * Outputs are row-major [instance][measurement], normalised like bk_evolve's. */
 typedef struct bk_batch_instance {
   int32_t n;           /* qubits: 14..30 (complex64) or 13..30 (complex128) */
