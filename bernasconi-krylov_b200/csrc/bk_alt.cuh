@@ -118,7 +118,7 @@ struct AltPlan {
   static constexpr int kThreads = 1 << (TB - KB);
   static constexpr int kWarps = kThreads / 32;
   static constexpr int kPer = 1 << KB;
-  static_assert(TB - KB >= 6 && 3 * KB >= TB && TB - KB <= 9, "three rounds cover the tile");
+  static_assert(TB - KB >= 5 && 3 * KB >= TB && TB - KB <= 9, "three rounds cover the tile");
   // lowest register bit and number of new tile bits of each round
   static constexpr int reg_lo(int r) { return r == 0 ? TB - KB : r == 1 ? TB - 2 * KB : 0; }
   static constexpr int act_hi(int r) { return r < 2 ? KB : TB - 2 * KB; }
@@ -133,7 +133,7 @@ struct AltPlan {
     constexpr int top = TB - (TB - KB - 5);  // warp bits [top, TB) of rounds 1 and 2
     if constexpr (r == 2) return (lane << KB) | (warp << top);
     constexpr int lo = TB - 2 * KB;          // tile bits below round 1's registers
-    if constexpr (lo == 2) {  // the 2^10-element tile
+    if constexpr (lo == 2 && TB == 10) {
       return (lane & 3u) | ((lane & 4u) << 6) | ((lane & 24u) << 3) | (warp << top);
     }
     return (lane & ((1u << lo) - 1u)) | ((lane >> lo) << (TB - KB)) | (warp << top);

@@ -1,6 +1,5 @@
-// Auxiliary kernels: E table, p_blind count, state init, the whole-state kernel
-// for n <= T (all steps in one launch), the plain per-qubit path, state export
-// and projective sampling.
+// Auxiliary kernels: E table, p_blind count, state init, the plain per-qubit path,
+// state export and projective sampling.
 #pragma once
 #include "bk_device.cuh"
 
@@ -62,104 +61,6 @@ __device__ __forceinline__ double2 amp_at(const double2* psi, uint32_t i) { retu
 __device__ __forceinline__ double2 amp_at(const Planar64* psi, uint32_t i) {
   const float* f = reinterpret_cast<const float*>(psi) + 4u * (i >> 1) + (i & 1u);
   return make_double2(f[0], f[2]);
-}
-
-// ---------------------------------------------------------------------------
-// Whole-state kernel (n <= T): one CTA keeps the 2^n amplitudes in shared
-// memory and runs every step (measure if flagged, D, Rx on each qubit) in one
-// launch. Per-step tangents, D scale factors, measure flags and result slots
-// come from device arrays.
-// ---------------------------------------------------------------------------
-template <class R>
-struct SmallParams {
-  typename AmpTraits<R>::amp* state;
-  int n, n_steps;
-  const R* t;            // n_steps tangents
-  const R* amp_scale;    // n_steps exact powers of two folded into D
-  const int* slot;       // n_steps + 1: results row, or -1
-  typename PhaseOf<R>::params phase;
-  int e0;
-  uint32_t s0;
-  double* results;
-  int inverse;           // 1: apply the adjoint step (butterflies with -t, then conj(D))
-  int measure_last;      // measure the entry at step n_steps (else the caller does later)
-};
-
-template <class R>
-__global__ void __launch_bounds__(kThreads, 1) small_state_kernel(const SmallParams<R> p) {
-  using amp = typename AmpTraits<R>::amp;
-  extern __shared__ __align__(1024) unsigned char smem[];
-  const int A = 1 << p.n;
-  amp* s = reinterpret_cast<amp*>(smem);
-  const auto tabs = PhaseOf<R>::stage(p.phase, smem);
-  s = reinterpret_cast<amp*>(smem + PhaseOf<R>::kSmemBytes);
-  uint16_t* E = reinterpret_cast<uint16_t*>(smem + PhaseOf<R>::kSmemBytes + (size_t)A * sizeof(amp));
-  __shared__ double red[3][kThreads / 32];
-  for (int i = threadIdx.x; i < A; i += kThreads) {
-    s[i] = p.state[i];
-    E[i] = (uint16_t)labs_energy((uint32_t)i, p.n);
-  }
-  __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int step = 0; step <= p.n_steps; ++step) {
-    const int slot = (step < p.n_steps || p.measure_last) ? p.slot[step] : -1;
-    if (slot >= 0) {
-      MeasureAcc acc;
-      for (int i = threadIdx.x; i < A; i += kThreads)
-        acc.add(norm2d(s[i]), (int)E[i] < p.e0, __popc((uint32_t)i ^ p.s0));
-      double a = warp_sum(acc.norm), b = warp_sum(acc.p_less), c = warp_sum(acc.d_h);
-      if (lane == 0) {
-        red[0][warp] = a;
-        red[1][warp] = b;
-        red[2][warp] = c;
-      }
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        double x = 0, y = 0, z = 0;
-        for (int w = 0; w < kThreads / 32; ++w) {
-          x += red[0][w];
-          y += red[1][w];
-          z += red[2][w];
-        }
-        p.results[4 * (size_t)slot + 0] = y;
-        p.results[4 * (size_t)slot + 1] = z;
-        p.results[4 * (size_t)slot + 2] = x;
-      }
-      __syncthreads();
-    }
-    if (step == p.n_steps) break;
-    const R t = p.inverse ? -p.t[step] : p.t[step];
-    if (!p.inverse) {
-      const R sc = p.amp_scale[step];
-      for (int i = threadIdx.x; i < A; i += kThreads) {
-        const int e = E[i];
-        amp v = PhaseOf<R>::apply(s[i], e, p.phase, tabs);
-        v.x *= sc;
-        v.y *= sc;
-        s[i] = v;
-      }
-      __syncthreads();
-    }
-    for (int q = 0; q < p.n; ++q) {
-      for (int k = threadIdx.x; k < A / 2; k += kThreads) {
-        const int a = ((k >> q) << (q + 1)) | (k & ((1 << q) - 1));
-        bfly(s[a], s[a | (1 << q)], t);
-      }
-      __syncthreads();
-    }
-    if (p.inverse) {
-      const R sc = p.amp_scale[step];
-      for (int i = threadIdx.x; i < A; i += kThreads) {
-        const int e = E[i];
-        amp v = PhaseOf<R>::apply_inverse(s[i], e, p.phase, tabs);
-        v.x *= sc;
-        v.y *= sc;
-        s[i] = v;
-      }
-      __syncthreads();
-    }
-  }
-  for (int i = threadIdx.x; i < A; i += kThreads) p.state[i] = s[i];
 }
 
 // ---------------------------------------------------------------------------

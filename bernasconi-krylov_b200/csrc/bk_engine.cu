@@ -32,6 +32,7 @@
 #include "bk_lanczos.cuh"
 #include "bk_persist.cuh"
 #include "bk_s23.cuh"
+#include "bk_small.cuh"
 
 using namespace bk;
 
@@ -106,6 +107,8 @@ struct bk_ctx {
   size_t alt_cap = 0;
   void* h_stage = nullptr;    // pinned staging of a run's uploads
   size_t stage_cap = 0;
+  void* h_out = nullptr;      // pinned room of a run's results
+  size_t out_cap = 0;
   std::map<std::pair<const void*, int>, int> occupancy;  // (kernel, dynamic smem) -> CTAs per SM
   uint32_t wait_polls = 0;    // persistent engine: polls of a dependency wait before it gives up (0 = default)
   uint64_t s23_checked = 0;   // fused strided pass geometry (np, a1, w2, lag) whose closed form was checked
@@ -372,46 +375,6 @@ int ensure_state(bk_ctx* c, int n, int prec) {
 }
 
 // Host side of the diagonal phase exp(-i angle_unit E).
-// complex64: E = h K + l; n_h table entries (the fewest in 16, 32, ..., 256 with
-// angle_unit (K - 1) <= 1/2 so the residual polynomials stay accurate);
-// h = umulhi(E, M) checked exact for every E <= Emax.
-int build_phase(bk_ctx* c, int n, double angle_unit, Phase32* P) {
-  const int emax = (n - 1) * n * (2 * n - 1) / 6;
-  int n_h = 16;
-  uint32_t K = 0;
-  for (;; n_h *= 2) {
-    if (n_h > kPhaseH)
-      return fail(c, BK_ERR_UNSUPPORTED, "phase angle per unit energy %g too large for the table", angle_unit);
-    K = std::max<uint32_t>(2u, (uint32_t)((emax + n_h) / n_h));  // ceil((emax + 1) / n_h), >= 2 so M fits 32 bits
-    if (std::fabs(angle_unit) * (double)(K - 1) <= 0.5) break;
-  }
-  const uint32_t M = (uint32_t)((((uint64_t)1 << 32) + K - 1) / K);
-  for (uint64_t e = 0; e <= (uint64_t)emax; ++e)
-    if (((e * M) >> 32) != e / K) return fail(c, BK_ERR_UNSUPPORTED, "no exact level split for n = %d", n);
-  std::vector<float2> hab((size_t)n_h);
-  std::vector<int> hq((size_t)n_h);
-  const double half_pi = 1.5707963267948966;
-  for (int h = 0; h < n_h; ++h) {
-    const double th = -angle_unit * (double)h * (double)K;
-    const double q = std::nearbyint(th / half_pi);
-    const double r = th - q * half_pi;  // |r| <= pi/4
-    hab[(size_t)h] = make_float2((float)(-std::tan(0.5 * r)), (float)std::sin(r));
-    hq[(size_t)h] = (int)(((long long)std::fmod(q, 4.0) + 4) % 4);
-  }
-  const size_t b1 = hab.size() * sizeof(float2), b2 = hq.size() * sizeof(int);
-  BK_TRY(ensure_buffer(c, &c->d_phase, &c->phase_cap, b1 + b2));
-  BK_CUDA(c, cudaMemcpyAsync(c->d_phase, hab.data(), b1, cudaMemcpyHostToDevice, c->stream));
-  BK_CUDA(c, cudaMemcpyAsync(static_cast<char*>(c->d_phase) + b1, hq.data(), b2, cudaMemcpyHostToDevice, c->stream));
-  BK_CUDA(c, cudaStreamSynchronize(c->stream));  // host vectors die at return
-  P->hab = reinterpret_cast<const float2*>(c->d_phase);
-  P->hq = reinterpret_cast<const int*>(static_cast<char*>(c->d_phase) + b1);
-  P->K = K;
-  P->M = M;
-  P->theta = (float)(-angle_unit);
-  P->theta_lo = (float)(-angle_unit - (double)P->theta);
-  P->n_h = n_h;
-  return BK_OK;
-}
 // complex128: E = 128 h + l, FP64 (cos, sin) tables.
 int build_phase(bk_ctx* c, int n, double angle_unit, Phase64* P) {
   const int emax = (n - 1) * n * (2 * n - 1) / 6;
@@ -1116,17 +1079,18 @@ int check_phase(bk_ctx* c, int n, double angle_unit) {
   return BK_OK;
 }
 
-// pinned host memory for a run's uploads (one copy, no staging by the driver)
-int ensure_stage(bk_ctx* c, size_t bytes) {
-  if (c->stage_cap >= bytes) return BK_OK;
-  if (c->h_stage) cudaFreeHost(c->h_stage);
-  c->h_stage = nullptr;
-  c->stage_cap = 0;
+// pinned host memory for a run's uploads and results (copied in one piece, not staged by the driver)
+int ensure_pinned(bk_ctx* c, void** ptr, size_t* cap, size_t bytes) {
+  if (*cap >= bytes) return BK_OK;
+  if (*ptr) cudaFreeHost(*ptr);
+  *ptr = nullptr;
+  *cap = 0;
   const size_t room = std::max<size_t>(bytes, 1 << 16);
-  BK_CUDA(c, cudaMallocHost(&c->h_stage, room));
-  c->stage_cap = room;
+  BK_CUDA(c, cudaMallocHost(ptr, room));
+  *cap = room;
   return BK_OK;
 }
+int ensure_stage(bk_ctx* c, size_t bytes) { return ensure_pinned(c, &c->h_stage, &c->stage_cap, bytes); }
 
 struct AltGeo {
   int tb = 0, w2 = 0, w3 = 0;
@@ -1347,6 +1311,86 @@ int evolve_alt(bk_ctx* c, const bk_evolve_params* p, const Schedule& S, double a
     }
     BK_TRY(alt_launch<R>(c, run, k0, k1, first, row0, rows));
     if (k1 > 0 && S.sample_pt[(size_t)k1] >= 0) BK_TRY(launch_sampling_t(c, psi, n, S.sample_pt[(size_t)k1], S.shots));
+    if (k1 == T) return BK_OK;
+    k0 = k1;
+  }
+}
+
+// ---------------------------------------------------------------------------
+// small statevectors (csrc/bk_small.cuh)
+// ---------------------------------------------------------------------------
+// Tile by the element bits np: 16 elements a thread from 2^10 elements on, 8 below
+// (more warps; one warp up to 2^8, smaller states padded).
+template <class R>
+const void* small_kernel_of(int np, int* threads, int* tile_bytes) {
+  *tile_bytes = 16 << std::max(np, 8);
+  *threads = np >= 10 ? 1 << (np - 4) : 1 << (std::max(np, 8) - 3);
+  switch (np) {
+    case 12: return reinterpret_cast<const void*>(small_kernel<R, 12, 4>);
+    case 11: return reinterpret_cast<const void*>(small_kernel<R, 11, 4>);
+    case 10: return reinterpret_cast<const void*>(small_kernel<R, 10, 4>);
+    case 9: return reinterpret_cast<const void*>(small_kernel<R, 9, 3>);
+    default: return reinterpret_cast<const void*>(small_kernel<R, 8, 3>);
+  }
+}
+
+template <class R>
+int evolve_small(bk_ctx* c, const bk_evolve_params* p, const Schedule& S, double angle_unit,
+                 const std::vector<R>& tans, const std::vector<R>& scales) {
+  using entry = typename AltPhase<R>::entry;
+  using amp = typename AmpTraits<R>::amp;
+  const int n = p->n, np = sizeof(R) == 4 ? n - 1 : n, T = p->n_steps;
+  SmallRun<R> P{};
+  const int n_j = alt_levels(n, &P.c0);
+  Bump b;
+  const size_t o_tab = b.take((size_t)(n_j + 1) * sizeof(entry));
+  const size_t o_step = b.take((size_t)(T + 1) * sizeof(SmallStep<R>));
+  const size_t up = b.off;
+  int threads = 0, tile = 0;
+  const void* fn = small_kernel_of<R>(np, &threads, &tile);
+  const size_t o_part = b.take((size_t)std::max(S.n_meas, 1) * 3 * (threads / 32) * sizeof(double));
+  BK_TRY(ensure_buffer(c, &c->d_small, &c->small_cap, b.off));
+  BK_TRY(ensure_stage(c, up));
+  char *h = static_cast<char*>(c->h_stage), *d = static_cast<char*>(c->d_small);
+  alt_table(n, angle_unit, reinterpret_cast<entry*>(h + o_tab), P.c0, n_j);
+  for (int k = 0; k <= T; ++k)
+    reinterpret_cast<SmallStep<R>*>(h + o_step)[k] = {k < T ? tans[(size_t)k] : (R)0, k < T ? scales[(size_t)k] : (R)1,
+                                                      S.slot[(size_t)k], 0};
+  BK_CUDA(c, cudaMemcpyAsync(d, h, up, cudaMemcpyHostToDevice, c->stream));
+  BK_TRY(allow_smem(c, fn, tile));
+  P.state = reinterpret_cast<amp*>(c->d_state);
+  P.E = c->d_E;
+  P.tab = reinterpret_cast<const entry*>(d + o_tab);
+  P.step = reinterpret_cast<const SmallStep<R>*>(d + o_step);
+  P.partials = reinterpret_cast<double*>(d + o_part);
+  P.results = c->d_results;
+  P.np = np;
+  P.e0 = (int)p->e0;
+  P.s0 = (uint32_t)(p->s0 & ((1ull << n) - 1ull));
+  // launches end at sampling points, which read psi_k from memory
+  auto launch = [&](int k0, int k1, bool first) -> int {
+    P.k0 = k0;
+    P.k1 = k1;
+    P.init = first ? 1 : 0;
+    P.meas_first = first ? 1 : 0;
+    P.row0 = P.rows = 0;
+    for (int k = k0; k <= k1; ++k)
+      if ((k > k0 || first) && S.slot[(size_t)k] >= 0 && P.rows++ == 0) P.row0 = S.slot[(size_t)k];
+    size_t ev = 0;
+    BK_TRY(ev_begin(c, "small_state", &ev));
+    void* args[] = {&P};
+    BK_CUDA(c, cudaLaunchKernel(fn, dim3(1), dim3((unsigned)threads), args, (size_t)tile, c->stream));
+    return ev_end(c, ev);
+  };
+  const amp* psi = reinterpret_cast<const amp*>(c->d_state);
+  int k0 = 0;
+  for (bool first = true;; first = false) {
+    // the first launch of a run that samples psi_0 only sets it up (and measures it)
+    int k1 = first && S.sample_pt[0] >= 0 ? 0 : k0 + 1;
+    while (k1 < T && S.sample_pt[(size_t)k1] < 0) ++k1;
+    k1 = std::min(k1, T);
+    BK_TRY(launch(k0, k1, first));
+    if (S.sample_pt[(size_t)k1] >= 0) BK_TRY(launch_sampling<amp>(c, psi, n, S.sample_pt[(size_t)k1], S.shots));
     if (k1 == T) return BK_OK;
     k0 = k1;
   }
@@ -1849,18 +1893,11 @@ int evolve_batch_t(bk_ctx* c, const bk_batch_params* bp, const bk_batch_instance
 template <class R>
 int evolve_fused(bk_ctx* c, const bk_evolve_params* p, const Schedule& S, double angle_unit,
                  std::vector<long double>* row_log2, long double* final_log2) {
-  using amp = typename AmpTraits<R>::amp;
   constexpr int T = AmpTraits<R>::kTileBits;
   const int n = p->n;
   const double dt = p->dt;
-  typename PhaseOf<R>::params phase{};
   const bool use_alt = n > T && c->engine_mode == 4 && alt_takes<R>(c, n);
-  if (use_alt)
-    BK_TRY(check_phase<R>(c, n, angle_unit));
-  else
-    BK_TRY(build_phase(c, n, angle_unit, &phase));
-  const int e0 = (int)p->e0;
-  const uint32_t s0 = (uint32_t)(p->s0 & ((1ull << n) - 1ull));
+  BK_TRY(check_phase<R>(c, n, angle_unit));
 
   // host schedule of the omitted cos^n factors and power-of-two rescales
   std::vector<R> tans((size_t)p->n_steps), scales((size_t)p->n_steps);
@@ -1888,74 +1925,7 @@ int evolve_fused(bk_ctx* c, const bk_evolve_params* p, const Schedule& S, double
   }
   *final_log2 = lg;
 
-  if (n <= T) {
-    // whole state in one CTA's shared memory; all steps between two sampling
-    // points in one launch
-    const size_t smem = PhaseOf<R>::kSmemBytes + (1ull << n) * (sizeof(amp) + 2);
-    const size_t bytes = tans.size() * sizeof(R) * 2 + S.slot.size() * sizeof(int) + 64;
-    BK_TRY(ensure_buffer(c, &c->d_small, &c->small_cap, bytes));
-    char* base = reinterpret_cast<char*>(c->d_small);
-    R* d_t = reinterpret_cast<R*>(base);
-    R* d_sc = d_t + tans.size();
-    int* d_slot = reinterpret_cast<int*>(base + tans.size() * sizeof(R) * 2);
-    if (!tans.empty()) {
-      BK_CUDA(c, cudaMemcpyAsync(d_t, tans.data(), tans.size() * sizeof(R), cudaMemcpyHostToDevice, c->stream));
-      BK_CUDA(c, cudaMemcpyAsync(d_sc, scales.data(), scales.size() * sizeof(R), cudaMemcpyHostToDevice, c->stream));
-    }
-    BK_CUDA(c, cudaMemcpyAsync(d_slot, S.slot.data(), S.slot.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream));
-    BK_TRY(allow_smem(c, reinterpret_cast<const void*>(small_state_kernel<R>),
-                      (int)(PhaseOf<R>::kSmemBytes + (1ull << T) * (sizeof(amp) + 2))));
-    // Segments end at sampling points: sampling reads psi_k before step k, so a
-    // segment runs steps [k0, k1) and leaves the measurement of step k1 to the
-    // next segment (measure_last = 0); the last segment measures its end.
-    int k0 = 0, search = 0;
-    while (true) {
-      int k1 = search;
-      while (k1 <= p->n_steps && S.sample_pt[(size_t)k1] < 0) ++k1;
-      const bool sample_here = (k1 <= p->n_steps);
-      SmallParams<R> sp;
-      sp.state = reinterpret_cast<amp*>(c->d_state);
-      sp.n = n;
-      sp.n_steps = (sample_here ? k1 : p->n_steps) - k0;
-      sp.t = d_t + k0;
-      sp.amp_scale = d_sc + k0;
-      sp.slot = d_slot + k0;
-      sp.phase = phase;
-      sp.e0 = e0;
-      sp.s0 = s0;
-      sp.results = c->d_results;
-      sp.inverse = 0;
-      sp.measure_last = sample_here ? 0 : 1;
-      if (sp.n_steps > 0 || sp.measure_last) {
-        size_t ev = 0;
-        BK_TRY(ev_begin(c, "small_state", &ev));
-        small_state_kernel<R><<<1, kThreads, smem, c->stream>>>(sp);
-        BK_CUDA(c, cudaGetLastError());
-        BK_TRY(ev_end(c, ev));
-      }
-      if (!sample_here) break;
-      BK_TRY(launch_sampling<amp>(c, reinterpret_cast<amp*>(c->d_state), n, S.sample_pt[(size_t)k1], S.shots));
-      k0 = k1;
-      search = k1 + 1;
-      if (k1 == p->n_steps) {
-        // sampling at the final step; its measurement follows in a zero-step launch
-        SmallParams<R> fp = sp;
-        fp.n_steps = 0;
-        fp.t = d_t;
-        fp.amp_scale = d_sc;
-        fp.slot = d_slot + k1;
-        fp.measure_last = 1;
-        size_t ev = 0;
-        BK_TRY(ev_begin(c, "small_state", &ev));
-        small_state_kernel<R><<<1, kThreads, smem, c->stream>>>(fp);
-        BK_CUDA(c, cudaGetLastError());
-        BK_TRY(ev_end(c, ev));
-        break;
-      }
-    }
-    return BK_OK;
-  }
-
+  if (n <= T) return evolve_small<R>(c, p, S, angle_unit, tans, scales);
   if (use_alt) return evolve_alt<R>(c, p, S, angle_unit, tans, scales);
   return evolve_persist<R>(c, p, S, angle_unit, tans, scales);
 }
@@ -2379,18 +2349,20 @@ int adjoint_t(bk_ctx* c, const bk_adjoint_params* p, const std::vector<double>& 
   return BK_OK;
 }
 
+// the error word a run has left: reported, and cleared for the next one
+int device_error(bk_ctx* c, int e) {
+  if (e == 0) return BK_OK;
+  cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream);
+  cudaMemsetAsync(c->d_ticket, 0, sizeof(unsigned int), c->stream);
+  cudaStreamSynchronize(c->stream);
+  if (e == DEV_TIMEOUT) return fail(c, BK_ERR_TIMEOUT, "a kernel's bounded wait for its tile load gave up");
+  return fail(c, BK_ERR_CUDA, "device error word %d", e);
+}
 int check_device_error(bk_ctx* c) {
   int e = 0;
   BK_CUDA(c, cudaMemcpyAsync(&e, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   BK_CUDA(c, cudaStreamSynchronize(c->stream));
-  if (e == DEV_TIMEOUT) {
-    cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream);
-    cudaMemsetAsync(c->d_ticket, 0, sizeof(unsigned int), c->stream);
-    cudaStreamSynchronize(c->stream);
-    return fail(c, BK_ERR_TIMEOUT, "a kernel's bounded wait for its tile load gave up");
-  }
-  if (e != 0) return fail(c, BK_ERR_CUDA, "device error word %d", e);
-  return BK_OK;
+  return device_error(c, e);
 }
 
 }  // namespace
@@ -2457,7 +2429,8 @@ int bk_destroy(bk_ctx* c) {
   for (void* p : {c->d_batch_state, c->d_batch, (void*)c->d_batch_results, c->d_persist, c->d_lam, c->d_ckpt,
                   c->d_adj, c->d_descent, c->d_lz, c->d_fsmap, c->d_alt})
     if (p) cudaFree(p);
-  if (c->h_stage) cudaFreeHost(c->h_stage);
+  for (void* p : {c->h_stage, c->h_out})
+    if (p) cudaFreeHost(p);
   for (auto& e : c->ev_pool) {
     cudaEventDestroy(e.first);
     cudaEventDestroy(e.second);
@@ -2788,12 +2761,17 @@ int bk_evolve(bk_ctx* c, const bk_evolve_params* p, double* p_less, double* d_h,
     BK_TRY(ensure_buffer(c, reinterpret_cast<void**>(&c->d_samples), &c->samples_cap, draws * sizeof(uint64_t)));
     BK_CUDA(c, cudaMemcpyAsync(c->d_rand, p->randnums, draws * sizeof(double), cudaMemcpyHostToDevice, c->stream));
   }
-  BK_CUDA(c, cudaMemsetAsync(c->d_ticket, 0, sizeof(unsigned int), c->stream));
-  BK_CUDA(c, cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
-  BK_CUDA(c, cudaMemsetAsync(c->d_state, 0, (1ull << n) * amp_bytes(p->precision), c->stream));
+  // a small run sets its basis state up itself and waits for nothing that could give up
+  const bool small = p->method == BK_FUSED && n <= T;
+  if (!small) {
+    BK_CUDA(c, cudaMemsetAsync(c->d_ticket, 0, sizeof(unsigned int), c->stream));
+    BK_CUDA(c, cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
+    BK_CUDA(c, cudaMemsetAsync(c->d_state, 0, (1ull << n) * amp_bytes(p->precision), c->stream));
+  }
   const uint32_t s0 = (uint32_t)(p->s0 & ((1ull << n) - 1ull));
   c->planar = (p->precision == BK_C64 && p->method == BK_FUSED && n > 13);
-  if (c->planar)
+  if (small) {
+  } else if (c->planar)
     set_basis_planar_kernel<<<1, 1, 0, c->stream>>>(reinterpret_cast<float*>(c->d_state), s0);
   else if (p->precision == BK_C64)
     set_basis_kernel<float2><<<1, 1, 0, c->stream>>>(reinterpret_cast<float2*>(c->d_state), s0);
@@ -2815,14 +2793,20 @@ int bk_evolve(bk_ctx* c, const bk_evolve_params* p, double* p_less, double* d_h,
     else
       BK_TRY(evolve_fused<double>(c, &q, S, angle_unit, &row_log2, &final_log2));
   }
-  std::vector<double> rows(4 * (size_t)S.n_meas);
+  // the rows and the error word come back through pinned memory, behind one wait
+  const size_t row_bytes = 4 * (size_t)S.n_meas * sizeof(double);
+  BK_TRY(ensure_pinned(c, &c->h_out, &c->out_cap, row_bytes + sizeof(int)));
+  const double* rows = static_cast<const double*>(c->h_out);
+  int* h_err = reinterpret_cast<int*>(static_cast<char*>(c->h_out) + row_bytes);
+  *h_err = 0;
   if (S.n_meas > 0)
-    BK_CUDA(c, cudaMemcpyAsync(rows.data(), c->d_results, rows.size() * sizeof(double), cudaMemcpyDeviceToHost,
-                               c->stream));
+    BK_CUDA(c, cudaMemcpyAsync(c->h_out, c->d_results, row_bytes, cudaMemcpyDeviceToHost, c->stream));
+  if (!small) BK_CUDA(c, cudaMemcpyAsync(h_err, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   if (S.n_pts > 0)
     BK_CUDA(c, cudaMemcpyAsync(p->samples_out, c->d_samples, (size_t)S.n_pts * S.shots * sizeof(uint64_t),
                                cudaMemcpyDeviceToHost, c->stream));
-  BK_TRY(check_device_error(c));
+  BK_CUDA(c, cudaStreamSynchronize(c->stream));
+  BK_TRY(device_error(c, *h_err));
   BK_TRY(collect_timing(c));
   c->have_state = true;
   c->last_planar = c->planar;

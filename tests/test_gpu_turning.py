@@ -101,3 +101,35 @@ def test_wait_limit_is_an_error_not_a_hang(eng):
         eng.set_option("wait_polls", 0)
     p, _, nn = eng.evolve(16, bk.select_trap(16, 3, 100, 0.3)[0], 0.35, 0.02, 4, precision=bk.BK_C128)
     assert np.max(np.abs(nn - 1.0)) <= 1e-12
+
+
+# the whole-state kernel (up to 13 / 12 qubits): every tile (2^8 padded to 2^12
+# elements), runs that end in either round layout, against the per-qubit path
+@pytest.mark.parametrize("precision", [bk.BK_C64, bk.BK_C128])
+@pytest.mark.parametrize("n", [1, 2, 3, 8, 9, 10, 11, 12, 13])
+@pytest.mark.parametrize("steps", [0, 1, 6, 7])
+def test_small_states_match_the_plain_path(eng, n, precision, steps):
+    if n == 13 and precision == bk.BK_C128:
+        pytest.skip("13 qubits in complex128 run in tiles")
+    s0, g = (0b1011001110101 & ((1 << n) - 1)), np.linspace(0.3, 0.5, steps)
+    a = eng.evolve(n, s0, g, 0.05, steps, precision=precision)
+    psi = eng.export_state(n)
+    b = eng.evolve(n, s0, g, 0.05, steps, precision=bk.BK_C128, method=bk.BK_PLAIN)
+    ref = eng.export_state(n)
+    c64 = precision == bk.BK_C64
+    assert np.max(np.abs(a[0] - b[0])) <= (C64_DP_BAR if c64 else BAR128)
+    assert np.max(np.abs(a[1] - b[1])) <= (C64_DH_BAR if c64 else BAR128 * n)
+    # complex64: 7 steps of at most 20 roundings of 6e-8 on amplitudes up to 1
+    assert np.max(np.abs(psi - ref)) <= (1e-5 if c64 else BAR128)
+
+
+@pytest.mark.parametrize("n", [5, 9, 12])
+def test_small_runs_split_at_sampling_points(eng, n):
+    s0 = 0b110100101110 & ((1 << n) - 1)
+    kw = dict(n=n, g=0.35, dt=0.05, t_max=1.0, verbose=False, num_sampling_seeds=1)
+    a = eng.sampler_run(s0, shots_per_point=0, num_sample_points=21, dt_sample=0.05, **kw)
+    b = eng.sampler_run(s0, shots_per_point=16, num_sample_points=7, record_trajectory=True, dt_trajectory=0.05, **kw)
+    # launches begin in round 0's layout: the sums of a step are the same terms, those
+    # of a step in the other layout are summed in another order
+    assert np.max(np.abs(a["p_less_history"] - b["p_less_history"])) <= BAR128
+    assert np.max(np.abs(a["dh_history"] - b["dh_history"])) <= BAR128 * n
