@@ -277,78 +277,155 @@ __global__ void dmin_sphere_kernel(int n, uint32_t s, int target, int d, unsigne
 
 // ---------------------------------------------------------------------------
 // Batched single-flip steepest descent (reference: batch_steepest_descent_kernel,
-// src/classical/classical.cuh:459-540; CPU form :625-712). One warp per start:
-// lane l scores the flips p = l, l + 32 from the shared autocorrelations C_k
-// (C_k + d_k(p))^2 summed over k, the warp keeps the lowest energy and, among
-// equal energies, the lowest p — the flip the sequential scan (first strictly
-// better) takes; lanes own C_k for k = l, l + 32 for the update. An iteration
-// costs n evaluations and runs only while evals + n <= budget, as in the reference.
+// src/classical/classical.cuh:459-540; CPU form :625-712). One warp per start: lane l
+// scores the flips p = l (and l + 32 from 33 spins on), the warp keeps the lowest
+// energy and, among equal energies, the lowest p — the flip the sequential scan (first
+// strictly better) takes. An iteration costs n evaluations and runs only while evals +
+// n <= budget, as in the reference.
+//
+// A flip of spin p changes every C_k by d_k = -2 s_p t_k, t_k = s_{p+k} + s_{p-k} (a
+// spin outside the chain counts 0), so the energy by
+//   sum_k d_k (2 C_k + d_k) = -4 s_p V + 4 Q,  V = sum_k C_k t_k,  Q = sum_k t_k^2.
+// V: with u_k, w_k the bits of the spins at p + k and p - k, t_k = (valid) - 2 (u_k +
+// w_k), so V = prefix sums of C - 2 sum_k C_k (u_k + w_k), and C_k (|C_k| < n, a byte)
+// against u_k + w_k (bytes) is four products an instruction (dp4a); the bytes stay in
+// registers and a flip of spin q changes one of them per lane, the one at |p - q|.
+// Q = n - 1 + 2 sum over the pairs inside the chain of s_{p+k} s_{p-k}: a popcount of
+// the chain against its mirror image. About 90 instructions an iteration up to 32
+// spins, where trying every flip with its n - 1 correlations took about 700
+// (B200, 65536 starts: n = 28 58 us against 268, n = 63 256 us against 1869).
 // ---------------------------------------------------------------------------
 constexpr int kDescentWarps = 8;
 
-__device__ __forceinline__ int spin_of(uint64_t x, int i) { return ((x >> i) & 1ull) ? -1 : 1; }
+__device__ __forceinline__ uint32_t bits_to_bytes(uint32_t b) { return (b * 0x00204081u) & 0x01010101u; }
 
+// HALVES = 1: up to 32 spins, 2: up to 63
+template <int HALVES>
+struct DescentWord;
+template <>
+struct DescentWord<1> {
+  using T = uint32_t;
+  __device__ static T rev(T x) { return __brev(x); }
+  __device__ static int popc(T x) { return __popc(x); }
+};
+template <>
+struct DescentWord<2> {
+  using T = unsigned long long;
+  __device__ static T rev(T x) { return __brevll(x); }
+  __device__ static int popc(T x) { return __popcll(x); }
+};
+
+template <int HALVES>
 __global__ void __launch_bounds__(32 * kDescentWarps)
     descent_kernel(int n, const uint64_t* __restrict__ starts, long long count, unsigned long long budget,
                    uint64_t* __restrict__ final_states, long long* __restrict__ final_energies,
                    unsigned long long* __restrict__ evals_out) {
-  __shared__ int Cs[kDescentWarps][64];
+  using W = DescentWord<HALVES>;
+  using T = typename W::T;
+  constexpr int kBits = 32 * HALVES, kWords = 8 * HALVES;  // chain bits, words of four C bytes
+  __shared__ __align__(16) signed char Cs[kDescentWarps][kBits];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const long long i = (long long)blockIdx.x * kDescentWarps + wib;
   if (i >= count) return;  // the whole warp leaves together
-  int* C = Cs[wib];
-  const uint64_t mask = (1ull << n) - 1ull;
-  uint64_t x = starts[i] & mask;
-  int part = 0;
-  for (int k = 1 + lane; k < n; k += 32) {
-    const int c = (n - k) - 2 * __popcll((x ^ (x >> k)) & ((1ull << (n - k)) - 1ull));
-    C[k] = c;
-    part += c * c;
-  }
+  signed char* C = Cs[wib];
+  const T mask = (T)~(T)0 >> (kBits - n);
+  T x = (T)starts[i] & mask;
+  int c[HALVES], e = 0;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-  int e = part;
+  for (int h = 0; h < HALVES; ++h) {
+    const int k = lane + 32 * h;
+    c[h] = 0;
+    if (k >= 1 && k < n) c[h] = (n - k) - 2 * W::popc((x ^ (x >> k)) & (mask >> k));
+    C[k] = (signed char)c[h];
+    e += c[h] * c[h];
+  }
+  e = __reduce_add_sync(0xffffffffu, e);
+  // bytes u_k + w_k of each of the lane's spins
+  uint32_t t[HALVES][kWords];
+#pragma unroll
+  for (int h = 0; h < HALVES; ++h) {
+    const int p = lane + 32 * h;
+    const T u = x >> p, w = W::rev(x) >> (kBits - 1 - p);
+#pragma unroll
+    for (int g = 0; g < kWords; ++g)
+      t[h][g] = bits_to_bytes((uint32_t)(u >> (4 * g)) & 15u) + bits_to_bytes((uint32_t)(w >> (4 * g)) & 15u);
+  }
   __syncwarp();
   unsigned long long evals = 1;
   while (evals + (unsigned long long)n <= budget) {
-    int best_e = e, best_p = 0x7fffffff;
-    for (int p = lane; p < n; p += 32) {
-      const int sp = spin_of(x, p);
-      int ne = 0;
-      for (int k = 1; k < n; ++k) {
-        int d = 0;
-        if (p + k < n) d -= 2 * sp * spin_of(x, p + k);
-        if (p - k >= 0) d -= 2 * sp * spin_of(x, p - k);
-        const int c = C[k] + d;
-        ne += c * c;
-      }
-      if (ne < best_e) {
-        best_e = ne;
-        best_p = p;
-      }
-    }
+    // prefix sums of C: lane l holds sum_{k <= l} C_k (second half: k <= l + 32)
+    int pre[HALVES];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const int oe = __shfl_xor_sync(0xffffffffu, best_e, o);
-      const int op = __shfl_xor_sync(0xffffffffu, best_p, o);
-      if (oe < best_e || (oe == best_e && op < best_p)) {
-        best_e = oe;
-        best_p = op;
+    for (int h = 0; h < HALVES; ++h) {
+      pre[h] = c[h];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, pre[h], o);
+        if (lane >= o) pre[h] += y;
+      }
+      if (h == 1) pre[1] += __shfl_sync(0xffffffffu, pre[0], 31);
+    }
+    int dot[HALVES];
+#pragma unroll
+    for (int h = 0; h < HALVES; ++h) dot[h] = 0;
+#pragma unroll
+    for (int g = 0; g < kWords; g += 4) {
+      const int4 q = *reinterpret_cast<const int4*>(C + 4 * g);  // the same address in every lane
+#pragma unroll
+      for (int h = 0; h < HALVES; ++h) {
+        dot[h] = __dp4a(q.x, (int)t[h][g], dot[h]);
+        dot[h] = __dp4a(q.y, (int)t[h][g + 1], dot[h]);
+        dot[h] = __dp4a(q.z, (int)t[h][g + 2], dot[h]);
+        dot[h] = __dp4a(q.w, (int)t[h][g + 3], dot[h]);
       }
     }
-    evals += (unsigned long long)n;
-    if (best_p == 0x7fffffff) break;  // no strictly better neighbour: a local minimum
-    const int sp = spin_of(x, best_p);
-    __syncwarp();
-    for (int k = 1 + lane; k < n; k += 32) {
-      int d = 0;
-      if (best_p + k < n) d -= 2 * sp * spin_of(x, best_p + k);
-      if (best_p - k >= 0) d -= 2 * sp * spin_of(x, best_p - k);
-      C[k] += d;
+    int key = 0x7fffffff;  // energy change * 64 + p
+    const T r = W::rev(x);
+#pragma unroll
+    for (int h = 0; h < HALVES; ++h) {
+      const int p = lane + 32 * h;
+      const int far = n - 1 - p;  // spins above p
+      int up = __shfl_sync(0xffffffffu, pre[0], far & 31);
+      if (HALVES == 2) {
+        const int hi = __shfl_sync(0xffffffffu, pre[HALVES - 1], far & 31);
+        if (far >= 32) up = hi;
+      }
+      if (p < n) {
+        const int m = min(p, far);
+        const T u = x >> p, w = r >> (kBits - 1 - p);
+        const int unlike = W::popc((u ^ w) & (T)((((T)1 << m) - 1) << 1));
+        const int V = up + pre[h] - 2 * dot[h];
+        const int Q = n - 1 + 2 * (m - 2 * unlike);
+        const int s = (u & 1) ? -1 : 1;
+        key = min(key, 4 * (Q - s * V) * 64 + p);
+      }
     }
+    key = __reduce_min_sync(0xffffffffu, key);
+    evals += (unsigned long long)n;
+    if (key >= 0) break;  // no strictly better neighbour: a local minimum
+    const int q = key & 63;
+    e += key >> 6;
+    const int sq = (int)((x >> q) & 1) ? -1 : 1;
     __syncwarp();
-    x ^= 1ull << best_p;
-    e = best_e;
+#pragma unroll
+    for (int h = 0; h < HALVES; ++h) {
+      const int k = lane + 32 * h;
+      // the lane as the correlation C_k
+      if (k >= 1 && k < n) {
+        int d = 0;
+        if (q + k < n) d += (int)((x >> (q + k)) & 1) ? -1 : 1;
+        if (q - k >= 0) d += (int)((x >> (q - k)) & 1) ? -1 : 1;
+        c[h] -= 2 * sq * d;
+        C[k] = (signed char)c[h];
+      }
+      // the lane as spin p = k: the byte at |p - q| moves with spin q's new bit
+      const int dist = k > q ? k - q : q - k;
+      const uint32_t step = dist == 0 ? 0u : (sq > 0 ? 1u : 0xFFFFFFFFu) << (8 * (dist & 3));
+#pragma unroll
+      for (int g = 0; g < kWords; ++g) t[h][g] += (dist >> 2) == g ? step : 0u;
+    }
+    x ^= (T)1 << q;
+    __syncwarp();
   }
   if (lane == 0) {
     final_states[i] = x;
