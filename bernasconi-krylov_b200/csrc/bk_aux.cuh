@@ -317,9 +317,9 @@ struct DescentWord<2> {
 
 template <int HALVES>
 __global__ void __launch_bounds__(32 * kDescentWarps)
-    descent_kernel(int n, const uint64_t* __restrict__ starts, long long count, unsigned long long budget,
-                   uint64_t* __restrict__ final_states, long long* __restrict__ final_energies,
-                   unsigned long long* __restrict__ evals_out) {
+    descent_kernel(int n, const typename DescentWord<HALVES>::T* __restrict__ starts, long long count,
+                   unsigned long long budget, typename DescentWord<HALVES>::T* __restrict__ final_states,
+                   int* __restrict__ final_energies, uint32_t* __restrict__ evals_out) {
   using W = DescentWord<HALVES>;
   using T = typename W::T;
   constexpr int kBits = 32 * HALVES, kWords = 8 * HALVES;  // chain bits, words of four C bytes
@@ -329,7 +329,7 @@ __global__ void __launch_bounds__(32 * kDescentWarps)
   if (i >= count) return;  // the whole warp leaves together
   signed char* C = Cs[wib];
   const T mask = (T)~(T)0 >> (kBits - n);
-  T x = (T)starts[i] & mask;
+  T x = starts[i] & mask;
   int c[HALVES], e = 0;
 #pragma unroll
   for (int h = 0; h < HALVES; ++h) {
@@ -430,7 +430,7 @@ __global__ void __launch_bounds__(32 * kDescentWarps)
   if (lane == 0) {
     final_states[i] = x;
     final_energies[i] = e;
-    if (evals_out) evals_out[i] = evals;
+    evals_out[i] = (uint32_t)evals;  // at most n flips' worth per energy level: far below 2^32
   }
 }
 

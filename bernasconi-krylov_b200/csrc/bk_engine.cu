@@ -17,6 +17,7 @@
 #include <iostream>
 #include <limits>
 #include <map>
+#include <mutex>
 #include <random>
 #include <string>
 #include <unordered_set>
@@ -61,6 +62,7 @@ struct TimingRec {
 
 struct bk_ctx {
   int device = 0;
+  bool counted = false;  // among the contexts that keep the process's pinned room
   cudaStream_t stream = nullptr;
   std::string last_error;
   // E table cache (per n), like the reference's ensure_cached_energies
@@ -105,10 +107,7 @@ struct bk_ctx {
   int adj_a1 = 0;             // adjoint reverse sweep A1: 0 = 12-bit, 1 = warp-local (element bits 0-8)
   void* d_alt = nullptr;      // turning passes: phase table, per-step arrays, partial sums, counters
   size_t alt_cap = 0;
-  void* h_stage = nullptr;    // pinned staging of a run's uploads
-  size_t stage_cap = 0;
-  void* h_out = nullptr;      // pinned room of a run's results
-  size_t out_cap = 0;
+  std::vector<char> h_stage;  // a run's uploads, put together for one copy
   std::map<std::pair<const void*, int>, int> occupancy;  // (kernel, dynamic smem) -> CTAs per SM
   uint32_t wait_polls = 0;    // persistent engine: polls of a dependency wait before it gives up (0 = default)
   uint64_t s23_checked = 0;   // fused strided pass geometry (np, a1, w2, lag) whose closed form was checked
@@ -1079,18 +1078,63 @@ int check_phase(bk_ctx* c, int n, double angle_unit) {
   return BK_OK;
 }
 
-// pinned host memory for a run's uploads and results (copied in one piece, not staged by the driver)
-int ensure_pinned(bk_ctx* c, void** ptr, size_t* cap, size_t bytes) {
-  if (*cap >= bytes) return BK_OK;
-  if (*ptr) cudaFreeHost(*ptr);
-  *ptr = nullptr;
-  *cap = 0;
-  const size_t room = std::max<size_t>(bytes, 1 << 16);
-  BK_CUDA(c, cudaMallocHost(ptr, room));
-  *cap = room;
-  return BK_OK;
+// Host memory of a run's uploads, kept warm between calls. Pageable: a small copy from
+// it is staged at once, and pinning memory costs milliseconds per context.
+char* stage(bk_ctx* c, size_t bytes) {
+  if (c->h_stage.size() < bytes) c->h_stage.resize(bytes);
+  return c->h_stage.data();
 }
-int ensure_stage(bk_ctx* c, size_t bytes) { return ensure_pinned(c, &c->h_stage, &c->stage_cap, bytes); }
+
+// One pinned room of 8 MB for the whole process, for the host arrays of large descent
+// batches: pinning it takes a millisecond or two, so it is not a context's own. One call
+// holds it at a time (another uses pageable memory meanwhile); it is taken on first use
+// and given back when the last context closes.
+class PinnedRoom {
+ public:
+  static constexpr size_t kBytes = (size_t)8 << 20;
+  void context_opened() {
+    std::lock_guard<std::mutex> l(m_);
+    ++contexts_;
+  }
+  void context_closed() {
+    std::lock_guard<std::mutex> l(m_);
+    if (--contexts_ == 0 && room_) {
+      cudaFreeHost(room_);
+      room_ = nullptr;
+    }
+  }
+  char* take(size_t bytes) {
+    std::lock_guard<std::mutex> l(m_);
+    if (bytes > kBytes || busy_) return nullptr;
+    if (!room_ && cudaHostAlloc(&room_, kBytes, cudaHostAllocPortable) != cudaSuccess) {
+      cudaGetLastError();
+      room_ = nullptr;
+      return nullptr;
+    }
+    busy_ = true;
+    return static_cast<char*>(room_);
+  }
+  void give_back() {
+    std::lock_guard<std::mutex> l(m_);
+    busy_ = false;
+  }
+
+ private:
+  std::mutex m_;
+  void* room_ = nullptr;
+  int contexts_ = 0;
+  bool busy_ = false;
+};
+PinnedRoom g_pinned;
+struct PinnedHold {  // the room for the length of a call
+  char* p;
+  explicit PinnedHold(size_t bytes) : p(g_pinned.take(bytes)) {}
+  PinnedHold(const PinnedHold&) = delete;
+  PinnedHold& operator=(const PinnedHold&) = delete;
+  ~PinnedHold() {
+    if (p) g_pinned.give_back();
+  }
+};
 
 struct AltGeo {
   int tb = 0, w2 = 0, w3 = 0;
@@ -1243,8 +1287,7 @@ int alt_prepare(bk_ctx* c, int n, uint64_t s0, int64_t e0, double angle_unit, co
   run->max_rows = (int)std::max<size_t>(kAltPartialBytes / row_bytes, 1);
   const size_t o_part = b.take(row_bytes * (size_t)std::max(1, std::min(S.n_meas, run->max_rows + 1)));
   BK_TRY(ensure_buffer(c, &c->d_alt, &c->alt_cap, b.off));
-  BK_TRY(ensure_stage(c, up));
-  char *h = static_cast<char*>(c->h_stage), *d = static_cast<char*>(c->d_alt);
+  char *h = stage(c, up), *d = static_cast<char*>(c->d_alt);
   alt_table(n, angle_unit, reinterpret_cast<entry*>(h + o_tab), D.c0, D.n_j);
   std::copy(tans.begin(), tans.end(), reinterpret_cast<R*>(h + o_tan));
   std::copy(scales.begin(), scales.end(), reinterpret_cast<R*>(h + o_sc));
@@ -1321,47 +1364,44 @@ int evolve_alt(bk_ctx* c, const bk_evolve_params* p, const Schedule& S, double a
 // ---------------------------------------------------------------------------
 // Tile by the element bits np: 16 elements a thread from 2^10 elements on, 8 below
 // (more warps; one warp up to 2^8, smaller states padded).
-template <class R>
 const void* small_kernel_of(int np, int* threads, int* tile_bytes) {
   *tile_bytes = 16 << std::max(np, 8);
   *threads = np >= 10 ? 1 << (np - 4) : 1 << (std::max(np, 8) - 3);
   switch (np) {
-    case 12: return reinterpret_cast<const void*>(small_kernel<R, 12, 4>);
-    case 11: return reinterpret_cast<const void*>(small_kernel<R, 11, 4>);
-    case 10: return reinterpret_cast<const void*>(small_kernel<R, 10, 4>);
-    case 9: return reinterpret_cast<const void*>(small_kernel<R, 9, 3>);
-    default: return reinterpret_cast<const void*>(small_kernel<R, 8, 3>);
+    case 12: return reinterpret_cast<const void*>(small_kernel<12, 4>);
+    case 11: return reinterpret_cast<const void*>(small_kernel<11, 4>);
+    case 10: return reinterpret_cast<const void*>(small_kernel<10, 4>);
+    case 9: return reinterpret_cast<const void*>(small_kernel<9, 3>);
+    default: return reinterpret_cast<const void*>(small_kernel<8, 3>);
   }
 }
 
-template <class R>
 int evolve_small(bk_ctx* c, const bk_evolve_params* p, const Schedule& S, double angle_unit,
-                 const std::vector<R>& tans, const std::vector<R>& scales) {
-  using entry = typename AltPhase<R>::entry;
-  using amp = typename AmpTraits<R>::amp;
-  const int n = p->n, np = sizeof(R) == 4 ? n - 1 : n, T = p->n_steps;
-  SmallRun<R> P{};
+                 const std::vector<double>& tans, const std::vector<double>& scales) {
+  using entry = double2;
+  using amp = double2;
+  const int n = p->n, np = n, T = p->n_steps;
+  SmallRun P{};
   const int n_j = alt_levels(n, &P.c0);
   Bump b;
   const size_t o_tab = b.take((size_t)(n_j + 1) * sizeof(entry));
-  const size_t o_step = b.take((size_t)(T + 1) * sizeof(SmallStep<R>));
+  const size_t o_step = b.take((size_t)(T + 1) * sizeof(SmallStep));
   const size_t up = b.off;
   int threads = 0, tile = 0;
-  const void* fn = small_kernel_of<R>(np, &threads, &tile);
+  const void* fn = small_kernel_of(np, &threads, &tile);
   const size_t o_part = b.take((size_t)std::max(S.n_meas, 1) * 3 * (threads / 32) * sizeof(double));
   BK_TRY(ensure_buffer(c, &c->d_small, &c->small_cap, b.off));
-  BK_TRY(ensure_stage(c, up));
-  char *h = static_cast<char*>(c->h_stage), *d = static_cast<char*>(c->d_small);
+  char *h = stage(c, up), *d = static_cast<char*>(c->d_small);
   alt_table(n, angle_unit, reinterpret_cast<entry*>(h + o_tab), P.c0, n_j);
   for (int k = 0; k <= T; ++k)
-    reinterpret_cast<SmallStep<R>*>(h + o_step)[k] = {k < T ? tans[(size_t)k] : (R)0, k < T ? scales[(size_t)k] : (R)1,
+    reinterpret_cast<SmallStep*>(h + o_step)[k] = {k < T ? tans[(size_t)k] : 0.0, k < T ? scales[(size_t)k] : 1.0,
                                                       S.slot[(size_t)k], 0};
   BK_CUDA(c, cudaMemcpyAsync(d, h, up, cudaMemcpyHostToDevice, c->stream));
   BK_TRY(allow_smem(c, fn, tile));
   P.state = reinterpret_cast<amp*>(c->d_state);
   P.E = c->d_E;
   P.tab = reinterpret_cast<const entry*>(d + o_tab);
-  P.step = reinterpret_cast<const SmallStep<R>*>(d + o_step);
+  P.step = reinterpret_cast<const SmallStep*>(d + o_step);
   P.partials = reinterpret_cast<double*>(d + o_part);
   P.results = c->d_results;
   P.np = np;
@@ -1426,17 +1466,6 @@ __global__ void set_basis_many_kernel(unsigned char* base, const unsigned long l
     reinterpret_cast<float*>(st)[4u * (s >> 1) + (s & 1u)] = 1.0f;
   else
     reinterpret_cast<double2*>(st)[s] = make_double2(1.0, 0.0);
-}
-
-// a host copy by several threads from 256 KB on (fresh pages of the destination fault in parallel)
-void copy_host(void* dst, const void* src, size_t bytes) {
-  constexpr size_t kPiece = (size_t)64 << 10;
-  const long long pieces = (long long)((bytes + kPiece - 1) / kPiece);
-#pragma omp parallel for schedule(static) if (bytes >= ((size_t)256 << 10))
-  for (long long i = 0; i < pieces; ++i) {
-    const size_t at = (size_t)i * kPiece;
-    std::memcpy(static_cast<char*>(dst) + at, static_cast<const char*>(src) + at, std::min(kPiece, bytes - at));
-  }
 }
 
 struct BatchGeo {
@@ -1529,8 +1558,7 @@ int batch_turning(bk_ctx* c, const std::vector<BatchGeo>& geo, int T, const std:
     part = std::max(part, (size_t)kv.second.groups * 2 * 3 * (size_t)std::max(n_meas, 1) * kv.second.G * sizeof(double));
   const size_t o_part = b.take(part);
   BK_TRY(ensure_buffer(c, &c->d_batch, &c->batch_cap, b.off));
-  BK_TRY(ensure_stage(c, up));
-  char *h = static_cast<char*>(c->h_stage), *d = static_cast<char*>(c->d_batch);
+  char *h = stage(c, up), *d = static_cast<char*>(c->d_batch);
   std::copy(tans.begin(), tans.end(), reinterpret_cast<R*>(h + o_tan));
   std::copy(scales.begin(), scales.end(), reinterpret_cast<R*>(h + o_scale));
   std::copy(slot.begin(), slot.end(), reinterpret_cast<int*>(h + o_slot));
@@ -1936,7 +1964,8 @@ int evolve_fused(bk_ctx* c, const bk_evolve_params* p, const Schedule& S, double
   }
   *final_log2 = lg;
 
-  if (n <= T) return evolve_small<R>(c, p, S, angle_unit, tans, scales);
+  if constexpr (sizeof(R) == 8)  // (complex64 runs of these sizes are complex128 ones: bk_evolve)
+    if (n <= T) return evolve_small(c, p, S, angle_unit, tans, scales);
   if (use_alt) return evolve_alt<R>(c, p, S, angle_unit, tans, scales);
   return evolve_persist<R>(c, p, S, angle_unit, tans, scales);
 }
@@ -2424,6 +2453,8 @@ int bk_create(int device, bk_ctx** out) {
   }
   cudaMemset(c->d_ticket, 0, sizeof(unsigned int));
   cudaMemset(c->d_err, 0, sizeof(int));
+  g_pinned.context_opened();
+  c->counted = true;
   *out = c;
   return BK_OK;
 }
@@ -2440,13 +2471,12 @@ int bk_destroy(bk_ctx* c) {
   for (void* p : {c->d_batch_state, c->d_batch, (void*)c->d_batch_results, c->d_persist, c->d_lam, c->d_ckpt,
                   c->d_adj, c->d_descent, c->d_lz, c->d_fsmap, c->d_alt})
     if (p) cudaFree(p);
-  for (void* p : {c->h_stage, c->h_out})
-    if (p) cudaFreeHost(p);
   for (auto& e : c->ev_pool) {
     cudaEventDestroy(e.first);
     cudaEventDestroy(e.second);
   }
   if (c->stream) cudaStreamDestroy(c->stream);
+  if (c->counted) g_pinned.context_closed();
   delete c;
   return BK_OK;
 }
@@ -2482,42 +2512,59 @@ int bk_steepest_descent_gpu(bk_ctx* c, int n, const uint64_t* starts, int64_t co
     return fail(c, BK_ERR_INVALID, "steepest descent: n = %d, count = %lld", n, (long long)count);
   if (count == 0) return BK_OK;
   BK_CUDA(c, cudaSetDevice(c->device));
-  const size_t cnt = (size_t)count;
-  BK_TRY(ensure_buffer(c, &c->d_descent, &c->descent_cap, cnt * 32));
-  uint64_t* d_start = static_cast<uint64_t*>(c->d_descent);
-  uint64_t* d_fs = d_start + cnt;
-  long long* d_fe = reinterpret_cast<long long*>(d_fs + cnt);
-  unsigned long long* d_ev = reinterpret_cast<unsigned long long*>(d_fe + cnt);
+  // The copies cost more than the descents (65536 starts of n = 28: 58 us of kernel, 210
+  // us of pageable copies of 8-byte words one array after another), so states up to 32
+  // spins, energies and evaluations cross as 4-byte words through pinned memory, the
+  // results in one copy, and the pages of the caller's arrays, mostly fresh ones, are
+  // touched while the GPU works. (Several threads would widen faster, but their idle
+  // spinning slows the host calls that follow.)
+  const size_t cnt = (size_t)count, word = n <= 32 ? 4 : 8;
+  const size_t need = cnt * (2 * word + 8) + 64;
+  BK_TRY(ensure_buffer(c, &c->d_descent, &c->descent_cap, need));
+  char* d = static_cast<char*>(c->d_descent);
+  const size_t o_fs = 0, o_fe = cnt * word, o_ev = o_fe + cnt * 4, o_st = (o_ev + cnt * 4 + 15) & ~(size_t)15;
   cudaStream_t st = c->stream;
-  // through pinned memory: a pageable copy is staged by the driver in one thread, and
-  // the callers' arrays are mostly fresh pages
-  // (65536 starts: 164 us in all against 267 us; up to 64 MB, the room stays with the context)
-  const bool pinned = cnt * 24 <= ((size_t)64 << 20);
-  if (pinned) {
-    BK_TRY(ensure_stage(c, cnt * 8));
-    BK_TRY(ensure_pinned(c, &c->h_out, &c->out_cap, cnt * 24));
-    copy_host(c->h_stage, starts, cnt * 8);
-  }
-  BK_CUDA(c, cudaMemcpyAsync(d_start, pinned ? c->h_stage : starts, cnt * 8, cudaMemcpyHostToDevice, st));
-  size_t e = 0;
-  BK_TRY(ev_begin(c, "descent", &e));
+  const unsigned long long budget = max_evals == 0 ? ~0ull : (unsigned long long)max_evals;
   const unsigned grid = (unsigned)((cnt + kDescentWarps - 1) / kDescentWarps);
-  (n <= 32 ? descent_kernel<1> : descent_kernel<2>)<<<grid, 32 * kDescentWarps, 0, st>>>(
-      n, d_start, (long long)count, max_evals == 0 ? ~0ull : (unsigned long long)max_evals, d_fs, d_fe, d_ev);
+  const size_t host_bytes = cnt * (word + 8);
+  std::vector<char> pageable;
+  PinnedHold pinned(host_bytes >= ((size_t)64 << 10) ? host_bytes : ~(size_t)0);
+  if (!pinned.p) pageable.resize(host_bytes);
+  char* h = pinned.p ? pinned.p : pageable.data();
+  size_t e = 0;
+  if (n <= 32) {
+    uint32_t* narrow = reinterpret_cast<uint32_t*>(h);
+    for (long long i = 0; i < (long long)cnt; ++i) narrow[i] = (uint32_t)starts[i];
+    BK_CUDA(c, cudaMemcpyAsync(d + o_st, narrow, cnt * 4, cudaMemcpyHostToDevice, st));
+  } else {
+    BK_CUDA(c, cudaMemcpyAsync(d + o_st, starts, cnt * 8, cudaMemcpyHostToDevice, st));
+  }
+  BK_TRY(ev_begin(c, "descent", &e));
+  if (n <= 32)
+    descent_kernel<1><<<grid, 32 * kDescentWarps, 0, st>>>(n, reinterpret_cast<const uint32_t*>(d + o_st), count, budget,
+                                                           reinterpret_cast<uint32_t*>(d + o_fs),
+                                                           reinterpret_cast<int*>(d + o_fe),
+                                                           reinterpret_cast<uint32_t*>(d + o_ev));
+  else
+    descent_kernel<2><<<grid, 32 * kDescentWarps, 0, st>>>(
+        n, reinterpret_cast<const unsigned long long*>(d + o_st), count, budget,
+        reinterpret_cast<unsigned long long*>(d + o_fs), reinterpret_cast<int*>(d + o_fe),
+        reinterpret_cast<uint32_t*>(d + o_ev));
   BK_CUDA(c, cudaGetLastError());
   BK_TRY(ev_end(c, e));
-  if (pinned) {
-    BK_CUDA(c, cudaMemcpyAsync(c->h_out, d_fs, cnt * 24, cudaMemcpyDeviceToHost, st));  // the three arrays lie together
-    BK_CUDA(c, cudaStreamSynchronize(st));
-    const char* h = static_cast<const char*>(c->h_out);
-    copy_host(fs, h, cnt * 8);
-    copy_host(fe, h + cnt * 8, cnt * 8);
-    if (ev) copy_host(ev, h + cnt * 16, cnt * 8);
-  } else {
-    BK_CUDA(c, cudaMemcpyAsync(fs, d_fs, cnt * 8, cudaMemcpyDeviceToHost, st));
-    BK_CUDA(c, cudaMemcpyAsync(fe, d_fe, cnt * 8, cudaMemcpyDeviceToHost, st));
-    if (ev) BK_CUDA(c, cudaMemcpyAsync(ev, d_ev, cnt * 8, cudaMemcpyDeviceToHost, st));
-    BK_CUDA(c, cudaStreamSynchronize(st));
+  if (pinned.p) BK_CUDA(c, cudaMemcpyAsync(h, d + o_fs, host_bytes, cudaMemcpyDeviceToHost, st));
+  for (void* out : {(void*)fs, (void*)fe, (void*)ev})
+    for (size_t at = 0; out && at < cnt * 8; at += 4096) static_cast<volatile char*>(out)[at] = 0;
+  if (!pinned.p) BK_CUDA(c, cudaMemcpyAsync(h, d + o_fs, host_bytes, cudaMemcpyDeviceToHost, st));
+  BK_CUDA(c, cudaStreamSynchronize(st));
+  const uint32_t* w_fs = reinterpret_cast<const uint32_t*>(h + o_fs);
+  const uint64_t* l_fs = reinterpret_cast<const uint64_t*>(h + o_fs);
+  const int* w_fe = reinterpret_cast<const int*>(h + o_fe);
+  const uint32_t* w_ev = reinterpret_cast<const uint32_t*>(h + o_ev);
+  for (long long i = 0; i < (long long)cnt; ++i) {
+    fs[i] = word == 4 ? w_fs[i] : l_fs[i];
+    fe[i] = w_fe[i];
+    if (ev) ev[i] = w_ev[i];
   }
   BK_TRY(collect_timing(c));
   return BK_OK;
@@ -2773,11 +2820,20 @@ int bk_evolve(bk_ctx* c, const bk_evolve_params* p, double* p_less, double* d_h,
   bk_evolve_params q = *p;
   q.e0 = e0;
   const double angle_unit = (p->diag_scale > 0.0) ? p->dt * p->diag_scale : p->dt / (double)n;
+  // Small complex64 runs compute in complex128: up to 18 qubits a step is latency, not
+  // arithmetic or bandwidth (us a step, complex64 / complex128 kernels: N = 9 0.66 /
+  // 0.61, 14 3.9 / 3.5, 16 4.6 / 3.9, 18 5.1 / 5.1, 19 5.7 / 8.0), and the results are
+  // the exact ones to 1e-13 instead of a random walk of FP32 roundings.
+  if (p->method == BK_FUSED && p->precision == BK_C64) BK_TRY(check_phase<float>(c, n, angle_unit));
+  if (p->precision == BK_C64 && p->method == BK_FUSED &&
+      (n <= 13 || (n <= 18 && c->engine_mode == 4 && c->e_recompute == 0)))
+    q.precision = BK_C128;
+  const int prec = q.precision;
 
   BK_CUDA(c, cudaSetDevice(c->device));
   BK_TRY(ensure_energy(c, n));
-  BK_TRY(ensure_state(c, n, p->precision));
-  const int T = tile_bits(p->precision);
+  BK_TRY(ensure_state(c, n, prec));
+  const int T = tile_bits(prec);
   const size_t grid = (n > T) ? (1ull << (n - T)) : 1;
   BK_TRY(ensure_buffer(c, reinterpret_cast<void**>(&c->d_partials), &c->partials_cap,
                        3 * std::max<size_t>(grid, kMeasureGrid) * sizeof(double)));
@@ -2794,14 +2850,14 @@ int bk_evolve(bk_ctx* c, const bk_evolve_params* p, double* p_less, double* d_h,
   if (!small) {
     BK_CUDA(c, cudaMemsetAsync(c->d_ticket, 0, sizeof(unsigned int), c->stream));
     BK_CUDA(c, cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
-    BK_CUDA(c, cudaMemsetAsync(c->d_state, 0, (1ull << n) * amp_bytes(p->precision), c->stream));
+    BK_CUDA(c, cudaMemsetAsync(c->d_state, 0, (1ull << n) * amp_bytes(prec), c->stream));
   }
   const uint32_t s0 = (uint32_t)(p->s0 & ((1ull << n) - 1ull));
-  c->planar = (p->precision == BK_C64 && p->method == BK_FUSED && n > 13);
+  c->planar = (prec == BK_C64 && p->method == BK_FUSED && n > 13);
   if (small) {
   } else if (c->planar)
     set_basis_planar_kernel<<<1, 1, 0, c->stream>>>(reinterpret_cast<float*>(c->d_state), s0);
-  else if (p->precision == BK_C64)
+  else if (prec == BK_C64)
     set_basis_kernel<float2><<<1, 1, 0, c->stream>>>(reinterpret_cast<float2*>(c->d_state), s0);
   else
     set_basis_kernel<double2><<<1, 1, 0, c->stream>>>(reinterpret_cast<double2*>(c->d_state), s0);
@@ -2816,30 +2872,27 @@ int bk_evolve(bk_ctx* c, const bk_evolve_params* p, double* p_less, double* d_h,
     else
       BK_TRY(evolve_plain<double>(c, &q, S, angle_unit));
   } else {
-    if (p->precision == BK_C64)
+    if (prec == BK_C64)
       BK_TRY(evolve_fused<float>(c, &q, S, angle_unit, &row_log2, &final_log2));
     else
       BK_TRY(evolve_fused<double>(c, &q, S, angle_unit, &row_log2, &final_log2));
   }
-  // the rows and the error word come back through pinned memory, behind one wait
-  const size_t row_bytes = 4 * (size_t)S.n_meas * sizeof(double);
-  BK_TRY(ensure_pinned(c, &c->h_out, &c->out_cap, row_bytes + sizeof(int)));
-  const double* rows = static_cast<const double*>(c->h_out);
-  int* h_err = reinterpret_cast<int*>(static_cast<char*>(c->h_out) + row_bytes);
-  *h_err = 0;
+  std::vector<double> rows(4 * (size_t)S.n_meas);
+  int err = 0;
   if (S.n_meas > 0)
-    BK_CUDA(c, cudaMemcpyAsync(c->h_out, c->d_results, row_bytes, cudaMemcpyDeviceToHost, c->stream));
-  if (!small) BK_CUDA(c, cudaMemcpyAsync(h_err, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    BK_CUDA(c, cudaMemcpyAsync(rows.data(), c->d_results, rows.size() * sizeof(double), cudaMemcpyDeviceToHost,
+                               c->stream));
+  if (!small) BK_CUDA(c, cudaMemcpyAsync(&err, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   if (S.n_pts > 0)
     BK_CUDA(c, cudaMemcpyAsync(p->samples_out, c->d_samples, (size_t)S.n_pts * S.shots * sizeof(uint64_t),
                                cudaMemcpyDeviceToHost, c->stream));
   BK_CUDA(c, cudaStreamSynchronize(c->stream));
-  BK_TRY(device_error(c, *h_err));
+  BK_TRY(device_error(c, err));
   BK_TRY(collect_timing(c));
   c->have_state = true;
   c->last_planar = c->planar;
   c->last_n = n;
-  c->last_prec = p->precision;
+  c->last_prec = prec;
   c->last_ordering = p->ordering;
   c->last_log2_scale = final_log2;
   c->last_angle_unit = angle_unit;

@@ -1,5 +1,5 @@
-// Small statevectors (complex64 up to 13 qubits, complex128 up to 12: at most 2^12
-// 16-byte elements): every step of a run in one CTA, the state in registers.
+// Small statevectors (up to 12 qubits, complex128 — complex64 runs of these sizes
+// compute in it too): every step of a run in one CTA, the state in registers.
 //
 // The element bits are split over the three rounds of a turning-pass tile
 // (bk_alt.cuh). A step goes through the rounds once and the next one comes back:
@@ -11,28 +11,26 @@
 // layouts' stay in registers, so D needs no energies and no table.
 //
 // Bound by FP64 arithmetic and the shared-memory pipe of the one SM at N = 12
-// complex128, by instruction latency at the smallest sizes. Measured on a B200 (a
-// step without / with measurement): N = 12 complex128 1.9 / 2.5 us, N = 9
-// complex64 0.7 / 1.1 us; the former kernel, a shared-memory round trip and a CTA barrier per qubit,
-// took 11.0 us and 2.6 us.
+// and by instruction latency at the smallest sizes. Measured on a B200 (a step without
+// / with measurement): N = 12 1.8 / 2.5 us, N = 9 0.6 / 0.9 us; the former kernel, a
+// shared-memory round trip and a CTA barrier per qubit, took 11.0 us at N = 12 and
+// 2.6 us at N = 9 in complex64.
 #pragma once
 #include "bk_alt.cuh"
 
 namespace bk {
 
 // what step k needs: read one step ahead, so no step waits for it
-template <class R>
 struct alignas(16) SmallStep {
-  R tan, scale;
+  double tan, scale;
   int slot;  // measurement row, or -1
   int pad;
 };
-template <class R>
 struct SmallRun {
-  typename AmpTraits<R>::amp* state;
+  double2* state;
   const uint16_t* E;
-  const typename AltPhase<R>::entry* tab;  // entry 0: no rotation, 1 + j: level c0 + 4 j
-  const SmallStep<R>* step;  // [steps + 1]
+  const double2* tab;  // entry 0: no rotation, 1 + j: level c0 + 4 j
+  const SmallStep* step;  // [steps + 1]
   double* partials;    // [rows][warps][3]
   double* results;     // [rows][4]
   int np;              // element bits (TB = 8: at most 8, the others dummies)
@@ -44,60 +42,11 @@ struct SmallRun {
   uint32_t s0;
 };
 
-// an element in the amplitude order of the small states' buffer
-__device__ __forceinline__ El<float>::T small_ld(const float2* s, uint32_t el) {
-  const float4 q = reinterpret_cast<const float4*>(s)[el];
-  return El<float>::T{make_float2(q.x, q.z), make_float2(q.y, q.w)};
-}
-__device__ __forceinline__ void small_st(float2* s, uint32_t el, const El<float>::T& v) {
-  reinterpret_cast<float4*>(s)[el] = make_float4(v.re.x, v.im.x, v.re.y, v.im.y);
-}
-__device__ __forceinline__ El<double>::T small_ld(const double2* s, uint32_t el) { return El<double>::T{s[el]}; }
-__device__ __forceinline__ void small_st(double2* s, uint32_t el, const El<double>::T& v) { s[el] = v.v; }
-// the basis state s0
-__device__ __forceinline__ void small_basis(El<float>::T& v, uint32_t el, uint32_t s0) {
-  v.re = make_float2(2u * el == s0 ? 1.f : 0.f, 2u * el + 1u == s0 ? 1.f : 0.f);
-  v.im = make_float2(0.f, 0.f);
-}
-__device__ __forceinline__ void small_basis(El<double>::T& v, uint32_t el, uint32_t s0) {
-  v.v = make_double2(el == s0 ? 1.0 : 0.0, 0.0);
-}
-
-// the phase of an element, ready to apply
-template <class R>
-struct SmallPhase;
-template <>
-struct SmallPhase<float> {
-  float2 a, b;
-  __device__ void set(const uint16_t* E, const float2* tab, uint32_t el, int c0, int e0, uint32_t& below, int j) {
-    const uint32_t e2 = reinterpret_cast<const uint32_t*>(E)[el], ea = e2 & 0xFFFFu, eb = e2 >> 16;
-    const float2 p = tab[1u + ((ea - (uint32_t)c0) >> 2)], q = tab[1u + ((eb - (uint32_t)c0) >> 2)];
-    a = make_float2(p.x, q.x);
-    b = make_float2(p.y, q.y);
-    below |= ((int)ea < e0 ? 1u : 0u) << (2 * j) | ((int)eb < e0 ? 2u : 0u) << (2 * j);
-  }
-  __device__ void apply(El<float>::T& v) const {
-    PhaseV<float>::shear2(v.re, v.im, a, b);
-    PhaseV<float>::shear2(v.re, v.im, a, b);
-  }
-};
-template <>
-struct SmallPhase<double> {
-  double2 cs;
-  __device__ void set(const uint16_t* E, const double2* tab, uint32_t el, int c0, int e0, uint32_t& below, int j) {
-    const uint32_t e = E[el];
-    cs = tab[1u + ((e - (uint32_t)c0) >> 2)];
-    below |= ((int)e < e0 ? 1u : 0u) << j;
-  }
-  __device__ void apply(El<double>::T& v) const {
-    v.v = make_double2(fma(v.v.x, cs.x, -v.v.y * cs.y), fma(v.v.x, cs.y, v.v.y * cs.x));
-  }
-};
-
-template <class R, int TB, int KB>
+template <int TB, int KB>
 struct SmallCta {
   using PL = AltPlan<TB, KB>;
-  using V = typename El<R>::T;
+  using R = double;
+  using V = El<R>::T;
   static constexpr int N = 1 << KB;
 
   // the rotations of round r's bits (TB = 8: those below np)
@@ -121,19 +70,10 @@ struct SmallCta {
     for (int j = 0; j < N; ++j) {
       const uint32_t el = pos | ((uint32_t)j << lo);
       const int q = j & 1;
-      if constexpr (sizeof(R) == 4) {
-        const uint32_t d = (el << 1) ^ s0;
-        const double w0 = (double)fmaf(v[j].re.x, v[j].re.x, v[j].im.x * v[j].im.x);
-        const double w1 = (double)fmaf(v[j].re.y, v[j].re.y, v[j].im.y * v[j].im.y);
-        n[q] += w0 + w1;
-        b[q] += ((below >> (2 * j)) & 1u ? w0 : 0.0) + ((below >> (2 * j + 1)) & 1u ? w1 : 0.0);
-        f[q] += fma(w0, alt_small(__popc(d)), w1 * alt_small(__popc(d ^ 1u)));
-      } else {
-        const double w = fma(v[j].v.x, v[j].v.x, v[j].v.y * v[j].v.y);
-        n[q] += w;
-        b[q] += (below >> j) & 1u ? w : 0.0;
-        f[q] = fma(w, alt_small(__popc(el ^ s0)), f[q]);
-      }
+      const double w = fma(v[j].v.x, v[j].v.x, v[j].v.y * v[j].v.y);
+      n[q] += w;
+      b[q] += (below >> j) & 1u ? w : 0.0;
+      f[q] = fma(w, alt_small(__popc(el ^ s0)), f[q]);
     }
     const double x = warp_sum(n[0] + n[1]), y = warp_sum(b[0] + b[1]), z = warp_sum(f[0] + f[1]);
     if ((threadIdx.x & 31u) == 0) {
@@ -144,9 +84,10 @@ struct SmallCta {
   }
 };
 
-template <class R, int TB, int KB>
-__global__ void __launch_bounds__(AltPlan<TB, KB>::kThreads, 1) small_kernel(const __grid_constant__ SmallRun<R> P) {
-  using C = SmallCta<R, TB, KB>;
+template <int TB, int KB>
+__global__ void __launch_bounds__(AltPlan<TB, KB>::kThreads, 1) small_kernel(const __grid_constant__ SmallRun P) {
+  using R = double;
+  using C = SmallCta<TB, KB>;
   using PL = typename C::PL;
   constexpr int N = C::N, L0 = PL::reg_lo(0);
   extern __shared__ __align__(128) unsigned char tile[];
@@ -155,17 +96,20 @@ __global__ void __launch_bounds__(AltPlan<TB, KB>::kThreads, 1) small_kernel(con
                  b2 = PL::template base<2>(lane, warp);
   const uint32_t size = TB > 8 ? 1u << TB : 1u << P.np;
   typename El<R>::T v[N];
-  SmallPhase<R> p0[N], p2[N];
+  double2 p0[N], p2[N];  // (cos, sin) of the elements' phases in round 0's and round 2's layout
   uint32_t below0 = 0u, below2 = 0u;
 #pragma unroll
   for (int j = 0; j < N; ++j) {
     const uint32_t el0 = b0 | ((uint32_t)j << L0), el2 = b2 | (uint32_t)j;
-    p0[j].set(P.E, P.tab, TB > 8 ? el0 : el0 & (size - 1u), P.c0, P.e0, below0, j);
-    p2[j].set(P.E, P.tab, TB > 8 ? el2 : el2 & (size - 1u), P.c0, P.e0, below2, j);
-    small_basis(v[j], el0, P.s0);
-    if (!P.init && (TB > 8 || el0 < size)) v[j] = small_ld(P.state, el0);
+    const int ea = P.E[TB > 8 ? el0 : el0 & (size - 1u)], eb = P.E[TB > 8 ? el2 : el2 & (size - 1u)];
+    p0[j] = P.tab[1 + ((ea - P.c0) >> 2)];
+    p2[j] = P.tab[1 + ((eb - P.c0) >> 2)];
+    below0 |= (ea < P.e0 ? 1u : 0u) << j;
+    below2 |= (eb < P.e0 ? 1u : 0u) << j;
+    v[j].v = make_double2(el0 == P.s0 ? 1.0 : 0.0, 0.0);
+    if (!P.init && (TB > 8 || el0 < size)) v[j].v = P.state[el0];
   }
-  SmallStep<R> now = P.step[P.k0];
+  SmallStep now = P.step[P.k0];
   if (!P.meas_first) now.slot = -1;
   auto row_of = [&](int slot) { return P.partials + 3 * ((size_t)(slot - P.row0) * PL::kWarps + warp); };
   uint32_t el_last = 0u;
@@ -180,8 +124,8 @@ __global__ void __launch_bounds__(AltPlan<TB, KB>::kThreads, 1) small_kernel(con
       now = P.step[k + 1];
 #pragma unroll
       for (int j = 0; j < N; ++j) {
-        p0[j].apply(v[j]);
-        El<R>::bfly_inner(v[j], t);
+        const double2 x = v[j].v;
+        v[j].v = make_double2(fma(x.x, p0[j].x, -x.y * p0[j].y), fma(x.x, p0[j].y, x.y * p0[j].x));
       }
       if (sc != (R)1) {
 #pragma unroll
@@ -206,8 +150,8 @@ __global__ void __launch_bounds__(AltPlan<TB, KB>::kThreads, 1) small_kernel(con
       now = P.step[k + 2];
 #pragma unroll
       for (int j = 0; j < N; ++j) {
-        p2[j].apply(v[j]);
-        El<R>::bfly_inner(v[j], t);
+        const double2 x = v[j].v;
+        v[j].v = make_double2(fma(x.x, p2[j].x, -x.y * p2[j].y), fma(x.x, p2[j].y, x.y * p2[j].x));
       }
       if (sc != (R)1) {
 #pragma unroll
@@ -227,7 +171,7 @@ __global__ void __launch_bounds__(AltPlan<TB, KB>::kThreads, 1) small_kernel(con
 #pragma unroll
   for (int j = 0; j < N; ++j) {
     const uint32_t el = el_last | ((uint32_t)j << lo_last);
-    if (TB > 8 || el < size) small_st(P.state, el, v[j]);
+    if (TB > 8 || el < size) P.state[el] = v[j].v;
   }
   __syncthreads();  // the partial rows of every warp
   for (int row = (int)threadIdx.x; row < P.rows; row += PL::kThreads) {

@@ -75,16 +75,19 @@ def test_sampling_points_do_not_change_the_series(eng, n, precision):
 @pytest.mark.parametrize("precision,ns", [(bk.BK_C64, [14, 19, 20, 21, 22, 24, 16, 16]), (bk.BK_C128, [13, 18, 19, 21, 22, 13]),
                                           (bk.BK_C64, [17] * 33)])
 def test_batch_matches_single_runs(eng, precision, ns):
-    """Groups of CTAs, one statevector each in turn: the states are those of the single
-    runs (sums over other CTA shares, so FP64 rounding apart)."""
+    """Groups of CTAs, one statevector each in turn: complex128, and complex64 from 19
+    qubits on, have the single runs' states (sums over other CTA shares, so FP64 rounding
+    apart); smaller complex64 single runs compute in complex128."""
     eng.set_option("engine_mode", 4)
     inst = [dict(n=n, s0=bk.select_trap(n, 30 + i, 40, 0.5)[0], g=0.2 + 0.01 * i) for i, n in enumerate(ns)]
     steps, meas = 9, [0, 1, 5, 9]
     p, d, nn = eng.evolve_batch(inst, 0.04, steps, measure=meas, precision=precision)
     for i, x in enumerate(inst):
         q, e, m = eng.evolve(x["n"], x["s0"], x["g"], 0.04, steps, measure=meas, precision=precision)
-        assert np.max(np.abs(p[i] - q)) <= BAR128 and np.max(np.abs(nn[i] - m)) <= BAR128
-        assert np.max(np.abs(d[i] - e)) <= BAR128 * x["n"]
+        same = precision == bk.BK_C128 or x["n"] >= 19
+        assert np.max(np.abs(p[i] - q)) <= (BAR128 if same else C64_DP_BAR)
+        assert np.max(np.abs(d[i] - e)) <= (BAR128 * x["n"] if same else C64_DH_BAR)
+        assert np.max(np.abs(nn[i] - m)) <= (BAR128 if same else 1e-5)
 
 
 def test_wait_limit_is_an_error_not_a_hang(eng):
@@ -109,8 +112,6 @@ def test_wait_limit_is_an_error_not_a_hang(eng):
 @pytest.mark.parametrize("n", [1, 2, 3, 8, 9, 10, 11, 12, 13])
 @pytest.mark.parametrize("steps", [0, 1, 6, 7])
 def test_small_states_match_the_plain_path(eng, n, precision, steps):
-    if n == 13 and precision == bk.BK_C128:
-        pytest.skip("13 qubits in complex128 run in tiles")
     s0, g = (0b1011001110101 & ((1 << n) - 1)), np.linspace(0.3, 0.5, steps)
     a = eng.evolve(n, s0, g, 0.05, steps, precision=precision)
     psi = eng.export_state(n)
@@ -119,8 +120,7 @@ def test_small_states_match_the_plain_path(eng, n, precision, steps):
     c64 = precision == bk.BK_C64
     assert np.max(np.abs(a[0] - b[0])) <= (C64_DP_BAR if c64 else BAR128)
     assert np.max(np.abs(a[1] - b[1])) <= (C64_DH_BAR if c64 else BAR128 * n)
-    # complex64: 7 steps of at most 20 roundings of 6e-8 on amplitudes up to 1
-    assert np.max(np.abs(psi - ref)) <= (1e-5 if c64 else BAR128)
+    assert np.max(np.abs(psi - ref)) <= BAR128  # complex64 runs of these sizes compute in complex128
 
 
 @pytest.mark.parametrize("n", [5, 9, 12])
