@@ -130,6 +130,19 @@ __device__ __forceinline__ void st_global_hint(void* p, double2 v, uint64_t poli
                : "memory");
 }
 
+__device__ __forceinline__ void st_global_hint(double* p, double v, uint64_t policy) {
+  asm volatile("st.global.L2::cache_hint.f64 [%0], %1, %2;" ::"l"(p), "d"(v), "l"(policy) : "memory");
+}
+// bulk_load with an L2 cache-policy hint
+__device__ __forceinline__ void bulk_load_hint(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar,
+                                               uint64_t policy) {
+  asm volatile(
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::"r"(
+          dst),
+      "l"(src), "r"(bytes), "r"(bar), "l"(policy)
+      : "memory");
+}
+
 // LABS energy (reference: src/labs_energy/labs_energy.hpp:121-132, and the device
 // form src/sampling/sampler.cuh:54-70), exact in integers.
 __device__ __forceinline__ int labs_energy(uint32_t x, int n) {

@@ -125,7 +125,7 @@ struct bk_ctx {
   size_t ckpt_cap = 0;
   void* d_adj = nullptr;      // adjoint: maps, descriptor, per-step arrays, partials
   size_t adj_cap = 0;
-  void* d_fsmap = nullptr;    // full-space strided pass: the tensor map of x (device memory, 64-byte aligned)
+  void* d_fsmap = nullptr;    // full-space tile passes: slab counters
   size_t fsmap_cap = 0;
   void* d_descent = nullptr;  // batched steepest descent: starts, final states, energies, evaluations
   size_t descent_cap = 0;
@@ -3372,11 +3372,56 @@ int bk_sample(bk_ctx* c, const double* randnums, int64_t shots, uint64_t* out) {
 // ---------------------------------------------------------------------------
 namespace {
 
-// n < 13: one CTA over the whole vector; else the block pass over index bits
-// [0, min(n, 23)) and, for n > 23, one strided tile pass over bits [23, n)
-// (w = n - 23 <= 7 bits, runs of 2^(13 - w) >= 64 doubles)
+// Product in tile passes, one launch (fs_turn_kernel): from 23 bits on (B200, us a call,
+// block pass / tile passes: n = 22 66 / 68, 23 113 / 110, 24 269 / 188, 27 1819 / 1272).
+constexpr int kFsTurnBits = 23;
+int fs_turn(bk_ctx* c, int n, double g, double scale, const double* x, double* y) {
+  const int r = n - kFsTileBits;  // index bits above the contiguous tile: 4 to 9 to each S set
+  const int w2 = r <= 9 ? 0 : std::min(r / 2, r > 16 ? 8 : 7), w1 = r - w2;
+  FtParams P{};
+  TmaDesc m1, m2;
+  BK_TRY(build_amp_map(c, const_cast<double*>(x), n, BK_C64, kFsTileBits - w1, kFsTileBits, w1, &m1));
+  if (w2 > 0) BK_TRY(build_amp_map(c, const_cast<double*>(x), n, BK_C64, kFsTileBits - w2, kFsTileBits + w1, w2, &m2));
+  P.map1 = m1.map;
+  P.map2 = w2 > 0 ? m2.map : m1.map;
+  P.mid1 = m1.mid_dim;
+  P.hi1 = m1.hi_dim;
+  P.mid2 = w2 > 0 ? m2.mid_dim : -1;
+  P.hi2 = w2 > 0 ? m2.hi_dim : -1;
+  P.x = x;
+  P.y = y;
+  P.E = c->d_E;
+  P.scale = scale;
+  P.g = g;
+  P.w1 = w1;
+  P.w2 = w2;
+  P.tiles = 1u << r;
+  P.slabs = 1u << w2;
+  // 2 lag 2^w1 tasks lie between a slab's A tiles and its S1 tiles: one and a half per CTA
+  // or more, so that the A tiles are done, but no more of x and y than L2 keeps (n = 28,
+  // lag 1 / 3: 2.60 / 2.94 ms)
+  P.lag = std::min<uint32_t>(P.slabs, std::max<uint32_t>(1u, ((uint32_t)c->num_sms * 3u / 2u + (1u << w1) - 1u) >> w1));
+  BK_TRY(ensure_buffer(c, &c->d_fsmap, &c->fsmap_cap, (P.slabs + 8) * sizeof(unsigned int)));
+  BK_CUDA(c, cudaMemsetAsync(c->d_fsmap, 0, (P.slabs + 8) * sizeof(unsigned int), c->stream));
+  P.done = static_cast<unsigned int*>(c->d_fsmap);
+  P.arrived = P.done + P.slabs;
+  P.abort = reinterpret_cast<int*>(P.done + P.slabs + 1);
+  P.err = c->d_err;
+  P.poll_limit = c->wait_polls > 0 ? c->wait_polls : kWaitPolls * 4u;
+  const void* fn = reinterpret_cast<const void*>(fs_turn_kernel);
+  BK_TRY(allow_smem(c, fn, kFtSmem));
+  size_t ev = 0;
+  BK_TRY(ev_begin(c, "fs_turn", &ev));
+  void* args[] = {&P};
+  BK_CUDA(c, cudaLaunchCooperativeKernel(fn, dim3(std::min<uint32_t>(2u * (uint32_t)c->num_sms, P.tiles)), dim3(kFtThreads),
+                                         args, (size_t)kFtSmem, c->stream));
+  return ev_end(c, ev);
+}
+
+// n < 13: one CTA over the whole vector; up to 22 bits the block pass, then tile passes
 int fs_matvec(bk_ctx* c, int n, double g, double scale, const double* x, double* y) {
   BK_TRY(ensure_energy(c, n));
+  if (n >= kFsTurnBits) return fs_turn(c, n, g, scale, x, y);
   const int tile_bytes = (1 << kFsTileBits) * (int)sizeof(double);
   size_t ev = 0;
   BK_TRY(ev_begin(c, n < kFsTileBits ? "fs_pass" : "fs_block", &ev));
@@ -3389,29 +3434,10 @@ int fs_matvec(bk_ctx* c, int n, double g, double scale, const double* x, double*
     return BK_OK;
   }
   BK_TRY(allow_smem(c, reinterpret_cast<const void*>(fs_block_kernel), tile_bytes));
-  BK_TRY(allow_smem(c, reinterpret_cast<const void*>(fs_tile_kernel), kFsTileSmem));
   const uint32_t tiles = 1u << (n - kFsTileBits);
-  fs_block_kernel<<<tiles, kFsThreads, tile_bytes, c->stream>>>(x, y, c->d_E, scale, g, std::min(n, kFsGatherBits),
-                                                                c->d_err);
+  fs_block_kernel<<<tiles, kFsThreads, tile_bytes, c->stream>>>(x, y, c->d_E, scale, g, n, c->d_err);
   BK_CUDA(c, cudaGetLastError());
-  BK_TRY(ev_end(c, ev));
-  if (n > kFsGatherBits) {
-    const int w = n - kFsGatherBits, cp = kFsTileBits - w, h0 = kFsGatherBits;
-    // x as 2^n doubles (8-byte TMA elements): runs of 2^cp, 2^w of them 2^h0 apart, tiles over bits [cp, h0)
-    TmaDesc xm;
-    BK_TRY(build_amp_map(c, const_cast<double*>(x), n, BK_C64, cp, h0, w, &xm));
-    if (xm.hi_dim >= 0 || (int)xm.mid_bits != h0 - cp)
-      return fail(c, BK_ERR_UNSUPPORTED, "full-space strided pass: tile geometry for n = %d", n);
-    BK_TRY(ensure_buffer(c, &c->d_fsmap, &c->fsmap_cap, sizeof(CUtensorMap)));
-    BK_CUDA(c, cudaMemcpyAsync(c->d_fsmap, &xm.map, sizeof(CUtensorMap), cudaMemcpyHostToDevice, c->stream));
-    BK_TRY(ev_begin(c, "fs_tile", &ev));
-    fs_tile_kernel<<<tiles, kFsThreads, kFsTileSmem, c->stream>>>(static_cast<const CUtensorMap*>(c->d_fsmap), y,
-                                                                   c->d_E, scale, g, cp, h0, h0 - cp,
-                                                                  xm.mid_dim, xm.hi_dim, 0, cp, c->d_err);
-    BK_CUDA(c, cudaGetLastError());
-    BK_TRY(ev_end(c, ev));
-  }
-  return BK_OK;
+  return ev_end(c, ev);
 }
 
 // the bounded waits' error word, cleared before and read after a full-space call
