@@ -6,14 +6,11 @@
 // (fullspace_matvec_kernel_d, :60-77). On a B200 the 126 MB L2 already serves
 // that form's neighbours up to ~2^23 states away, and the DRAM cost is the far
 // neighbours. Here one product is:
-//   block pass (fs_block_kernel): 8192-state blocks, the block of x staged in
-//     shared memory by a bulk copy for the 13 low-bit neighbours, bits 13..22 as
-//     coalesced sweeps of the partner blocks (L2 hits: partners <= 32 MB away),
-//     the diagonal from the cached uint16 E table, y stored streaming;
-//   strided pass (fs_tile_kernel, n > 23): tiles of index bits [0, 13 - w) u
-//     [23, n), w = n - 23 <= 7 (runs of >= 64 doubles) loaded as one tensor-map
-//     box, y -= g sum x[i ^ 2^j] for the far bits with every partner inside the tile.
-// DRAM per state: x, E, y once (18 B) plus x, y, y (24 B) for the far bits.
+//   up to 22 bits a block pass (fs_block_kernel): 8192-state blocks, the block of x
+//     staged in shared memory by a bulk copy for the 13 low-bit neighbours, the others
+//     as coalesced sweeps of the partner blocks (L2 hits), the diagonal from the cached
+//     uint16 E table;
+//   beyond, tile passes in one launch (fs_turn_kernel).
 //
 // Lanczos steps (the driver's cuBLAS calls, :437-482) are fused element-wise
 // kernels with per-block partial sums reduced in a fixed order (deterministic).
@@ -54,74 +51,11 @@ __global__ void __launch_bounds__(kFsThreads) fs_pass_kernel(const double* __res
 
 
 constexpr int kFsPer = (1 << kFsTileBits) / kFsThreads;  // 32 tile positions per thread
-constexpr int kFsTileSmem = (1 << kFsTileBits) * (int)sizeof(double) + 128;  // strided pass: tile + alignment slack
-
-// A neighbour-sum pass over a full 8192-double tile (the strided pass): the tile
-// of x arrives as ONE tensor-map box (runs of 2^cp contiguous doubles, 2^w of
-// them 2^h0 doubles apart) while every thread prefetches its 32 values of y (or
-// of scale * E when first) into registers, so each SM keeps > 100 KB of loads in
-// flight; then the neighbour sums over tile bits [act_lo, 13) are read from
-// shared memory. (One bulk copy per run was measured 3-5x slower per byte than
-// one box for runs of a few hundred bytes.)
-__global__ void __launch_bounds__(kFsThreads, 2) fs_tile_kernel(const CUtensorMap* __restrict__ xmap,
-                                                                double* __restrict__ y,
-                                                                const uint16_t* __restrict__ E, double scale, double g,
-                                                                int cp, int h0, int mb, int md, int hd, int first,
-                                                                int act_lo, int* err) {
-  // the tensor copy's destination must sit on a 128-byte boundary: the dynamic
-  // area gets 128 bytes of slack (kFsTileSmem) and the tile is aligned here
-  extern __shared__ __align__(128) unsigned char fs_raw[];
-  double* ft = reinterpret_cast<double*>(fs_raw + ((128u - (smem_addr(fs_raw) & 127u)) & 127u));
-  __shared__ __align__(8) uint64_t bar;
-  const uint32_t tid = threadIdx.x, tile = blockIdx.x;
-  if ((smem_addr(ft) & 127u) != 0u) {  // cannot happen after the alignment above; never issue a misaligned copy
-    if (tid == 0) atomicCAS(err, 0, DEV_BAD_LAUNCH);
-    return;
-  }
-  const int w = kFsTileBits - cp;
-  const uint32_t mid = tile & ((1u << mb) - 1u), hi = tile >> mb;
-  const uint64_t base = ((uint64_t)mid << cp) | ((uint64_t)hi << (h0 + w));
-  const uint32_t lo_mask = (1u << cp) - 1u;
-  const uint32_t fb = smem_addr(&bar);
-  if (tid == 0) {
-    mbar_init(fb, 1);
-    fence_barrier_init();
-    mbar_arrive_expect_tx(fb, 8u << kFsTileBits);
-    tma_load_5d_hint(smem_addr(ft), xmap, tile_coord(0, md, (int)mid, hd, (int)hi),
-                     tile_coord(1, md, (int)mid, hd, (int)hi), tile_coord(2, md, (int)mid, hd, (int)hi),
-                     tile_coord(3, md, (int)mid, hd, (int)hi), tile_coord(4, md, (int)mid, hd, (int)hi), fb,
-                     policy_evict_first());
-  }
-  // no thread may poll the barrier before thread 0 has initialised it
-  __syncthreads();
-  double pre[kFsPer];
-#pragma unroll
-  for (int k = 0; k < kFsPer; ++k) {
-    const uint32_t p = tid + kFsThreads * (uint32_t)k;
-    const uint64_t gi = base | (p & lo_mask) | ((uint64_t)(p >> cp) << h0);
-    pre[k] = first ? scale * (double)E[gi] : y[gi];
-  }
-  const bool ok = mbar_wait_bounded(fb, 0, err);
-  if (__syncthreads_or(!ok)) return;
-#pragma unroll
-  for (int k = 0; k < kFsPer; ++k) {
-    const uint32_t p = tid + kFsThreads * (uint32_t)k;
-    double s = 0.0;
-    for (int b = act_lo; b < kFsTileBits; ++b) s += ft[p ^ (1u << b)];
-    const uint64_t gi = base | (p & lo_mask) | ((uint64_t)(p >> cp) << h0);
-    y[gi] = first ? pre[k] * ft[p] - g * s : pre[k] - g * s;
-  }
-}
-
-// First pass for n >= 13: CTA = one 8192-state block (index bits 0-12). The
-// block of x arrives in shared memory by one 64 KB bulk copy; the 13 low-bit
-// neighbours are read there. Each bit j in [13, n_gather) pairs the block with
-// the block 2^(j-13) away, read as one coalesced sweep (32 loads in flight per
-// thread) into register accumulators: with blocks in index order and at most 512
-// blocks (32 MB) between partners (n_gather <= 23), the partner is still in the
-// 126 MB L2, so DRAM sees x, E and y once; y is stored streaming (evict-first) so
-// it does not push x out of L2. Bits >= n_gather go to a strided tile pass.
-
+// Up to 22 bits: CTA = one 8192-state block (index bits 0-12). The block of x arrives
+// in shared memory by one 64 KB bulk copy; the 13 low-bit neighbours are read there.
+// Each bit j from 13 on pairs the block with the block 2^(j-13) away, read as one
+// coalesced sweep (32 loads in flight per thread) into register accumulators: the
+// partner is in L2 (x is 32 MB at most).
 __global__ void __launch_bounds__(kFsThreads, 2) fs_block_kernel(const double* __restrict__ x, double* __restrict__ y,
                                                                  const uint16_t* __restrict__ E, double scale, double g,
                                                                  int n_gather, int* err) {
@@ -162,17 +96,19 @@ __global__ void __launch_bounds__(kFsThreads, 2) fs_block_kernel(const double* _
 }
 
 // ---------------------------------------------------------------------------
-// Product in tile passes, one cooperative launch (n >= 20). The index bits are split
-// into A = [0, 13), S1 = [13, 13 + w1) and S2 = the w2 bits above (none up to n = 20);
+// Product in tile passes, one cooperative launch (n >= 23). The index bits are split
+// into A = [0, 13), S1 = [13, 13 + w1) and S2 = the w2 bits above;
 // a tile is 8192 doubles of x, an S tile 2^w rows of 2^(13 - w) contiguous ones:
 //   1. S2 over the whole vector:  y  = -g sum_S2
 //   2. slab by slab (the 2^(13 + w1) states of one value of the S2 bits):
 //      A:  y += scale E x - g sum_A;   S1: y -= g sum_S1
 // S1 of a slab is queued `lag` slabs behind its A tiles, so x and y of the slab are
 // still in L2: DRAM sees x twice, y twice written and once read and E once, 42 bytes a
-// state. (Sweeping the ten bits above A through L2, 80 bytes a state of L2 reads, took
-// 1.35 of the 1.81 ms of N = 27.) A tile's x is loaded (TMA) once the tile before it is
-// summed, two CTAs an SM overlapping their loads and sums; a thread keeps the 32 doubles of the top five tile bits in
+// state (measured: 41.6). Sweeping the ten bits above A through L2 instead, 80 bytes a
+// state of L2 reads, took 1.82 ms at N = 27 with the far bits' pass; this takes 1.27 ms,
+// bound by the chain of one tile (x, y, sums from shared memory, stores), which the two
+// CTAs of an SM hide from each other in part. A tile's x is loaded (TMA) once the tile
+// before it is summed; a thread keeps the 32 doubles of the top five tile bits in
 // registers, so those neighbours need no shared-memory read, and reads the others from
 // the tile. Tasks are dealt to the CTAs in order; a slab's counter is awaited only by
 // S1 tiles, whose CTA owes nothing while it waits. Every wait is bounded.
