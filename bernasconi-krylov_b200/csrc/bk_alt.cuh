@@ -347,11 +347,8 @@ __device__ __forceinline__ void alt_turn(typename El<R>::T (&v)[1 << KB], unsign
     for (int i = 0; i < 8; ++i) {
       AltPhase<R>::apply(v[j0 + i], ev[i], P);
       El<R>::bfly_inner(v[j0 + i], T.t_post);
+      El<R>::scale(v[j0 + i], T.scale);  // 1 in most steps, and exact; a branch around it costs registers
     }
-  }
-  if (T.scale != (R)1) {
-#pragma unroll
-    for (int j = 0; j < (1 << KB); ++j) El<R>::scale(v[j], T.scale);
   }
   alt_rotate<R, TB, KB, CP == TB ? 0 : CP, r>(v, T.t_post);
 }

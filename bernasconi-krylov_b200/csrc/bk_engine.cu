@@ -24,8 +24,8 @@
 #include <unordered_map>
 #include <vector>
 
-#include "bk_adjoint.cuh"
 #define BK_ALT_REDUCE
+#include "bk_adj_turn.cuh"
 #include "bk_alt.cuh"
 #include "bk_aux.cuh"
 #include "bk_engine.h"
@@ -1158,6 +1158,16 @@ bool alt_geometry(int np, AltGeo* g) {
   g->w3 = rest - g->w2;
   return true;
 }
+// The reverse sweep's dual tiles: two sets up to 2^21 elements, three beyond (2^13-element
+// tiles of both vectors do not fit in shared memory).
+bool adj_geometry(int np, AltGeo* g) {
+  if (np < kElemBits + 1 || np > 30) return false;
+  g->tb = np <= 18 ? 10 : 12;
+  const int rest = np - g->tb;
+  g->w2 = np <= 21 ? rest : (rest + 1) / 2;
+  g->w3 = rest - g->w2;
+  return true;
+}
 template <class R>
 bool alt_takes(const bk_ctx* c, int n) {
   AltGeo g;
@@ -2056,6 +2066,132 @@ AdjKernel<R> adj_table_kernel(bool warp_a1) {
     return adj_kernel<R>(warp_a1, 0);
 }
 
+// A checkpoint put back after reverse step after_j (checkpoint ck; a, b undo the scales of
+// the rebuilt and of the stored vector).
+struct AdjReset {
+  int after_j, ck;
+  double a, b;
+};
+
+// The reverse sweep in turning passes (csrc/bk_adj_turn.cuh) behind a forward run already
+// enqueued: lambda_T, the passes (a launch per stretch between checkpoints), the cross terms
+// of every step. Waits for the stream; row and e_fwd are the forward run's result and error.
+template <class R>
+int adj_reverse_turning(bk_ctx* c, int n, int T, const AltRun<R>& fwd, const typename PhaseV<R>::params& reset_phase,
+                        const std::vector<R>& t_rev, const std::vector<R>& sc_rev, const std::vector<double>& lg_rev,
+                        const std::vector<AdjReset>& resets, int objective, int64_t e0, uint32_t s0,
+                        const unsigned char* ckpt, std::vector<double>* cross, double* drift, double* rev_ms,
+                        double* row, int* e_fwd, cudaEvent_t* ev) {
+  constexpr bool kC64 = sizeof(R) == 4;
+  const int np = kC64 ? n - 1 : n;
+  const size_t n_el = 1ull << np, sbytes = n_el * 16;
+  cudaStream_t st = c->stream;
+  AltGeo geo;
+  adj_geometry(np, &geo);
+  const int three = geo.w3 > 0 ? 1 : 0, n_seg = (int)resets.size() + 1;
+  const int n_rows = (three ? 2 : 1) * (T + 1) + n_seg;
+  AdjRun<R> D{};
+  BK_TRY(alt_maps(c, c->d_state, np, geo, D.map[0], D.set));
+  BK_TRY(alt_maps(c, c->d_lam, np, geo, D.map[1], D.set));
+  D.vec[0] = static_cast<unsigned char*>(c->d_state);
+  D.vec[1] = static_cast<unsigned char*>(c->d_lam);
+  D.E = c->d_E;
+  D.tab = fwd.D.tab;  // the forward run's phase table
+  D.n_j = fwd.D.n_j;
+  D.c0 = fwd.D.c0;
+  D.n_tiles = 1u << (np - geo.tb);
+  D.m0 = kC64 ? 1 : 0;
+  D.width[0] = geo.tb;
+  D.width[1] = geo.w2;
+  D.width[2] = geo.w3;
+  const void* fn = kC64 ? adj_turn_kernel_f32(geo.tb, geo.w2, geo.w3) : adj_turn_kernel_f64(geo.tb, geo.w2, geo.w3);
+  const int entry = (int)sizeof(typename AltPhase<R>::entry), threads = geo.tb == 10 ? 64 : 256;
+  const int smem = geo.tb == 10 ? AdjTurnSmem<10>::bytes(D.n_j, entry) : AdjTurnSmem<12>::bytes(D.n_j, entry);
+  BK_TRY(allow_smem(c, fn, smem));
+  int per_sm = 0;
+  BK_TRY(ctas_per_sm(c, fn, threads, smem, &per_sm));
+  if (per_sm < 1) return fail(c, BK_ERR_CUDA, "reverse turning pass: no room for a CTA (%d bytes of shared memory)", smem);
+  const uint32_t G = std::min<uint32_t>(D.n_tiles, (uint32_t)(per_sm * c->num_sms));
+  Bump b;
+  const size_t o_tan = b.take((size_t)T * sizeof(R));
+  const size_t o_sc = b.take((size_t)T * sizeof(R));
+  const size_t o_lg = b.take((size_t)T * sizeof(double));
+  const size_t o_row = b.take((size_t)T * sizeof(int));
+  const size_t o_ctr = b.take((size_t)n_seg * 128 + 64);
+  const size_t up = b.off;
+  const size_t o_cross = b.take((size_t)T * sizeof(double));
+  const size_t o_dev = b.take(std::max<size_t>(resets.size(), 1) * kResetGrid * sizeof(double));
+  const size_t o_part = b.take((size_t)n_rows * G * 2 * sizeof(double));
+  BK_TRY(ensure_buffer(c, &c->d_adj, &c->adj_cap, b.off));
+  char *h = stage(c, up), *d = static_cast<char*>(c->d_adj);
+  std::copy(t_rev.begin(), t_rev.end(), reinterpret_cast<R*>(h + o_tan));
+  std::copy(sc_rev.begin(), sc_rev.end(), reinterpret_cast<R*>(h + o_sc));
+  std::copy(lg_rev.begin(), lg_rev.end(), reinterpret_cast<double*>(h + o_lg));
+  std::memset(h + o_ctr, 0, (size_t)n_seg * 128 + 64);
+  std::vector<int> seg_end;
+  for (const AdjReset& r : resets) seg_end.push_back(r.after_j + 1);
+  seg_end.push_back(T);
+  for (int j = 0, s = 0; j < T; ++j) {
+    while (j >= seg_end[(size_t)s]) ++s;
+    reinterpret_cast<int*>(h + o_row)[j] = s + (three ? 2 : 1) * j;
+  }
+  BK_CUDA(c, cudaMemcpyAsync(d, h, up, cudaMemcpyHostToDevice, st));
+  D.tan = reinterpret_cast<const R*>(d + o_tan);
+  D.scale = reinterpret_cast<const R*>(d + o_sc);
+  D.lg = reinterpret_cast<const double*>(d + o_lg);
+  D.partials = reinterpret_cast<double*>(d + o_part);
+  int* abort_w = reinterpret_cast<int*>(d + o_ctr + (size_t)n_seg * 128);
+  BK_CUDA(c, cudaEventRecord(ev[2], st));
+  adj_lambda_init_kernel<R><<<(unsigned)std::min<size_t>((n_el + 255) / 256, (size_t)kResetGrid), 256, 0, st>>>(
+      D.vec[0], D.vec[1], c->d_E, (uint32_t)n_el, objective, (int)e0, s0);
+  BK_CUDA(c, cudaGetLastError());
+  double* d_dev = reinterpret_cast<double*>(d + o_dev);
+  for (int s = 0, j0 = 0; s < n_seg; ++s) {
+    D.j0 = j0;
+    D.j1 = seg_end[(size_t)s];
+    D.row0 = s;
+    AltBarrier B{reinterpret_cast<unsigned int*>(d + o_ctr + (size_t)s * 128), c->d_err, abort_w,
+                 c->wait_polls > 0 ? c->wait_polls : kWaitPolls * 4u};
+    size_t e = 0;
+    BK_TRY(ev_begin(c, "adj_turn", &e));
+    void* args[] = {&D, &B};
+    BK_CUDA(c, cudaLaunchCooperativeKernel(fn, dim3(G), dim3((unsigned)threads), args, (size_t)smem, st));
+    BK_TRY(ev_end(c, e));
+    if (s < n_seg - 1) {
+      const AdjReset& r = resets[(size_t)s];
+      BK_TRY(ev_begin(c, "adj_reset", &e));
+      adj_reset_kernel<R><<<kResetGrid, kComputeThreads, 0, st>>>(D.vec[0], ckpt + (size_t)r.ck * sbytes, c->d_E,
+                                                                  (uint32_t)n_el, reset_phase, r.a, r.b,
+                                                                  d_dev + (size_t)s * kResetGrid);
+      BK_CUDA(c, cudaGetLastError());
+      BK_TRY(ev_end(c, e));
+    }
+    j0 = D.j1;
+  }
+  adj_cross_kernel<<<(T + 3) / 4, 128, 0, st>>>(D.partials, T, (int)G, three, reinterpret_cast<const int*>(d + o_row),
+                                                reinterpret_cast<double*>(d + o_cross));
+  BK_CUDA(c, cudaGetLastError());
+  BK_CUDA(c, cudaEventRecord(ev[3], st));
+  cross->assign((size_t)T, 0.0);
+  std::vector<double> dev(resets.size() * kResetGrid);
+  BK_CUDA(c, cudaMemcpyAsync(cross->data(), d + o_cross, (size_t)T * sizeof(double), cudaMemcpyDeviceToHost, st));
+  if (!dev.empty())
+    BK_CUDA(c, cudaMemcpyAsync(dev.data(), d_dev, dev.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
+  BK_CUDA(c, cudaMemcpyAsync(row, c->d_results, 4 * sizeof(double), cudaMemcpyDeviceToHost, st));
+  BK_CUDA(c, cudaMemcpyAsync(e_fwd, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
+  BK_CUDA(c, cudaStreamSynchronize(st));
+  BK_TRY(collect_timing(c));
+  float ms = 0.f;
+  BK_CUDA(c, cudaEventElapsedTime(&ms, ev[2], ev[3]));
+  *rev_ms = ms;
+  for (size_t r = 0; r < resets.size(); ++r) {
+    double s = 0.0;
+    for (int i = 0; i < kResetGrid; ++i) s += dev[r * kResetGrid + (size_t)i];
+    *drift = std::max(*drift, std::sqrt(s));
+  }
+  return BK_OK;
+}
+
 // Forward run with checkpoints every K steps (persistent engine), lambda_T = W
 // psi_T, then the reverse sweep: per reverse step one dual A1 / S2 / S3 launch
 // each, a checkpoint put back every K steps. grad_step[k] = dO/dg_k.
@@ -2125,13 +2261,16 @@ int adjoint_t(bk_ctx* c, const bk_adjoint_params* p, const std::vector<double>& 
     }
   } guard{ev};
 
+  // turning passes: the forward run as bk_evolve's, the reverse sweep unless the warp-local
+  // A1 layout is asked for
+  const bool turning = c->engine_mode == 4 && alt_takes<R>(c, n);
+  const bool rev_turning = turning && c->adj_a1 == 0;
   PersistRun<R> run;
-  BK_TRY(persist_prepare<R>(c, &q, S, angle_unit, tans, scales, &run));
+  if (!rev_turning || n_ckpt > 0) BK_TRY(persist_prepare<R>(c, &q, S, angle_unit, tans, scales, &run));
   unsigned char* ckpt = static_cast<unsigned char*>(c->d_ckpt);
   grad_step->assign((size_t)T, 0.0);
   // forward: one persistent launch per window of K steps, psi copied to a
   // checkpoint between windows; enqueued without host synchronisation
-  const bool turning = c->engine_mode == 4 && alt_takes<R>(c, n);  // bk_evolve's choice
   AltRun<R> arun;
   if (turning) BK_TRY(alt_prepare<R>(c, n, p->s0, e0, angle_unit, S, tans, scales, &arun));
   int* fwd_err = turning ? c->d_err : run.err;
@@ -2218,6 +2357,25 @@ int adjoint_t(bk_ctx* c, const bk_adjoint_params* p, const std::vector<double>& 
       resets.push_back(Reset{j, m - 1, (double)std::exp2(-lp), (double)std::exp2(-lgf[(size_t)k])});
       lp = lgf[(size_t)k];
     }
+  }
+
+  if (rev_turning) {
+    std::vector<AdjReset> rs;
+    for (const Reset& r : resets) rs.push_back({r.after_j, r.ck, r.a, r.b});
+    std::vector<double> cross;
+    double drift = 0.0, rev_ms = 0.0;
+    BK_TRY(enqueue_forward());
+    BK_TRY(adj_reverse_turning<R>(c, n, T, arun, run.phase, t_rev, sc_rev, lg_rev, rs, p->objective, e0, s0, ckpt, &cross,
+                                  &drift, &rev_ms, row, &e_fwd, ev));
+    BK_TRY(finish_forward());
+    for (int j = 0; j < T; ++j)
+      (*grad_step)[(size_t)(T - 1 - j)] =
+          (double)(-2.0L * (long double)p->dt * (long double)cross[(size_t)j] * std::exp2(-wlog2[(size_t)j]));
+    if (stats) {
+      stats->reverse_ms = rev_ms;
+      stats->max_drift = drift;
+    }
+    return BK_OK;
   }
 
   // device layout
@@ -2515,9 +2673,8 @@ int bk_steepest_descent_gpu(bk_ctx* c, int n, const uint64_t* starts, int64_t co
   // The copies cost more than the descents (65536 starts of n = 28: 58 us of kernel, 210
   // us of pageable copies of 8-byte words one array after another), so states up to 32
   // spins, energies and evaluations cross as 4-byte words through pinned memory, the
-  // results in one copy, and the pages of the caller's arrays, mostly fresh ones, are
-  // touched while the GPU works. (Several threads would widen faster, but their idle
-  // spinning slows the host calls that follow.)
+  // results in one copy, and the host threads widen them into the caller's arrays, whose
+  // fresh pages then fault in parallel (120 us the call; 285 us with one thread).
   const size_t cnt = (size_t)count, word = n <= 32 ? 4 : 8;
   const size_t need = cnt * (2 * word + 8) + 64;
   BK_TRY(ensure_buffer(c, &c->d_descent, &c->descent_cap, need));
@@ -2534,6 +2691,7 @@ int bk_steepest_descent_gpu(bk_ctx* c, int n, const uint64_t* starts, int64_t co
   size_t e = 0;
   if (n <= 32) {
     uint32_t* narrow = reinterpret_cast<uint32_t*>(h);
+#pragma omp parallel for schedule(static) if (cnt >= 16384)
     for (long long i = 0; i < (long long)cnt; ++i) narrow[i] = (uint32_t)starts[i];
     BK_CUDA(c, cudaMemcpyAsync(d + o_st, narrow, cnt * 4, cudaMemcpyHostToDevice, st));
   } else {
@@ -2552,15 +2710,13 @@ int bk_steepest_descent_gpu(bk_ctx* c, int n, const uint64_t* starts, int64_t co
         reinterpret_cast<uint32_t*>(d + o_ev));
   BK_CUDA(c, cudaGetLastError());
   BK_TRY(ev_end(c, e));
-  if (pinned.p) BK_CUDA(c, cudaMemcpyAsync(h, d + o_fs, host_bytes, cudaMemcpyDeviceToHost, st));
-  for (void* out : {(void*)fs, (void*)fe, (void*)ev})
-    for (size_t at = 0; out && at < cnt * 8; at += 4096) static_cast<volatile char*>(out)[at] = 0;
-  if (!pinned.p) BK_CUDA(c, cudaMemcpyAsync(h, d + o_fs, host_bytes, cudaMemcpyDeviceToHost, st));
+  BK_CUDA(c, cudaMemcpyAsync(h, d + o_fs, host_bytes, cudaMemcpyDeviceToHost, st));
   BK_CUDA(c, cudaStreamSynchronize(st));
   const uint32_t* w_fs = reinterpret_cast<const uint32_t*>(h + o_fs);
   const uint64_t* l_fs = reinterpret_cast<const uint64_t*>(h + o_fs);
   const int* w_fe = reinterpret_cast<const int*>(h + o_fe);
   const uint32_t* w_ev = reinterpret_cast<const uint32_t*>(h + o_ev);
+#pragma omp parallel for schedule(static) if (cnt >= 16384)
   for (long long i = 0; i < (long long)cnt; ++i) {
     fs[i] = word == 4 ? w_fs[i] : l_fs[i];
     fe[i] = w_fe[i];
@@ -2951,18 +3107,21 @@ int bk_adjoint(bk_ctx* c, const bk_adjoint_params* p, double* value_out, double*
   BK_CUDA(c, cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
   const size_t sbytes = (1ull << n) * amp_bytes(p->precision);
   // checkpoints: every K steps strictly inside (0, T); K enlarged until they fit
-  size_t free_b = 0, total_b = 0;
-  BK_CUDA(c, cudaMemGetInfo(&free_b, &total_b));
-  const size_t reserve = (size_t)1 << 30;
-  const size_t avail = free_b + c->lam_cap + c->ckpt_cap;
-  if (avail < sbytes + reserve) return fail(c, BK_ERR_OOM, "adjoint: no room for the adjoint statevector");
   int K = p->checkpoint_every;
   const bool auto_k = K <= 0;
   if (auto_k) K = 128;
   auto n_ck = [&](int k) { return T > 0 ? (T - 1) / k : 0; };
-  while (sbytes * (size_t)(1 + n_ck(K)) + reserve > avail) {
-    if (!auto_k) return fail(c, BK_ERR_OOM, "adjoint: %d checkpoints of %zu bytes do not fit", n_ck(K), sbytes);
-    K *= 2;
+  // (the free memory is asked for only when the buffers of an earlier call do not suffice)
+  if (c->lam_cap < sbytes || c->ckpt_cap < sbytes * (size_t)n_ck(K)) {
+    size_t free_b = 0, total_b = 0;
+    BK_CUDA(c, cudaMemGetInfo(&free_b, &total_b));
+    const size_t reserve = (size_t)1 << 30;
+    const size_t avail = free_b + c->lam_cap + c->ckpt_cap;
+    if (avail < sbytes + reserve) return fail(c, BK_ERR_OOM, "adjoint: no room for the adjoint statevector");
+    while (sbytes * (size_t)(1 + n_ck(K)) + reserve > avail) {
+      if (!auto_k) return fail(c, BK_ERR_OOM, "adjoint: %d checkpoints of %zu bytes do not fit", n_ck(K), sbytes);
+      K *= 2;
+    }
   }
   const int n_ckpt = n_ck(K);
   BK_TRY(ensure_buffer(c, &c->d_lam, &c->lam_cap, sbytes));

@@ -133,3 +133,31 @@ def test_small_runs_split_at_sampling_points(eng, n):
     # of a step in the other layout are summed in another order
     assert np.max(np.abs(a["p_less_history"] - b["p_less_history"])) <= BAR128
     assert np.max(np.abs(a["dh_history"] - b["dh_history"])) <= BAR128 * n
+
+
+# the reverse sweep's tiles: 2^10 (13, 14, 18 element bits: a set of 3, 4, 8 bits), 2^12
+# with two sets (19, 20, 21) and with three (22, 23, 25), against the launch-per-pass sweep;
+# checkpoints that split the sweep into stretches of odd and even length
+@pytest.mark.parametrize("n", [13, 14, 18, 19, 20, 21, 22, 23, 25])
+def test_reverse_sweep_matches_the_launch_per_pass_sweep(eng, n):
+    T, g = 11, np.linspace(0.3, 0.42, 11)
+    bits, e0 = bk.select_trap(n, 13, 100, 0.3)
+    out = []
+    for mode in (1, 4):
+        eng.set_option("engine_mode", mode)
+        out.append([eng.adjoint(n, bits, g, 0.04, T, e0=e0, precision=bk.BK_C128, checkpoint_every=K)[:2] for K in (64, 4, 3)])
+    for a, b in zip(*out):
+        # FP64 rounding of ~32 T rotations on sums of products of amplitudes of norm 1
+        assert abs(a[0] - b[0]) <= BAR128
+        assert np.max(np.abs(a[1] - b[1])) <= 1e-11 * max(1e-3, np.max(np.abs(a[1])))
+
+
+@pytest.mark.parametrize("n", [14, 20, 22, 24])
+def test_reverse_sweep_complex64(eng, n):
+    T, g = 8, np.linspace(0.3, 0.42, 8)
+    bits, e0 = bk.select_trap(n, 13, 100, 0.3)
+    eng.set_option("engine_mode", 4)
+    a = eng.adjoint(n, bits, g, 0.04, T, e0=e0, precision=bk.BK_C64, checkpoint_every=3)
+    b = eng.adjoint(n, bits, g, 0.04, T, e0=e0, precision=bk.BK_C128, checkpoint_every=3)
+    assert np.max(np.abs(a[1] - b[1])) <= 1e-4 * np.max(np.abs(b[1]))  # the complex64 gradient's bar
+    assert a[2]["max_drift"] <= 1e-5
