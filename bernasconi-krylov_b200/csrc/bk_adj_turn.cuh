@@ -44,8 +44,8 @@ struct AdjPhaseInv;  // D^dagger on both vectors' element
 template <>
 struct AdjPhaseInv<float> {
   __device__ static void apply(El<float>::T& v, El<float>::T& u, uint32_t e2, const AltTab& t) {
-    const float2 H0 = *reinterpret_cast<const float2*>(t.base + (((e2 & 0xFFFFu) - t.c0) >> 2) * t.stride);
-    const float2 H1 = *reinterpret_cast<const float2*>(t.base + (((e2 >> 16) - t.c0) >> 2) * t.stride);
+    const float2 H0 = *reinterpret_cast<const float2*>(t.base + (e2 & 0xFFFFu) * t.per_e);
+    const float2 H1 = *reinterpret_cast<const float2*>(t.base + (e2 >> 16) * t.per_e);
     const float2 A = make_float2(-H0.x, -H1.x), B = make_float2(-H0.y, -H1.y);
     PhaseV<float>::shear2(v.re, v.im, A, B);
     PhaseV<float>::shear2(v.re, v.im, A, B);
@@ -56,7 +56,7 @@ struct AdjPhaseInv<float> {
 template <>
 struct AdjPhaseInv<double> {
   __device__ static void apply(El<double>::T& v, El<double>::T& u, uint32_t e, const AltTab& t) {
-    const double2 cs = *reinterpret_cast<const double2*>(t.base + ((e - t.c0) >> 2) * t.stride);
+    const double2 cs = *reinterpret_cast<const double2*>(t.base + e * t.per_e);
     v.v = make_double2(fma(v.v.x, cs.x, v.v.y * cs.y), fma(-v.v.x, cs.y, v.v.y * cs.x));
     u.v = make_double2(fma(u.v.x, cs.x, u.v.y * cs.y), fma(-u.v.x, cs.y, u.v.y * cs.x));
   }
@@ -65,7 +65,7 @@ struct AdjPhaseInv<double> {
 struct AdjCtl {
   uint64_t full_bar;
   int stop, inflight;
-  double w[16];      // round weights of the pass: [0, 4) finishing, [4, 8) starting (4: at the turn)
+  double w[16];      // round weights of the pass: [0, 4) finishing, [4, 8) starting; 8, 9: of the lane bit
   double acc[16][2];
 };
 template <int TB>
@@ -78,7 +78,7 @@ struct AdjTurnSmem {
 // round r's cross terms and rotations of the set's bits, on both vectors
 template <class R, int TB, int KB, int LO, int r>
 __device__ __forceinline__ double adj_round(typename El<R>::T (&v)[1 << KB], typename El<R>::T (&u)[1 << KB], R t,
-                                            double weight) {
+                                            double weight, double lane_weight = 0.0) {
   constexpr int lo = AltPlan<TB, KB>::reg_lo(r);
   CrossAcc<R> ca;
 #pragma unroll
@@ -89,14 +89,36 @@ __device__ __forceinline__ double adj_round(typename El<R>::T (&v)[1 << KB], typ
         if (!(j & (1 << k))) ca.pair(v[j], v[j | (1 << k)], u[j], u[j | (1 << k)]);
     }
   }
-  alt_rotate<R, TB, KB, LO, r>(v, t);
-  alt_rotate<R, TB, KB, LO, r>(u, t);
-  return weight * ca.take();
+  double sum = weight * ca.take();
+  if constexpr (r == 1 && alt_lane_bit(TB, KB, LO)) {
+    // the registers' bits, then the bit across lanes (each thread adds its own ordered term)
+#pragma unroll
+    for (int k = 0; k < KB; ++k) {
+#pragma unroll
+      for (int j = 0; j < (1 << KB); ++j)
+        if (!(j & (1 << k))) {
+          El<R>::bfly(v[j], v[j | (1 << k)], t);
+          El<R>::bfly(u[j], u[j | (1 << k)], t);
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < (1 << KB); ++j) {
+      const typename El<R>::T pv = El<R>::shfl_xor(v[j], 1 << LO), pu = El<R>::shfl_xor(u[j], 1 << LO);
+      ca.one(pv, u[j]);
+      El<R>::bfly_partner(v[j], pv, t);
+      El<R>::bfly_partner(u[j], pu, t);
+    }
+    sum += weight * lane_weight * ca.take();
+  } else {
+    alt_rotate<R, TB, KB, LO, r>(v, t);
+    alt_rotate<R, TB, KB, LO, r>(u, t);
+  }
+  return sum;
 }
 // qubits of a set that round r rotates
 __host__ __device__ constexpr int adj_round_bits(int TB, int KB, int LO, int r) {
   const int lo = r == 0 ? TB - KB : r == 1 ? TB - 2 * KB : 0, hi = lo + (r < 2 ? KB : TB - 2 * KB);
-  return hi <= LO ? 0 : hi - (lo > LO ? lo : LO);
+  return (hi <= LO ? 0 : hi - (lo > LO ? lo : LO)) + (r == 1 && alt_lane_bit(TB, KB, LO) ? 1 : 0);
 }
 
 template <class R, int TB, int KB>
@@ -193,12 +215,14 @@ struct AdjCta {
         w = round_weight(m, D.lg[j]);
       }
       ctl().w[threadIdx.x] = w;
+      // the lane bit of round 1 comes after its KB register bits
+      if (threadIdx.x == 0u) ctl().w[8] = pre ? round_weight(KB, D.lg[j - 1]) : 0.0;
+      if (threadIdx.x == 4u) ctl().w[9] = post ? round_weight(KB, D.lg[j]) : 0.0;
     }
     __syncthreads();
     const volatile double(&wt)[16] = ctl().w;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    constexpr uint32_t kEntry = sizeof(typename AltPhase<R>::entry);
-    const AltTab P{tab() + (phase ? kEntry : 0u), phase ? kEntry : 0u, (uint32_t)D.c0};
+    const AltTab P = alt_tab<R>(tab(), phase, (uint32_t)D.c0);
     const uint32_t b0 = PL::template base<0>(lane, warp);
     double fin = 0.0, sta = 0.0;
     unsigned char *sp = stage, *sl = lam();
@@ -233,7 +257,7 @@ struct AdjCta {
           }
           sta += wt[7] * ca.take();
         }
-        sta += adj_round<R, TB, KB, LO, r>(v, u, t_post, wt[4 + r]);
+        sta += adj_round<R, TB, KB, LO, r>(v, u, t_post, wt[4 + r], wt[9]);
       };
       if constexpr (RT == 0) {
         at_turn(b0, std::integral_constant<int, 0>{});
@@ -247,7 +271,7 @@ struct AdjCta {
         const uint32_t b1 = PL::template base<1>(lane, warp);
         alt_load<R, TB, KB, 1, true>(sp, v, b1);
         alt_load<R, TB, KB, 1, true>(sl, u, b1);
-        fin += adj_round<R, TB, KB, LO, 1>(v, u, t_pre, wt[1]);
+        fin += adj_round<R, TB, KB, LO, 1>(v, u, t_pre, wt[1], wt[8]);
         if constexpr (RT == 1) {
           at_turn(b1, std::integral_constant<int, 1>{});
         } else {
@@ -264,7 +288,7 @@ struct AdjCta {
           __syncwarp();
           alt_load<R, TB, KB, 1, true>(sp, v, b1);
           alt_load<R, TB, KB, 1, true>(sl, u, b1);
-          sta += adj_round<R, TB, KB, LO, 1>(v, u, t_post, wt[5]);
+          sta += adj_round<R, TB, KB, LO, 1>(v, u, t_post, wt[5], wt[9]);
         }
         alt_store<R, TB, KB, 1>(sp, v, b1);
         alt_store<R, TB, KB, 1>(sl, u, b1);

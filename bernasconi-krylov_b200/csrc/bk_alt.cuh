@@ -43,15 +43,15 @@ namespace bk {
 template <class R>
 struct AltPhase;
 struct AltTab {
-  const unsigned char* base;
-  uint32_t stride, c0;
+  const unsigned char* base;  // where E = 0 would be
+  uint32_t per_e;             // bytes per unit of E (an entry per 4 units), or 0
 };
 template <>
 struct AltPhase<float> {
   using entry = float2;  // {-tan(r/4), sin(r/2)}: two half-angle shear rotations
   __device__ static void apply(El<float>::T& v, uint32_t e2, const AltTab& t) {
-    const float2 H0 = *reinterpret_cast<const float2*>(t.base + (((e2 & 0xFFFFu) - t.c0) >> 2) * t.stride);
-    const float2 H1 = *reinterpret_cast<const float2*>(t.base + (((e2 >> 16) - t.c0) >> 2) * t.stride);
+    const float2 H0 = *reinterpret_cast<const float2*>(t.base + (e2 & 0xFFFFu) * t.per_e);
+    const float2 H1 = *reinterpret_cast<const float2*>(t.base + (e2 >> 16) * t.per_e);
     const float2 A = make_float2(H0.x, H1.x), B = make_float2(H0.y, H1.y);
     PhaseV<float>::shear2(v.re, v.im, A, B);
     PhaseV<float>::shear2(v.re, v.im, A, B);
@@ -61,10 +61,17 @@ template <>
 struct AltPhase<double> {
   using entry = double2;  // {cos r, sin r}
   __device__ static void apply(El<double>::T& v, uint32_t e, const AltTab& t) {
-    const double2 cs = *reinterpret_cast<const double2*>(t.base + ((e - t.c0) >> 2) * t.stride);
+    const double2 cs = *reinterpret_cast<const double2*>(t.base + e * t.per_e);
     v.v = make_double2(fma(v.v.x, cs.x, -v.v.y * cs.y), fma(v.v.x, cs.y, v.v.y * cs.x));
   }
 };
+
+// the table at `tab` (shared memory), or its entry 0 for every E
+template <class R>
+__device__ __forceinline__ AltTab alt_tab(const unsigned char* tab, bool on, uint32_t c0) {
+  constexpr uint32_t kEntry = sizeof(typename AltPhase<R>::entry), kPerE = kEntry / 4u;
+  return on ? AltTab{tab + kEntry - c0 * kPerE, kPerE} : AltTab{tab, 0u};
+}
 
 // TMA coordinates of a set's tiles: the dimensions of the tile id's two parts.
 struct AltSet {
@@ -168,6 +175,11 @@ __device__ __forceinline__ void alt_store(unsigned char* s, const typename El<R>
 #pragma unroll
   for (int j = 0; j < (1 << KB); ++j) El<R>::st(s + 16u * (sb ^ swz<double>((uint32_t)j << lo)), v[j]);
 }
+// A set one bit wider than two rounds hold: its lowest bit, tile bit CP, is lane bit CP in
+// round 1 (whose lanes run over the bits below its registers), so it is rotated across
+// lanes instead of in a round of its own (two more trips through shared memory).
+__host__ __device__ constexpr bool alt_lane_bit(int TB, int KB, int CP) { return TB - CP == 2 * KB + 1 && CP > 0; }
+
 // the rotations of round r's new bits that belong to the set (tile bits >= cp)
 template <class R, int TB, int KB, int CP, int r>
 __device__ __forceinline__ void alt_rotate(typename El<R>::T (&v)[1 << KB], R t) {
@@ -178,6 +190,13 @@ __device__ __forceinline__ void alt_rotate(typename El<R>::T (&v)[1 << KB], R t)
 #pragma unroll
       for (int j = 0; j < (1 << KB); ++j)
         if (!(j & (1 << k))) El<R>::bfly(v[j], v[j | (1 << k)], t);
+    }
+  }
+  if constexpr (r == 1 && alt_lane_bit(TB, KB, CP)) {
+#pragma unroll
+    for (int j = 0; j < (1 << KB); ++j) {
+      const typename El<R>::T q = El<R>::shfl_xor(v[j], 1 << CP);
+      El<R>::bfly_partner(v[j], q, t);
     }
   }
 }
@@ -336,9 +355,11 @@ __device__ __forceinline__ void alt_turn(typename El<R>::T (&v)[1 << KB], unsign
                                          const AltTurn<R>& T, uint32_t tile_base, uint32_t base,
                                          const unsigned char* tab, const AltMeas& M) {
   cp_async_wait();
-  if (T.meas) alt_measure<R, TB, KB, CP, H0, r>(v, tile, es, *M.e0, *M.s0, tile_base, base, M.acc3);
-  constexpr uint32_t kEntry = sizeof(typename AltPhase<R>::entry);
-  const AltTab P{tab + (T.post ? kEntry : 0u), T.post ? kEntry : 0u, T.c0};
+  if (T.meas) {
+    alt_measure<R, TB, KB, CP, H0, r>(v, tile, es, *M.e0, *M.s0, tile_base, base, M.acc3);
+    alt_load<R, TB, KB, r, true>(tile, v, base);  // the measurement needs the registers
+  }
+  const AltTab P = alt_tab<R>(tab, T.post, T.c0);
 #pragma unroll
   for (int j0 = 0; j0 < (1 << KB); j0 += 8) {
     uint32_t ev[8];
@@ -347,20 +368,33 @@ __device__ __forceinline__ void alt_turn(typename El<R>::T (&v)[1 << KB], unsign
     for (int i = 0; i < 8; ++i) {
       AltPhase<R>::apply(v[j0 + i], ev[i], P);
       El<R>::bfly_inner(v[j0 + i], T.t_post);
-      El<R>::scale(v[j0 + i], T.scale);  // 1 in most steps, and exact; a branch around it costs registers
     }
+  }
+  if (T.scale != (R)1) {
+#pragma unroll
+    for (int j = 0; j < (1 << KB); ++j) El<R>::scale(v[j], T.scale);
   }
   alt_rotate<R, TB, KB, CP == TB ? 0 : CP, r>(v, T.t_post);
 }
 
 // the round a pass turns in (CP = TB: the A set)
 __host__ __device__ constexpr int alt_turn_round(int TB, int KB, int CP) {
-  return CP == TB ? 2 : (TB - CP + KB - 1) / KB - 1;
+  return CP == TB ? 2 : alt_lane_bit(TB, KB, CP) ? 1 : (TB - CP + KB - 1) / KB - 1;
 }
 
 // A turning pass on one staged tile (CP = TB: a tile of the A set). `wait()` returns
 // when the tile has landed, `stage_free()` runs in every thread after a barrier
 // behind the last shared-memory read.
+// 2^10-element tiles are read straight into round 0's registers: a CTA has one of them a
+// pass (or little more), so there is nothing to load ahead, and the copy through shared
+// memory with its barrier is latency on top of the exchange's.
+constexpr bool alt_direct(int TB) { return TB == 10; }
+template <class R>
+__device__ __forceinline__ typename El<R>::T alt_ldcg(const unsigned char* p) {
+  const float4 q = __ldcg(reinterpret_cast<const float4*>(p));  // other SMs write it: never from L1
+  return El<R>::ld(&q);
+}
+
 template <class R, int TB, int KB, int CP, int H0, class W, class F>
 __device__ __forceinline__ void alt_tile_turn(unsigned char* tile, unsigned char* state, const AltTurn<R>& T,
                                               uint32_t tile_base, const unsigned char* tab, unsigned char* es,
@@ -371,8 +405,15 @@ __device__ __forceinline__ void alt_tile_turn(unsigned char* tile, unsigned char
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const uint32_t b0 = PL::template base<0>(lane, warp);
   typename El<R>::T v[1 << KB];
-  wait();
-  alt_load<R, TB, KB, 0, false>(tile, v, b0);
+  if constexpr (alt_direct(TB)) {
+    const unsigned char* g = state + 16ull * (tile_base | alt_index<CP, H0>(b0));
+#pragma unroll
+    for (int j = 0; j < (1 << KB); ++j)
+      v[j] = alt_ldcg<R>(g + 16ull * alt_index<CP, H0>((uint32_t)j << PL::reg_lo(0)));
+  } else {
+    wait();
+    alt_load<R, TB, KB, 0, false>(tile, v, b0);
+  }
   if constexpr (RT == 0) {
     alt_rotate<R, TB, KB, LO, 0>(v, T.t_pre);
     if (T.meas) __syncwarp();  // the measurement's swizzled slots were other lanes' linear ones
@@ -540,6 +581,7 @@ struct AltCta {
   }
 
   __device__ __forceinline__ void issue(int map, uint32_t tile) {
+    if constexpr (alt_direct(TB)) return;
     if (threadIdx.x == 0 && tile < D.n_tiles && !ctl().stop) {
       alt_issue(D.set[map], maps() + map, tile, kBytes, stage, bar());
       ctl().inflight = 1;
@@ -616,7 +658,11 @@ struct AltCta {
   // ... then the next pass's first tile
   __device__ __forceinline__ bool next_pass(int map) {
     if (!group_barrier()) return false;
-    issue(map, rank);
+    if constexpr (alt_direct(TB)) {
+      if (__syncthreads_or(ctl().stop)) return false;  // thread 0 has seen every CTA's stores
+    } else {
+      issue(map, rank);
+    }
     return true;
   }
   __device__ __forceinline__ void stage_table() {
@@ -799,7 +845,7 @@ const void* alt_kernel_table(int tb, int w2, int w3, bool batch) {
     case 0xA80: return alt_pick<R, 10, 4, 8, 0>(batch);
     case 0xC70: return alt_pick<R, 12, 4, 7, 0>(batch);
     case 0xC80: return alt_pick<R, 12, 4, 8, 0>(batch);
-    case 0xD80: return alt_pick<R, 13, 5, 8, 0>(batch);
+    case 0xC90: return alt_pick<R, 12, 4, 9, 0>(batch);
     case 0xD90: return alt_pick<R, 13, 5, 9, 0>(batch);
     case 0xDA0: return alt_pick<R, 13, 5, 10, 0>(batch);
     case 0xC66: return alt_pick<R, 12, 4, 6, 6>(batch);

@@ -1144,15 +1144,15 @@ struct AltGeo {
 //   np <= 18: 2^10-element tiles, a 64-thread CTA each, two sets. The barrier and the
 //     exchange through L2 bound these sizes, so small tiles on many SMs win (np = 18:
 //     5.7 / 5.1 against 16.5 / 14.6 for a launch per pass).
-//   np <= 20: 2^12-element tiles, two CTAs an SM, two sets (np = 20: 12.3 / 12.2
-//     against 22.8 / 20.6).
+//   np <= 21: 2^12-element tiles, two CTAs an SM, two sets (np = 20: 12.3 / 12.2
+//     against 22.8 / 20.6 for a launch per pass; np = 21, a set of nine bits with one of
+//     them across lanes: 23.8 / 22.7 against 26.0 / 23.7 with 2^13-element tiles).
 //   np <= 23: 2^13-element tiles with 32 elements a thread, so that two sets still do
-//     (one pass a step): np = 21 25.4 / 23.9 against 27.8 / 26.7 with 2^12-element
-//     tiles and a 9-bit second set, np = 23 94 / 86 against 103 / 110 with three sets.
+//     (one pass a step): np = 23 94 / 86 against 103 / 110 with three sets.
 //   beyond: 2^12-element tiles, three sets (two passes a step).
 bool alt_geometry(int np, AltGeo* g) {
   if (np < kElemBits + 1 || np > 30) return false;
-  g->tb = np <= 18 ? 10 : np <= 20 || np > 23 ? 12 : 13;
+  g->tb = np <= 18 ? 10 : np <= 21 || np > 23 ? 12 : 13;
   const int rest = np - g->tb;
   g->w2 = np <= 23 ? rest : (rest + 1) / 2;
   g->w3 = rest - g->w2;
@@ -3297,19 +3297,14 @@ int bk_sampler_run(bk_ctx* c, const bk_sampler_config* cfg, uint64_t start_bits,
   const size_t n_draws = drawn.size();
   std::vector<int> shot_e(n_draws), shot_d(n_draws);
   if (n_draws > 0) {
-    void* scratch = nullptr;
-    BK_CUDA(c, cudaMallocAsync(&scratch, n_draws * 2 * sizeof(int), c->stream));
-    int* d_e = static_cast<int*>(scratch);
+    BK_TRY(ensure_buffer(c, &c->d_io, &c->io_cap, n_draws * 2 * sizeof(int)));
+    int* d_e = static_cast<int*>(c->d_io);
     int* d_f = d_e + n_draws;
     shot_stats_kernel<<<(unsigned)((n_draws + 255) / 256), 256, 0, c->stream>>>(
         c->d_samples, (long long)n_draws, n, (unsigned long long)(start_bits & ((1ull << n) - 1ull)), d_e, d_f);
-    const cudaError_t le = cudaGetLastError();
-    cudaError_t ce = cudaMemcpyAsync(shot_e.data(), d_e, n_draws * sizeof(int), cudaMemcpyDeviceToHost, c->stream);
-    if (ce == cudaSuccess)
-      ce = cudaMemcpyAsync(shot_d.data(), d_f, n_draws * sizeof(int), cudaMemcpyDeviceToHost, c->stream);
-    cudaFreeAsync(scratch, c->stream);
-    BK_CUDA(c, le);
-    BK_CUDA(c, ce);
+    BK_CUDA(c, cudaGetLastError());
+    BK_CUDA(c, cudaMemcpyAsync(shot_e.data(), d_e, n_draws * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    BK_CUDA(c, cudaMemcpyAsync(shot_d.data(), d_f, n_draws * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     BK_CUDA(c, cudaStreamSynchronize(c->stream));
   }
   std::vector<bk_seed_stats> ss((size_t)n_seeds);
