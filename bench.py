@@ -56,7 +56,7 @@ def parse():
     ap.add_argument("--no-compare", action="store_true")
     ap.add_argument("--engine-mode", type=int, default=None,
                     help="0 persistent, 1 one launch per pass, 2 A1 launch + fused strided launch, "
-                         "3 the same with the fused strided pass in two self-served groups")
+                         "3 the same with the fused strided pass in two self-served groups, 4 turning passes")
     ap.add_argument("--workload", choices=["large", "batched", "adjoint", "matvec"], default="large",
                     help="large: the N=28 headline; batched: 512 instances (64 traps x 8 g), N in {16,18,20,22}")
     ap.add_argument("--slab-lag", type=int, default=None)
@@ -330,7 +330,7 @@ def run_batched(a):
     value = amp_steps * a.steps / dev_s
     # the same 512 instances one after another, each through its own launches
     seq = {}
-    for mode in (1, 0):
+    for mode in (1, 0, tune.TURNING):
         eng.set_option("engine_mode", mode)
         eng.evolve(inst[0]["n"], inst[0]["s0"], inst[0]["g"], a.dt, 4, measure=[0], e0=inst[0]["e0"])
         torch.cuda.synchronize(dev)
@@ -340,16 +340,17 @@ def run_batched(a):
             eng.evolve(d["n"], d["s0"], d["g"], a.dt, steps_t, measure=meas, e0=d["e0"], precision=bk.BK_C64)
         e1_.record(stream)
         torch.cuda.synchronize(dev)
-        seq["sequential_" + ("one_launch_per_pass" if mode == 1 else "persistent_per_instance")] = \
-            amp_steps / (e0_.elapsed_time(e1_) / 1e3)
+        name = {1: "one_launch_per_pass", 0: "persistent_per_instance"}.get(mode, "turning_per_instance")
+        seq["sequential_" + name] = amp_steps / (e0_.elapsed_time(e1_) / 1e3)
     best_seq = max(seq.values())
-    # roofline: one persistent launch per bench step runs all 500 steps of all
-    # 512 instances; algorithmic bytes 32 per amplitude-step (two complex64
-    # read + write passes), timed by the CUDA events bracketing the launches
+    # roofline: one launch per size and bench step runs all 500 steps of that size's
+    # instances; algorithmic bytes 32 per amplitude-step (the two complex64
+    # read + write passes of the two-round-trip model; turning passes of these
+    # sizes need one), timed by the CUDA events bracketing the launches
     peak, peak_kind = measured_peaks()
     launch_s = dev_s / a.steps
     alg = 32.0 * amp_steps
-    roof = {"bound": "hbm", "kernel": "persist_kernel (batched, one graph launch per bench step)",
+    roof = {"bound": "hbm", "kernel": "alt_batch_kernel (turning passes, one cooperative launch per size)",
             "achieved": alg / launch_s / 1e9, "peak": peak, "unit": "GB/s", "frac": alg / launch_s / 1e9 / peak,
             "peak_source": peak_kind, "algorithmic_bytes_per_launch": alg, "avg_launch_ms": 1e3 * launch_s,
             "traffic": None,
@@ -362,15 +363,15 @@ def run_batched(a):
             "data": "synthetic (64 seeded traps x 8 g, no dataset)",
             "config": {"workload": "512 instances = 64 traps (lowest 5% of 1000 descents, N uniform in "
                                    "{16,18,20,22}, seed 2024) x 8 g in linspace(0.2, 0.5, 8); dt=0.02, 500 Trotter "
-                                   "steps, P_< and <d_H> every step; one persistent launch through a captured "
-                                   "CUDA graph per bench step",
+                                   "steps, P_< and <d_H> every step; one cooperative launch per size and "
+                                   "bench step",
                        "instances": len(inst), "trotter_steps_per_step": steps_t,
                        "tuning": {"lag": lag, "source": lag_src},
                        "amp_steps_per_step": amp_steps},
             "compare": dict(seq, batched_over_best_sequential=value / best_seq),
             "e2e": {"value": amp_steps * a.steps / wall, "unit": UNIT, "h2d_bytes_per_step": 24 * len(inst) + 501,
                     "d2h_bytes_per_step": 3 * 8 * len(inst) * 501},
-            "clocks": clocks.summary(), "roofline": roof, "gpu_launches": a.steps,
+            "clocks": clocks.summary(), "roofline": roof, "gpu_launches": a.steps * len(set(d["n"] for d in inst)),
             "check": {"p_less_mean_last": float(np.mean(p[:, -1])), "norm_max_dev": float(np.max(np.abs(nn - 1)))}}
     eng.close()
     if not a.no_cpu_baseline:
@@ -550,8 +551,9 @@ def run_matvec(a):
     per = dev_s / (a.steps * reps)
     peak, peak_kind = measured_peaks()
     alg = 18.0 * states  # x and y once (8 B each) and E once (2 B) per product
-    fb_, ft_ = kt.get("fs_block", (0, 0.0)), kt.get("fs_tile", (0, 0.0))
-    fs = (fb_[0] + ft_[0], fb_[1] + ft_[1])
+    fs, tp_ = kt.get("fs_turn", (0, 0.0)), kt.get("fs_pass", (0, 0.0))
+    fb_ = kt.get("fs_block", (0, 0.0))
+    fs = (fs[0] + tp_[0] + fb_[0], fs[1] + tp_[1] + fb_[1])
     # CPU baseline: the oracle's per-state restatement (OpenMP, all host cores) at N = 24
     nc, xc = 24, np.random.default_rng(1).standard_normal(1 << 24)
     O.fullspace_matvec(nc, 0.35, xc)
@@ -566,15 +568,15 @@ def run_matvec(a):
             "config": {"workload": f"y = (E/N) x - 0.35 sum_j x[i ^ 2^j] over 2^{n} states, FP64, 10 products per "
                                    "bench step", "n": n, "products_per_step": reps,
                        "l2": f"x and y {8 * states / 2**30:.1f} GiB each > 126 MB L2, no flush needed",
-                       "passes": "block pass over 8192-state blocks (index bits 0-12 in shared memory, bits 13-22 "
-                                 "as L2 sweeps of partner blocks), then for n > 23 one strided tile pass over "
-                                 "bits [23, n) (each tile one tensor-map box)",
+                       "passes": "one cooperative launch from 23 bits on: a tile pass over the highest bits, then "
+                                 "slab by slab the middle bits and the lowest ones with the diagonal, the slab held "
+                                 "in L2 between the two; below, one block pass over 8192-state blocks",
                        "design_dram_bytes_per_state": 42},
-            "roofline": {"bound": "hbm", "kernel": "fs_block + fs_tile (all passes of one product)",
+            "roofline": {"bound": "hbm", "kernel": "fs_turn (one launch per product)",
                          "achieved": alg / per / 1e9,
                          "peak": peak, "unit": "GB/s", "frac": alg / per / 1e9 / peak, "peak_source": peak_kind,
                          "algorithmic_bytes_per_launch": alg, "avg_launch_ms": 1e3 * per, "traffic": None,
-                         "block_pass_avg_ms": fb_[1] / max(fb_[0], 1), "strided_pass_avg_ms": ft_[1] / max(ft_[0], 1)},
+                         "launches_per_product": fs[0] / reps},
             "cpu_baseline": {"value": cpu_rate, "unit": "states/s", "cores": os.cpu_count(), "kind": "port",
                              "sample": "3 products at N = 24 by the oracle's per-state restatement "
                                        "(oracle/trotter_oracle.cpp orc_fullspace_matvec, OpenMP)"},
@@ -676,9 +678,10 @@ def main():
     # ---- roofline of the dominant kernel ----
     S = 8 if prec == bk.BK_C64 else 16
     # algorithmic bytes per launch: a pass reads and writes the state once (2 S per
-    # amplitude); one persistent launch runs all T Trotter steps of a call (4 S per
-    # amplitude-step: two such passes per step)
+    # amplitude); one persistent or turning launch runs all T Trotter steps of a call
+    # (4 S per amplitude-step: two such passes per step)
     per_launch_bytes = {"measure": S, "plain_phase": 2 * S, "plain_rx": 2 * S, "persist": 4 * S * T,
+                        "turn": 4 * S * T,
                         "tile_a1": 2 * S, "tile_s2": 2 * S, "tile_s3": 2 * S, "tile_m": S}
     dom = max(timing.items(), key=lambda kv: kv[1][1])
     dname, (dl, dms) = dom
