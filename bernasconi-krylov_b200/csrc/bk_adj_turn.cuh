@@ -12,8 +12,9 @@
 // step rotated before it; a pass sums two steps' terms, one partial pair per CTA and
 // pass, added up in index order by adj_cross_kernel.
 //
-// Measured on a B200 (reverse us a step, complex64 / complex128): N = 20 ADJ20, 22
-// ADJ22, 24 ADJ24; bound by the latency of a tile's rounds at eight warps an SM.
+// Measured on a B200 (reverse us a step, complex64 / complex128): N = 20 17.7 / 28.3, 22
+// 64 / 128, 24 253 / 446, against 24.5 / 39, 73 / 186 and 359 / 626 for a launch per pass
+// and set; bound by the latency of a tile's rounds at eight warps an SM.
 #pragma once
 #include "bk_adjoint.cuh"
 #include "bk_alt.cuh"

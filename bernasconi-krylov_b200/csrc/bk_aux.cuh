@@ -213,7 +213,7 @@ __global__ void sample_kernel(const A* __restrict__ psi, uint32_t count, const d
   const uint32_t base = lo << kSampleChunkBits;
   const uint32_t len = min(1u << kSampleChunkBits, count - base);
   // the chunk's 32 blocks of 128 states: coalesced sums, lane b keeps block b's (a lane
-  // walking its own 128 states took 20 of the 85 us of a sampling point at n = 16)
+  // walking its own 128 states made a sampling point at n = 16 85 us instead of 70)
   double part = 0.0;
   for (uint32_t b = 0; b < 32u; ++b) {
     if (b * 128u >= len) break;

@@ -1146,9 +1146,9 @@ struct AltGeo {
 //     5.7 / 5.1 against 16.5 / 14.6 for a launch per pass).
 //   np <= 21: 2^12-element tiles, two CTAs an SM, two sets (np = 20: 12.3 / 12.2
 //     against 22.8 / 20.6 for a launch per pass; np = 21, a set of nine bits with one of
-//     them across lanes: 23.8 / 22.7 against 26.0 / 23.7 with 2^13-element tiles).
+//     them across lanes: 23.0 / 22.6 against 26.0 / 23.7 with 2^13-element tiles).
 //   np <= 23: 2^13-element tiles with 32 elements a thread, so that two sets still do
-//     (one pass a step): np = 23 94 / 86 against 103 / 110 with three sets.
+//     (one pass a step): np = 23 97 / 88 against 103 / 110 with three sets.
 //   beyond: 2^12-element tiles, three sets (two passes a step).
 bool alt_geometry(int np, AltGeo* g) {
   if (np < kElemBits + 1 || np > 30) return false;

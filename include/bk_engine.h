@@ -279,7 +279,9 @@ int bk_d_min(bk_ctx* ctx, int n, uint64_t bits, int64_t target, int max_d, int* 
  *       statevector (two from 25 qubits in complex64, 24 in complex128, on), all
  *       of them in one cooperative launch; complex64 takes its phase from the full
  *       per-energy table; the knobs below do not apply to it, and with
- *       BK_OPT_E_SOURCE = 1 mode 0 runs; bk_adjoint's forward run follows it,
+ *       BK_OPT_E_SOURCE = 1 mode 0 runs; bk_adjoint's forward run follows it, and
+ *       its reverse sweep too unless BK_OPT_ADJ_A1 = 1; complex64 runs up to 18
+ *       qubits compute in complex128 (no slower there) and report its sums,
  *       0 = persistent dataflow kernel (all steps in one launch,
  *       L2 hand-off between the A1 and S2 tasks), 1 = one grid launch per pass,
  *       2 = a grid launch for the A1 pass and ONE persistent launch for both
@@ -414,8 +416,8 @@ int bk_measure_noalloc(int n, int precision, const void* d_state, int64_t e0, ui
  * diag = scale * E(s) as in :388-392). x and y are 16-byte aligned device pointers on
  * the context's device and must not alias; the call runs on the context's stream and returns
  * after it has finished (the caller's own work on x must be complete before).
- * method: BK_FUSED = tile passes over 64 KB shared-memory tiles (x read once per
- * pass), BK_PLAIN = the reference's one-thread-per-state form (comparison).
+ * method: BK_FUSED = tile passes over 64 KB shared-memory tiles (from 23 bits on
+ * one cooperative launch of three index sets, 42 bytes of DRAM a state), BK_PLAIN = the reference's one-thread-per-state form (comparison).
  *
  * bk_fullspace_lanczos: the reference's Diagonalizer::solve_fullspace_lanczos
  * (diagonalizer.cuh:377-416 with run_gpu_lanczos_internal :418-560): plain Lanczos
