@@ -17,7 +17,7 @@
 #include <iostream>
 #include <limits>
 #include <map>
-#include <mutex>
+#include <memory>
 #include <random>
 #include <string>
 #include <unordered_set>
@@ -62,7 +62,6 @@ struct TimingRec {
 
 struct bk_ctx {
   int device = 0;
-  bool counted = false;  // among the contexts that keep the process's pinned room
   cudaStream_t stream = nullptr;
   std::string last_error;
   // E table cache (per n), like the reference's ensure_cached_energies
@@ -1084,57 +1083,6 @@ char* stage(bk_ctx* c, size_t bytes) {
   if (c->h_stage.size() < bytes) c->h_stage.resize(bytes);
   return c->h_stage.data();
 }
-
-// One pinned room of 8 MB for the whole process, for the host arrays of large descent
-// batches: pinning it takes a millisecond or two, so it is not a context's own. One call
-// holds it at a time (another uses pageable memory meanwhile); it is taken on first use
-// and given back when the last context closes.
-class PinnedRoom {
- public:
-  static constexpr size_t kBytes = (size_t)8 << 20;
-  void context_opened() {
-    std::lock_guard<std::mutex> l(m_);
-    ++contexts_;
-  }
-  void context_closed() {
-    std::lock_guard<std::mutex> l(m_);
-    if (--contexts_ == 0 && room_) {
-      cudaFreeHost(room_);
-      room_ = nullptr;
-    }
-  }
-  char* take(size_t bytes) {
-    std::lock_guard<std::mutex> l(m_);
-    if (bytes > kBytes || busy_) return nullptr;
-    if (!room_ && cudaHostAlloc(&room_, kBytes, cudaHostAllocPortable) != cudaSuccess) {
-      cudaGetLastError();
-      room_ = nullptr;
-      return nullptr;
-    }
-    busy_ = true;
-    return static_cast<char*>(room_);
-  }
-  void give_back() {
-    std::lock_guard<std::mutex> l(m_);
-    busy_ = false;
-  }
-
- private:
-  std::mutex m_;
-  void* room_ = nullptr;
-  int contexts_ = 0;
-  bool busy_ = false;
-};
-PinnedRoom g_pinned;
-struct PinnedHold {  // the room for the length of a call
-  char* p;
-  explicit PinnedHold(size_t bytes) : p(g_pinned.take(bytes)) {}
-  PinnedHold(const PinnedHold&) = delete;
-  PinnedHold& operator=(const PinnedHold&) = delete;
-  ~PinnedHold() {
-    if (p) g_pinned.give_back();
-  }
-};
 
 struct AltGeo {
   int tb = 0, w2 = 0, w3 = 0;
@@ -2611,8 +2559,6 @@ int bk_create(int device, bk_ctx** out) {
   }
   cudaMemset(c->d_ticket, 0, sizeof(unsigned int));
   cudaMemset(c->d_err, 0, sizeof(int));
-  g_pinned.context_opened();
-  c->counted = true;
   *out = c;
   return BK_OK;
 }
@@ -2634,7 +2580,6 @@ int bk_destroy(bk_ctx* c) {
     cudaEventDestroy(e.second);
   }
   if (c->stream) cudaStreamDestroy(c->stream);
-  if (c->counted) g_pinned.context_closed();
   delete c;
   return BK_OK;
 }
@@ -2672,9 +2617,10 @@ int bk_steepest_descent_gpu(bk_ctx* c, int n, const uint64_t* starts, int64_t co
   BK_CUDA(c, cudaSetDevice(c->device));
   // The copies cost more than the descents (65536 starts of n = 28: 58 us of kernel, 210
   // us of pageable copies of 8-byte words one array after another), so states up to 32
-  // spins, energies and evaluations cross as 4-byte words through pinned memory, the
-  // results in one copy, and the host threads widen them into the caller's arrays, whose
-  // fresh pages then fault in parallel (120 us the call; 285 us with one thread).
+  // spins, energies and evaluations cross as 4-byte words, the results in one copy, and
+  // the host threads widen them into the caller's arrays, whose fresh pages then fault in
+  // parallel: 230 us a call, 450 a context's first (450 and 850 with the words as the
+  // caller has them). Pinned memory makes that 120, but pinning takes 4 to 11 ms of the first.
   const size_t cnt = (size_t)count, word = n <= 32 ? 4 : 8;
   const size_t need = cnt * (2 * word + 8) + 64;
   BK_TRY(ensure_buffer(c, &c->d_descent, &c->descent_cap, need));
@@ -2684,10 +2630,9 @@ int bk_steepest_descent_gpu(bk_ctx* c, int n, const uint64_t* starts, int64_t co
   const unsigned long long budget = max_evals == 0 ? ~0ull : (unsigned long long)max_evals;
   const unsigned grid = (unsigned)((cnt + kDescentWarps - 1) / kDescentWarps);
   const size_t host_bytes = cnt * (word + 8);
-  std::vector<char> pageable;
-  PinnedHold pinned(host_bytes >= ((size_t)64 << 10) ? host_bytes : ~(size_t)0);
-  if (!pinned.p) pageable.resize(host_bytes);
-  char* h = pinned.p ? pinned.p : pageable.data();
+  // the context keeps up to 8 MB of it warm; a larger batch returns its own
+  std::unique_ptr<char[]> own(host_bytes > ((size_t)8 << 20) ? new char[host_bytes] : nullptr);
+  char* h = own ? own.get() : stage(c, host_bytes);
   size_t e = 0;
   if (n <= 32) {
     uint32_t* narrow = reinterpret_cast<uint32_t*>(h);

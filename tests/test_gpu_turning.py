@@ -7,6 +7,7 @@ of rounding on amplitudes of norm 1: 1e-13 absolute on P_< and the norm, n times
 that on <d_H>. complex64: the engine's own bars (conftest)."""
 import numpy as np
 import pytest
+import torch
 
 import bk_b200 as bk
 from tests.conftest import C64_DH_BAR, C64_DP_BAR
@@ -35,8 +36,8 @@ def _both(eng, n, precision, steps, **kw):
 
 # element bits: 13 / 18 (first and last of the 2^10 tiles), 14, 15 (a set of 4 and of 5
 # bits: turn in the first and in the second round), 19, 20, 21, 23 and the three-set
-# sizes from 24 on
-@pytest.mark.parametrize("n", [13, 14, 15, 18, 19, 20, 21, 23, 24, 25])
+# sizes from 24 on, up to the widest sets (30: 9 + 9 bits)
+@pytest.mark.parametrize("n", [13, 14, 15, 16, 17, 18, 19, 20, 21, 22, 23, 24, 25, 26, 27, 28, 29, 30])
 @pytest.mark.parametrize("steps", [1, 6])
 def test_sizes_match_the_tile_passes_c128(eng, n, steps):
     a, b = _both(eng, n, bk.BK_C128, steps)
@@ -45,7 +46,7 @@ def test_sizes_match_the_tile_passes_c128(eng, n, steps):
     assert np.max(np.abs(a[2] - b[2])) <= BAR128
 
 
-@pytest.mark.parametrize("n", [14, 19, 20, 22, 24, 25, 27])
+@pytest.mark.parametrize("n", [14, 19, 20, 21, 22, 23, 24, 25, 26, 27, 28, 29, 30])
 def test_sizes_match_the_tile_passes_c64(eng, n):
     a, b = _both(eng, n, bk.BK_C64, 7, measure=[0, 3, 7])
     assert np.max(np.abs(a[0] - b[0])) <= C64_DP_BAR
@@ -138,7 +139,7 @@ def test_small_runs_split_at_sampling_points(eng, n):
 # the reverse sweep's tiles: 2^10 (13, 14, 18 element bits: a set of 3, 4, 8 bits), 2^12
 # with two sets (19, 20, 21) and with three (22, 23, 25), against the launch-per-pass sweep;
 # checkpoints that split the sweep into stretches of odd and even length
-@pytest.mark.parametrize("n", [13, 14, 18, 19, 20, 21, 22, 23, 25])
+@pytest.mark.parametrize("n", [13, 14, 16, 17, 18, 19, 20, 21, 22, 23, 24, 25, 26, 27, 28])
 def test_reverse_sweep_matches_the_launch_per_pass_sweep(eng, n):
     T, g = 11, np.linspace(0.3, 0.42, 11)
     bits, e0 = bk.select_trap(n, 13, 100, 0.3)
@@ -161,3 +162,18 @@ def test_reverse_sweep_complex64(eng, n):
     b = eng.adjoint(n, bits, g, 0.04, T, e0=e0, precision=bk.BK_C128, checkpoint_every=3)
     assert np.max(np.abs(a[1] - b[1])) <= 1e-4 * np.max(np.abs(b[1]))  # the complex64 gradient's bar
     assert a[2]["max_drift"] <= 1e-5
+
+
+# the full-space product in tile passes (from 23 bits on): every split of the far bits,
+# against the per-state form on the same vectors
+@pytest.mark.parametrize("n", [23, 24, 25, 26, 27, 28, 29, 30])
+def test_full_space_tile_passes_match_the_per_state_form(eng, n):
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.randn(1 << n, generator=gen, device="cuda", dtype=torch.float64)
+    y, ref = torch.empty_like(x), torch.empty_like(x)
+    torch.cuda.synchronize()
+    eng.fullspace_matvec(n, 0.35, x, y)
+    eng.fullspace_matvec(n, 0.35, x, ref, method=bk.BK_PLAIN)
+    # n + 1 terms summed in another order
+    bound = 1e-14 * (n + 1) * float(ref.abs().max())
+    assert float(y.sub_(ref).abs().max()) <= bound
