@@ -219,7 +219,8 @@ __global__ void __launch_bounds__(kFtThreads, 2) fs_turn_kernel(const __grid_con
   bool joined = !two;  // phase 1 is behind every CTA
   FtTask t = ft_task(P, blockIdx.x);
   issue(t);
-  for (uint32_t it = 0; t.kind != FT_END; ++it) {
+  uint32_t it = 0;
+  for (; t.kind != FT_END; ++it) {
     const FtTask nt = ft_task(P, blockIdx.x + (it + 1u) * gridDim.x);
     if (t.kind != FT_S2 && (!joined || t.kind == FT_S1)) {
       // y of phase 1 from every CTA, or of the slab's A tiles
@@ -233,7 +234,7 @@ __global__ void __launch_bounds__(kFtThreads, 2) fs_turn_kernel(const __grid_con
         if (!ok) *stop = 1;
       }
       joined = true;
-      __syncthreads();
+      if (__syncthreads_or(*stop)) break;
     }
     // where the thread's doubles live: tile position p = tid + 256 j
     const int w = t.kind == FT_A ? 0 : t.kind == FT_S1 ? P.w1 : P.w2;
@@ -263,7 +264,7 @@ __global__ void __launch_bounds__(kFtThreads, 2) fs_turn_kernel(const __grid_con
       };
       fetch(0);
       fetch(1);
-      if (!*stop && !mbar_wait_bounded(fb, it & 1u, P.err)) *stop = 1;
+      if (!mbar_wait_bounded(fb, it & 1u, P.err)) *stop = 1;
       double x[kFtPer];
 #pragma unroll
       for (int j = 0; j < kFtPer; ++j) x[j] = ft[tid + kFtThreads * j];
@@ -290,7 +291,7 @@ __global__ void __launch_bounds__(kFtThreads, 2) fs_turn_kernel(const __grid_con
       };
       fetch(0);
       fetch(1);
-      if (!*stop && !mbar_wait_bounded(fb, it & 1u, P.err)) *stop = 1;
+      if (!mbar_wait_bounded(fb, it & 1u, P.err)) *stop = 1;
       double x[kFtPer];
 #pragma unroll
       for (int j = 0; j < kFtPer; ++j) x[j] = ft[tid + kFtThreads * j];
@@ -314,12 +315,11 @@ __global__ void __launch_bounds__(kFtThreads, 2) fs_turn_kernel(const __grid_con
     // (the barrier above is behind every store of the task)
     if (tid == 0 && t.kind == FT_A) red_release_add(P.done + t.slab, 1u);
     t = nt;
-    if (__syncthreads_or(*stop)) {
-      // a failed run: a copy on its way lands before the CTA leaves
-      if (tid == 0) mbar_wait_bounded(fb, (it + 1u) & 1u, P.err);
-      break;
-    }
+    if (__syncthreads_or(*stop)) break;
   }
+  // a failed run: the copy of task `it` (phase it) may still be on its way, and lands before
+  // the CTA leaves; none was issued behind it, stop was set first
+  if (tid == 0 && *stop) mbar_wait_bounded(fb, it & 1u, P.err);
 }
 
 // The reference's form (diagonalizer.cuh:60-77): one thread per state, its n
