@@ -108,7 +108,7 @@ struct bk_ctx {
   size_t alt_cap = 0;
   std::vector<char> h_stage;  // a run's uploads, put together for one copy
   std::map<std::pair<const void*, int>, int> occupancy;  // (kernel, dynamic smem) -> CTAs per SM
-  uint32_t wait_polls = 0;    // persistent engine: polls of a dependency wait before it gives up (0 = default)
+  uint32_t wait_polls = 0;    // polls of a pass barrier's or dependency's wait before it gives up (0 = default)
   uint64_t s23_checked = 0;   // fused strided pass geometry (np, a1, w2, lag) whose closed form was checked
   int64_t hold_step = -1;     // test hook: launch step whose dependency can never be met (-1 = off)
   std::map<int, uint16_t*> batch_E;  // E tables of batched runs, per n
@@ -1167,6 +1167,10 @@ int alt_set(bk_ctx* c, void* state, int np, int cp, int h0, int w, CUtensorMap* 
   return BK_OK;
 }
 
+// The test hook in turning passes: a launch's arrival counter starts one short of zero, so
+// that its first pass barrier is never met.
+bool held(const bk_ctx* c, int64_t k0, int64_t k1) { return c->hold_step >= k0 && c->hold_step < k1; }
+
 constexpr size_t kAltPartialBytes = (size_t)64 << 20;  // partial sums of one launch (more rows: more launches)
 
 // levels of the phase table for n
@@ -1279,7 +1283,8 @@ int alt_launch(bk_ctx* c, AltRun<R>& r, int k0, int k1, bool first, int row0, in
   r.D.k1 = k1;
   r.D.row0 = row0;
   r.D.meas_first = first ? 1 : 0;
-  if (!first) BK_CUDA(c, cudaMemsetAsync(r.B.ctr, 0, sizeof(unsigned int), st));
+  const bool hold = held(c, k0, k1);
+  if (!first || hold) BK_CUDA(c, cudaMemsetAsync(r.B.ctr, hold ? 0xFF : 0, sizeof(unsigned int), st));
   size_t ev = 0;
   BK_TRY(ev_begin(c, "turn", &ev));
   void* args[] = {&r.D, &r.I, &r.B};
@@ -1541,7 +1546,7 @@ int batch_turning(bk_ctx* c, const std::vector<BatchGeo>& geo, int T, const std:
   for (auto& kv : classes) {
     Class& k = kv.second;
     alt_table(k.n, k.angle_unit, reinterpret_cast<entry*>(h + k.o_tab), k.D.c0, k.D.n_j);
-    std::memset(h + k.o_ctr, 0, (size_t)k.groups * 128);
+    std::memset(h + k.o_ctr, held(c, 0, T) ? 0xFF : 0, (size_t)k.groups * 128);
     uint16_t* dE = nullptr;
     BK_TRY(batch_energy(c, k.n, &dE));
     k.D.E = dE;
@@ -2079,6 +2084,9 @@ int adj_reverse_turning(bk_ctx* c, int n, int T, const AltRun<R>& fwd, const typ
   std::vector<int> seg_end;
   for (const AdjReset& r : resets) seg_end.push_back(r.after_j + 1);
   seg_end.push_back(T);
+  for (int s = 0; s < n_seg; ++s)
+    if (held(c, (int64_t)T + (s > 0 ? seg_end[(size_t)s - 1] : 0), (int64_t)T + seg_end[(size_t)s]))
+      std::memset(h + o_ctr + (size_t)s * 128, 0xFF, sizeof(unsigned int));
   for (int j = 0, s = 0; j < T; ++j) {
     while (j >= seg_end[(size_t)s]) ++s;
     reinterpret_cast<int*>(h + o_row)[j] = s + (three ? 2 : 1) * j;
@@ -2501,7 +2509,7 @@ int device_error(bk_ctx* c, int e) {
   cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream);
   cudaMemsetAsync(c->d_ticket, 0, sizeof(unsigned int), c->stream);
   cudaStreamSynchronize(c->stream);
-  if (e == DEV_TIMEOUT) return fail(c, BK_ERR_TIMEOUT, "a kernel's bounded wait for its tile load gave up");
+  if (e == DEV_TIMEOUT) return fail(c, BK_ERR_TIMEOUT, "a bounded device wait gave up (a tile's load or a pass barrier)");
   return fail(c, BK_ERR_CUDA, "device error word %d", e);
 }
 int check_device_error(bk_ctx* c) {
@@ -3507,6 +3515,7 @@ int fs_turn(bk_ctx* c, int n, double g, double scale, const double* x, double* y
   P.abort = reinterpret_cast<int*>(P.done + P.slabs + 1);
   P.err = c->d_err;
   P.poll_limit = c->wait_polls > 0 ? c->wait_polls : kWaitPolls * 4u;
+  if (c->hold_step >= 0) BK_CUDA(c, cudaMemsetAsync(P.arrived, 0xFF, sizeof(unsigned int), c->stream));
   const void* fn = reinterpret_cast<const void*>(fs_turn_kernel);
   BK_TRY(allow_smem(c, fn, kFtSmem));
   size_t ev = 0;

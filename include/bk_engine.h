@@ -306,13 +306,18 @@ int bk_d_min(bk_ctx* ctx, int n, uint64_t bits, int64_t target, int max_d, int* 
  *   BK_OPT_ADJ_A1: bk_adjoint's reverse sweep, 1 = the warp-local A1 layout for
  *       both statevectors (element bits 0-8, strided passes from bit 9; up to 27
  *       element bits), 0 (default) = the 12-bit A1 of the forward geometry;
- *   BK_OPT_WAIT_POLLS: persistent engine, polls of one dependency wait before
- *       it gives up with BK_ERR_TIMEOUT (1000 .. 2^24; 0 = the default 2^24);
- *   BK_OPT_TEST_HOLD_STEP: failure-path test hook, off (-1) by default: in the
- *       persistent engine (BK_OPT_ENGINE_MODE 0), the A1 tasks of this step of a
- *       launch wait for one completion more than can arrive, as if a producer
- *       were lost; the bounded wait runs out, every CTA leaves, and bk_evolve
- *       returns BK_ERR_TIMEOUT with the context still usable;
+ *   BK_OPT_WAIT_POLLS: polls of one dependency wait (persistent engine) or pass
+ *       barrier (turning passes, full-space tile passes) before it gives up with
+ *       BK_ERR_TIMEOUT (1000 .. 2^24; 0 = the default 2^24);
+ *   BK_OPT_TEST_HOLD_STEP: failure-path test hook, off (-1) by default. Turning
+ *       passes: the first pass barrier of the launch that covers this step is
+ *       short of one arrival, as if a CTA were lost (bk_evolve above 12 qubits,
+ *       bk_evolve_batch, bk_adjoint; steps n_steps + j are those of bk_adjoint's
+ *       reverse sweep, in its order). Full-space tile passes (23 bits on): any
+ *       value from 0 on does so. Persistent engine (BK_OPT_ENGINE_MODE 0): the A1
+ *       tasks of this step of a launch wait for one completion more than can
+ *       arrive. The bounded wait runs out, every CTA leaves, and the call returns
+ *       BK_ERR_TIMEOUT with the context still usable;
  *   BK_OPT_PHASE_TABLE: complex64, per-pass schedules (modes 1 and 2), every
  *       A1 kernel: 1 = the diagonal phase of every energy level from one
  *       table entry (E = floor(n/2) mod 4 for every LABS energy, so at most 2139
