@@ -20,7 +20,7 @@ LIB = os.path.join(LIB_DIR, "libbk_b200.so")
 SOURCES = ["csrc/bk_engine.cu", "csrc/bk_alt_f32.cu", "csrc/bk_alt_f64.cu", "csrc/bk_adj_turn_f32.cu", "csrc/bk_adj_turn_f64.cu",
            "csrc/bk_noalloc.cu"]
 HEADERS = ["csrc/bk_device.cuh", "csrc/bk_fused.cuh", "csrc/bk_aux.cuh", "csrc/bk_persist.cuh", "csrc/bk_adjoint.cuh", "csrc/bk_lanczos.cuh", "csrc/bk_s23.cuh", "csrc/bk_alt.cuh", "csrc/bk_small.cuh",
-           "csrc/bk_adj_turn.cuh"]
+           "csrc/bk_adj_turn.cuh", "csrc/bk_stage.hpp"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",
          "--expt-relaxed-constexpr", "-Xcompiler", "-fPIC,-fopenmp", "-ccbin", "/usr/bin/g++",

@@ -34,6 +34,7 @@
 #include "bk_persist.cuh"
 #include "bk_s23.cuh"
 #include "bk_small.cuh"
+#include "bk_stage.hpp"
 
 using namespace bk;
 
@@ -59,6 +60,17 @@ struct TimingRec {
 };
 
 }  // namespace
+
+// The copies enqueued so far: an event on the context's stream.
+struct StreamFence {
+  cudaStream_t stream = nullptr;
+  cudaEvent_t event = nullptr;
+  bool mark() {
+    if (!event && cudaEventCreateWithFlags(&event, cudaEventDisableTiming) != cudaSuccess) return false;
+    return cudaEventRecord(event, stream) == cudaSuccess;
+  }
+  bool wait() { return cudaEventSynchronize(event) == cudaSuccess; }
+};
 
 struct bk_ctx {
   int device = 0;
@@ -106,7 +118,7 @@ struct bk_ctx {
   int adj_a1 = 0;             // adjoint reverse sweep A1: 0 = 12-bit, 1 = warp-local (element bits 0-8)
   void* d_alt = nullptr;      // turning passes: phase table, per-step arrays, partial sums, counters
   size_t alt_cap = 0;
-  std::vector<char> h_stage;  // a run's uploads, put together for one copy
+  StageRoom<StreamFence> h_stage;  // a run's uploads, put together for one copy
   std::map<std::pair<const void*, int>, int> occupancy;  // (kernel, dynamic smem) -> CTAs per SM
   uint32_t wait_polls = 0;    // polls of a pass barrier's or dependency's wait before it gives up (0 = default)
   uint64_t s23_checked = 0;   // fused strided pass geometry (np, a1, w2, lag) whose closed form was checked
@@ -1077,11 +1089,13 @@ int check_phase(bk_ctx* c, int n, double angle_unit) {
   return BK_OK;
 }
 
-// Host memory of a run's uploads, kept warm between calls. Pageable: a small copy from
-// it is staged at once, and pinning memory costs milliseconds per context.
-char* stage(bk_ctx* c, size_t bytes) {
-  if (c->h_stage.size() < bytes) c->h_stage.resize(bytes);
-  return c->h_stage.data();
+// Room for a run's uploads (bk_stage.hpp); `staged` after the copies from it.
+int stage(bk_ctx* c, size_t bytes, char** out) {
+  *out = c->h_stage.take(bytes);
+  return *out ? BK_OK : fail(c, BK_ERR_OOM, "no host memory for %zu bytes of uploads", bytes);
+}
+int staged(bk_ctx* c) {
+  return c->h_stage.sent() ? BK_OK : fail(c, BK_ERR_CUDA, "the uploads' event: %s", cudaGetErrorString(cudaGetLastError()));
 }
 
 struct AltGeo {
@@ -1249,13 +1263,15 @@ int alt_prepare(bk_ctx* c, int n, uint64_t s0, int64_t e0, double angle_unit, co
   run->max_rows = (int)std::max<size_t>(kAltPartialBytes / row_bytes, 1);
   const size_t o_part = b.take(row_bytes * (size_t)std::max(1, std::min(S.n_meas, run->max_rows + 1)));
   BK_TRY(ensure_buffer(c, &c->d_alt, &c->alt_cap, b.off));
-  char *h = stage(c, up), *d = static_cast<char*>(c->d_alt);
+  char *h = nullptr, *d = static_cast<char*>(c->d_alt);
+  BK_TRY(stage(c, up, &h));
   alt_table(n, angle_unit, reinterpret_cast<entry*>(h + o_tab), D.c0, D.n_j);
   std::copy(tans.begin(), tans.end(), reinterpret_cast<R*>(h + o_tan));
   std::copy(scales.begin(), scales.end(), reinterpret_cast<R*>(h + o_sc));
   std::copy(S.slot.begin(), S.slot.end(), reinterpret_cast<int*>(h + o_slot));
   std::memset(h + o_ctr, 0, 64);
   BK_CUDA(c, cudaMemcpyAsync(d, h, up, cudaMemcpyHostToDevice, c->stream));
+  BK_TRY(staged(c));
   D.E = c->d_E;
   D.tab = reinterpret_cast<const entry*>(d + o_tab);
   D.slot = reinterpret_cast<const int*>(d + o_slot);
@@ -1354,12 +1370,14 @@ int evolve_small(bk_ctx* c, const bk_evolve_params* p, const Schedule& S, double
   const void* fn = small_kernel_of(np, &threads, &tile);
   const size_t o_part = b.take((size_t)std::max(S.n_meas, 1) * 3 * (threads / 32) * sizeof(double));
   BK_TRY(ensure_buffer(c, &c->d_small, &c->small_cap, b.off));
-  char *h = stage(c, up), *d = static_cast<char*>(c->d_small);
+  char *h = nullptr, *d = static_cast<char*>(c->d_small);
+  BK_TRY(stage(c, up, &h));
   alt_table(n, angle_unit, reinterpret_cast<entry*>(h + o_tab), P.c0, n_j);
   for (int k = 0; k <= T; ++k)
     reinterpret_cast<SmallStep*>(h + o_step)[k] = {k < T ? tans[(size_t)k] : 0.0, k < T ? scales[(size_t)k] : 1.0,
                                                       S.slot[(size_t)k], 0};
   BK_CUDA(c, cudaMemcpyAsync(d, h, up, cudaMemcpyHostToDevice, c->stream));
+  BK_TRY(staged(c));
   BK_TRY(allow_smem(c, fn, tile));
   P.state = reinterpret_cast<amp*>(c->d_state);
   P.E = c->d_E;
@@ -1521,7 +1539,8 @@ int batch_turning(bk_ctx* c, const std::vector<BatchGeo>& geo, int T, const std:
     part = std::max(part, (size_t)kv.second.groups * 2 * 3 * (size_t)std::max(n_meas, 1) * kv.second.G * sizeof(double));
   const size_t o_part = b.take(part);
   BK_TRY(ensure_buffer(c, &c->d_batch, &c->batch_cap, b.off));
-  char *h = stage(c, up), *d = static_cast<char*>(c->d_batch);
+  char *h = nullptr, *d = static_cast<char*>(c->d_batch);
+  BK_TRY(stage(c, up, &h));
   std::copy(tans.begin(), tans.end(), reinterpret_cast<R*>(h + o_tan));
   std::copy(scales.begin(), scales.end(), reinterpret_cast<R*>(h + o_scale));
   std::copy(slot.begin(), slot.end(), reinterpret_cast<int*>(h + o_slot));
@@ -1559,6 +1578,7 @@ int batch_turning(bk_ctx* c, const std::vector<BatchGeo>& geo, int T, const std:
   size_t ev = 0;
   BK_TRY(ev_begin(c, "batch", &ev));
   BK_CUDA(c, cudaMemcpyAsync(d, h, up, cudaMemcpyHostToDevice, st));
+  BK_TRY(staged(c));
   BK_CUDA(c, cudaMemsetAsync(state, 0, state_bytes, st));
   set_basis_many_kernel<<<(n_inst + 127) / 128, 128, 0, st>>>(state, reinterpret_cast<unsigned long long*>(d + o_offs),
                                                               reinterpret_cast<unsigned int*>(d + o_idx), c64 ? 1 : 0,
@@ -2076,7 +2096,8 @@ int adj_reverse_turning(bk_ctx* c, int n, int T, const AltRun<R>& fwd, const typ
   const size_t o_dev = b.take(std::max<size_t>(resets.size(), 1) * kResetGrid * sizeof(double));
   const size_t o_part = b.take((size_t)n_rows * G * 2 * sizeof(double));
   BK_TRY(ensure_buffer(c, &c->d_adj, &c->adj_cap, b.off));
-  char *h = stage(c, up), *d = static_cast<char*>(c->d_adj);
+  char *h = nullptr, *d = static_cast<char*>(c->d_adj);
+  BK_TRY(stage(c, up, &h));
   std::copy(t_rev.begin(), t_rev.end(), reinterpret_cast<R*>(h + o_tan));
   std::copy(sc_rev.begin(), sc_rev.end(), reinterpret_cast<R*>(h + o_sc));
   std::copy(lg_rev.begin(), lg_rev.end(), reinterpret_cast<double*>(h + o_lg));
@@ -2092,6 +2113,7 @@ int adj_reverse_turning(bk_ctx* c, int n, int T, const AltRun<R>& fwd, const typ
     reinterpret_cast<int*>(h + o_row)[j] = s + (three ? 2 : 1) * j;
   }
   BK_CUDA(c, cudaMemcpyAsync(d, h, up, cudaMemcpyHostToDevice, st));
+  BK_TRY(staged(c));
   D.tan = reinterpret_cast<const R*>(d + o_tan);
   D.scale = reinterpret_cast<const R*>(d + o_sc);
   D.lg = reinterpret_cast<const double*>(d + o_lg);
@@ -2565,6 +2587,7 @@ int bk_create(int device, bk_ctx** out) {
     bk_destroy(c);
     return BK_ERR_CUDA;
   }
+  c->h_stage.fence().stream = c->stream;
   cudaMemset(c->d_ticket, 0, sizeof(unsigned int));
   cudaMemset(c->d_err, 0, sizeof(int));
   *out = c;
@@ -2587,6 +2610,7 @@ int bk_destroy(bk_ctx* c) {
     cudaEventDestroy(e.first);
     cudaEventDestroy(e.second);
   }
+  if (c->h_stage.fence().event) cudaEventDestroy(c->h_stage.fence().event);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
   return BK_OK;
@@ -2639,14 +2663,21 @@ int bk_steepest_descent_gpu(bk_ctx* c, int n, const uint64_t* starts, int64_t co
   const unsigned grid = (unsigned)((cnt + kDescentWarps - 1) / kDescentWarps);
   const size_t host_bytes = cnt * (word + 8);
   // the context keeps up to 8 MB of it warm; a larger batch returns its own
-  std::unique_ptr<char[]> own(host_bytes > ((size_t)8 << 20) ? new char[host_bytes] : nullptr);
-  char* h = own ? own.get() : stage(c, host_bytes);
+  std::unique_ptr<char[]> own;
+  char* h = nullptr;
+  if (host_bytes > ((size_t)8 << 20)) {
+    own.reset(h = new (std::nothrow) char[host_bytes]);
+    if (!h) return fail(c, BK_ERR_OOM, "no host memory for %zu bytes of uploads", host_bytes);
+  } else {
+    BK_TRY(stage(c, host_bytes, &h));
+  }
   size_t e = 0;
   if (n <= 32) {
     uint32_t* narrow = reinterpret_cast<uint32_t*>(h);
 #pragma omp parallel for schedule(static) if (cnt >= 16384)
     for (long long i = 0; i < (long long)cnt; ++i) narrow[i] = (uint32_t)starts[i];
     BK_CUDA(c, cudaMemcpyAsync(d + o_st, narrow, cnt * 4, cudaMemcpyHostToDevice, st));
+    if (!own) BK_TRY(staged(c));
   } else {
     BK_CUDA(c, cudaMemcpyAsync(d + o_st, starts, cnt * 8, cudaMemcpyHostToDevice, st));
   }
