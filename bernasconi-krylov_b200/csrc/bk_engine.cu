@@ -506,6 +506,38 @@ struct Log2Memo {
   }
 };
 
+// A run's steps one after another: the tangent the kernels use, the exact power of two
+// applied before it, and the log2 of the state's omitted scale.
+template <class R>
+struct StepTurns {
+  int n;
+  double dt;
+  long double lg = 0.0L;  // before the step about to be taken
+  double last_g = 0.0, exact = 0.0;
+  double missed = 0.0;    // the angle by which the tangents so far fall short
+  Log2Memo<R> memo;
+  StepTurns(int n_, double dt_) : n(n_), dt(dt_) {}
+  void next(double g, R* tan, R* scale) {
+    if (g != last_g) exact = std::tan((last_g = g) * dt);
+    // The rounding of a step's tangent is made up for in the next one, so a run's total
+    // rotation is not off by its number of steps times one rounding. Tangents do not add:
+    // what was missed is an angle, tan(a + d) = (tan a + d) / (1 - d tan a) up to d^2
+    // (complex128: d = 0; complex64: |d| < 6e-8).
+    const double under = 1.0 - missed * exact;
+    const double want = under != 0.0 ? (exact + missed) / under : exact;
+    *tan = (R)want;
+    const double t = (double)*tan;
+    missed = std::isfinite(t) ? (want - t) / (1.0 + want * t) : 0.0;
+    *scale = (R)1;
+    if (lg >= (long double)kRescaleLog2) {
+      *scale = (R)std::ldexp(1.0, -kRescaleLog2);
+      lg -= (long double)kRescaleLog2;
+    }
+    // each butterfly multiplies the norm^2 of its pair by 1 + t^2, t the value the kernel uses
+    lg += 0.5L * (long double)n * memo.log2_1t2(*tan);
+  }
+};
+
 struct Schedule {
   std::vector<double> g;        // per step
   std::vector<int> slot;        // per step (n_steps + 1): measurement row or -1
@@ -1652,26 +1684,13 @@ int evolve_batch_t(bk_ctx* c, const bk_batch_params* bp, const bk_batch_instance
   std::vector<R> tans((size_t)n_inst * std::max(T, 1)), scales((size_t)n_inst * std::max(T, 1));
   std::vector<long double> row_log2((size_t)n_inst * std::max(n_meas, 1), 0.0L);
   for (int i = 0; i < n_inst; ++i) {
-    long double lg = 0.0L;
-    double carry = 0.0, last_g = 0.0, exact = 0.0;
-    Log2Memo<R> memo;
+    StepTurns<R> turns(geo[(size_t)i].n, bp->dt);
     for (int k = 0; k <= T; ++k) {
-      if (slot[(size_t)k] >= 0) row_log2[(size_t)i * n_meas + slot[(size_t)k]] = lg;
+      if (slot[(size_t)k] >= 0) row_log2[(size_t)i * n_meas + slot[(size_t)k]] = turns.lg;
       if (k == T) break;
       const double gk = inst[i].g ? inst[i].g[k] : inst[i].g_const;
       if (!is_finite(gk)) return fail(c, BK_ERR_INVALID, "instance %d: g[%d] not finite", i, k);
-      if (gk != last_g) exact = std::tan((last_g = gk) * bp->dt);
-      const double want = exact + carry;  // as in evolve_fused
-      const R tf = (R)want;
-      carry = want - (double)tf;
-      R sc = (R)1;
-      if (lg >= (long double)kRescaleLog2) {
-        sc = (R)std::ldexp(1.0, -kRescaleLog2);
-        lg -= (long double)kRescaleLog2;
-      }
-      tans[(size_t)i * T + k] = tf;
-      scales[(size_t)i * T + k] = sc;
-      lg += 0.5L * (long double)geo[(size_t)i].n * memo.log2_1t2(tf);
+      turns.next(gk, &tans[(size_t)i * T + k], &scales[(size_t)i * T + k]);
     }
   }
   bool turning = c->engine_mode == 4 && c->e_recompute == 0;
@@ -1917,35 +1936,18 @@ int evolve_fused(bk_ctx* c, const bk_evolve_params* p, const Schedule& S, double
                  std::vector<long double>* row_log2, long double* final_log2) {
   constexpr int T = AmpTraits<R>::kTileBits;
   const int n = p->n;
-  const double dt = p->dt;
   const bool use_alt = n > T && c->engine_mode == 4 && alt_takes<R>(c, n);
   BK_TRY(check_phase<R>(c, n, angle_unit));
 
   // host schedule of the omitted cos^n factors and power-of-two rescales
   std::vector<R> tans((size_t)p->n_steps), scales((size_t)p->n_steps);
   row_log2->assign((size_t)S.n_meas, 0.0L);
-  long double lg = 0.0L;
-  double carry = 0.0;
+  StepTurns<R> turns(n, p->dt);
   for (int k = 0; k <= p->n_steps; ++k) {
-    if (S.slot[(size_t)k] >= 0) (*row_log2)[(size_t)S.slot[(size_t)k]] = lg;
-    if (k == p->n_steps) break;
-    const double gd = S.g[(size_t)k] * dt;
-    // the rounding of a step's tangent is made up for in the next ones, so a run's
-    // total rotation is not off by its number of steps times one rounding
-    const double want = std::tan(gd) + carry;
-    tans[(size_t)k] = (R)want;
-    carry = want - (double)tans[(size_t)k];
-    R sc = (R)1;
-    if (lg >= (long double)kRescaleLog2) {
-      sc = (R)std::ldexp(1.0, -kRescaleLog2);
-      lg -= (long double)kRescaleLog2;
-    }
-    scales[(size_t)k] = sc;
-    // each butterfly multiplies the norm^2 of its pair by 1 + t^2, t the value the kernel uses
-    const long double tf = (long double)tans[(size_t)k];
-    lg += 0.5L * (long double)n * std::log2(1.0L + tf * tf);
+    if (S.slot[(size_t)k] >= 0) (*row_log2)[(size_t)S.slot[(size_t)k]] = turns.lg;
+    if (k < p->n_steps) turns.next(S.g[(size_t)k], &tans[(size_t)k], &scales[(size_t)k]);
   }
-  *final_log2 = lg;
+  *final_log2 = turns.lg;
 
   if constexpr (sizeof(R) == 8)  // (complex64 runs of these sizes are complex128 ones: bk_evolve)
     if (n <= T) return evolve_small(c, p, S, angle_unit, tans, scales);
@@ -2194,22 +2196,10 @@ int adjoint_t(bk_ctx* c, const bk_adjoint_params* p, const std::vector<double>& 
   S.sample_pt.assign((size_t)T + 1, -1);
   std::vector<R> tans((size_t)T), scales((size_t)T);
   std::vector<long double> lgf((size_t)T + 1, 0.0L);
-  long double lg = 0.0L;
-  double carry = 0.0;
+  StepTurns<R> turns(n, p->dt);
   for (int k = 0; k <= T; ++k) {
-    lgf[(size_t)k] = lg;
-    if (k == T) break;
-    const double want = std::tan(g_step[(size_t)k] * p->dt) + carry;  // as in evolve_fused
-    tans[(size_t)k] = (R)want;
-    carry = want - (double)tans[(size_t)k];
-    R sc = (R)1;
-    if (lg >= (long double)kRescaleLog2) {
-      sc = (R)std::ldexp(1.0, -kRescaleLog2);
-      lg -= (long double)kRescaleLog2;
-    }
-    scales[(size_t)k] = sc;
-    const long double tf = (long double)tans[(size_t)k];
-    lg += 0.5L * (long double)n * std::log2(1.0L + tf * tf);
+    lgf[(size_t)k] = turns.lg;
+    if (k < T) turns.next(g_step[(size_t)k], &tans[(size_t)k], &scales[(size_t)k]);
   }
   bk_evolve_params q{};
   q.n = n;
