@@ -293,7 +293,8 @@ class Engine:
 
     def evolve_batch(self, instances, dt, n_steps, measure=None, precision=BK_C64, use_graph=True, lag=0,
                      diag_scale=0.0):
-        """Many statevectors in one launch per size (one persistent launch in engine modes 0 to 3).
+        """Many statevectors in one launch per size (one persistent launch in engine modes 0 to 3);
+        each instance's rows are those of its own ``evolve``, bit for bit.
 
         ``instances``: sequence of dicts with n, s0 and either g (scalar) or a per-step
         schedule; optional e0. Returns (p_less, d_h, norm) as [instance, measurement]."""

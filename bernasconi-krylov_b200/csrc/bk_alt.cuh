@@ -84,9 +84,10 @@ struct AltRunDesc {
   const uint16_t* E;
   const typename AltPhase<R>::entry* tab;
   const int* slot;     // [steps + 1] measurement row, or -1
-  double* partials;    // [rows][G][3]: norm, P_<, <d_H> of one CTA's tiles
+  double* partials;    // [rows][units][3]: norm, P_<, <d_H> of a unit's elements
   AltSet set[3];       // the A set, the S sets
   uint32_t n_tiles;
+  uint32_t units;      // units of a measured row: a warp's share of a tile, with three sets a CTA's tiles
   int n_j, c0;         // levels of the phase table (after its entry 0), lowest level
   int k0, k1;          // steps [k0, k1)
   int row0;            // first measurement row of `partials`
@@ -109,7 +110,7 @@ struct AltBatch {
   const AltInst<R>* inst;
   int n_inst, n_rows;
   uint32_t G;
-  size_t part_stride;  // doubles of one partial-sum buffer ([n_rows][G][3]); every group has two
+  size_t part_stride;  // doubles of one partial-sum buffer ([n_rows][units][3]); every group has two
 };
 
 // Barrier over the G CTAs of a run; `ctr` counts arrivals over all passes.
@@ -307,11 +308,13 @@ __device__ __forceinline__ void alt_weights(const El<double>::T& v, uint32_t e, 
   f = n * alt_small(__popc(el ^ s0));
 }
 
-// a warp's sums, and where the threshold and the trap are (read by the passes that measure)
+// where the threshold and the trap are (read by the passes that measure), and where a
+// warp's sums go: put(norm, P_<, <d_H>) by its lane 0
+template <class Put>
 struct AltMeas {
-  double* acc3;
   const int* e0;
   const uint32_t* s0;
+  Put put;
 };
 
 // Measurement of the thread's elements at the turn: rolled, from the thread's own
@@ -319,10 +322,10 @@ struct AltMeas {
 // that measure nothing neither registers nor instruction cache. Unrolled on the
 // register copies it pushed the 2^12-element kernels into spills, which go to L2:
 // next to the tile the L1 has little room.
-template <class R, int TB, int KB, int CP, int H0, int r>
+template <class R, int TB, int KB, int CP, int H0, int r, class Put>
 __device__ __forceinline__ void alt_measure(const typename El<R>::T (&v)[1 << KB], unsigned char* tile,
                                             const unsigned char* es, int e0, uint32_t s0, uint32_t tile_base,
-                                            uint32_t base, double* acc3) {
+                                            uint32_t base, const Put& put) {
   constexpr int lo = AltPlan<TB, KB>::reg_lo(r);
   alt_store<R, TB, KB, r>(tile, v, base);
   const uint32_t sb = swz<double>(base), g0 = tile_base | alt_index<CP, H0>(base);
@@ -343,20 +346,16 @@ __device__ __forceinline__ void alt_measure(const typename El<R>::T (&v)[1 << KB
     flips += (f4[0] + f4[1]) + (f4[2] + f4[3]);
   }
   const double a = warp_sum(norm), b = warp_sum(below), c = warp_sum(flips);
-  if ((threadIdx.x & 31u) == 0) {  // the warp's sums over the CTA's tiles of this pass
-    acc3[0] += a;
-    acc3[1] += b;
-    acc3[2] += c;
-  }
+  if ((threadIdx.x & 31u) == 0) put(a, b, c);
 }
 
-template <class R, int TB, int KB, int CP, int H0, int r>
+template <class R, int TB, int KB, int CP, int H0, int r, class Put>
 __device__ __forceinline__ void alt_turn(typename El<R>::T (&v)[1 << KB], unsigned char* tile, const unsigned char* es,
                                          const AltTurn<R>& T, uint32_t tile_base, uint32_t base,
-                                         const unsigned char* tab, const AltMeas& M) {
+                                         const unsigned char* tab, const AltMeas<Put>& M) {
   cp_async_wait();
   if (T.meas) {
-    alt_measure<R, TB, KB, CP, H0, r>(v, tile, es, *M.e0, *M.s0, tile_base, base, M.acc3);
+    alt_measure<R, TB, KB, CP, H0, r>(v, tile, es, *M.e0, *M.s0, tile_base, base, M.put);
     alt_load<R, TB, KB, r, true>(tile, v, base);  // the measurement needs the registers
   }
   const AltTab P = alt_tab<R>(tab, T.post, T.c0);
@@ -395,10 +394,10 @@ __device__ __forceinline__ typename El<R>::T alt_ldcg(const unsigned char* p) {
   return El<R>::ld(&q);
 }
 
-template <class R, int TB, int KB, int CP, int H0, class W, class F>
+template <class R, int TB, int KB, int CP, int H0, class Put, class W, class F>
 __device__ __forceinline__ void alt_tile_turn(unsigned char* tile, unsigned char* state, const AltTurn<R>& T,
                                               uint32_t tile_base, const unsigned char* tab, unsigned char* es,
-                                              const AltMeas& M, W&& wait, F&& stage_free) {
+                                              const AltMeas<Put>& M, W&& wait, F&& stage_free) {
   using PL = AltPlan<TB, KB>;
   constexpr int RT = alt_turn_round(TB, KB, CP);
   constexpr int LO = CP == TB ? 0 : CP;  // lowest tile bit of the set
@@ -531,7 +530,7 @@ struct AltCtl {
   uint64_t full_bar;
   int stop;      // the run has failed: every thread leaves at the end of the pass
   int inflight;  // thread 0: a tile's copy is on its way
-  double acc[16][3];  // per warp: norm, P_<, <d_H> of the pass
+  double acc[16][3];  // per warp: norm, P_<, <d_H> of the pass (three sets); batch: of a row's units
   // batch: the statevector the group works on
   const CUtensorMap* map;
   unsigned char* state;
@@ -572,12 +571,12 @@ struct AltCta {
   __device__ __forceinline__ const R* tans() const { return kBatch ? static_cast<const R*>(ctl().tan) : I.tan; }
   __device__ __forceinline__ const R* scales() const { return kBatch ? static_cast<const R*>(ctl().scale) : I.scale; }
   __device__ __forceinline__ const CUtensorMap* maps() const { return kBatch ? ctl().map : I.map; }
-  __device__ __forceinline__ AltMeas meas() const {
-    double* a = const_cast<double*>(&ctl().acc[threadIdx.x >> 5][0]);
+  template <class Put>
+  __device__ __forceinline__ AltMeas<Put> meas(const Put& put) const {
     if constexpr (kBatch)
-      return AltMeas{a, const_cast<const int*>(&ctl().e0), const_cast<const uint32_t*>(&ctl().s0)};
+      return AltMeas<Put>{const_cast<const int*>(&ctl().e0), const_cast<const uint32_t*>(&ctl().s0), put};
     else
-      return AltMeas{a, &I.e0, &I.s0};
+      return AltMeas<Put>{&I.e0, &I.s0, put};
   }
 
   __device__ __forceinline__ void issue(int map, uint32_t tile) {
@@ -609,8 +608,12 @@ struct AltCta {
     AltE<R, TB, KB, CP, H0, RT>::fetch(D.E, alt_tile_base<TB, CP, H0>(tile),
                                        PL::template base<RT>(threadIdx.x & 31u, threadIdx.x >> 5), smem_addr(es()));
   }
-  // the turning pass of step k on the tiles of set `s` (E of the first one already fetched)
-  template <int CP, int H0>
+  // The turning pass of step k on the tiles of set `s` (E of the first one already fetched).
+  // kTiles: a measured row keeps the sums of every warp of every tile, so they are added up
+  // in the same order whatever the number of CTAs, and a statevector of a batch measures what
+  // its own run does, bit for bit. Three sets (never in a group of a batch) keep the sums of
+  // a CTA: 24 bytes a warp and tile are 6 MB a row at N = 28.
+  template <int CP, int H0, bool kTiles>
   __device__ __forceinline__ void turn(int s, int k) {
     AltTurn<R> T;
     const bool pre = k > D.k0;
@@ -621,19 +624,38 @@ struct AltCta {
     T.c0 = (uint32_t)D.c0;
     const int slot = (pre || D.meas_first) ? D.slot[k] : -1;
     T.meas = slot >= 0;
-    const AltMeas M = meas();
-    if (T.meas && (threadIdx.x & 31u) == 0) M.acc3[0] = M.acc3[1] = M.acc3[2] = 0.0;
+    auto unit = [&](uint32_t u) {
+      return (kBatch ? ctl().partials : D.partials) + 3 * ((size_t)(slot - D.row0) * D.units + u);
+    };
+    if (!kTiles && T.meas && (threadIdx.x & 31u) == 0) {
+      volatile double(&a)[3] = ctl().acc[threadIdx.x >> 5];
+      a[0] = a[1] = a[2] = 0.0;
+    }
     for (uint32_t tile = rank; tile < D.n_tiles; tile += G) {
-      alt_tile_turn<R, TB, KB, CP, H0>(stage, state(), T, alt_tile_base<TB, CP, H0>(tile), tab(), es(), M,
+      auto put = [&](double a, double b, double c) {
+        const uint32_t warp = threadIdx.x >> 5;
+        if constexpr (kTiles) {
+          double* o = unit(tile * PL::kWarps + warp);
+          o[0] = a;
+          o[1] = b;
+          o[2] = c;
+        } else {
+          volatile double(&acc)[3] = ctl().acc[warp];
+          acc[0] = acc[0] + a;
+          acc[1] = acc[1] + b;
+          acc[2] = acc[2] + c;
+        }
+      };
+      alt_tile_turn<R, TB, KB, CP, H0>(stage, state(), T, alt_tile_base<TB, CP, H0>(tile), tab(), es(), meas(put),
                                        [&]() { wait(); }, [&]() { issue(s, tile + G); });
       fetch_e<CP, H0>(tile + G);  // after the stores, when the registers are free
     }
-    if (T.meas) {
+    if (!kTiles && T.meas) {
       __syncthreads();
       if (threadIdx.x < 3u) {
         double x = 0;
         for (int w = 0; w < PL::kWarps; ++w) x += ctl().acc[w][threadIdx.x];
-        (kBatch ? ctl().partials : D.partials)[3 * ((size_t)(slot - D.row0) * G + rank) + threadIdx.x] = x;
+        unit(rank)[threadIdx.x] = x;
       }
     }
   }
@@ -694,11 +716,11 @@ __device__ __forceinline__ bool alt_run2(AltCta<R, TB, KB, kBatch>& C) {
   C.issue(D.k0 & 1, C.rank);
   for (int k = D.k0;; ++k) {
     if (k & 1) {
-      C.template turn<TB - W, TB>(1, k);
+      C.template turn<TB - W, TB, true>(1, k);
       if (k == D.k1) return true;
       C.template fetch_e<TB, TB>(C.rank);
     } else {
-      C.template turn<TB, TB>(0, k);
+      C.template turn<TB, TB, true>(0, k);
       if (k == D.k1) return true;
       C.template fetch_e<TB - W, TB>(C.rank);
     }
@@ -716,15 +738,40 @@ __device__ __forceinline__ bool alt_run3(AltCta<R, 12, 4, kBatch>& C) {
   C.issue(1 + (D.k0 & 1), C.rank);
   for (int k = D.k0;; ++k) {
     if (k & 1)
-      C.template turn<C3, H3>(2, k);
+      C.template turn<C3, H3, false>(2, k);
     else
-      C.template turn<C2, TB>(1, k);
+      C.template turn<C2, TB, false>(1, k);
     if (k == D.k1) return true;
     if (!C.next_pass(0)) return false;
     C.plain(0, k);
     if (k & 1) C.template fetch_e<C2, TB>(C.rank); else C.template fetch_e<C3, H3>(C.rank);
     if (!C.next_pass(1 + ((k + 1) & 1))) return false;
   }
+}
+
+// The sums of a measured row's units, by a CTA of as many threads as the passes' and in the
+// same order wherever it runs: in thread 0.
+template <int TB>
+constexpr int kAltRowThreads = TB == 10 ? AltPlan<10, 4>::kThreads : AltPlan<12, 4>::kThreads;
+template <int kRow>
+__device__ __forceinline__ void alt_row_sum(const double* part, uint32_t units, volatile double (*red)[3], double (&s)[3]) {
+  const uint32_t t = threadIdx.x;
+  s[0] = s[1] = s[2] = 0.0;
+#pragma unroll 4
+  for (uint32_t u = t; u < units; u += kRow)
+#pragma unroll
+    for (int q = 0; q < 3; ++q) s[q] += __ldcg(&part[3 * (size_t)u + q]);
+#pragma unroll
+  for (int q = 0; q < 3; ++q) s[q] = warp_sum(s[q]);
+  __syncthreads();  // the last row's sums have been read
+  if ((t & 31u) == 0)
+#pragma unroll
+    for (int q = 0; q < 3; ++q) red[t >> 5][q] = s[q];
+  __syncthreads();
+  if (t == 0)
+    for (int w = 1; w < kRow / 32; ++w)
+#pragma unroll
+      for (int q = 0; q < 3; ++q) s[q] += red[w][q];
 }
 
 __device__ __forceinline__ unsigned char* alt_stage(unsigned char* raw) {
@@ -749,7 +796,7 @@ __global__ void __launch_bounds__(AltPlan<TB, KB>::kThreads, TB == 10 ? 6 : TB =
 
 // Many statevectors of one size: groups of Q.G CTAs work through them on their own,
 // each with its own barrier, so a small statevector's barriers and waits overlap
-// those of the other groups. Results are reduced by the group (CTA sums in index
+// those of the other groups. Results are reduced by the group (units in index
 // order) after the statevector's last pass, from one of two partial-sum buffers:
 // the next use of a buffer lies behind the barriers of the statevector between.
 template <class R, int TB, int KB, int W2, int W3>
@@ -761,7 +808,6 @@ __global__ void __launch_bounds__(AltPlan<TB, KB>::kThreads, TB == 10 ? 6 : TB =
   AltCta<R, TB, KB, true> C{D, *Q.inst, B, B.ctr + 32u * group, blockIdx.x % Q.G, Q.G, alt_stage(smem_raw)};
   C.begin();
   C.stage_table();
-  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   uint32_t turn = 0;
   bool ok = true;
   for (int i = (int)group; ok && i < Q.n_inst; i += (int)n_groups, ++turn) {
@@ -784,14 +830,11 @@ __global__ void __launch_bounds__(AltPlan<TB, KB>::kThreads, TB == 10 ? 6 : TB =
       ok = alt_run3<R, W2, W3>(C);
     if (!ok || !(ok = C.group_barrier())) break;
     if (__syncthreads_or(C.ctl().stop)) break;  // also: thread 0 has seen every CTA's partial sums
-    for (int row = (int)(C.rank * AltPlan<TB, KB>::kWarps + warp); row < Q.n_rows; row += (int)(Q.G * AltPlan<TB, KB>::kWarps)) {
-      double s[3] = {0, 0, 0};
-      for (uint32_t j = lane; j < Q.G; j += 32u)
-#pragma unroll
-        for (int q = 0; q < 3; ++q) s[q] += __ldcg(&part[3 * ((size_t)row * Q.G + j) + q]);
-#pragma unroll
-      for (int q = 0; q < 3; ++q) s[q] = warp_sum(s[q]);
-      if (lane == 0) {
+    static_assert(kAltRowThreads<TB == 13 ? 12 : TB> == AltPlan<TB, KB>::kThreads, "the CTA sums a row");
+    for (int row = (int)C.rank; row < Q.n_rows; row += (int)Q.G) {
+      double s[3];
+      alt_row_sum<AltPlan<TB, KB>::kThreads>(part + 3 * (size_t)row * D.units, D.units, C.ctl().acc, s);
+      if (threadIdx.x == 0) {
         I.results[4 * (size_t)row + 0] = s[1];
         I.results[4 * (size_t)row + 1] = s[2];
         I.results[4 * (size_t)row + 2] = s[0];
@@ -803,18 +846,15 @@ __global__ void __launch_bounds__(AltPlan<TB, KB>::kThreads, TB == 10 ? 6 : TB =
 }
 
 #ifdef BK_ALT_REDUCE  // defined by the one source that launches it
-// results[row0 + row] = sum over the G CTAs of a run in index order (one warp a row)
-__global__ void __launch_bounds__(128) alt_reduce_kernel(const double* __restrict__ partials, int rows, int G,
-                                                         double* __restrict__ results) {
-  const int row = (int)(blockIdx.x * 4 + (threadIdx.x >> 5)), lane = (int)(threadIdx.x & 31);
-  if (row >= rows) return;
-  double s[3] = {0, 0, 0};
-  for (int i = lane; i < G; i += 32)
-#pragma unroll
-    for (int q = 0; q < 3; ++q) s[q] += partials[3 * ((size_t)row * G + i) + q];
-#pragma unroll
-  for (int q = 0; q < 3; ++q) s[q] = warp_sum(s[q]);
-  if (lane == 0) {
+// results[row0 + row] = sum over a row's units in a fixed order (a CTA a row)
+template <int kRow>
+__global__ void __launch_bounds__(kRow)
+    alt_reduce_kernel(const double* __restrict__ partials, uint32_t units, double* __restrict__ results) {
+  __shared__ volatile double red[16][3];
+  const int row = (int)blockIdx.x;
+  double s[3];
+  alt_row_sum<kRow>(partials + 3 * (size_t)row * units, units, red, s);
+  if (threadIdx.x == 0) {
     results[4 * (size_t)row + 0] = s[1];
     results[4 * (size_t)row + 1] = s[2];
     results[4 * (size_t)row + 2] = s[0];

@@ -1255,7 +1255,20 @@ int alt_kernel_ready(bk_ctx* c, const AltGeo& geo, bool batch, int n_j, const vo
   return BK_OK;
 }
 
-// A prepared run over c->d_state: geometry, uploads and the kernel; alt_launch
+// Units of a measured row's partial sums (bk_alt.cuh), for G CTAs a statevector.
+uint32_t alt_units(const AltGeo& g, uint32_t n_tiles, uint32_t G) {
+  return g.w3 > 0 ? G : n_tiles * (g.tb == 10 ? AltPlan<10, 4>::kWarps : AltPlan<12, 4>::kWarps);
+}
+static_assert(AltPlan<13, 5>::kWarps == AltPlan<12, 4>::kWarps, "both tiles have eight warps");
+
+// A statevector, its energies and where its rows go.
+struct AltTarget {
+  void* state;
+  const uint16_t* E;
+  double* results;  // [measurement rows][4]
+};
+
+// A prepared run over a target: geometry, uploads and the kernel; alt_launch
 // runs any range of its steps.
 template <class R>
 struct AltRun {
@@ -1266,22 +1279,27 @@ struct AltRun {
   int smem = 0, threads = 0;
   uint32_t G = 0;
   int max_rows = 1;  // measurement rows the partial sums of one launch have room for
+  int tb = 0;
+  double* results = nullptr;
 };
 
 template <class R>
-int alt_prepare(bk_ctx* c, int n, uint64_t s0, int64_t e0, double angle_unit, const Schedule& S,
+int alt_prepare(bk_ctx* c, const AltTarget& at, int n, uint64_t s0, int64_t e0, double angle_unit, const Schedule& S,
                 const std::vector<R>& tans, const std::vector<R>& scales, AltRun<R>* run) {
   using entry = typename AltPhase<R>::entry;
   const int np = sizeof(R) == 4 ? n - 1 : n, T = (int)tans.size();
   AltGeo geo;
   if (!alt_geometry(np, &geo)) return fail(c, BK_ERR_UNSUPPORTED, "turning passes: n = %d", n);
   AltRunDesc<R>& D = run->D;
-  BK_TRY(alt_maps(c, c->d_state, np, geo, run->I.map, D.set));
+  BK_TRY(alt_maps(c, at.state, np, geo, run->I.map, D.set));
   D.n_j = alt_levels(n, &D.c0);
   D.n_tiles = 1u << (np - geo.tb);
   int per_sm = 0;
   BK_TRY(alt_kernel_ready<R>(c, geo, false, D.n_j, &run->fn, &run->smem, &run->threads, &per_sm));
   run->G = std::min<uint32_t>(D.n_tiles, (uint32_t)(per_sm * c->num_sms));
+  run->tb = geo.tb;
+  run->results = at.results;
+  D.units = alt_units(geo, D.n_tiles, run->G);
 
   // one upload: phase table, tangents, rescales, measurement rows, zeroed counters
   Bump b;
@@ -1291,7 +1309,7 @@ int alt_prepare(bk_ctx* c, int n, uint64_t s0, int64_t e0, double angle_unit, co
   const size_t o_slot = b.take((size_t)(T + 1) * sizeof(int));
   const size_t o_ctr = b.take(64);
   const size_t up = b.off;
-  const size_t row_bytes = 3 * sizeof(double) * (size_t)run->G;
+  const size_t row_bytes = 3 * sizeof(double) * (size_t)D.units;
   run->max_rows = (int)std::max<size_t>(kAltPartialBytes / row_bytes, 1);
   const size_t o_part = b.take(row_bytes * (size_t)std::max(1, std::min(S.n_meas, run->max_rows + 1)));
   BK_TRY(ensure_buffer(c, &c->d_alt, &c->alt_cap, b.off));
@@ -1304,12 +1322,12 @@ int alt_prepare(bk_ctx* c, int n, uint64_t s0, int64_t e0, double angle_unit, co
   std::memset(h + o_ctr, 0, 64);
   BK_CUDA(c, cudaMemcpyAsync(d, h, up, cudaMemcpyHostToDevice, c->stream));
   BK_TRY(staged(c));
-  D.E = c->d_E;
+  D.E = at.E;
   D.tab = reinterpret_cast<const entry*>(d + o_tab);
   D.slot = reinterpret_cast<const int*>(d + o_slot);
   D.partials = reinterpret_cast<double*>(d + o_part);
   AltInst<R>& I = run->I;
-  I.state = static_cast<unsigned char*>(c->d_state);
+  I.state = static_cast<unsigned char*>(at.state);
   I.tan = reinterpret_cast<const R*>(d + o_tan);
   I.scale = reinterpret_cast<const R*>(d + o_sc);
   I.e0 = (int)e0;
@@ -1339,21 +1357,20 @@ int alt_launch(bk_ctx* c, AltRun<R>& r, int k0, int k1, bool first, int row0, in
   BK_CUDA(c, cudaLaunchCooperativeKernel(r.fn, dim3(r.G), dim3((unsigned)r.threads), args, (size_t)r.smem, st));
   BK_TRY(ev_end(c, ev));
   if (rows > 0) {
-    alt_reduce_kernel<<<(rows + 3) / 4, 128, 0, st>>>(r.D.partials, rows, (int)r.G, c->d_results + 4 * (size_t)row0);
+    double* out = r.results + 4 * (size_t)row0;
+    if (r.tb == 10)
+      alt_reduce_kernel<kAltRowThreads<10>><<<rows, kAltRowThreads<10>, 0, st>>>(r.D.partials, r.D.units, out);
+    else
+      alt_reduce_kernel<kAltRowThreads<12>><<<rows, kAltRowThreads<12>, 0, st>>>(r.D.partials, r.D.units, out);
     BK_CUDA(c, cudaGetLastError());
   }
   return BK_OK;
 }
 
-template <class R>
-int evolve_alt(bk_ctx* c, const bk_evolve_params* p, const Schedule& S, double angle_unit, const std::vector<R>& tans,
-               const std::vector<R>& scales) {
-  using Samp = typename std::conditional<sizeof(R) == 4, Planar64, double2>::type;
-  const int n = p->n, T = p->n_steps;
-  const Samp* psi = reinterpret_cast<const Samp*>(c->d_state);
-  AltRun<R> run;
-  BK_TRY(alt_prepare<R>(c, n, p->s0, p->e0, angle_unit, S, tans, scales, &run));
-  if (S.sample_pt[0] >= 0) BK_TRY(launch_sampling_t(c, psi, n, S.sample_pt[0], S.shots));
+// All T steps of a prepared run; sample(point) at its sampling points.
+template <class R, class F>
+int alt_steps(bk_ctx* c, AltRun<R>& run, const Schedule& S, int T, F&& sample) {
+  if (S.sample_pt[0] >= 0) BK_TRY(sample(S.sample_pt[0]));
   // segments end at sampling points (which read psi_k) and where the partial sums' room ends
   int k0 = 0;
   for (bool first = true;; first = false) {
@@ -1364,10 +1381,21 @@ int evolve_alt(bk_ctx* c, const bk_evolve_params* p, const Schedule& S, double a
       if (k == T || (k > k0 && (S.sample_pt[(size_t)k] >= 0 || rows >= run.max_rows))) break;
     }
     BK_TRY(alt_launch<R>(c, run, k0, k1, first, row0, rows));
-    if (k1 > 0 && S.sample_pt[(size_t)k1] >= 0) BK_TRY(launch_sampling_t(c, psi, n, S.sample_pt[(size_t)k1], S.shots));
+    if (k1 > 0 && S.sample_pt[(size_t)k1] >= 0) BK_TRY(sample(S.sample_pt[(size_t)k1]));
     if (k1 == T) return BK_OK;
     k0 = k1;
   }
+}
+
+template <class R>
+int evolve_alt(bk_ctx* c, const bk_evolve_params* p, const Schedule& S, double angle_unit, const std::vector<R>& tans,
+               const std::vector<R>& scales) {
+  using Samp = typename std::conditional<sizeof(R) == 4, Planar64, double2>::type;
+  const Samp* psi = reinterpret_cast<const Samp*>(c->d_state);
+  AltRun<R> run;
+  BK_TRY(alt_prepare<R>(c, AltTarget{c->d_state, c->d_E, c->d_results}, p->n, p->s0, p->e0, angle_unit, S, tans, scales,
+                        &run));
+  return alt_steps<R>(c, run, S, p->n_steps, [&](int pt) { return launch_sampling_t(c, psi, p->n, pt, S.shots); });
 }
 
 // ---------------------------------------------------------------------------
@@ -1449,8 +1477,18 @@ int evolve_small(bk_ctx* c, const bk_evolve_params* p, const Schedule& S, double
   }
 }
 
+// the error word a run has left: reported, and cleared for the next one
+int device_error(bk_ctx* c, int e) {
+  if (e == 0) return BK_OK;
+  cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream);
+  cudaMemsetAsync(c->d_ticket, 0, sizeof(unsigned int), c->stream);
+  cudaStreamSynchronize(c->stream);
+  if (e == DEV_TIMEOUT) return fail(c, BK_ERR_TIMEOUT, "a bounded device wait gave up (a tile's load or a pass barrier)");
+  return fail(c, BK_ERR_CUDA, "device error word %d", e);
+}
+
 // ---------------------------------------------------------------------------
-// batched evolution (persistent engine over many statevectors)
+// batched evolution (turning passes, or the persistent engine over many statevectors)
 // ---------------------------------------------------------------------------
 int batch_energy(bk_ctx* c, int n, uint16_t** out) {
   auto it = c->batch_E.find(n);
@@ -1489,13 +1527,12 @@ struct BatchGeo {
 };
 
 // rows [instance][measurement] of the device -> the caller's arrays, scales taken out
-template <class R>
-void batch_rows(const std::vector<double>& rows, const std::vector<long double>& row_log2, double* p_less, double* d_h,
-                double* norm_out) {
+void batch_rows(bool c64, const std::vector<double>& rows, const std::vector<long double>& row_log2, double* p_less,
+                double* d_h, double* norm_out) {
   for (size_t r = 0; r < rows.size() / 4; ++r) {
     const long double f = std::exp2(-2.0L * row_log2[r]);
     // complex64: expectation values of the normalised state (see bk_evolve)
-    const long double nrm = (sizeof(R) == 4 && rows[4 * r + 2] > 0.0) ? (long double)rows[4 * r + 2] * f : 1.0L;
+    const long double nrm = (c64 && rows[4 * r + 2] > 0.0) ? (long double)rows[4 * r + 2] * f : 1.0L;
     p_less[r] = (double)((long double)rows[4 * r + 0] * f / nrm);
     d_h[r] = (double)((long double)rows[4 * r + 1] * f / nrm);
     if (norm_out) norm_out[r] = (double)((long double)rows[4 * r + 2] * f);
@@ -1509,8 +1546,7 @@ void batch_rows(const std::vector<double>& rows, const std::vector<long double>&
 // one after another (about 9 us for a tile of each of an SM's resident CTAs).
 template <class R>
 int batch_turning(bk_ctx* c, const std::vector<BatchGeo>& geo, int T, const std::vector<int>& slot, int n_meas,
-                  const std::vector<R>& tans, const std::vector<R>& scales, size_t state_bytes,
-                  const std::vector<long double>& row_log2, double* p_less, double* d_h, double* norm_out) {
+                  const std::vector<R>& tans, const std::vector<R>& scales, size_t state_bytes, double* rows) {
   using entry = typename AltPhase<R>::entry;
   constexpr bool c64 = sizeof(R) == 4;
   const int n_inst = (int)geo.size();
@@ -1543,6 +1579,7 @@ int batch_turning(bk_ctx* c, const std::vector<BatchGeo>& geo, int T, const std:
     alt_geometry(np, &k.geo);
     k.D.n_j = alt_levels(k.n, &k.D.c0);
     k.D.n_tiles = 1u << (np - k.geo.tb);
+    k.D.units = alt_units(k.geo, k.D.n_tiles, 0);
     BK_TRY(alt_kernel_ready<R>(c, k.geo, true, k.D.n_j, &k.fn, &k.smem, &k.threads, &k.per_sm));
     const uint32_t slots = (uint32_t)(k.per_sm * c->num_sms);
     double best = 0;
@@ -1568,7 +1605,7 @@ int batch_turning(bk_ctx* c, const std::vector<BatchGeo>& geo, int T, const std:
   const size_t up = b.off;
   size_t part = 0;  // the classes run one after another: one room for their partial sums
   for (auto& kv : classes)
-    part = std::max(part, (size_t)kv.second.groups * 2 * 3 * (size_t)std::max(n_meas, 1) * kv.second.G * sizeof(double));
+    part = std::max(part, (size_t)kv.second.groups * 2 * 3 * (size_t)std::max(n_meas, 1) * kv.second.D.units * sizeof(double));
   const size_t o_part = b.take(part);
   BK_TRY(ensure_buffer(c, &c->d_batch, &c->batch_cap, b.off));
   char *h = nullptr, *d = static_cast<char*>(c->d_batch);
@@ -1619,38 +1656,34 @@ int batch_turning(bk_ctx* c, const std::vector<BatchGeo>& geo, int T, const std:
   for (auto& kv : classes) {
     Class& k = kv.second;
     AltBatch<R> Q{reinterpret_cast<const AltInst<R>*>(d + o_inst) + k.first, k.n_inst, n_meas, k.G,
-                  3 * (size_t)std::max(n_meas, 1) * k.G};
+                  3 * (size_t)std::max(n_meas, 1) * k.D.units};
     AltBarrier B{reinterpret_cast<unsigned int*>(d + k.o_ctr), reinterpret_cast<int*>(d + o_glob),
                  reinterpret_cast<int*>(d + o_glob + 4), c->wait_polls > 0 ? c->wait_polls : kWaitPolls * 4u};
     void* args[] = {&k.D, &Q, &B};
     BK_CUDA(c, cudaLaunchCooperativeKernel(k.fn, dim3(k.G * k.groups), dim3((unsigned)k.threads), args, (size_t)k.smem, st));
   }
   BK_TRY(ev_end(c, ev));
-  std::vector<double> rows((size_t)n_inst * n_meas * 4);
   int e = 0;
   BK_CUDA(c, cudaMemcpyAsync(&e, d + o_glob, sizeof(int), cudaMemcpyDeviceToHost, st));
-  if (!rows.empty())
-    BK_CUDA(c, cudaMemcpyAsync(rows.data(), c->d_batch_results, rows.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
+  if (n_meas > 0)
+    BK_CUDA(c, cudaMemcpyAsync(rows, c->d_batch_results, (size_t)n_inst * n_meas * 4 * sizeof(double),
+                               cudaMemcpyDeviceToHost, st));
   BK_CUDA(c, cudaStreamSynchronize(st));
   BK_TRY(collect_timing(c));
   if (e != 0) return fail(c, BK_ERR_TIMEOUT, "batched turning passes: a bounded device wait gave up (%d)", e);
-  batch_rows<R>(rows, row_log2, p_less, d_h, norm_out);
   return BK_OK;
 }
 
-template <class R>
-int evolve_batch_t(bk_ctx* c, const bk_batch_params* bp, const bk_batch_instance* inst, int n_inst,
-                   double* p_less, double* d_h, double* norm_out) {
-  const bool c64 = sizeof(R) == 4;
-  const int T = bp->n_steps;
-  std::vector<int> slot((size_t)T + 1, -1);
-  int n_meas = 0;
-  for (int k = 0; k <= T; ++k)
-    if (bp->measure == nullptr || bp->measure[k]) slot[(size_t)k] = n_meas++;
-  if (n_meas > 0 && (!p_less || !d_h)) return fail(c, BK_ERR_INVALID, "output arrays are NULL");
-
-  std::vector<BatchGeo> geo((size_t)n_inst);
-  size_t state_bytes = 0;
+// A batch's rows and instances; refuses what a batch does not take.
+int batch_geometry(bk_ctx* c, const bk_batch_params* bp, const bk_batch_instance* inst, int n_inst, bool outputs,
+                   std::vector<int>* slot, int* n_meas, std::vector<BatchGeo>* geo) {
+  const bool c64 = bp->precision == BK_C64;
+  slot->assign((size_t)bp->n_steps + 1, -1);
+  *n_meas = 0;
+  for (int k = 0; k <= bp->n_steps; ++k)
+    if (bp->measure == nullptr || bp->measure[k]) (*slot)[(size_t)k] = (*n_meas)++;
+  if (*n_meas > 0 && !outputs) return fail(c, BK_ERR_INVALID, "output arrays are NULL");
+  geo->resize((size_t)n_inst);
   for (int i = 0; i < n_inst; ++i) {
     const bk_batch_instance& b = inst[i];
     BatchGeo g{};
@@ -1670,10 +1703,175 @@ int evolve_batch_t(bk_ctx* c, const bk_batch_params* bp, const bk_batch_instance
     if (e0 < 0) e0 = host_energy(b.n, g.s0);
     g.e0 = (int)e0;
     g.angle_unit = (bp->diag_scale > 0.0) ? bp->dt * bp->diag_scale : bp->dt / (double)b.n;
-    g.state_off = state_bytes;
-    state_bytes += (1ull << b.n) * (c64 ? 8 : 16);
-    geo[(size_t)i] = g;
+    (*geo)[(size_t)i] = g;
     if (b.g == nullptr && !is_finite(b.g_const)) return fail(c, BK_ERR_INVALID, "instance %d: g not finite", i);
+  }
+  return BK_OK;
+}
+
+// Up to 18 qubits complex64 runs in turning passes compute in complex128: a step is latency
+// there, not arithmetic or bandwidth (us a step, complex64 / complex128 kernels: N = 14
+// 3.9 / 3.5, 16 4.6 / 3.9, 18 5.1 / 5.1, 19 5.7 / 8.0), and the results are the exact ones to
+// 1e-13 instead of a random walk of FP32 roundings. The members of a batch follow, so that
+// each is its own single run: where members fill the GPU the wider state costs them
+// (200 x N = 14 1.15 -> 1.48 ms, 200 x N = 16 2.35 -> 3.88, 100 x N = 18 3.66 -> 7.35 for 24
+// measured steps; three members of N = 16 take 0.21 ms either way).
+bool widened(const bk_ctx* c, int n) { return n <= 18 && c->engine_mode == 4 && c->e_recompute == 0; }
+
+// A batch in turning passes (the default mode): what bk_evolve computes for each member.
+// Members of a size that one group of CTAs takes share a cooperative launch per size
+// (batch_turning); larger ones fill the GPU and run one after another.
+struct BatchRun {
+  bk_ctx* c;
+  const bk_batch_params* bp;
+  const bk_batch_instance* inst;
+  std::vector<int> slot;
+  int n_meas = 0;
+  std::vector<BatchGeo> geo;
+  std::vector<double> rows;            // [instance][measurement][4]
+  std::vector<long double> row_log2;   // [instance][measurement]
+
+  // tangents, rescales and scale logs of the members `ids`, one after another
+  template <class R>
+  int turns(const std::vector<int>& ids, std::vector<R>* tans, std::vector<R>* scales) {
+    const int T = bp->n_steps;
+    tans->resize(ids.size() * (size_t)T);
+    scales->resize(ids.size() * (size_t)T);
+    for (size_t m = 0; m < ids.size(); ++m) {
+      const size_t i = (size_t)ids[m];
+      StepTurns<R> t(geo[i].n, bp->dt);
+      for (int k = 0; k <= T; ++k) {
+        if (slot[(size_t)k] >= 0) row_log2[i * (size_t)n_meas + (size_t)slot[(size_t)k]] = t.lg;
+        if (k < T)
+          t.next(inst[i].g ? inst[i].g[k] : inst[i].g_const, &(*tans)[m * (size_t)T + k], &(*scales)[m * (size_t)T + k]);
+      }
+    }
+    return BK_OK;
+  }
+  template <class R>
+  int members(const std::vector<int>& ids) {
+    std::vector<R> tans, scales;
+    BK_TRY(turns(ids, &tans, &scales));
+    std::vector<BatchGeo> g;
+    size_t bytes = 0;
+    for (int i : ids) {
+      g.push_back(geo[(size_t)i]);
+      g.back().np = sizeof(R) == 4 ? g.back().n - 1 : g.back().n;
+      g.back().state_off = bytes;
+      bytes += (16ull << g.back().np);
+    }
+    std::vector<double> r(ids.size() * (size_t)n_meas * 4);
+    BK_TRY(batch_turning<R>(c, g, bp->n_steps, slot, n_meas, tans, scales, bytes, r.data()));
+    const size_t per = (size_t)n_meas * 4;
+    for (size_t m = 0; m < ids.size(); ++m)
+      std::copy(r.begin() + (long)(m * per), r.begin() + (long)((m + 1) * per), rows.begin() + (long)((size_t)ids[m] * per));
+    return BK_OK;
+  }
+  template <class R>
+  int alone(int i) {
+    std::vector<R> tans, scales;
+    BK_TRY(turns(std::vector<int>{i}, &tans, &scales));
+    const BatchGeo& g = geo[(size_t)i];
+    const int T = bp->n_steps;
+    Schedule S;
+    S.slot = slot;
+    S.n_meas = n_meas;
+    S.sample_pt.assign((size_t)T + 1, -1);
+    uint16_t* dE = nullptr;
+    BK_TRY(batch_energy(c, g.n, &dE));
+    BK_CUDA(c, cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
+    BK_CUDA(c, cudaMemsetAsync(c->d_batch_state, 0, (1ull << g.n) * (sizeof(R) * 2), c->stream));
+    if (sizeof(R) == 4)
+      set_basis_planar_kernel<<<1, 1, 0, c->stream>>>(static_cast<float*>(c->d_batch_state), g.s0);
+    else
+      set_basis_kernel<double2><<<1, 1, 0, c->stream>>>(static_cast<double2*>(c->d_batch_state), g.s0);
+    BK_CUDA(c, cudaGetLastError());
+    AltRun<R> run;
+    BK_TRY(alt_prepare<R>(c, AltTarget{c->d_batch_state, dE, c->d_batch_results}, g.n, g.s0, g.e0, g.angle_unit, S, tans,
+                          scales, &run));
+    BK_TRY(alt_steps<R>(c, run, S, T, [](int) { return BK_OK; }));
+    int err = 0;
+    BK_CUDA(c, cudaMemcpyAsync(&err, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    if (n_meas > 0)
+      BK_CUDA(c, cudaMemcpyAsync(rows.data() + (size_t)i * n_meas * 4, c->d_batch_results,
+                                 (size_t)n_meas * 4 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    BK_CUDA(c, cudaStreamSynchronize(c->stream));
+    BK_TRY(device_error(c, err));
+    return collect_timing(c);
+  }
+};
+
+int evolve_batch_turning(bk_ctx* c, const bk_batch_params* bp, const bk_batch_instance* inst, int n_inst,
+                         double* p_less, double* d_h, double* norm_out) {
+  const bool c64 = bp->precision == BK_C64;
+  BatchRun B{c, bp, inst};
+  BK_TRY(batch_geometry(c, bp, inst, n_inst, p_less && d_h, &B.slot, &B.n_meas, &B.geo));
+  for (int i = 0; i < n_inst && bp->n_steps > 0; ++i)
+    for (int k = 0; inst[i].g && k < bp->n_steps; ++k)
+      if (!is_finite(inst[i].g[k])) return fail(c, BK_ERR_INVALID, "instance %d: g[%d] not finite", i, k);
+  if (c64)
+    for (const BatchGeo& g : B.geo) BK_TRY(check_phase<float>(c, g.n, g.angle_unit));
+  // who runs where, and the room of their states
+  enum { kWide, kOwn, kAlone };
+  std::vector<int> part[3];
+  auto bytes_of = [&](int i, int w) { return (size_t)(c64 && w != kWide ? 8 : 16) << B.geo[(size_t)i].n; };
+  for (int i = 0; i < n_inst; ++i) {
+    const BatchGeo& g = B.geo[(size_t)i];
+    const bool wide = c64 && widened(c, g.n);
+    AltGeo ag;
+    alt_geometry(wide ? g.n : g.np, &ag);
+    part[ag.w3 > 0 ? kAlone : wide ? kWide : kOwn].push_back(i);
+  }
+  size_t room = 0, want = 0;
+  for (int w : {kWide, kOwn}) {
+    size_t sum = 0;
+    for (int i : part[w]) sum += bytes_of(i, w);
+    want = std::max(want, sum);
+  }
+  for (int w : {kWide, kOwn, kAlone})
+    for (int i : part[w]) room = std::max(room, bytes_of(i, w));
+  if (want > c->batch_state_cap) {
+    // all of a part at once where that fits, else in pieces: a member's result is the same in any
+    size_t free_b = 0, total_b = 0;
+    BK_CUDA(c, cudaMemGetInfo(&free_b, &total_b));
+    const size_t spare = (size_t)1 << 30;  // tables, rows, partial sums
+    const size_t avail = free_b + c->batch_state_cap;
+    want = std::min(want, avail > spare ? avail - spare : 0);
+  }
+  room = std::max(room, want);
+  BK_TRY(ensure_buffer(c, &c->d_batch_state, &c->batch_state_cap, room));
+  BK_TRY(ensure_buffer(c, reinterpret_cast<void**>(&c->d_batch_results), &c->batch_results_cap,
+                       std::max<size_t>((size_t)n_inst * B.n_meas * 4, 1) * sizeof(double)));
+  B.rows.resize((size_t)n_inst * B.n_meas * 4);
+  B.row_log2.assign((size_t)n_inst * std::max(B.n_meas, 1), 0.0L);
+  for (int w : {kWide, kOwn})
+    for (size_t at = 0; at < part[w].size();) {
+      std::vector<int> ids;
+      for (size_t sum = 0; at < part[w].size(); ++at) {
+        sum += bytes_of(part[w][at], w);
+        if (!ids.empty() && sum > room) break;
+        ids.push_back(part[w][at]);
+      }
+      BK_TRY((c64 && w == kOwn) ? B.members<float>(ids) : B.members<double>(ids));
+    }
+  for (int i : part[kAlone]) BK_TRY(c64 ? B.alone<float>(i) : B.alone<double>(i));
+  batch_rows(c64, B.rows, B.row_log2, p_less, d_h, norm_out);
+  return BK_OK;
+}
+
+template <class R>
+int evolve_batch_t(bk_ctx* c, const bk_batch_params* bp, const bk_batch_instance* inst, int n_inst,
+                   double* p_less, double* d_h, double* norm_out) {
+  const bool c64 = sizeof(R) == 4;
+  const int T = bp->n_steps;
+  std::vector<int> slot;
+  int n_meas = 0;
+  std::vector<BatchGeo> geo;
+  BK_TRY(batch_geometry(c, bp, inst, n_inst, p_less && d_h, &slot, &n_meas, &geo));
+  size_t state_bytes = 0;
+  for (BatchGeo& g : geo) {
+    g.state_off = state_bytes;
+    state_bytes += (1ull << g.n) * (c64 ? 8 : 16);
   }
   BK_TRY(ensure_buffer(c, &c->d_batch_state, &c->batch_state_cap, state_bytes));
   BK_TRY(ensure_buffer(c, reinterpret_cast<void**>(&c->d_batch_results), &c->batch_results_cap,
@@ -1693,17 +1891,6 @@ int evolve_batch_t(bk_ctx* c, const bk_batch_params* bp, const bk_batch_instance
       turns.next(gk, &tans[(size_t)i * T + k], &scales[(size_t)i * T + k]);
     }
   }
-  bool turning = c->engine_mode == 4 && c->e_recompute == 0;
-  for (const BatchGeo& g : geo) {
-    AltGeo ag;
-    turning = turning && alt_geometry(g.np, &ag) && alt_kernel_of<R>(ag, true) != nullptr;
-  }
-  if (turning) {
-    if constexpr (sizeof(R) == 4)
-      for (const BatchGeo& g : geo) BK_TRY(check_phase<R>(c, g.n, g.angle_unit));
-    return batch_turning<R>(c, geo, T, slot, n_meas, tans, scales, state_bytes, row_log2, p_less, d_h, norm_out);
-  }
-
   // phase tables per distinct n
   std::map<int, std::vector<unsigned char>> tables;
   std::map<int, typename PhaseV<R>::params> phase_of;
@@ -1925,7 +2112,7 @@ int evolve_batch_t(bk_ctx* c, const bk_batch_params* bp, const bk_batch_instance
   BK_CUDA(c, cudaStreamSynchronize(st));
   BK_TRY(collect_timing(c));
   if (e != 0) return fail(c, BK_ERR_TIMEOUT, "batched persistent engine: a bounded device wait gave up (%d)", e);
-  batch_rows<R>(rows, row_log2, p_less, d_h, norm_out);
+  batch_rows(sizeof(R) == 4, rows, row_log2, p_less, d_h, norm_out);
   return BK_OK;
 }
 
@@ -2240,7 +2427,7 @@ int adjoint_t(bk_ctx* c, const bk_adjoint_params* p, const std::vector<double>& 
   // forward: one persistent launch per window of K steps, psi copied to a
   // checkpoint between windows; enqueued without host synchronisation
   AltRun<R> arun;
-  if (turning) BK_TRY(alt_prepare<R>(c, n, p->s0, e0, angle_unit, S, tans, scales, &arun));
+  if (turning) BK_TRY(alt_prepare<R>(c, AltTarget{c->d_state, c->d_E, c->d_results}, n, p->s0, e0, angle_unit, S, tans, scales, &arun));
   int* fwd_err = turning ? c->d_err : run.err;
   auto enqueue_forward = [&]() -> int {
     BK_CUDA(c, cudaEventRecord(ev[0], st));
@@ -2515,15 +2702,6 @@ int adjoint_t(bk_ctx* c, const bk_adjoint_params* p, const std::vector<double>& 
   return BK_OK;
 }
 
-// the error word a run has left: reported, and cleared for the next one
-int device_error(bk_ctx* c, int e) {
-  if (e == 0) return BK_OK;
-  cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream);
-  cudaMemsetAsync(c->d_ticket, 0, sizeof(unsigned int), c->stream);
-  cudaStreamSynchronize(c->stream);
-  if (e == DEV_TIMEOUT) return fail(c, BK_ERR_TIMEOUT, "a bounded device wait gave up (a tile's load or a pass barrier)");
-  return fail(c, BK_ERR_CUDA, "device error word %d", e);
-}
 int check_device_error(bk_ctx* c) {
   int e = 0;
   BK_CUDA(c, cudaMemcpyAsync(&e, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
@@ -2950,13 +3128,11 @@ int bk_evolve(bk_ctx* c, const bk_evolve_params* p, double* p_less, double* d_h,
   bk_evolve_params q = *p;
   q.e0 = e0;
   const double angle_unit = (p->diag_scale > 0.0) ? p->dt * p->diag_scale : p->dt / (double)n;
-  // Small complex64 runs compute in complex128: up to 18 qubits a step is latency, not
-  // arithmetic or bandwidth (us a step, complex64 / complex128 kernels: N = 9 0.66 /
-  // 0.61, 14 3.9 / 3.5, 16 4.6 / 3.9, 18 5.1 / 5.1, 19 5.7 / 8.0), and the results are
-  // the exact ones to 1e-13 instead of a random walk of FP32 roundings.
+  // Small complex64 runs compute in complex128: `widened`, and up to 13 qubits, where the
+  // whole run is one CTA's, in every mode (N = 9: 0.66 us a step in complex64, 0.61 here).
   if (p->method == BK_FUSED && p->precision == BK_C64) BK_TRY(check_phase<float>(c, n, angle_unit));
   if (p->precision == BK_C64 && p->method == BK_FUSED &&
-      (n <= 13 || (n <= 18 && c->engine_mode == 4 && c->e_recompute == 0)))
+      (n <= 13 || widened(c, n)))
     q.precision = BK_C128;
   const int prec = q.precision;
 
@@ -3425,6 +3601,7 @@ int bk_evolve_batch(bk_ctx* c, const bk_batch_params* p, const bk_batch_instance
     return fail(c, BK_ERR_INVALID, "invalid batch parameters");
   if (p->precision != BK_C64 && p->precision != BK_C128) return fail(c, BK_ERR_INVALID, "precision %d", p->precision);
   BK_CUDA(c, cudaSetDevice(c->device));
+  if (c->engine_mode == 4 && c->e_recompute == 0) return evolve_batch_turning(c, p, inst, n_inst, p_less, d_h, norm);
   if (p->precision == BK_C64) return evolve_batch_t<float>(c, p, inst, n_inst, p_less, d_h, norm);
   return evolve_batch_t<double>(c, p, inst, n_inst, p_less, d_h, norm);
 }

@@ -158,13 +158,16 @@ int bk_evolve(bk_ctx* ctx, const bk_evolve_params* p, double* p_less, double* d_
 /* ---- Batched evolution: many statevectors in one call ----
  *
  * Every instance has its own n, trap and field; all share dt, the step count and
- * the measurement schedule. Up to 24 qubits (complex64) or 23 (complex128) the
+ * the measurement schedule, and every instance's rows are those of its own
+ * bk_evolve call, bit for bit. Up to 24 qubits (complex64) or 23 (complex128) the
  * instances of one size share a cooperative launch of turning passes, each worked
- * on by a group of CTAs with its own barrier (use_graph and lag do not apply).
- * With a larger instance, with E recomputed, or in BK_OPT_ENGINE_MODE 0 to 3 the
- * tile tasks of all instances run in ONE persistent kernel (launched through a
- * captured CUDA graph when use_graph is set), interleaved so that each
- * statevector's A1 output is re-read from L2.
+ * on by a group of CTAs with its own barrier; larger ones fill the GPU and run one
+ * after another (use_graph and lag do not apply). Instances whose states do not
+ * fit the free memory together run in several launches.
+ * With E recomputed, or in BK_OPT_ENGINE_MODE 0 to 3, the tile tasks of all
+ * instances run in ONE persistent kernel (launched through a captured CUDA graph
+ * when use_graph is set), interleaved so that each statevector's A1 output is
+ * re-read from L2; their states are held together.
  * Outputs are row-major [instance][measurement], normalised like bk_evolve's. */
 typedef struct bk_batch_instance {
   int32_t n;           /* qubits: 14..30 (complex64) or 13..30 (complex128) */
@@ -280,8 +283,8 @@ int bk_d_min(bk_ctx* ctx, int n, uint64_t bits, int64_t target, int max_d, int* 
  *       of them in one cooperative launch; complex64 takes its phase from the full
  *       per-energy table; the knobs below do not apply to it, and with
  *       BK_OPT_E_SOURCE = 1 mode 0 runs; bk_adjoint's forward run follows it, and
- *       its reverse sweep too unless BK_OPT_ADJ_A1 = 1; complex64 runs up to 18
- *       qubits compute in complex128 (no slower there) and report its sums,
+ *       its reverse sweep too unless BK_OPT_ADJ_A1 = 1; complex64 runs and
+ *       batch members up to 18 qubits compute in complex128 and report its sums,
  *       0 = persistent dataflow kernel (all steps in one launch,
  *       L2 hand-off between the A1 and S2 tasks), 1 = one grid launch per pass,
  *       2 = a grid launch for the A1 pass and ONE persistent launch for both
