@@ -108,7 +108,7 @@ struct alignas(64) AltInst {
 template <class R>
 struct AltBatch {
   const AltInst<R>* inst;
-  int n_inst, n_rows;
+  int n_inst, n_rows;  // n_rows: of this launch, from row D.row0 on
   uint32_t G;
   size_t part_stride;  // doubles of one partial-sum buffer ([n_rows][units][3]); every group has two
 };
@@ -835,9 +835,10 @@ __global__ void __launch_bounds__(AltPlan<TB, KB>::kThreads, TB == 10 ? 6 : TB =
       double s[3];
       alt_row_sum<AltPlan<TB, KB>::kThreads>(part + 3 * (size_t)row * D.units, D.units, C.ctl().acc, s);
       if (threadIdx.x == 0) {
-        I.results[4 * (size_t)row + 0] = s[1];
-        I.results[4 * (size_t)row + 1] = s[2];
-        I.results[4 * (size_t)row + 2] = s[0];
+        double* out = I.results + 4 * (size_t)(D.row0 + row);
+        out[0] = s[1];
+        out[1] = s[2];
+        out[2] = s[0];
       }
     }
     __syncthreads();

@@ -1367,23 +1367,31 @@ int alt_launch(bk_ctx* c, AltRun<R>& r, int k0, int k1, bool first, int row0, in
   return BK_OK;
 }
 
+// The steps of one launch from k0 on: up to a sampling point (which reads psi_k) or to where
+// the room of the partial sums, max_rows + 1 measured rows, ends.
+struct Stretch {
+  int k1, row0, rows;
+};
+Stretch stretch_from(int k0, bool first, int T, const std::vector<int>& slot, const std::vector<int>& sample_pt, int max_rows) {
+  Stretch s{k0, 0, 0};
+  for (int k = k0;; ++k) {
+    if ((k > k0 || first) && slot[(size_t)k] >= 0 && s.rows++ == 0) s.row0 = slot[(size_t)k];
+    s.k1 = k;
+    if (k == T || (k > k0 && ((!sample_pt.empty() && sample_pt[(size_t)k] >= 0) || s.rows >= max_rows))) return s;
+  }
+}
+
 // All T steps of a prepared run; sample(point) at its sampling points.
 template <class R, class F>
 int alt_steps(bk_ctx* c, AltRun<R>& run, const Schedule& S, int T, F&& sample) {
   if (S.sample_pt[0] >= 0) BK_TRY(sample(S.sample_pt[0]));
-  // segments end at sampling points (which read psi_k) and where the partial sums' room ends
   int k0 = 0;
   for (bool first = true;; first = false) {
-    int row0 = 0, rows = 0, k1 = k0;
-    for (int k = k0;; ++k) {
-      if ((k > k0 || first) && S.slot[(size_t)k] >= 0 && rows++ == 0) row0 = S.slot[(size_t)k];
-      k1 = k;
-      if (k == T || (k > k0 && (S.sample_pt[(size_t)k] >= 0 || rows >= run.max_rows))) break;
-    }
-    BK_TRY(alt_launch<R>(c, run, k0, k1, first, row0, rows));
-    if (k1 > 0 && S.sample_pt[(size_t)k1] >= 0) BK_TRY(sample(S.sample_pt[(size_t)k1]));
-    if (k1 == T) return BK_OK;
-    k0 = k1;
+    const Stretch s = stretch_from(k0, first, T, S.slot, S.sample_pt, run.max_rows);
+    BK_TRY(alt_launch<R>(c, run, k0, s.k1, first, s.row0, s.rows));
+    if (s.k1 > 0 && S.sample_pt[(size_t)s.k1] >= 0) BK_TRY(sample(S.sample_pt[(size_t)s.k1]));
+    if (s.k1 == T) return BK_OK;
+    k0 = s.k1;
   }
 }
 
@@ -1552,7 +1560,7 @@ int batch_turning(bk_ctx* c, const std::vector<BatchGeo>& geo, int T, const std:
   const int n_inst = (int)geo.size();
   cudaStream_t st = c->stream;
   struct Class {
-    int n = 0, per_sm = 0, smem = 0, threads = 0, n_inst = 0, first = 0;
+    int n = 0, per_sm = 0, smem = 0, threads = 0, n_inst = 0, first = 0, max_rows = 1;
     uint32_t G = 1, groups = 1;
     AltGeo geo;
     const void* fn = nullptr;
@@ -1603,9 +1611,18 @@ int batch_turning(bk_ctx* c, const std::vector<BatchGeo>& geo, int T, const std:
   }
   const size_t o_glob = b.take(64);
   const size_t up = b.off;
-  size_t part = 0;  // the classes run one after another: one room for their partial sums
-  for (auto& kv : classes)
-    part = std::max(part, (size_t)kv.second.groups * 2 * 3 * (size_t)std::max(n_meas, 1) * kv.second.D.units * sizeof(double));
+  // The classes run one after another: one room for their partial sums, bounded (a measured
+  // row of 64 members of N = 14 takes 98 KB over its groups: at 100000 rows 10 GB), so a
+  // long schedule runs in several launches, one pass more each; a quarter of the states'
+  // room keeps them rare for the batches of many members, whose rows are the largest.
+  size_t part = 0;
+  const size_t part_most = std::max(kAltPartialBytes, state_bytes / 4);
+  for (auto& kv : classes) {
+    Class& k = kv.second;
+    const size_t row_bytes = (size_t)k.groups * 2 * 3 * k.D.units * sizeof(double);
+    k.max_rows = (int)std::max<size_t>(part_most / row_bytes, 1);
+    part = std::max(part, row_bytes * (size_t)std::max(1, std::min(n_meas, k.max_rows + 1)));
+  }
   const size_t o_part = b.take(part);
   BK_TRY(ensure_buffer(c, &c->d_batch, &c->batch_cap, b.off));
   char *h = nullptr, *d = static_cast<char*>(c->d_batch);
@@ -1634,15 +1651,13 @@ int batch_turning(bk_ctx* c, const std::vector<BatchGeo>& geo, int T, const std:
   for (auto& kv : classes) {
     Class& k = kv.second;
     alt_table(k.n, k.angle_unit, reinterpret_cast<entry*>(h + k.o_tab), k.D.c0, k.D.n_j);
-    std::memset(h + k.o_ctr, held(c, 0, T) ? 0xFF : 0, (size_t)k.groups * 128);
+    std::memset(h + k.o_ctr, 0, (size_t)k.groups * 128);
     uint16_t* dE = nullptr;
     BK_TRY(batch_energy(c, k.n, &dE));
     k.D.E = dE;
     k.D.tab = reinterpret_cast<const entry*>(d + k.o_tab);
     k.D.slot = reinterpret_cast<const int*>(d + o_slot);
     k.D.partials = reinterpret_cast<double*>(d + o_part);
-    k.D.k1 = T;
-    k.D.meas_first = 1;
   }
   size_t ev = 0;
   BK_TRY(ev_begin(c, "batch", &ev));
@@ -1655,12 +1670,22 @@ int batch_turning(bk_ctx* c, const std::vector<BatchGeo>& geo, int T, const std:
   BK_CUDA(c, cudaGetLastError());
   for (auto& kv : classes) {
     Class& k = kv.second;
-    AltBatch<R> Q{reinterpret_cast<const AltInst<R>*>(d + o_inst) + k.first, k.n_inst, n_meas, k.G,
-                  3 * (size_t)std::max(n_meas, 1) * k.D.units};
+    AltBatch<R> Q{reinterpret_cast<const AltInst<R>*>(d + o_inst) + k.first, k.n_inst, 0, k.G,
+                  3 * (size_t)std::max(1, std::min(n_meas, k.max_rows + 1)) * k.D.units};
     AltBarrier B{reinterpret_cast<unsigned int*>(d + k.o_ctr), reinterpret_cast<int*>(d + o_glob),
                  reinterpret_cast<int*>(d + o_glob + 4), c->wait_polls > 0 ? c->wait_polls : kWaitPolls * 4u};
-    void* args[] = {&k.D, &Q, &B};
-    BK_CUDA(c, cudaLaunchCooperativeKernel(k.fn, dim3(k.G * k.groups), dim3((unsigned)k.threads), args, (size_t)k.smem, st));
+    for (bool first = true; first || k.D.k0 < T; first = false) {
+      const Stretch s = stretch_from(k.D.k0, first, T, slot, {}, k.max_rows);
+      k.D.k1 = s.k1;
+      k.D.row0 = s.row0;
+      k.D.meas_first = first ? 1 : 0;
+      Q.n_rows = s.rows;
+      const bool hold = held(c, k.D.k0, s.k1);
+      if (!first || hold) BK_CUDA(c, cudaMemsetAsync(B.ctr, hold ? 0xFF : 0, (size_t)k.groups * 128, st));
+      void* args[] = {&k.D, &Q, &B};
+      BK_CUDA(c, cudaLaunchCooperativeKernel(k.fn, dim3(k.G * k.groups), dim3((unsigned)k.threads), args, (size_t)k.smem, st));
+      k.D.k0 = s.k1;
+    }
   }
   BK_TRY(ev_end(c, ev));
   int e = 0;
@@ -1834,9 +1859,9 @@ int evolve_batch_turning(bk_ctx* c, const bk_batch_params* bp, const bk_batch_in
     // all of a part at once where that fits, else in pieces: a member's result is the same in any
     size_t free_b = 0, total_b = 0;
     BK_CUDA(c, cudaMemGetInfo(&free_b, &total_b));
-    const size_t spare = (size_t)1 << 30;  // tables, rows, partial sums
+    const size_t spare = (size_t)1 << 30;  // tables, rows, partial sums (these up to a quarter of the states)
     const size_t avail = free_b + c->batch_state_cap;
-    want = std::min(want, avail > spare ? avail - spare : 0);
+    want = std::min(want, avail > spare ? (avail - spare) / 5 * 4 : 0);
   }
   room = std::max(room, want);
   BK_TRY(ensure_buffer(c, &c->d_batch_state, &c->batch_state_cap, room));

@@ -1,0 +1,55 @@
+"""Device memory of long schedules: partial sums take a bounded room, whatever the number of
+measured rows or steps, and a run that is cut into launches for it gives the same rows."""
+import numpy as np
+import pytest
+import torch
+
+import bk_b200 as bk
+
+pytestmark = pytest.mark.gpu
+
+MIB = 1 << 20
+
+
+def _held(call):
+    """Device bytes a fresh engine holds after `call`, and its result."""
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    with bk.Engine(0) as eng:
+        out = call(eng)
+        return before - torch.cuda.mem_get_info()[0], out
+
+
+def test_batch_of_many_measured_rows():
+    n, steps, count = 14, 20000, 64
+    inst = [dict(n=n, s0=bk.select_trap(n, 30 + i, 40, 0.5)[0], g=0.2 + 0.002 * i) for i in range(count)]
+
+    def call(eng):
+        got = eng.evolve_batch(inst, 0.02, steps, precision=bk.BK_C64)
+        return got, [eng.evolve(n, x["s0"], x["g"], 0.02, steps, precision=bk.BK_C64) for x in (inst[0], inst[37])]
+
+    held, (got, ones) = _held(call)
+    # rows 41 MB, tangents and rescales 20 MB, states 17 MB, the single run's rows and sums
+    # 66 MB, 64 MiB of partial sums (all rows at once: 530 MB in sums by CTA, 2 GB by tile)
+    assert held <= 320 * MIB
+    for i, one in zip((0, 37), ones):
+        for a, b in zip(got, one):
+            assert np.array_equal(a[i], b)
+
+
+def test_batch_that_does_not_fit_at_once():
+    """States that the free memory does not hold together run in several launches."""
+    inst = [dict(n=22, s0=bk.select_trap(22, 30 + i, 40, 0.5)[0], g=0.3 + 0.01 * i) for i in range(40)]
+    with bk.Engine(0) as eng:
+        want = eng.evolve_batch(inst, 0.04, 3, precision=bk.BK_C128)
+    torch.cuda.empty_cache()
+    free = torch.cuda.mem_get_info()[0]
+    held = torch.empty(free - 3 * 1024 * MIB, dtype=torch.uint8, device="cuda")  # 40 states are 2.7 GB
+    try:
+        with bk.Engine(0) as eng:
+            got = eng.evolve_batch(inst, 0.04, 3, precision=bk.BK_C128)
+    finally:
+        del held
+        torch.cuda.empty_cache()
+    for a, b in zip(got, want):
+        assert np.array_equal(a, b)
