@@ -37,7 +37,7 @@ struct AdjRun {
   int m0;              // qubits rotated at the turn itself (complex64: amplitude bit 0)
   int width[3];        // qubits of each set
   int j0, j1;          // reverse steps [j0, j1)
-  int row0;            // partial row of pass 0 (a segment's passes have rows of their own)
+  int row0;            // partial row of the sweep's pass 0 (a launch's passes have rows of their own)
 };
 
 template <class R>

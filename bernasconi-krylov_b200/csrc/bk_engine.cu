@@ -2275,8 +2275,7 @@ int adj_reverse_turning(bk_ctx* c, int n, int T, const AltRun<R>& fwd, const typ
   cudaStream_t st = c->stream;
   AltGeo geo;
   adj_geometry(np, &geo);
-  const int three = geo.w3 > 0 ? 1 : 0, n_seg = (int)resets.size() + 1;
-  const int n_rows = (three ? 2 : 1) * (T + 1) + n_seg;
+  const int three = geo.w3 > 0 ? 1 : 0, mult = three ? 2 : 1;  // passes a step
   AdjRun<R> D{};
   BK_TRY(alt_maps(c, c->d_state, np, geo, D.map[0], D.set));
   BK_TRY(alt_maps(c, c->d_lam, np, geo, D.map[1], D.set));
@@ -2299,32 +2298,56 @@ int adj_reverse_turning(bk_ctx* c, int n, int T, const AltRun<R>& fwd, const typ
   BK_TRY(ctas_per_sm(c, fn, threads, smem, &per_sm));
   if (per_sm < 1) return fail(c, BK_ERR_CUDA, "reverse turning pass: no room for a CTA (%d bytes of shared memory)", smem);
   const uint32_t G = std::min<uint32_t>(D.n_tiles, (uint32_t)(per_sm * c->num_sms));
+  // Launches: the stretches between checkpoints, cut where the partial sums' room ends (a row
+  // a pass, 16 bytes a CTA: 5 KB a step at N = 24, a gigabyte at 200000 steps). The rows of
+  // the launches up to one that ends the room are summed behind it, and the room is used again.
+  struct Launch {
+    int j0, j1, row0;  // steps, first row
+    int reset;         // checkpoint put back behind it, or -1
+    bool sum;          // the cross terms of the steps so far are summed behind it
+  };
+  std::vector<Launch> runs;
+  const int max_rows = (int)std::max<size_t>(kAltPartialBytes / ((size_t)G * 2 * sizeof(double)), (size_t)mult + 1);
+  int used = 0, most = 0;
+  for (size_t s = 0, r = resets.size(); s <= r; ++s) {
+    const int end = s < r ? resets[s].after_j + 1 : T;
+    for (int j0 = s > 0 ? resets[s - 1].after_j + 1 : 0; j0 < end;) {
+      int steps = std::min(end - j0, (max_rows - used - 1) / mult);
+      if (steps < 1) {
+        runs.back().sum = true;
+        used = 0;
+        steps = std::min(end - j0, (max_rows - 1) / mult);
+      }
+      runs.push_back({j0, j0 + steps, used, -1, false});
+      used += mult * steps + 1;
+      most = std::max(most, used);
+      j0 += steps;
+    }
+    if (s < r) runs.back().reset = (int)s;
+  }
+  runs.back().sum = true;
+  const size_t n_run = runs.size();
   Bump b;
   const size_t o_tan = b.take((size_t)T * sizeof(R));
   const size_t o_sc = b.take((size_t)T * sizeof(R));
   const size_t o_lg = b.take((size_t)T * sizeof(double));
   const size_t o_row = b.take((size_t)T * sizeof(int));
-  const size_t o_ctr = b.take((size_t)n_seg * 128 + 64);
+  const size_t o_ctr = b.take(n_run * 128 + 64);
   const size_t up = b.off;
   const size_t o_cross = b.take((size_t)T * sizeof(double));
   const size_t o_dev = b.take(std::max<size_t>(resets.size(), 1) * kResetGrid * sizeof(double));
-  const size_t o_part = b.take((size_t)n_rows * G * 2 * sizeof(double));
+  const size_t o_part = b.take((size_t)most * G * 2 * sizeof(double));
   BK_TRY(ensure_buffer(c, &c->d_adj, &c->adj_cap, b.off));
   char *h = nullptr, *d = static_cast<char*>(c->d_adj);
   BK_TRY(stage(c, up, &h));
   std::copy(t_rev.begin(), t_rev.end(), reinterpret_cast<R*>(h + o_tan));
   std::copy(sc_rev.begin(), sc_rev.end(), reinterpret_cast<R*>(h + o_sc));
   std::copy(lg_rev.begin(), lg_rev.end(), reinterpret_cast<double*>(h + o_lg));
-  std::memset(h + o_ctr, 0, (size_t)n_seg * 128 + 64);
-  std::vector<int> seg_end;
-  for (const AdjReset& r : resets) seg_end.push_back(r.after_j + 1);
-  seg_end.push_back(T);
-  for (int s = 0; s < n_seg; ++s)
-    if (held(c, (int64_t)T + (s > 0 ? seg_end[(size_t)s - 1] : 0), (int64_t)T + seg_end[(size_t)s]))
-      std::memset(h + o_ctr + (size_t)s * 128, 0xFF, sizeof(unsigned int));
-  for (int j = 0, s = 0; j < T; ++j) {
-    while (j >= seg_end[(size_t)s]) ++s;
-    reinterpret_cast<int*>(h + o_row)[j] = s + (three ? 2 : 1) * j;
+  std::memset(h + o_ctr, 0, n_run * 128 + 64);
+  for (size_t i = 0; i < n_run; ++i) {
+    const Launch& l = runs[i];
+    if (held(c, (int64_t)T + l.j0, (int64_t)T + l.j1)) std::memset(h + o_ctr + i * 128, 0xFF, sizeof(unsigned int));
+    for (int j = l.j0; j < l.j1; ++j) reinterpret_cast<int*>(h + o_row)[j] = l.row0 + mult * (j - l.j0);
   }
   BK_CUDA(c, cudaMemcpyAsync(d, h, up, cudaMemcpyHostToDevice, st));
   BK_TRY(staged(c));
@@ -2332,37 +2355,43 @@ int adj_reverse_turning(bk_ctx* c, int n, int T, const AltRun<R>& fwd, const typ
   D.scale = reinterpret_cast<const R*>(d + o_sc);
   D.lg = reinterpret_cast<const double*>(d + o_lg);
   D.partials = reinterpret_cast<double*>(d + o_part);
-  int* abort_w = reinterpret_cast<int*>(d + o_ctr + (size_t)n_seg * 128);
+  int* abort_w = reinterpret_cast<int*>(d + o_ctr + n_run * 128);
   BK_CUDA(c, cudaEventRecord(ev[2], st));
   adj_lambda_init_kernel<R><<<(unsigned)std::min<size_t>((n_el + 255) / 256, (size_t)kResetGrid), 256, 0, st>>>(
       D.vec[0], D.vec[1], c->d_E, (uint32_t)n_el, objective, (int)e0, s0);
   BK_CUDA(c, cudaGetLastError());
   double* d_dev = reinterpret_cast<double*>(d + o_dev);
-  for (int s = 0, j0 = 0; s < n_seg; ++s) {
-    D.j0 = j0;
-    D.j1 = seg_end[(size_t)s];
-    D.row0 = s;
-    AltBarrier B{reinterpret_cast<unsigned int*>(d + o_ctr + (size_t)s * 128), c->d_err, abort_w,
+  int summed = 0;
+  for (size_t i = 0; i < n_run; ++i) {
+    const Launch& l = runs[i];
+    D.j0 = l.j0;
+    D.j1 = l.j1;
+    D.row0 = l.row0 - mult * l.j0;  // the kernel counts its rows by passes of the whole sweep
+    AltBarrier B{reinterpret_cast<unsigned int*>(d + o_ctr + i * 128), c->d_err, abort_w,
                  c->wait_polls > 0 ? c->wait_polls : kWaitPolls * 4u};
     size_t e = 0;
     BK_TRY(ev_begin(c, "adj_turn", &e));
     void* args[] = {&D, &B};
     BK_CUDA(c, cudaLaunchCooperativeKernel(fn, dim3(G), dim3((unsigned)threads), args, (size_t)smem, st));
     BK_TRY(ev_end(c, e));
-    if (s < n_seg - 1) {
-      const AdjReset& r = resets[(size_t)s];
+    if (l.reset >= 0) {
+      const AdjReset& r = resets[(size_t)l.reset];
       BK_TRY(ev_begin(c, "adj_reset", &e));
       adj_reset_kernel<R><<<kResetGrid, kComputeThreads, 0, st>>>(D.vec[0], ckpt + (size_t)r.ck * sbytes, c->d_E,
                                                                   (uint32_t)n_el, reset_phase, r.a, r.b,
-                                                                  d_dev + (size_t)s * kResetGrid);
+                                                                  d_dev + (size_t)l.reset * kResetGrid);
       BK_CUDA(c, cudaGetLastError());
       BK_TRY(ev_end(c, e));
     }
-    j0 = D.j1;
+    if (l.sum) {
+      const int count = l.j1 - summed;
+      adj_cross_kernel<<<(count + 3) / 4, 128, 0, st>>>(D.partials, count, (int)G, three,
+                                                        reinterpret_cast<const int*>(d + o_row) + summed,
+                                                        reinterpret_cast<double*>(d + o_cross) + summed);
+      BK_CUDA(c, cudaGetLastError());
+      summed = l.j1;
+    }
   }
-  adj_cross_kernel<<<(T + 3) / 4, 128, 0, st>>>(D.partials, T, (int)G, three, reinterpret_cast<const int*>(d + o_row),
-                                                reinterpret_cast<double*>(d + o_cross));
-  BK_CUDA(c, cudaGetLastError());
   BK_CUDA(c, cudaEventRecord(ev[3], st));
   cross->assign((size_t)T, 0.0);
   std::vector<double> dev(resets.size() * kResetGrid);

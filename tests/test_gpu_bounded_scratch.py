@@ -53,3 +53,36 @@ def test_batch_that_does_not_fit_at_once():
         torch.cuda.empty_cache()
     for a, b in zip(got, want):
         assert np.array_equal(a, b)
+
+
+def test_gradient_of_many_steps():
+    """One stretch of reverse steps (no checkpoint), cut for the room of its partial sums."""
+    n, steps = 18, 60000
+    bits, e0 = bk.select_trap(n, 3, 100, 0.3)
+
+    def call(eng):
+        return eng.adjoint(n, bits, [0.3], 0.02, steps, e0=e0, precision=bk.BK_C128, checkpoint_every=1 << 30,
+                           per_step=True)
+
+    held, (value, _, st) = _held(call)
+    # both vectors 8 MB, per-step arrays 2 MB, 64 MiB of partial sums (all passes': 246 MB)
+    assert held <= 128 * MIB
+    with bk.Engine(0) as eng:
+        ref, _, rst = eng.adjoint(n, bits, [0.3], 0.02, steps, e0=e0, precision=bk.BK_C128, checkpoint_every=1000,
+                                  per_step=True)
+    # the same steps with psi put back from checkpoints: FP64 rounding of 60000 steps of 36
+    # rotations, 1.5e-13 an amplitude as a walk, 2e-10 in one direction
+    assert value == ref
+    assert np.max(np.abs(st["grad_steps"] - rst["grad_steps"])) <= 1e-9 * np.max(np.abs(rst["grad_steps"]))
+
+
+@pytest.mark.parametrize("n", [18, 22])
+def test_cut_sweeps_give_the_same_gradient(n):
+    """Checkpoints that cut the sweep in stretches of 1, 3 and 7 steps."""
+    T, g = 15, np.linspace(0.3, 0.42, 15)
+    bits, e0 = bk.select_trap(n, 13, 100, 0.3)
+    with bk.Engine(0) as eng:
+        out = [eng.adjoint(n, bits, g, 0.04, T, e0=e0, precision=bk.BK_C128, checkpoint_every=K) for K in (64, 7, 3, 1)]
+    for v, grad, _ in out[1:]:
+        assert v == out[0][0]
+        assert np.max(np.abs(grad - out[0][1])) <= 1e-11 * np.max(np.abs(out[0][1]))
