@@ -2444,7 +2444,7 @@ int adjoint_t(bk_ctx* c, const bk_adjoint_params* p, const std::vector<double>& 
   }
   bk_evolve_params q{};
   q.n = n;
-  q.precision = p->precision;
+  q.precision = kC64 ? BK_C64 : BK_C128;
   q.method = BK_FUSED;
   q.s0 = p->s0;
   q.e0 = e0;
@@ -3306,32 +3306,40 @@ int bk_adjoint(bk_ctx* c, const bk_adjoint_params* p, double* value_out, double*
   const double angle_unit = (p->diag_scale > 0.0) ? p->dt * p->diag_scale : p->dt / (double)n;
   BK_CUDA(c, cudaSetDevice(c->device));
   BK_TRY(ensure_energy(c, n));
-  BK_TRY(ensure_state(c, n, p->precision));
-  BK_TRY(ensure_buffer(c, reinterpret_cast<void**>(&c->d_results), &c->results_cap, 4 * sizeof(double)));
-  BK_CUDA(c, cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
-  const size_t sbytes = (1ull << n) * amp_bytes(p->precision);
+  // the precision of bk_evolve's run of this size, whose value the forward run returns
+  // (unless checkpoints asked for fit in complex64 alone)
+  int prec = p->precision == BK_C64 && widened(c, n) ? BK_C128 : p->precision;
+  BK_TRY(ensure_state(c, n, prec));
   // checkpoints: every K steps strictly inside (0, T); K enlarged until they fit
-  int K = p->checkpoint_every;
-  const bool auto_k = K <= 0;
-  if (auto_k) K = 128;
+  const bool auto_k = p->checkpoint_every <= 0;
+  int K = auto_k ? 128 : p->checkpoint_every;
   auto n_ck = [&](int k) { return T > 0 ? (T - 1) / k : 0; };
+  size_t sbytes = (1ull << n) * amp_bytes(prec);
   // (the free memory is asked for only when the buffers of an earlier call do not suffice)
   if (c->lam_cap < sbytes || c->ckpt_cap < sbytes * (size_t)n_ck(K)) {
     size_t free_b = 0, total_b = 0;
     BK_CUDA(c, cudaMemGetInfo(&free_b, &total_b));
     const size_t reserve = (size_t)1 << 30;
     const size_t avail = free_b + c->lam_cap + c->ckpt_cap;
+    auto fits = [&]() { return sbytes * (size_t)(1 + n_ck(K)) + reserve <= avail; };
+    if (!auto_k && prec != p->precision && !fits()) {
+      prec = p->precision;
+      sbytes = (1ull << n) * amp_bytes(prec);
+      BK_TRY(ensure_state(c, n, prec));
+    }
     if (avail < sbytes + reserve) return fail(c, BK_ERR_OOM, "adjoint: no room for the adjoint statevector");
-    while (sbytes * (size_t)(1 + n_ck(K)) + reserve > avail) {
+    while (!fits()) {
       if (!auto_k) return fail(c, BK_ERR_OOM, "adjoint: %d checkpoints of %zu bytes do not fit", n_ck(K), sbytes);
       K *= 2;
     }
   }
   const int n_ckpt = n_ck(K);
+  BK_TRY(ensure_buffer(c, reinterpret_cast<void**>(&c->d_results), &c->results_cap, 4 * sizeof(double)));
+  BK_CUDA(c, cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
   BK_TRY(ensure_buffer(c, &c->d_lam, &c->lam_cap, sbytes));
   if (n_ckpt > 0) BK_TRY(ensure_buffer(c, &c->d_ckpt, &c->ckpt_cap, sbytes * (size_t)n_ckpt));
   std::vector<double> gs;
-  if (p->precision == BK_C64)
+  if (prec == BK_C64)
     BK_TRY(adjoint_t<float>(c, p, g_step, e0, angle_unit, K, n_ckpt, value_out, &gs, stats));
   else
     BK_TRY(adjoint_t<double>(c, p, g_step, e0, angle_unit, K, n_ckpt, value_out, &gs, stats));

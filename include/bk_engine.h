@@ -283,8 +283,10 @@ int bk_d_min(bk_ctx* ctx, int n, uint64_t bits, int64_t target, int max_d, int* 
  *       of them in one cooperative launch; complex64 takes its phase from the full
  *       per-energy table; the knobs below do not apply to it, and with
  *       BK_OPT_E_SOURCE = 1 mode 0 runs; bk_adjoint's forward run follows it, and
- *       its reverse sweep too unless BK_OPT_ADJ_A1 = 1; complex64 runs and
- *       batch members up to 18 qubits compute in complex128 and report its sums,
+ *       its reverse sweep too unless BK_OPT_ADJ_A1 = 1; complex64 runs,
+ *       batch members and gradients up to 18 qubits compute in complex128 and
+ *       report its sums (a gradient whose checkpoint_every fits the memory in
+ *       complex64 alone excepted),
  *       0 = persistent dataflow kernel (all steps in one launch,
  *       L2 hand-off between the A1 and S2 tasks), 1 = one grid launch per pass,
  *       2 = a grid launch for the A1 pass and ONE persistent launch for both
