@@ -3306,6 +3306,7 @@ int bk_adjoint(bk_ctx* c, const bk_adjoint_params* p, double* value_out, double*
   const double angle_unit = (p->diag_scale > 0.0) ? p->dt * p->diag_scale : p->dt / (double)n;
   BK_CUDA(c, cudaSetDevice(c->device));
   BK_TRY(ensure_energy(c, n));
+  if (p->precision == BK_C64) BK_TRY(check_phase<float>(c, n, angle_unit));
   // the precision of bk_evolve's run of this size, whose value the forward run returns
   // (unless checkpoints asked for fit in complex64 alone)
   int prec = p->precision == BK_C64 && widened(c, n) ? BK_C128 : p->precision;

@@ -1,6 +1,7 @@
 """The gradient's value is that of the run bk_evolve makes of the same schedule, in the default
 mode: complex64 schedules up to 18 qubits compute in complex128 in both (they differed by
-FP32 rounding, and TrotterObjective's value changed with requires_grad)."""
+FP32 rounding, and TrotterObjective's value changed with requires_grad), and both refuse the
+phase angles that the complex64 level table does not hold."""
 import numpy as np
 import pytest
 
@@ -37,3 +38,14 @@ def test_single_precision_request_is_the_double_gradient(eng, n):
     a = eng.adjoint(n, bits, g, 0.05, 12, e0=e0, precision=bk.BK_C64, checkpoint_every=5)
     b = eng.adjoint(n, bits, g, 0.05, 12, e0=e0, precision=bk.BK_C128, checkpoint_every=5)
     assert a[0] == b[0] and np.array_equal(a[1], b[1])
+
+
+@pytest.mark.parametrize("n,checkpoint_every", [(16, 64), (20, 64), (20, 2)])
+def test_angles_beyond_the_level_table_are_refused(eng, n, checkpoint_every):
+    bits, e0 = bk.select_trap(n, 12, 100, 0.3)
+    for call in (lambda: eng.evolve(n, bits, 0.3, 0.05, 4, e0=e0, precision=bk.BK_C64, diag_scale=4.0),
+                 lambda: eng.adjoint(n, bits, [0.3], 0.05, 4, e0=e0, precision=bk.BK_C64, diag_scale=4.0,
+                                     checkpoint_every=checkpoint_every)):
+        with pytest.raises(bk.BkError) as e:
+            call()
+        assert e.value.status == bk._lib.BK_ERR_UNSUPPORTED
