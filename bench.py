@@ -308,11 +308,12 @@ def run_batched(a):
     stream = torch.cuda.ExternalStream(eng.stream_handle(), device=dev)
     meas = range(0, steps_t + 1)
     from bk_b200 import tune
-    lag = tune.batch_lag(eng, inst)
+    chosen = tune.apply_batch(eng, inst)
     lag_src = "autotuner cache (bk_b200/tuning/b200.json)"
-    if lag is None:
-        lag = tune.tune_batch(eng, inst, a.dt, steps_t, measure=meas, write=False)["best"]["lag"]
+    if chosen is None:
+        chosen = tune.tune_batch(eng, inst, a.dt, steps_t, measure=meas, write=False)["best"]
         lag_src = "autotuner sweep at start-up (untimed)"
+    lag, turning = chosen["lag"], chosen["engine_mode"] == tune.TURNING
     for _ in range(max(a.warmup, 1)):
         eng.evolve_batch(inst, a.dt, steps_t, measure=meas, precision=bk.BK_C64, use_graph=True, lag=lag)
     torch.cuda.synchronize(dev)
@@ -328,6 +329,11 @@ def run_batched(a):
         wall = time.perf_counter() - t0
     dev_s = ev0.elapsed_time(ev1) / 1e3
     value = amp_steps * a.steps / dev_s
+    # launches of one call, counted in an untimed one
+    eng.set_kernel_timing(True)
+    eng.evolve_batch(inst, a.dt, steps_t, measure=meas, precision=bk.BK_C64, use_graph=True, lag=lag)
+    launches = sum(count for count, _ in eng.kernel_timing().values())
+    eng.set_kernel_timing(False)
     # the same 512 instances one after another, each through its own launches
     seq = {}
     for mode in (1, 0, tune.TURNING):
@@ -343,19 +349,19 @@ def run_batched(a):
         name = {1: "one_launch_per_pass", 0: "persistent_per_instance"}.get(mode, "turning_per_instance")
         seq["sequential_" + name] = amp_steps / (e0_.elapsed_time(e1_) / 1e3)
     best_seq = max(seq.values())
-    # roofline: one launch per size and bench step runs all 500 steps of that size's
-    # instances; algorithmic bytes 32 per amplitude-step (the two complex64
-    # read + write passes of the two-round-trip model; turning passes of these
-    # sizes need one), timed by the CUDA events bracketing the launches
+    # roofline: algorithmic bytes 16 per amplitude-step (a complex64 amplitude read and
+    # written once a step), timed by the CUDA events bracketing the launches
     peak, peak_kind = measured_peaks()
     launch_s = dev_s / a.steps
-    alg = 32.0 * amp_steps
-    roof = {"bound": "hbm", "kernel": "alt_batch_kernel (turning passes, one cooperative launch per size)",
+    alg = 16.0 * amp_steps
+    roof = {"bound": "hbm", "kernel": "alt_batch_kernel (turning passes, cooperative launches per size)" if turning else
+            "persist_kernel (one persistent launch)",
             "achieved": alg / launch_s / 1e9, "peak": peak, "unit": "GB/s", "frac": alg / launch_s / 1e9 / peak,
-            "peak_source": peak_kind, "algorithmic_bytes_per_launch": alg, "avg_launch_ms": 1e3 * launch_s,
+            "peak_source": peak_kind, "algorithmic_bytes_per_launch": alg / launches, "avg_launch_ms": 1e3 * launch_s / launches,
             "traffic": None,
-            "l2": "each statevector is 0.5-32 MiB (N = 16-22, complex64); the tasks of a few statevectors in flight "
-                  "fit the 126 MB L2, so part of the traffic is served from L2 and the HBM fraction is nominal"}
+            "l2": "each statevector is 1-32 MiB (N = 16-22; up to 18 qubits held in complex128); those of a few "
+                  "instances in flight fit the 126 MB L2, so part of the traffic is served from L2 and the HBM "
+                  "fraction is nominal"}
     line = {"metric": "Batched Trotter amp-steps/s (512 instances, N in {16,18,20,22}, complex64)", "value": value,
             "unit": UNIT, "n_gpus": 1, "steps": a.steps, "warmup": a.warmup,
             "ms_per_step": 1e3 * dev_s / a.steps, "higher_is_better": True, "scaling": "weak",
@@ -363,15 +369,14 @@ def run_batched(a):
             "data": "synthetic (64 seeded traps x 8 g, no dataset)",
             "config": {"workload": "512 instances = 64 traps (lowest 5% of 1000 descents, N uniform in "
                                    "{16,18,20,22}, seed 2024) x 8 g in linspace(0.2, 0.5, 8); dt=0.02, 500 Trotter "
-                                   "steps, P_< and <d_H> every step; one cooperative launch per size and "
-                                   "bench step",
+                                   "steps, P_< and <d_H> every step",
                        "instances": len(inst), "trotter_steps_per_step": steps_t,
-                       "tuning": {"lag": lag, "source": lag_src},
+                       "tuning": dict(chosen, source=lag_src),
                        "amp_steps_per_step": amp_steps},
             "compare": dict(seq, batched_over_best_sequential=value / best_seq),
             "e2e": {"value": amp_steps * a.steps / wall, "unit": UNIT, "h2d_bytes_per_step": 24 * len(inst) + 501,
                     "d2h_bytes_per_step": 3 * 8 * len(inst) * 501},
-            "clocks": clocks.summary(), "roofline": roof, "gpu_launches": a.steps * len(set(d["n"] for d in inst)),
+            "clocks": clocks.summary(), "roofline": roof, "gpu_launches": a.steps * launches,
             "check": {"p_less_mean_last": float(np.mean(p[:, -1])), "norm_max_dev": float(np.max(np.abs(nn - 1)))}}
     eng.close()
     if not a.no_cpu_baseline:

@@ -23,8 +23,9 @@ Knobs (engine options, include/bk_engine.h):
                each energy level from a full table (E = floor(n/2) mod 4 for
                every LABS energy) as two half-angle shear rotations, 0 = level
                table and residual polynomials.
-For the batched engine the knob is the task-block lag between a statevector
-slab's A1 and S2 tasks.
+For the batched engine the knobs are the engine mode (turning passes, or the
+persistent kernel) and, for the latter, the task-block lag between a
+statevector slab's A1 and S2 tasks.
 
 Each candidate is timed with CUDA events on the engine's stream over `steps`
 Trotter steps after `warmup` (the state of a large N is far larger than L2, so
@@ -42,8 +43,8 @@ from ._lib import BK_C64, BK_C128
 
 DEFAULT_CACHE = os.path.join(os.path.dirname(os.path.abspath(__file__)), "tuning", "b200.json")
 KNOBS = ("engine_mode", "slab_lag", "split_w2", "e_source", "a1_wide", "phase_table")
-DEFAULTS = {"engine_mode": 0, "slab_lag": 3, "split_w2": 0, "e_source": 0, "a1_wide": 0, "phase_table": 0}
 TURNING = 4  # the engine's default schedule
+DEFAULTS = {"engine_mode": TURNING, "slab_lag": 3, "split_w2": 0, "e_source": 0, "a1_wide": 0, "phase_table": 0}
 ELEM_BITS = 12  # element bits of one 64 KB tile
 
 
@@ -158,11 +159,11 @@ def tune(eng, n, precision=BK_C64, steps=20, warmup=4, cache_path=None, trap=Non
         results.append(dict(cfg, amp_steps_per_s=measure(eng, n, precision, cfg, bits, e0, steps, warmup)))
     best = max(results, key=lambda r: r["amp_steps_per_s"])
     # a swept schedule is worth setting only where it beats the engine's own choice
-    turning = dict(DEFAULTS, engine_mode=TURNING)
-    own = measure(eng, n, precision, turning, bits, e0, steps, warmup)
-    chosen = turning if own > best["amp_steps_per_s"] else {k: best.get(k, DEFAULTS[k]) for k in KNOBS}
-    entry = {"best": chosen, "amp_steps_per_s": best["amp_steps_per_s"], "turning_amp_steps_per_s": own,
-             "steps": steps, "candidates": results}
+    own = measure(eng, n, precision, DEFAULTS, bits, e0, steps, warmup)
+    swept = best["amp_steps_per_s"]
+    chosen = dict(DEFAULTS) if own > swept else {k: best.get(k, DEFAULTS[k]) for k in KNOBS}
+    entry = {"best": chosen, "amp_steps_per_s": max(own, swept), "turning_amp_steps_per_s": own,
+             "swept_amp_steps_per_s": swept, "steps": steps, "candidates": results}
     if write:
         cache = load_cache(cache_path)
         cache.setdefault(device_key(eng.device), {})[entry_key(n, precision)] = entry
@@ -177,7 +178,7 @@ def apply(eng, n, precision=BK_C64, cache_path=None):
     entry = cache.get(device_key(eng.device), {}).get(entry_key(n, precision))
     if entry is None:
         return None
-    apply_config(eng, entry["best"])
+    apply_config(eng, dict({"engine_mode": 0}, **entry["best"]))  # an entry without a mode was timed in mode 0
     return entry["best"]
 
 
@@ -188,21 +189,36 @@ def batch_key(instances, precision):
 
 def tune_batch(eng, instances, dt, n_steps, measure=None, precision=BK_C64, lags=(1, 2, 3, 4, 6, 8), cache_path=None,
                write=True):
-    """Times the batched engine for each task-block lag; returns and caches the best."""
+    """Times turning passes and, in the persistent engine, each task-block lag; returns the
+    entry, caches it and leaves the engine in the best one's mode."""
     results = []
     t = _timer(eng)
-    for lag in lags:
+    for mode, lag in [(TURNING, 0)] + [(0, lag) for lag in lags]:
+        eng.set_option("engine_mode", mode)
         eng.evolve_batch(instances, dt, n_steps, measure=measure, precision=precision, use_graph=True, lag=lag)
         sec = t(lambda: eng.evolve_batch(instances, dt, n_steps, measure=measure, precision=precision,
                                          use_graph=True, lag=lag))
-        results.append(dict(lag=lag, amp_steps_per_s=float(sum(1 << d["n"] for d in instances)) * n_steps / sec))
+        results.append(dict(engine_mode=mode, lag=lag,
+                            amp_steps_per_s=float(sum(1 << d["n"] for d in instances)) * n_steps / sec))
     best = max(results, key=lambda r: r["amp_steps_per_s"])
-    entry = {"best": {"lag": best["lag"]}, "amp_steps_per_s": best["amp_steps_per_s"], "candidates": results}
+    entry = {"best": {"engine_mode": best["engine_mode"], "lag": best["lag"]},
+             "amp_steps_per_s": best["amp_steps_per_s"], "candidates": results}
+    eng.set_option("engine_mode", best["engine_mode"])
     if write:
         cache = load_cache(cache_path)
         cache.setdefault(device_key(eng.device), {})[batch_key(instances, precision)] = entry
         save_cache(cache, cache_path)
     return entry
+
+
+def apply_batch(eng, instances, precision=BK_C64, cache_path=None):
+    """Sets the cached best engine mode for this batch; returns {"engine_mode", "lag"} or None
+    (also for an entry that names no mode: its lag belongs to a mode it was not timed against)."""
+    entry = load_cache(cache_path).get(device_key(eng.device), {}).get(batch_key(instances, precision))
+    if entry is None or "engine_mode" not in entry["best"]:
+        return None
+    eng.set_option("engine_mode", entry["best"]["engine_mode"])
+    return entry["best"]
 
 
 def batch_lag(eng, instances, precision=BK_C64, cache_path=None):

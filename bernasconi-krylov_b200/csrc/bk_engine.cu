@@ -1659,8 +1659,6 @@ int batch_turning(bk_ctx* c, const std::vector<BatchGeo>& geo, int T, const std:
     k.D.slot = reinterpret_cast<const int*>(d + o_slot);
     k.D.partials = reinterpret_cast<double*>(d + o_part);
   }
-  size_t ev = 0;
-  BK_TRY(ev_begin(c, "batch", &ev));
   BK_CUDA(c, cudaMemcpyAsync(d, h, up, cudaMemcpyHostToDevice, st));
   BK_TRY(staged(c));
   BK_CUDA(c, cudaMemsetAsync(state, 0, state_bytes, st));
@@ -1682,12 +1680,14 @@ int batch_turning(bk_ctx* c, const std::vector<BatchGeo>& geo, int T, const std:
       Q.n_rows = s.rows;
       const bool hold = held(c, k.D.k0, s.k1);
       if (!first || hold) BK_CUDA(c, cudaMemsetAsync(B.ctr, hold ? 0xFF : 0, (size_t)k.groups * 128, st));
+      size_t ev = 0;
+      BK_TRY(ev_begin(c, "batch", &ev));
       void* args[] = {&k.D, &Q, &B};
       BK_CUDA(c, cudaLaunchCooperativeKernel(k.fn, dim3(k.G * k.groups), dim3((unsigned)k.threads), args, (size_t)k.smem, st));
+      BK_TRY(ev_end(c, ev));
       k.D.k0 = s.k1;
     }
   }
-  BK_TRY(ev_end(c, ev));
   int e = 0;
   BK_CUDA(c, cudaMemcpyAsync(&e, d + o_glob, sizeof(int), cudaMemcpyDeviceToHost, st));
   if (n_meas > 0)
