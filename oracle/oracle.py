@@ -119,8 +119,11 @@ def random_states(n, seed, count):
 
 
 def steepest_descent(n, start, max_evals=0, use_ref=False):
-    L = ref_lib() if use_ref else lib()
-    fn = L.ref_steepest_descent if use_ref else L.orc_steepest_descent
+    """(final state, energy, evaluations, steps) of one descent. use_ref asks for the reference's own
+    compiled code; where oracle/_ref was not built the restatement stands in for it (the two are
+    compared bit for bit where it was)."""
+    R = ref_lib() if use_ref else None
+    fn = R.ref_steepest_descent if R is not None else lib().orc_steepest_descent
     fs, fe, ev, st = ctypes.c_uint64(), ctypes.c_int64(), ctypes.c_uint64(), ctypes.c_int64()
     fn(n, start, max_evals, ctypes.byref(fs), ctypes.byref(fe), ctypes.byref(ev), ctypes.byref(st))
     return int(fs.value), int(fe.value), int(ev.value), int(st.value)
