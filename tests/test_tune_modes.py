@@ -46,7 +46,7 @@ def test_rate_beside_a_choice_is_its_own(eng, tmp_path, monkeypatch, turning):
                         else 10.0 + 0.01 * next(rates))
     e = tune.tune(eng, 22, bk.BK_C64, trap=(1, 1), cache_path=str(tmp_path / "t.json"))
     swept = max(c["amp_steps_per_s"] for c in e["candidates"])
-    assert e["amp_steps_per_s"] == max(turning, swept)
+    assert e["best_amp_steps_per_s"] == max(turning, swept)
     assert (e["best"]["engine_mode"] == tune.TURNING) == (turning > swept)
     assert e["best"]["engine_mode"] == eng.options["engine_mode"]
 
@@ -74,7 +74,7 @@ def test_committed_rates_belong_to_the_committed_choices():
     for entries in tune.load_cache().values():
         for key, e in entries.items():
             if "turning_amp_steps_per_s" in e:
-                own = "turning" if e["best"]["engine_mode"] == tune.TURNING else "swept"
-                assert e["amp_steps_per_s"] == e[own + "_amp_steps_per_s"], key
+                own = "turning_amp_steps_per_s" if e["best"]["engine_mode"] == tune.TURNING else "amp_steps_per_s"
+                assert e["best_amp_steps_per_s"] == e[own], key
             if key.startswith("batch/"):
                 assert "engine_mode" in e["best"], key
