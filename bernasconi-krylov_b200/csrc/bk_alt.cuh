@@ -871,7 +871,9 @@ const void* alt_kernel_f64(int tb, int w2, int w3, bool batch);
 
 template <class R, int TB, int KB, int W2, int W3>
 const void* alt_pick(bool batch) {
-  if constexpr (W3 == 0)  // larger statevectors fill the GPU one at a time
+  // larger statevectors fill the GPU one at a time, complex64 members up to 18 qubits
+  // (W2 < 8 of the 2^10-element tiles) compute in complex128
+  if constexpr (W3 == 0 && !(sizeof(R) == 4 && TB == 10 && W2 < 8))
     if (batch) return reinterpret_cast<const void*>(alt_batch_kernel<R, TB, KB, W2, W3>);
   return batch ? nullptr : reinterpret_cast<const void*>(alt_kernel<R, TB, KB, W2, W3>);
 }
