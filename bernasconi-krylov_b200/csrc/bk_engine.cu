@@ -2763,6 +2763,65 @@ int check_device_error(bk_ctx* c) {
   return device_error(c, e);
 }
 
+// Starts of one kernel. A larger batch goes through the same warm room piece by piece: 10^6
+// starts 2.9 ms a call, 5.0 a context's first. With a room for all of them, 12 fresh MB, 6.3 to
+// 7.5 and 7 to 9, more than the 5.5 that the 8-byte copies of the whole batch could take.
+constexpr int64_t kDescentPiece = (int64_t)1 << 17;
+
+// The copies cost more than the descents (65536 starts of n = 28: 58 us of kernel, 210
+// us of pageable copies of 8-byte words one array after another), so states up to 32
+// spins, energies and evaluations cross as 4-byte words, the results in one copy, and
+// the host threads widen them into the caller's arrays, whose fresh pages then fault in
+// parallel: 230 us a call, 300 a context's first (450 and 800 with the words as the
+// caller has them). Pinned memory makes that 120, but pinning takes 4 to 11 ms of the first.
+int descend_piece(bk_ctx* c, int n, const uint64_t* starts, size_t cnt, unsigned long long budget, uint64_t* fs,
+                  int64_t* fe, uint64_t* ev) {
+  const size_t word = n <= 32 ? 4 : 8;
+  BK_TRY(ensure_buffer(c, &c->d_descent, &c->descent_cap, cnt * (2 * word + 8) + 64));
+  char* d = static_cast<char*>(c->d_descent);
+  const size_t o_fs = 0, o_fe = cnt * word, o_ev = o_fe + cnt * 4, o_st = (o_ev + cnt * 4 + 15) & ~(size_t)15;
+  cudaStream_t st = c->stream;
+  const unsigned grid = (unsigned)((cnt + kDescentWarps - 1) / kDescentWarps);
+  const size_t host_bytes = cnt * (word + 8);
+  char* h = nullptr;
+  BK_TRY(stage(c, host_bytes, &h));
+  size_t e = 0;
+  if (n <= 32) {
+    uint32_t* narrow = reinterpret_cast<uint32_t*>(h);
+#pragma omp parallel for schedule(static) if (cnt >= 16384)
+    for (long long i = 0; i < (long long)cnt; ++i) narrow[i] = (uint32_t)starts[i];
+    BK_CUDA(c, cudaMemcpyAsync(d + o_st, narrow, cnt * 4, cudaMemcpyHostToDevice, st));
+    BK_TRY(staged(c));
+  } else {
+    BK_CUDA(c, cudaMemcpyAsync(d + o_st, starts, cnt * 8, cudaMemcpyHostToDevice, st));
+  }
+  BK_TRY(ev_begin(c, "descent", &e));
+  if (n <= 32)
+    descent_kernel<1><<<grid, 32 * kDescentWarps, 0, st>>>(
+        n, reinterpret_cast<const uint32_t*>(d + o_st), (long long)cnt, budget, reinterpret_cast<uint32_t*>(d + o_fs),
+        reinterpret_cast<int*>(d + o_fe), reinterpret_cast<uint32_t*>(d + o_ev));
+  else
+    descent_kernel<2><<<grid, 32 * kDescentWarps, 0, st>>>(
+        n, reinterpret_cast<const unsigned long long*>(d + o_st), (long long)cnt, budget,
+        reinterpret_cast<unsigned long long*>(d + o_fs), reinterpret_cast<int*>(d + o_fe),
+        reinterpret_cast<uint32_t*>(d + o_ev));
+  BK_CUDA(c, cudaGetLastError());
+  BK_TRY(ev_end(c, e));
+  BK_CUDA(c, cudaMemcpyAsync(h, d + o_fs, host_bytes, cudaMemcpyDeviceToHost, st));
+  BK_CUDA(c, cudaStreamSynchronize(st));
+  const uint32_t* w_fs = reinterpret_cast<const uint32_t*>(h + o_fs);
+  const uint64_t* l_fs = reinterpret_cast<const uint64_t*>(h + o_fs);
+  const int* w_fe = reinterpret_cast<const int*>(h + o_fe);
+  const uint32_t* w_ev = reinterpret_cast<const uint32_t*>(h + o_ev);
+#pragma omp parallel for schedule(static) if (cnt >= 16384)
+  for (long long i = 0; i < (long long)cnt; ++i) {
+    fs[i] = word == 4 ? w_fs[i] : l_fs[i];
+    fe[i] = w_fe[i];
+    if (ev) ev[i] = w_ev[i];
+  }
+  return collect_timing(c);
+}
+
 }  // namespace
 
 // ============================================================================
@@ -2869,66 +2928,10 @@ int bk_steepest_descent_gpu(bk_ctx* c, int n, const uint64_t* starts, int64_t co
     return fail(c, BK_ERR_INVALID, "steepest descent: n = %d, count = %lld", n, (long long)count);
   if (count == 0) return BK_OK;
   BK_CUDA(c, cudaSetDevice(c->device));
-  // The copies cost more than the descents (65536 starts of n = 28: 58 us of kernel, 210
-  // us of pageable copies of 8-byte words one array after another), so states up to 32
-  // spins, energies and evaluations cross as 4-byte words, the results in one copy, and
-  // the host threads widen them into the caller's arrays, whose fresh pages then fault in
-  // parallel: 230 us a call, 450 a context's first (450 and 850 with the words as the
-  // caller has them). Pinned memory makes that 120, but pinning takes 4 to 11 ms of the first.
-  const size_t cnt = (size_t)count, word = n <= 32 ? 4 : 8;
-  const size_t need = cnt * (2 * word + 8) + 64;
-  BK_TRY(ensure_buffer(c, &c->d_descent, &c->descent_cap, need));
-  char* d = static_cast<char*>(c->d_descent);
-  const size_t o_fs = 0, o_fe = cnt * word, o_ev = o_fe + cnt * 4, o_st = (o_ev + cnt * 4 + 15) & ~(size_t)15;
-  cudaStream_t st = c->stream;
   const unsigned long long budget = max_evals == 0 ? ~0ull : (unsigned long long)max_evals;
-  const unsigned grid = (unsigned)((cnt + kDescentWarps - 1) / kDescentWarps);
-  const size_t host_bytes = cnt * (word + 8);
-  // the context keeps up to 8 MB of it warm; a larger batch returns its own
-  std::unique_ptr<char[]> own;
-  char* h = nullptr;
-  if (host_bytes > ((size_t)8 << 20)) {
-    own.reset(h = new (std::nothrow) char[host_bytes]);
-    if (!h) return fail(c, BK_ERR_OOM, "no host memory for %zu bytes of uploads", host_bytes);
-  } else {
-    BK_TRY(stage(c, host_bytes, &h));
-  }
-  size_t e = 0;
-  if (n <= 32) {
-    uint32_t* narrow = reinterpret_cast<uint32_t*>(h);
-#pragma omp parallel for schedule(static) if (cnt >= 16384)
-    for (long long i = 0; i < (long long)cnt; ++i) narrow[i] = (uint32_t)starts[i];
-    BK_CUDA(c, cudaMemcpyAsync(d + o_st, narrow, cnt * 4, cudaMemcpyHostToDevice, st));
-    if (!own) BK_TRY(staged(c));
-  } else {
-    BK_CUDA(c, cudaMemcpyAsync(d + o_st, starts, cnt * 8, cudaMemcpyHostToDevice, st));
-  }
-  BK_TRY(ev_begin(c, "descent", &e));
-  if (n <= 32)
-    descent_kernel<1><<<grid, 32 * kDescentWarps, 0, st>>>(n, reinterpret_cast<const uint32_t*>(d + o_st), count, budget,
-                                                           reinterpret_cast<uint32_t*>(d + o_fs),
-                                                           reinterpret_cast<int*>(d + o_fe),
-                                                           reinterpret_cast<uint32_t*>(d + o_ev));
-  else
-    descent_kernel<2><<<grid, 32 * kDescentWarps, 0, st>>>(
-        n, reinterpret_cast<const unsigned long long*>(d + o_st), count, budget,
-        reinterpret_cast<unsigned long long*>(d + o_fs), reinterpret_cast<int*>(d + o_fe),
-        reinterpret_cast<uint32_t*>(d + o_ev));
-  BK_CUDA(c, cudaGetLastError());
-  BK_TRY(ev_end(c, e));
-  BK_CUDA(c, cudaMemcpyAsync(h, d + o_fs, host_bytes, cudaMemcpyDeviceToHost, st));
-  BK_CUDA(c, cudaStreamSynchronize(st));
-  const uint32_t* w_fs = reinterpret_cast<const uint32_t*>(h + o_fs);
-  const uint64_t* l_fs = reinterpret_cast<const uint64_t*>(h + o_fs);
-  const int* w_fe = reinterpret_cast<const int*>(h + o_fe);
-  const uint32_t* w_ev = reinterpret_cast<const uint32_t*>(h + o_ev);
-#pragma omp parallel for schedule(static) if (cnt >= 16384)
-  for (long long i = 0; i < (long long)cnt; ++i) {
-    fs[i] = word == 4 ? w_fs[i] : l_fs[i];
-    fe[i] = w_fe[i];
-    if (ev) ev[i] = w_ev[i];
-  }
-  BK_TRY(collect_timing(c));
+  for (int64_t at = 0; at < count; at += kDescentPiece)
+    BK_TRY(descend_piece(c, n, starts + at, (size_t)std::min(kDescentPiece, count - at), budget, fs + at, fe + at,
+                         ev ? ev + at : nullptr));
   return BK_OK;
 }
 
