@@ -1436,7 +1436,10 @@ int evolve_small(bk_ctx* c, const bk_evolve_params* p, const Schedule& S, double
   const size_t up = b.off;
   int threads = 0, tile = 0;
   const void* fn = small_kernel_of(np, &threads, &tile);
-  const size_t o_part = b.take((size_t)std::max(S.n_meas, 1) * 3 * (threads / 32) * sizeof(double));
+  // a launch's rows have a bounded room (350000 of them at N = 12); a longer run takes several
+  const size_t row_bytes = 3 * (size_t)(threads / 32) * sizeof(double);
+  const int max_rows = (int)(kAltPartialBytes / row_bytes);
+  const size_t o_part = b.take((size_t)std::max(1, std::min(S.n_meas, max_rows + 1)) * row_bytes);
   BK_TRY(ensure_buffer(c, &c->d_small, &c->small_cap, b.off));
   char *h = nullptr, *d = static_cast<char*>(c->d_small);
   BK_TRY(stage(c, up, &h));
@@ -1457,14 +1460,13 @@ int evolve_small(bk_ctx* c, const bk_evolve_params* p, const Schedule& S, double
   P.e0 = (int)p->e0;
   P.s0 = (uint32_t)(p->s0 & ((1ull << n) - 1ull));
   // launches end at sampling points, which read psi_k from memory
-  auto launch = [&](int k0, int k1, bool first) -> int {
+  auto launch = [&](int k0, const Stretch& s, bool first) -> int {
     P.k0 = k0;
-    P.k1 = k1;
+    P.k1 = s.k1;
     P.init = first ? 1 : 0;
     P.meas_first = first ? 1 : 0;
-    P.row0 = P.rows = 0;
-    for (int k = k0; k <= k1; ++k)
-      if ((k > k0 || first) && S.slot[(size_t)k] >= 0 && P.rows++ == 0) P.row0 = S.slot[(size_t)k];
+    P.row0 = s.row0;
+    P.rows = s.rows;
     size_t ev = 0;
     BK_TRY(ev_begin(c, "small_state", &ev));
     void* args[] = {&P};
@@ -1475,10 +1477,10 @@ int evolve_small(bk_ctx* c, const bk_evolve_params* p, const Schedule& S, double
   int k0 = 0;
   for (bool first = true;; first = false) {
     // the first launch of a run that samples psi_0 only sets it up (and measures it)
-    int k1 = first && S.sample_pt[0] >= 0 ? 0 : k0 + 1;
-    while (k1 < T && S.sample_pt[(size_t)k1] < 0) ++k1;
-    k1 = std::min(k1, T);
-    BK_TRY(launch(k0, k1, first));
+    const int T1 = first && S.sample_pt[0] >= 0 ? 0 : T;
+    const Stretch s = stretch_from(k0, first, T1, S.slot, S.sample_pt, max_rows);
+    BK_TRY(launch(k0, s, first));
+    const int k1 = s.k1;
     if (S.sample_pt[(size_t)k1] >= 0) BK_TRY(launch_sampling<amp>(c, psi, n, S.sample_pt[(size_t)k1], S.shots));
     if (k1 == T) return BK_OK;
     k0 = k1;

@@ -86,3 +86,16 @@ def test_cut_sweeps_give_the_same_gradient(n):
     for v, grad, _ in out[1:]:
         assert v == out[0][0]
         assert np.max(np.abs(grad - out[0][1])) <= 1e-11 * np.max(np.abs(out[0][1]))
+
+
+def test_small_run_of_many_measured_rows():
+    n, steps, every = 12, 1000000, 1000
+    bits, e0 = bk.select_trap(n, 3, 100, 0.3)
+    held, got = _held(lambda eng: eng.evolve(n, bits, 0.3, 0.02, steps, e0=e0, precision=bk.BK_C128))
+    # rows 32 MB, steps 32 MB, 64 MiB of partial sums (all rows': 192 MB)
+    assert held <= 160 * MIB
+    with bk.Engine(0) as eng:
+        ref = eng.evolve(n, bits, 0.3, 0.02, steps, measure=range(0, steps + 1, every), e0=e0, precision=bk.BK_C128)
+    # one run cut in launches, one whole: the same rotations, sums in another order
+    for a, b in zip(got, ref):
+        assert np.max(np.abs(a[::every] - b)) <= 1e-13 * n
