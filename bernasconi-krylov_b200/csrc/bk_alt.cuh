@@ -24,7 +24,7 @@
 //
 // What bounds it (B200): up to 2^23 elements shared memory and its latency (N = 23
 // complex64: shared-memory pipe 52%, issue 26% of peak at 16 warps an SM; a step of
-// N = 19 is 5.6 us against 27 us for the persistent task engine, N = 22 23 against
+// N = 19 is 5.4 us against 27 us for the persistent task engine, N = 22 23 against
 // 37); beyond, DRAM: N = 28 complex64 1.54 ms a step = 5.6 TB/s over its two passes
 // (2.09 ms with a pass per set and the strided passes fused through L2).
 //

@@ -1137,8 +1137,8 @@ struct AltGeo {
 // complex64 / complex128):
 //   np <= 18: 2^10-element tiles, a 64-thread CTA each, two sets. The barrier and the
 //     exchange through L2 bound these sizes, so small tiles on many SMs win (np = 18:
-//     5.7 / 5.1 against 16.5 / 14.6 for a launch per pass).
-//   np <= 21: 2^12-element tiles, two CTAs an SM, two sets (np = 20: 12.3 / 12.2
+//     5.4 / 4.9 against 16.5 / 14.6 for a launch per pass).
+//   np <= 21: 2^12-element tiles, two CTAs an SM, two sets (np = 20: 11.9 / 11.9
 //     against 22.8 / 20.6 for a launch per pass; np = 21, a set of nine bits with one of
 //     them across lanes: 23.0 / 22.6 against 26.0 / 23.7 with 2^13-element tiles).
 //   np <= 23: 2^13-element tiles with 32 elements a thread, so that two sets still do

@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(kFsThreads, 2) fs_block_kernel(const double* _
 //      A:  y += scale E x - g sum_A;   S1: y -= g sum_S1
 // S1 of a slab is queued `lag` slabs behind its A tiles, so x and y of the slab are
 // still in L2: DRAM sees x twice, y twice written and once read and E once, 42 bytes a
-// state (measured: 41.6). Sweeping the ten bits above A through L2 instead, 80 bytes a
+// state (43.6 in a profile at N = 27). Sweeping the ten bits above A through L2 instead, 80 bytes a
 // state of L2 reads, took 1.82 ms at N = 27 with the far bits' pass; this takes 1.27 ms,
 // bound by the chain of one tile (x, y, sums from shared memory, stores), which the two
 // CTAs of an SM hide from each other in part. A tile's x is loaded (TMA) once the tile
