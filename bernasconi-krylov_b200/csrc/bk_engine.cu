@@ -61,15 +61,10 @@ struct TimingRec {
 
 }  // namespace
 
-// The copies enqueued so far: an event on the context's stream.
+// The copies enqueued so far: everything on the context's stream.
 struct StreamFence {
   cudaStream_t stream = nullptr;
-  cudaEvent_t event = nullptr;
-  bool mark() {
-    if (!event && cudaEventCreateWithFlags(&event, cudaEventDisableTiming) != cudaSuccess) return false;
-    return cudaEventRecord(event, stream) == cudaSuccess;
-  }
-  bool wait() { return cudaEventSynchronize(event) == cudaSuccess; }
+  bool wait() { return cudaStreamSynchronize(stream) == cudaSuccess; }
 };
 
 struct bk_ctx {
@@ -119,6 +114,7 @@ struct bk_ctx {
   void* d_alt = nullptr;      // turning passes: phase table, per-step arrays, partial sums, counters
   size_t alt_cap = 0;
   StageRoom<StreamFence> h_stage;  // a run's uploads, put together for one copy
+  StageRoom<StreamFence> h_sweep;  // a gradient's second upload, for its reverse sweep
   std::map<std::pair<const void*, int>, int> occupancy;  // (kernel, dynamic smem) -> CTAs per SM
   uint32_t wait_polls = 0;    // polls of a pass barrier's or dependency's wait before it gives up (0 = default)
   uint64_t s23_checked = 0;   // fused strided pass geometry (np, a1, w2, lag) whose closed form was checked
@@ -1121,13 +1117,16 @@ int check_phase(bk_ctx* c, int n, double angle_unit) {
   return BK_OK;
 }
 
-// Room for a run's uploads (bk_stage.hpp); `staged` after the copies from it.
-int stage(bk_ctx* c, size_t bytes, char** out) {
-  *out = c->h_stage.take(bytes);
+// Room for a run's uploads (bk_stage.hpp); `wait_stream` settles it.
+int stage(bk_ctx* c, StageRoom<StreamFence>& room, size_t bytes, char** out) {
+  *out = room.take(bytes);
   return *out ? BK_OK : fail(c, BK_ERR_OOM, "no host memory for %zu bytes of uploads", bytes);
 }
-int staged(bk_ctx* c) {
-  return c->h_stage.sent() ? BK_OK : fail(c, BK_ERR_CUDA, "the uploads' event: %s", cudaGetErrorString(cudaGetLastError()));
+int wait_stream(bk_ctx* c) {
+  BK_CUDA(c, cudaStreamSynchronize(c->stream));
+  c->h_stage.settled();
+  c->h_sweep.settled();
+  return BK_OK;
 }
 
 struct AltGeo {
@@ -1314,14 +1313,13 @@ int alt_prepare(bk_ctx* c, const AltTarget& at, int n, uint64_t s0, int64_t e0, 
   const size_t o_part = b.take(row_bytes * (size_t)std::max(1, std::min(S.n_meas, run->max_rows + 1)));
   BK_TRY(ensure_buffer(c, &c->d_alt, &c->alt_cap, b.off));
   char *h = nullptr, *d = static_cast<char*>(c->d_alt);
-  BK_TRY(stage(c, up, &h));
+  BK_TRY(stage(c, c->h_stage, up, &h));
   alt_table(n, angle_unit, reinterpret_cast<entry*>(h + o_tab), D.c0, D.n_j);
   std::copy(tans.begin(), tans.end(), reinterpret_cast<R*>(h + o_tan));
   std::copy(scales.begin(), scales.end(), reinterpret_cast<R*>(h + o_sc));
   std::copy(S.slot.begin(), S.slot.end(), reinterpret_cast<int*>(h + o_slot));
   std::memset(h + o_ctr, 0, 64);
   BK_CUDA(c, cudaMemcpyAsync(d, h, up, cudaMemcpyHostToDevice, c->stream));
-  BK_TRY(staged(c));
   D.E = at.E;
   D.tab = reinterpret_cast<const entry*>(d + o_tab);
   D.slot = reinterpret_cast<const int*>(d + o_slot);
@@ -1442,13 +1440,12 @@ int evolve_small(bk_ctx* c, const bk_evolve_params* p, const Schedule& S, double
   const size_t o_part = b.take((size_t)std::max(1, std::min(S.n_meas, max_rows + 1)) * row_bytes);
   BK_TRY(ensure_buffer(c, &c->d_small, &c->small_cap, b.off));
   char *h = nullptr, *d = static_cast<char*>(c->d_small);
-  BK_TRY(stage(c, up, &h));
+  BK_TRY(stage(c, c->h_stage, up, &h));
   alt_table(n, angle_unit, reinterpret_cast<entry*>(h + o_tab), P.c0, n_j);
   for (int k = 0; k <= T; ++k)
     reinterpret_cast<SmallStep*>(h + o_step)[k] = {k < T ? tans[(size_t)k] : 0.0, k < T ? scales[(size_t)k] : 1.0,
                                                       S.slot[(size_t)k], 0};
   BK_CUDA(c, cudaMemcpyAsync(d, h, up, cudaMemcpyHostToDevice, c->stream));
-  BK_TRY(staged(c));
   BK_TRY(allow_smem(c, fn, tile));
   P.state = reinterpret_cast<amp*>(c->d_state);
   P.E = c->d_E;
@@ -1628,7 +1625,7 @@ int batch_turning(bk_ctx* c, const std::vector<BatchGeo>& geo, int T, const std:
   const size_t o_part = b.take(part);
   BK_TRY(ensure_buffer(c, &c->d_batch, &c->batch_cap, b.off));
   char *h = nullptr, *d = static_cast<char*>(c->d_batch);
-  BK_TRY(stage(c, up, &h));
+  BK_TRY(stage(c, c->h_stage, up, &h));
   std::copy(tans.begin(), tans.end(), reinterpret_cast<R*>(h + o_tan));
   std::copy(scales.begin(), scales.end(), reinterpret_cast<R*>(h + o_scale));
   std::copy(slot.begin(), slot.end(), reinterpret_cast<int*>(h + o_slot));
@@ -1662,7 +1659,6 @@ int batch_turning(bk_ctx* c, const std::vector<BatchGeo>& geo, int T, const std:
     k.D.partials = reinterpret_cast<double*>(d + o_part);
   }
   BK_CUDA(c, cudaMemcpyAsync(d, h, up, cudaMemcpyHostToDevice, st));
-  BK_TRY(staged(c));
   BK_CUDA(c, cudaMemsetAsync(state, 0, state_bytes, st));
   set_basis_many_kernel<<<(n_inst + 127) / 128, 128, 0, st>>>(state, reinterpret_cast<unsigned long long*>(d + o_offs),
                                                               reinterpret_cast<unsigned int*>(d + o_idx), c64 ? 1 : 0,
@@ -1695,7 +1691,7 @@ int batch_turning(bk_ctx* c, const std::vector<BatchGeo>& geo, int T, const std:
   if (n_meas > 0)
     BK_CUDA(c, cudaMemcpyAsync(rows, c->d_batch_results, (size_t)n_inst * n_meas * 4 * sizeof(double),
                                cudaMemcpyDeviceToHost, st));
-  BK_CUDA(c, cudaStreamSynchronize(st));
+  BK_TRY(wait_stream(c));
   BK_TRY(collect_timing(c));
   if (e != 0) return fail(c, BK_ERR_TIMEOUT, "batched turning passes: a bounded device wait gave up (%d)", e);
   return BK_OK;
@@ -1822,7 +1818,7 @@ struct BatchRun {
     if (n_meas > 0)
       BK_CUDA(c, cudaMemcpyAsync(rows.data() + (size_t)i * n_meas * 4, c->d_batch_results,
                                  (size_t)n_meas * 4 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    BK_CUDA(c, cudaStreamSynchronize(c->stream));
+    BK_TRY(wait_stream(c));
     BK_TRY(device_error(c, err));
     return collect_timing(c);
   }
@@ -2341,7 +2337,7 @@ int adj_reverse_turning(bk_ctx* c, int n, int T, const AltRun<R>& fwd, const typ
   const size_t o_part = b.take((size_t)most * G * 2 * sizeof(double));
   BK_TRY(ensure_buffer(c, &c->d_adj, &c->adj_cap, b.off));
   char *h = nullptr, *d = static_cast<char*>(c->d_adj);
-  BK_TRY(stage(c, up, &h));
+  BK_TRY(stage(c, c->h_sweep, up, &h));
   std::copy(t_rev.begin(), t_rev.end(), reinterpret_cast<R*>(h + o_tan));
   std::copy(sc_rev.begin(), sc_rev.end(), reinterpret_cast<R*>(h + o_sc));
   std::copy(lg_rev.begin(), lg_rev.end(), reinterpret_cast<double*>(h + o_lg));
@@ -2352,7 +2348,6 @@ int adj_reverse_turning(bk_ctx* c, int n, int T, const AltRun<R>& fwd, const typ
     for (int j = l.j0; j < l.j1; ++j) reinterpret_cast<int*>(h + o_row)[j] = l.row0 + mult * (j - l.j0);
   }
   BK_CUDA(c, cudaMemcpyAsync(d, h, up, cudaMemcpyHostToDevice, st));
-  BK_TRY(staged(c));
   D.tan = reinterpret_cast<const R*>(d + o_tan);
   D.scale = reinterpret_cast<const R*>(d + o_sc);
   D.lg = reinterpret_cast<const double*>(d + o_lg);
@@ -2402,7 +2397,7 @@ int adj_reverse_turning(bk_ctx* c, int n, int T, const AltRun<R>& fwd, const typ
     BK_CUDA(c, cudaMemcpyAsync(dev.data(), d_dev, dev.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
   BK_CUDA(c, cudaMemcpyAsync(row, c->d_results, 4 * sizeof(double), cudaMemcpyDeviceToHost, st));
   BK_CUDA(c, cudaMemcpyAsync(e_fwd, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
-  BK_CUDA(c, cudaStreamSynchronize(st));
+  BK_TRY(wait_stream(c));
   BK_TRY(collect_timing(c));
   float ms = 0.f;
   BK_CUDA(c, cudaEventElapsedTime(&ms, ev[2], ev[3]));
@@ -2523,7 +2518,7 @@ int adjoint_t(bk_ctx* c, const bk_adjoint_params* p, const std::vector<double>& 
     BK_TRY(enqueue_forward());
     BK_CUDA(c, cudaMemcpyAsync(row, c->d_results, sizeof(row), cudaMemcpyDeviceToHost, st));
     BK_CUDA(c, cudaMemcpyAsync(&e_fwd, fwd_err, sizeof(int), cudaMemcpyDeviceToHost, st));
-    BK_CUDA(c, cudaStreamSynchronize(st));
+    BK_TRY(wait_stream(c));
     return finish_forward();
   }
 
@@ -2734,7 +2729,7 @@ int adjoint_t(bk_ctx* c, const bk_adjoint_params* p, const std::vector<double>& 
   // the forward's result row is untouched by the sweep: read it with the rest
   BK_CUDA(c, cudaMemcpyAsync(row, c->d_results, sizeof(row), cudaMemcpyDeviceToHost, st));
   BK_CUDA(c, cudaMemcpyAsync(&e_fwd, fwd_err, sizeof(int), cudaMemcpyDeviceToHost, st));
-  BK_CUDA(c, cudaStreamSynchronize(st));
+  BK_TRY(wait_stream(c));
   BK_TRY(finish_forward());
   if (e_dev != 0) return fail(c, BK_ERR_TIMEOUT, "adjoint sweep: a bounded device wait gave up (%d)", e_dev);
   BK_TRY(collect_timing(c));
@@ -2786,14 +2781,13 @@ int descend_piece(bk_ctx* c, int n, const uint64_t* starts, size_t cnt, unsigned
   const unsigned grid = (unsigned)((cnt + kDescentWarps - 1) / kDescentWarps);
   const size_t host_bytes = cnt * (word + 8);
   char* h = nullptr;
-  BK_TRY(stage(c, host_bytes, &h));
+  BK_TRY(stage(c, c->h_stage, host_bytes, &h));
   size_t e = 0;
   if (n <= 32) {
     uint32_t* narrow = reinterpret_cast<uint32_t*>(h);
 #pragma omp parallel for schedule(static) if (cnt >= 16384)
     for (long long i = 0; i < (long long)cnt; ++i) narrow[i] = (uint32_t)starts[i];
     BK_CUDA(c, cudaMemcpyAsync(d + o_st, narrow, cnt * 4, cudaMemcpyHostToDevice, st));
-    BK_TRY(staged(c));
   } else {
     BK_CUDA(c, cudaMemcpyAsync(d + o_st, starts, cnt * 8, cudaMemcpyHostToDevice, st));
   }
@@ -2810,7 +2804,7 @@ int descend_piece(bk_ctx* c, int n, const uint64_t* starts, size_t cnt, unsigned
   BK_CUDA(c, cudaGetLastError());
   BK_TRY(ev_end(c, e));
   BK_CUDA(c, cudaMemcpyAsync(h, d + o_fs, host_bytes, cudaMemcpyDeviceToHost, st));
-  BK_CUDA(c, cudaStreamSynchronize(st));
+  BK_TRY(wait_stream(c));
   const uint32_t* w_fs = reinterpret_cast<const uint32_t*>(h + o_fs);
   const uint64_t* l_fs = reinterpret_cast<const uint64_t*>(h + o_fs);
   const int* w_fe = reinterpret_cast<const int*>(h + o_fe);
@@ -2870,7 +2864,7 @@ int bk_create(int device, bk_ctx** out) {
     bk_destroy(c);
     return BK_ERR_CUDA;
   }
-  c->h_stage.fence().stream = c->stream;
+  c->h_stage.fence().stream = c->h_sweep.fence().stream = c->stream;
   cudaMemset(c->d_ticket, 0, sizeof(unsigned int));
   cudaMemset(c->d_err, 0, sizeof(int));
   *out = c;
@@ -2893,7 +2887,6 @@ int bk_destroy(bk_ctx* c) {
     cudaEventDestroy(e.first);
     cudaEventDestroy(e.second);
   }
-  if (c->h_stage.fence().event) cudaEventDestroy(c->h_stage.fence().event);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
   return BK_OK;
@@ -3251,7 +3244,7 @@ int bk_evolve(bk_ctx* c, const bk_evolve_params* p, double* p_less, double* d_h,
   if (S.n_pts > 0)
     BK_CUDA(c, cudaMemcpyAsync(p->samples_out, c->d_samples, (size_t)S.n_pts * S.shots * sizeof(uint64_t),
                                cudaMemcpyDeviceToHost, c->stream));
-  BK_CUDA(c, cudaStreamSynchronize(c->stream));
+  BK_TRY(wait_stream(c));
   BK_TRY(device_error(c, err));
   BK_TRY(collect_timing(c));
   c->have_state = true;

@@ -2,10 +2,12 @@
 //
 // Pageable: a small copy from it is staged at once, and pinning memory costs milliseconds
 // per context. Whether an asynchronous copy has read its pageable source when it returns is
-// the driver's choice, and one call can upload twice (a gradient: its forward run, then its
-// reverse sweep), so the room is handed out again only when the copies made from it are
-// behind: `Fence::mark` follows them on the stream, `Fence::wait` waits for the mark.
-// Not initialised: zero-filling touched every page once more.
+// the driver's choice, so the room is handed out again only when the copies made from it are
+// behind: the caller says `settled` where it has waited for the stream anyway, and a `take`
+// that finds them unsettled (a call that ended in an error) waits with `Fence::wait`. A call
+// with two uploads before its first wait (a gradient) has a room for each: an event behind
+// every upload cost each call a microsecond. Not initialised: zero-filling touched every
+// page once more.
 #pragma once
 #include <cstddef>
 #include <memory>
@@ -20,7 +22,7 @@ class StageRoom {
   // At least `bytes`, or nullptr: no memory, or the copies from it failed.
   char* take(size_t bytes) {
     if (sent_ && !fence_.wait()) return nullptr;
-    sent_ = false;
+    sent_ = true;  // until settled: copies from it may be on their way
     if (bytes > size_) {
       room_.reset();
       size_ = 0;
@@ -30,11 +32,8 @@ class StageRoom {
     }
     return room_.get();
   }
-  // The copies that read what `take` gave have been enqueued.
-  bool sent() {
-    sent_ = true;
-    return fence_.mark();
-  }
+  // The stream has been waited for since the last `take`.
+  void settled() { sent_ = false; }
   Fence& fence() { return fence_; }
 
  private:
